@@ -262,7 +262,9 @@ def test_rope_angles_at_large_positions():
 
 
 @pytest.mark.parametrize("M,N,K,cap", [(1, 1, 1, 0.0), (3, 70, 33, 0.0), (64, 64, 16, 0.0), (65, 130, 100, 5.0),
-                                       (8, 384, 96, 15.0), (200, 96, 320, 0.0)])
+                                       (8, 384, 96, 15.0), (200, 96, 320, 0.0),
+                                       # both tile shapes, with and without 16-byte rows, the last tiles ragged
+                                       (63, 65, 20, 0.0), (1300, 1920, 36, 0.0), (1301, 1921, 37, 5.0)])
 def test_gemm_f32(M, N, K, cap):
     x = rnd((M, K), torch.float32, 14)
     w = rnd((N, K), torch.float32, 15)
