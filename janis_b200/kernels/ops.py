@@ -158,6 +158,9 @@ def mixers():
         lib.janis_group_norm.argtypes = [P, P, I, P, F, P, F, I, P, I, I, I, P]
         lib.janis_round_rows.argtypes = [P, P, ctypes.c_size_t, P]
         lib.janis_selective_scan.argtypes = [P, I, I, I, P, I, I, P, P, I, P, I, I, I, P, P, I, I, P, P, P, P, I, P, P, I, I, I, I, I, P, P]
+        lib.janis_duality_scan_takes.argtypes = [P, I, I, P, I, I, I, P, P, I, I, I, I]
+        lib.janis_duality_scan_takes.restype = I
+        lib.janis_duality_scan.argtypes = [P, I, I, P, I, I, P, P, P, I, I, I, P, P, P, P, P, I, P, P, I, I, I, I, P]
         lib.janis_selective_scan_set_lanes.argtypes = [I]
         lib.janis_selective_scan_set_lanes.restype = None
         lib.janis_selective_scan_set_form.argtypes = [I]
@@ -1234,6 +1237,18 @@ def selective_scan(u, u_off: int, dt, dt_off: int, dt_bias, A, a_per_state: bool
     if scratch.numel() < need:
         raise KernelError(f"selective_scan: scratch of {scratch.numel()} floats, {need} wanted")
     lib = mixers()
+    # The chunked form on the tensor cores where it takes the sizes.  It costs what a chunk of 64 tokens costs however few a
+    # sequence brings; below DUALITY_TOKENS tokens a sequence the scan is quicker.
+    if dtype == torch.bfloat16 and z is None and not a_per_state and _scan_form in (0, 3) \
+            and (T >= DUALITY_TOKENS * n_seq or _scan_form == 3) \
+            and lib.janis_duality_scan_takes(u.data_ptr(), u.shape[1], int(u_off), bc.data_ptr(), bc.shape[1], int(b_off), int(c_off),
+                                             state.data_ptr(), out.data_ptr(), C, N, int(ch_per_head), int(ch_per_group)):
+        _check(lib, lib.janis_duality_scan(
+            u.data_ptr(), u.shape[1], int(u_off), dt.data_ptr(), dt.shape[1], int(dt_off), dt_bias.data_ptr(), A.data_ptr(),
+            bc.data_ptr(), bc.shape[1], int(b_off), int(c_off), D.data_ptr(), seq_slot.data_ptr(), seq_first_row.data_ptr(),
+            seq_start.data_ptr(), seq_end.data_ptr(), n_seq, state.data_ptr(), out.data_ptr(), C, N, int(ch_per_head),
+            int(ch_per_group), _stream()))
+        return out
     _check(lib, lib.janis_selective_scan(
         u.data_ptr(), _DT[dtype], u.shape[1], int(u_off), dt.data_ptr(), dt.shape[1], int(dt_off), dt_bias.data_ptr(),
         A.data_ptr(), 1 if a_per_state else 0, bc.data_ptr(), bc.shape[1], int(b_off), int(c_off), D.data_ptr(),
@@ -1241,6 +1256,10 @@ def selective_scan(u, u_off: int, dt, dt_off: int, dt_bias, A, a_per_state: bool
         seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), n_seq, state.data_ptr(), out.data_ptr(),
         C, N, int(ch_per_head), int(ch_per_group), T, scratch.data_ptr(), _stream()), kernels=2)
     return out
+
+
+DUALITY_TOKENS = 8
+_scan_form = 0
 
 
 def selective_scan_scratch_floats(n_tok: int, heads: int) -> int:
@@ -1255,9 +1274,12 @@ def selective_scan_set_lanes(lanes: int = 0) -> None:
 
 def selective_scan_set_form(form: int = 0) -> None:
     """0: a step in which a sequence brings several tokens runs the form that stages tiles of B and C in shared memory
-    where the sizes allow it and there are 64 states a channel or more (the default); 1: always the form that keeps a
-    tile's inputs in registers; 2: the staged form wherever the sizes allow it.  For tests."""
-    mixers().janis_selective_scan_set_form(int(form))
+    where the sizes allow it and there are 64 states a channel or more, or with one decay a head the chunked form (the
+    default); 1: always the form that keeps a tile's inputs in registers; 2: the staged form wherever the sizes allow
+    it; 3: the chunked form wherever the sizes allow it.  For tests."""
+    global _scan_form
+    _scan_form = int(form)
+    mixers().janis_selective_scan_set_form(int(form) if form != 3 else 0)
 
 
 def gate_group_norm(o, rows, z_off: int, weight, eps: float, n_groups: int, out):

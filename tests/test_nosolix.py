@@ -356,6 +356,40 @@ def test_scan_kernel_against_its_statement(dtype, C, N, cph, cpg, per_state, gat
 
 
 @GPU
+@pytest.mark.parametrize("C,N,cph,cpg", [(128, 128, 64, 64), (64, 32, 16, 64), (96, 32, 48, 96), (128, 64, 128, 128), (64, 128, 32, 32)])
+@pytest.mark.parametrize("lens", [[64, 1, 200, 17], [63, 65, 16, 128]])
+def test_chunked_duality_scan_against_its_statement(C, N, cph, cpg, lens):
+    """The chunked form at the edges of its chunks and tiles, from zero and from stored states, with a padding sequence, with
+    heads that forget at once (decays that leave nothing, in sums of thousands) beside heads that keep everything."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    starts, slots = [0, 30, 5, 0], [3, 0, 1, -1]
+    _, seq_slot, first, seq_start, seq_end, T = _tables(lens, starts, slots)
+    heads, groups = C // cph, C // cpg
+    g = torch.Generator().manual_seed(C * N + lens[0])
+    u = torch.randn(T, C + 8, generator=g).bfloat16()
+    dt = (torch.randn(T, heads + 3, generator=g) * 2.0).bfloat16()
+    bc = torch.randn(T, 2 * groups * N + 8, generator=g).bfloat16()
+    dt_bias, D = torch.randn(heads, generator=g) - 1.0, torch.randn(heads, generator=g)
+    A = -torch.exp(torch.linspace(-9.0, 6.0, heads)) if heads > 1 else -torch.ones(1)
+    state = torch.randn(4, C, N, generator=g)
+    want, want_state = torch.zeros(T, C), state.clone()
+    args = lambda dev, st, out: (dev(u), 8, dev(dt), 3, dev(dt_bias), dev(A), False, dev(bc), 8, 8 + groups * N, dev(D), None, 0,
+                                 dev(seq_slot), dev(first), dev(seq_start), dev(seq_end), len(lens), st, out, C, N, cph, cpg)
+    R.selective_scan(*args(lambda x: x, want_state, want))
+    for form in (3, 2):
+        ops.selective_scan_set_form(form)
+        try:
+            got, got_state = torch.full((T, C), float("nan"), device="cuda"), state.clone().cuda()
+            ops.selective_scan(*args(lambda x: x.cuda(), got_state, got))
+        finally:
+            ops.selective_scan_set_form(0)
+        _close(got, want, torch.float32, f"scan, form {form}", f32=5e-5)
+        _close(got_state, want_state, torch.float32, "the state left behind", f32=5e-5)
+        assert torch.equal(got_state[2].cpu(), state[2]), "a slot that is not in the step keeps its state"
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_small_kernels_against_their_statements(dtype):
     from janis_b200.kernels import ops
