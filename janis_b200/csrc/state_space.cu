@@ -13,6 +13,8 @@
 // delta, the decays, the state and o are float whatever the projections are stored in.  The state lives in the
 // cache, [slots, C, N] floats per line: a step loads it, runs its tokens in order and writes it back; sequences
 // without a slot (padding) start from zero and store nothing.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace janis {
@@ -21,10 +23,28 @@ __device__ __forceinline__ float silu_f(float v) { return v / (1.0f + expf(-v));
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 // A state that remembers hundreds of tokens is multiplied by decays just below 1, where a float holds exp(x) to
-// 6e-8 only and an error of one sign in every step adds up over the steps.  So the decay is kept as exp(x) - 1, which
-// expm1f gives to its own last bit however small it is, and the step is S + (S (exp(x) - 1) + input): the bracket is
+// 6e-8 only and an error of one sign in every step adds up over the steps.  So the decay is kept as exp(x) - 1, good
+// to its own last bit however small it is, and the step is S + (S (exp(x) - 1) + input): the bracket is
 // small against S and its rounding does not count; what remains is the one rounding of the sum.
 __device__ __forceinline__ float decay_minus_one(float x) { return expm1f(x); }
+
+// The same for x <= 0 without a branch, for the selective scan's prompts, which form one per state and token and do little else.
+// x = j ln 2 + f with a whole j (Cody and Waite's reduction: ln 2 in two floats), e^f - 1 is its Taylor series up to f^8 (the
+// next term is 6e-10 of the sum at |f| = ln 2 / 2), and 2^j (e^f - 1) + (2^j - 1) has one rounding: within 0.87 units in the
+// last place of exp(x) - 1, as compared with 64 bits over all negative floats' exponents.
+__device__ __forceinline__ float shrink_minus_one(float x) {
+    x = x < -30.f ? -30.f : x;                            // (-1 there already; a NaN stays one)
+    const float t = fmaf(x, 1.44269504f, 12582912.f), j = t - 12582912.f;      // x / ln 2 rounded, and in the low bits of t
+    const float f = fmaf(j, -1.42860682e-6f, fmaf(j, -0.693145751953125f, x));
+    float p = fmaf(1.f / 40320.f, f, 1.f / 5040.f);
+    p = fmaf(p, f, 1.f / 720.f);
+    p = fmaf(p, f, 1.f / 120.f);
+    p = fmaf(p, f, 1.f / 24.f);
+    p = fmaf(p, f, 1.f / 6.f);
+    p = fmaf(p, f, 0.5f);
+    const float q = fmaf(f * f, p, f), s = __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
+    return fmaf(s, q, s - 1.f);
+}
 __device__ __forceinline__ float decayed(float S, float grow, float input) { return S + fmaf(S, grow, input); }
 
 // ---------------------------------------------------------------------------
@@ -518,6 +538,142 @@ selective_scan_staged_kernel(const T* __restrict__ u_rows, const T* __restrict__
     }
 }
 
+// The selective scan of a long prompt, in pieces.  One token after another leaves the GPU waiting: 4,608 channels of 16 states
+// are 36,864 threads at two states each, whose every token is a chain of some 900 cycles.  So a sequence is cut into pieces of
+// equal length: the first kernel runs every piece but a sequence's last from a state of zero and keeps the state it ends with
+// and the sum of its step sizes; the second goes over the pieces of a sequence, S <- S e^(A sum) + what the piece left, and
+// puts the state each one starts from in its place; the third runs every piece from there and writes the results.  The
+// decays are formed twice, but a thread keeps all the states of a channel, so that nothing is passed between lanes and
+// what a token costs beside its states is paid once, and there are pieces enough to fill the SMs' issue slots, which bound it.
+// 4,608 channels, 16 states, against selective_scan_kernel: one sequence of 2,048 tokens 1,105 -> 390 us, 300 tokens 148 -> 74,
+// 128 tokens 66 -> 47 (64 tokens 39 -> 46: the launcher leaves short steps to the other kernel); eight of 512 1,200 -> 677.
+template <typename T, int N, bool LOCAL>
+__global__ void __launch_bounds__(128)
+selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ bc_rows, const T* __restrict__ z_rows,
+                            const float* __restrict__ delta, const float* __restrict__ A, const float* __restrict__ D, ScanShape g,
+                            int piece, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
+                            const int* __restrict__ seq_start, const int* __restrict__ seq_end, float* __restrict__ state,
+                            float* __restrict__ ends, float* __restrict__ sums, void* __restrict__ out_raw) {
+    const int seq = blockIdx.z, p = blockIdx.y, c_raw = blockIdx.x * 128 + threadIdx.x, C = g.C;
+    const bool live = c_raw < C, gated = g.gated != 0;
+    const int c = live ? c_raw : C - 1, head = c / g.cph, group = c / g.cpg;
+    grid_dependents_launch();
+    const int slot = seq_slot[seq], first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq];
+    const int t0 = p * piece, n_tok = min(piece, n_all - t0);
+    if (n_tok <= 0 || (LOCAL && t0 + piece >= n_all)) return;
+    const int row0 = first + t0;
+    const size_t place = (size_t)(first / piece + seq + p);
+    float Ar[N], S[N];
+#pragma unroll
+    for (int k = 0; k < N; k += 4) Vec16<float>::load(A + (size_t)head * N + k, Ar + k);
+    const float Dh = LOCAL ? 0.f : D[head];
+    grid_dependency_wait();
+    const float* from = LOCAL ? nullptr : ends + (place * C + c) * N;
+#pragma unroll
+    for (int k = 0; k < N; k += 4) {
+        if (!LOCAL) Vec16<float>::load(from + k, S + k);
+        else S[k] = S[k + 1] = S[k + 2] = S[k + 3] = 0.f;
+    }
+    const T* pu = u_rows + (size_t)row0 * g.u_stride + g.u_off + c;
+    const T* pz = gated ? z_rows + (size_t)row0 * g.z_stride + g.z_off + c : nullptr;
+    const T* pb = bc_rows + (size_t)row0 * g.bc_stride + g.b_off + group * N;
+    const int c_from_b = g.c_off - g.b_off;
+    const float* pd = delta + (size_t)row0 * g.heads + head;
+    T* out_t = reinterpret_cast<T*>(out_raw) + (size_t)row0 * C + c;
+    float* out_f = reinterpret_cast<float*>(out_raw) + (size_t)row0 * C + c;
+    // a token's inputs as they are stored, asked for a token ahead
+    constexpr int RAW = N * (int)sizeof(T) / 16;
+    struct Token {
+        float d;
+        T u, z;
+        uint4 B[RAW], C[RAW];
+    };
+    auto fetch = [&](int t, Token& x) {
+        x.d = pd[(size_t)t * g.heads];
+        x.u = pu[(size_t)t * g.u_stride];
+        if (!LOCAL && gated) x.z = pz[(size_t)t * g.z_stride];
+        const uint4* b = reinterpret_cast<const uint4*>(pb + (size_t)t * g.bc_stride);
+        const uint4* cc = reinterpret_cast<const uint4*>(pb + (size_t)t * g.bc_stride + c_from_b);
+#pragma unroll
+        for (int i = 0; i < RAW; ++i) {
+            x.B[i] = b[i];
+            if (!LOCAL) x.C[i] = cc[i];
+        }
+    };
+    bool shrinks = true;
+#pragma unroll
+    for (int k = 0; k < N; ++k) shrinks = shrinks && !(Ar[k] > 0.f);
+    shrinks = __syncthreads_and(shrinks);                    // (step sizes are positive: no decay is above 1)
+    float sum = 0.f;
+    auto run = [&](auto all_shrink) {
+        Token now, next;
+        fetch(0, now);
+        for (int t = 0; t < n_tok; ++t) {
+            if (t + 1 < n_tok) fetch(t + 1, next);
+            float B[N];
+            load_run<T, N, true>(reinterpret_cast<const T*>(now.B), B);
+            const float uu = to_float(now.u), du = now.d * uu;
+            sum += now.d;
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const float x = now.d * Ar[k];
+                S[k] = decayed(S[k], decltype(all_shrink)::value ? shrink_minus_one(x) : decay_minus_one(x), du * B[k]);
+            }
+            if (!LOCAL) {
+                float Cc[N], acc0 = 0.f, acc1 = 0.f;
+                load_run<T, N, true>(reinterpret_cast<const T*>(now.C), Cc);
+#pragma unroll
+                for (int k = 0; k < N; k += 2) {
+                    acc0 = fmaf(S[k], Cc[k], acc0);
+                    acc1 = fmaf(S[k + 1], Cc[k + 1], acc1);
+                }
+                if (live) {
+                    const float y = fmaf(Dh, uu, acc0 + acc1);
+                    const size_t at = (size_t)(unsigned)t * C;
+                    if (gated) out_t[at] = from_float<T>(y * silu_f(to_float(now.z)));
+                    else out_f[at] = y;
+                }
+            }
+            now = next;
+        }
+    };
+    if (shrinks) run(std::true_type());
+    else run(std::false_type());
+    if (!live) return;
+    if (LOCAL) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) Vec16<float>::store(ends + (place * C + c) * N + k, S + k);
+        sums[place * C + c] = sum;
+    } else if (t0 + piece >= n_all && slot >= 0) {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) Vec16<float>::store(state + ((size_t)slot * C + c) * N + k, S + k);
+    }
+}
+
+// A thread per (sequence, channel, state)
+template <int N>
+__global__ void __launch_bounds__(256)
+selective_scan_carry_kernel(const float* __restrict__ A, int C, int cph, int piece, const int* __restrict__ seq_slot,
+                            const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                            const float* __restrict__ state, float* __restrict__ ends, const float* __restrict__ sums) {
+    const int seq = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, c = i / N, k = i - c * N;
+    grid_dependents_launch();
+    const int slot = seq_slot[seq], first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq];
+    if (c >= C || n_all <= 0) return;
+    const float a = A[(size_t)(c / cph) * N + k];
+    grid_dependency_wait();
+    float S = slot >= 0 ? state[((size_t)slot * C + c) * N + k] : 0.f;
+    const size_t place = (size_t)(first / piece + seq);
+    const int pieces = (n_all + piece - 1) / piece;
+    for (int p = 0; p < pieces; ++p) {
+        float* e = ends + ((place + p) * C + c) * N + k;
+        const bool last = p + 1 == pieces;                       // (the last piece leaves nothing here)
+        const float end = last ? 0.f : *e, sum = last ? 0.f : sums[(place + p) * C + c];
+        *e = S;
+        if (!last) S = decayed(S, decay_minus_one(sum * a), end);
+    }
+}
+
 // y[t, part] = x / sqrt(mean(x^2) + eps) * w with x = o * silu(z): a CTA per (token, part)
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -666,13 +822,34 @@ static int scan_launch(const void* u, const void* bc, const void* z, const float
     return fail("selective_scan: %d states a channel are above %d", g.N, 32 * 16);
 }
 
+// Floats of scratch for a sequence's pieces beside the 2 n_tok heads of the step sizes, a piece.
+static long long scan_piece_floats(int C, int N) { return (long long)C * (N + 1); }
+
+template <typename T, int N>
+static int scan_pieces_launch(const void* u, const void* bc, const void* z, const float* delta, const float* A, const float* D, ScanShape g,
+                              int piece, int n_tok, const int* seq_slot, const int* seq_first_row, const int* seq_start,
+                              const int* seq_end, int n_seq, float* state, float* ends, float* sums, void* out, cudaStream_t stream) {
+    const int pieces = (n_tok + piece - 1) / piece;
+    const dim3 grid((g.C + 127) / 128, pieces, n_seq), block(128);
+    if (launch_kernel("selective_scan", selective_scan_piece_kernel<T, N, true>, grid, block, 0, stream, 1, (const T*)u, (const T*)bc,
+                      (const T*)z, delta, A, D, g, piece, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out))
+        return 1;
+    if (launch_kernel("selective_scan_carry", selective_scan_carry_kernel<N>, dim3((g.C * N + 255) / 256, n_seq), dim3(256), 0, stream, 1,
+                      A, g.C, g.cph, piece, seq_slot, seq_first_row, seq_start, seq_end, (const float*)state, ends, (const float*)sums))
+        return 1;
+    return launch_kernel("selective_scan", selective_scan_piece_kernel<T, N, false>, grid, block, 0, stream, 1, (const T*)u, (const T*)bc,
+                         (const T*)z, delta, A, D, g, piece, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out);
+}
+
 JANIS_EXPORT long long janis_selective_scan_scratch(int n_tok, int heads) { return 2LL * n_tok * heads; }
+
+constexpr int SCAN_PIECES_FROM = 128;  // tokens of a step
 
 static int scan_lanes_forced = 0;      // lanes a channel fixed by a test or a tuning run (0: chosen per launch)
 
 JANIS_EXPORT void janis_selective_scan_set_lanes(int lanes) { scan_lanes_forced = lanes; }
 
-static int scan_form_forced = 0;       // 0: the prompt form with its tiles in shared memory where it fits and pays; 1: never; 2: wherever it fits (tests)
+static int scan_form_forced = 0;       // 0: the prompt form with its tiles in shared memory where it fits and pays; 1: never; 2: wherever it fits; 4: in pieces wherever that fits (tests)
 
 JANIS_EXPORT void janis_selective_scan_set_form(int form) { scan_form_forced = form; }
 
@@ -681,7 +858,7 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
                                       int bc_stride, int b_off, int c_off, const float* D, const void* z, int z_stride,
                                       int z_off, const int* seq_slot, const int* seq_first_row, const int* seq_start,
                                       const int* seq_end, int n_seq, float* state, void* out, int C, int N, int cph,
-                                      int cpg, int n_tok, float* scratch, cudaStream_t stream) {
+                                      int cpg, int n_tok, float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (n_seq <= 0 || n_tok <= 0) return 0;
     if (C <= 0 || N <= 0 || cph <= 0 || cpg <= 0 || C % cph || C % cpg)
         return fail("selective_scan: %d channels, %d states, %d a head, %d a group", C, N, cph, cpg);
@@ -747,10 +924,39 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
     const size_t n = (size_t)n_tok * g.heads, want = (n + 255) / 256;
     const dim3 sgrid((unsigned)(want < 148 * 8 ? want : 148 * 8)), sblock(256);
     const float* A_head = a_per_state ? nullptr : A;
+    // The prompt in pieces (see the kernel) where the states a channel and the alignment allow it and the scratch has room: as
+    // many pieces as give an SM 16 warps, of 8 tokens or more.
+    int piece = 0;
+    if (a_per_state && (N == 8 || N == 16) && scan_form_forced != 1 && scan_form_forced != 2 && !scan_lanes_forced &&
+        (n_tok >= SCAN_PIECES_FROM || scan_form_forced == 4) && (dtype == JANIS_BF16 || dtype == JANIS_F32) && n_seq <= 65535) {
+        const int epp = 16 / (int)esz;
+        const bool aligned = (((uintptr_t)bc | (uintptr_t)A | (uintptr_t)state | (uintptr_t)scratch) & 15) == 0 && bc_stride % epp == 0 &&
+                             b_off % epp == 0 && c_off % epp == 0 && (size_t)n_tok * g.heads % 2 == 0 && C % 4 == 0;
+        const long long room = (scratch_floats - 2LL * n_tok * g.heads) / scan_piece_floats(C, N) - n_seq;
+        if (aligned && room >= 2) {
+            long long want = (148LL * 16 * 32 + C - 1) / C;
+            if (want > room) want = room;
+            if (want < 2) want = 2;
+            long long length = (n_tok + want - 1) / want;
+            // with two warps a quarter of an SM from the sequences alone, those of up to twice the mean length stay whole: the
+            // second run costs more than the shorter chains give
+            if ((long long)n_seq * C >= 148LL * 4 * 2 * 32 && length < (2LL * n_tok + n_seq - 1) / n_seq) length = (2LL * n_tok + n_seq - 1) / n_seq;
+            piece = length < 8 ? 8 : (int)length;
+        }
+    }
+    float* ends = scratch + 2 * (size_t)n_tok * g.heads;
+    float* sums = piece > 0 ? ends + ((size_t)(n_tok / piece) + n_seq) * C * N : nullptr;
+#define JANIS_SCAN_PIECES(T)                                                                                                  \
+    if (piece > 0)                                                                                                             \
+        return N == 8 ? scan_pieces_launch<T, 8>(u, bc, z, delta, A, D, g, piece, n_tok, seq_slot, seq_first_row, seq_start,     \
+                                                 seq_end, n_seq, state, ends, sums, out, stream)                                 \
+                      : scan_pieces_launch<T, 16>(u, bc, z, delta, A, D, g, piece, n_tok, seq_slot, seq_first_row, seq_start,    \
+                                                  seq_end, n_seq, state, ends, sums, out, stream);
     if (dtype == JANIS_F32) {
         if (launch_kernel("scan_steps", scan_steps_kernel<float>, sgrid, sblock, 0, stream, 1, (const float*)dt, dt_stride, dt_off,
                           dt_bias, A_head, delta, grow, g.heads, n))
             return 1;
+        JANIS_SCAN_PIECES(float)
         return a_per_state ? scan_launch<float, true>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream)
                            : scan_launch<float, false>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream);
     }
@@ -758,9 +964,11 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
         if (launch_kernel("scan_steps", scan_steps_kernel<bf16>, sgrid, sblock, 0, stream, 1, (const bf16*)dt, dt_stride, dt_off,
                           dt_bias, A_head, delta, grow, g.heads, n))
             return 1;
+        JANIS_SCAN_PIECES(bf16)
         return a_per_state ? scan_launch<bf16, true>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream)
                            : scan_launch<bf16, false>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream);
     }
+#undef JANIS_SCAN_PIECES
     return fail("selective_scan: unknown dtype %d", dtype);
 }
 

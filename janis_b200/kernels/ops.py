@@ -157,7 +157,7 @@ def mixers():
         lib.janis_head_linear.argtypes = [P, I, I, I, I, P, P, I, I, I, I, I, I, I, I, P]
         lib.janis_group_norm.argtypes = [P, P, I, P, F, P, F, I, P, I, I, I, P]
         lib.janis_round_rows.argtypes = [P, P, ctypes.c_size_t, P]
-        lib.janis_selective_scan.argtypes = [P, I, I, I, P, I, I, P, P, I, P, I, I, I, P, P, I, I, P, P, P, P, I, P, P, I, I, I, I, I, P, P]
+        lib.janis_selective_scan.argtypes = [P, I, I, I, P, I, I, P, P, I, P, I, I, I, P, P, I, I, P, P, P, P, I, P, P, I, I, I, I, I, P, c_longlong, P]
         lib.janis_duality_scan_takes.argtypes = [P, I, I, P, I, I, I, P, P, I, I, I, I]
         lib.janis_duality_scan_takes.restype = I
         lib.janis_duality_scan.argtypes = [P, I, I, P, I, I, P, P, P, I, I, I, P, P, P, P, P, I, P, P, I, I, I, I, P]
@@ -1212,7 +1212,8 @@ def selective_scan(u, u_off: int, dt, dt_off: int, dt_bias, A, a_per_state: bool
     [heads].  With z ([T, *], the gate's channels at z_off) out [T, C] takes o * silu(z) in the activations' type;
     without, out is float32 o.  state float32 [slots, C, N] is read and written back for slots >= 0.  A first kernel
     forms delta (and, with one A per head, exp(delta A) - 1) once per (token, head) into scratch (float32, at least
-    `selective_scan_scratch_floats`; allocated here when not given)."""
+    `selective_scan_scratch_floats`; allocated here when not given); what the scratch holds beyond that lets a prompt with
+    decays per state run in pieces at the same time (N + 1 floats a channel and piece, and as much for every sequence)."""
     T = u.shape[0]
     heads = C // ch_per_head
     dtype = u.dtype
@@ -1254,7 +1255,7 @@ def selective_scan(u, u_off: int, dt, dt_off: int, dt_bias, A, a_per_state: bool
         A.data_ptr(), 1 if a_per_state else 0, bc.data_ptr(), bc.shape[1], int(b_off), int(c_off), D.data_ptr(),
         z.data_ptr() if z is not None else None, z.shape[1] if z is not None else 0, int(z_off), seq_slot.data_ptr(),
         seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), n_seq, state.data_ptr(), out.data_ptr(),
-        C, N, int(ch_per_head), int(ch_per_group), T, scratch.data_ptr(), _stream()), kernels=2)
+        C, N, int(ch_per_head), int(ch_per_group), T, scratch.data_ptr(), scratch.numel(), _stream()), kernels=2)
     return out
 
 
@@ -1276,7 +1277,8 @@ def selective_scan_set_form(form: int = 0) -> None:
     """0: a step in which a sequence brings several tokens runs the form that stages tiles of B and C in shared memory
     where the sizes allow it and there are 64 states a channel or more, or with one decay a head the chunked form (the
     default); 1: always the form that keeps a tile's inputs in registers; 2: the staged form wherever the sizes allow
-    it; 3: the chunked form wherever the sizes allow it.  For tests."""
+    it; 3: the chunked form wherever the sizes allow it; 4: with decays per state in pieces wherever the sizes and the
+    scratch allow it.  For tests."""
     global _scan_form
     _scan_form = int(form)
     mixers().janis_selective_scan_set_form(int(form) if form != 3 else 0)

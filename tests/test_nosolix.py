@@ -391,6 +391,46 @@ def test_chunked_duality_scan_against_its_statement(C, N, cph, cpg, lens):
 
 @GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("C,N,cph,cpg,gated", [(260, 16, 1, 260, True), (128, 8, 1, 64, True), (64, 16, 4, 64, False)])
+@pytest.mark.parametrize("pieces", [2, 7, 300])
+def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, pieces):
+    """Room for 2, 7 and 300 pieces of 220 tokens (the last one: pieces of 8 tokens): sequences of one piece and of many, on a
+    border of pieces and beside it, from zero and from stored states, with a padding sequence."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    lens, starts, slots = [120, 1, 8, 81, 10], [0, 30, 5, 0, 0], [3, 0, 1, 4, -1]
+    _, seq_slot, first, seq_start, seq_end, T = _tables(lens, starts, slots)
+    heads, groups = C // cph, C // cpg
+    g = torch.Generator().manual_seed(C + N + pieces)
+    u, z = torch.randn(T, C + 8, generator=g).to(dtype), torch.randn(T, C, generator=g).to(dtype)
+    dt = (torch.randn(T, heads, generator=g) * 2.0).to(dtype)
+    bc = torch.randn(T, 2 * groups * N + 8, generator=g).to(dtype)
+    dt_bias, D = torch.randn(heads, generator=g) - 2.0, torch.randn(heads, generator=g)
+    A = -torch.exp(3.0 * torch.randn(heads, N, generator=g) - 1.0)
+    state = torch.randn(6, C, N, generator=g)
+    out_dtype = dtype if gated else torch.float32
+    want, want_state = torch.zeros(T, C, dtype=out_dtype), state.clone()
+    args = lambda dev, st, out: (dev(u), 8, dev(dt), 0, dev(dt_bias), dev(A), True, dev(bc), 8, 8 + groups * N, dev(D),
+                                 dev(z) if gated else None, 0, dev(seq_slot), dev(first), dev(seq_start), dev(seq_end),
+                                 len(lens), st, out, C, N, cph, cpg)
+    R.selective_scan(*args(lambda x: x, want_state, want))
+    floats = ops.selective_scan_scratch_floats(T, heads) + (pieces + len(lens)) * C * (N + 1)
+    scratch = torch.full((floats + 64,), float("nan"), device="cuda")
+    ops.selective_scan_set_form(4)
+    try:
+        got, got_state = torch.full((T, C), float("nan"), dtype=out_dtype, device="cuda"), state.clone().cuda()
+        ops.selective_scan(*args(lambda x: x.cuda(), got_state, got), scratch=scratch[:floats])
+    finally:
+        ops.selective_scan_set_form(0)
+    own = 2 * T * heads                                       # behind the step sizes: what the first piece starts from
+    assert scratch[floats:].isnan().all() and not scratch[own:own + C * N].isnan().any(), "the pieces' room, and no more"
+    _close(got, want, out_dtype, f"scan in {pieces} pieces", f32=5e-5)
+    _close(got_state, want_state, torch.float32, "the state left behind", f32=5e-5)
+    assert torch.equal(got_state[[2, 5]].cpu(), state[[2, 5]]), "a slot that is not in the step keeps its state"
+
+
+@GPU
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_small_kernels_against_their_statements(dtype):
     from janis_b200.kernels import ops
     from tests import kernel_refs as R
