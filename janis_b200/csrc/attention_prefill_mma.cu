@@ -370,6 +370,44 @@ attn_prefill_merge_kernel(const float* __restrict__ partial, const int* __restri
     }
 }
 
+// The keys and values that a step of continued sequences sees, side by side: position p of sequence s in row
+// seq_end[0] + .. + seq_end[s - 1] + p of `all`, its nkv key heads, then its value heads; earlier positions from the cache line,
+// the step's own from its buffer.  Positions that no query of the step sees (they lie before a window's or a chunk's first
+// tile of BN keys) keep what the row held.  2 nkv HD elements a row are read and written once, 16 bytes a thread: at 4 key
+// heads of 256 3,000 positions are 25 MB of traffic, a few microseconds, and the tcgen05 kernel then runs as on a whole
+// prompt; reading its tiles from the pages it would have to gather rows of the ring one by one.
+constexpr int GATHER_ROWS = 8;
+
+__global__ void __launch_bounds__(256)
+gather_keys_values_kernel(const bf16* __restrict__ kv_src, int kv_row_elems, int kv_k_head0, int nkv,
+                          const int* __restrict__ seq_first_row, const int* __restrict__ seq_end, int n_seq, int window,
+                          CachedPrefix cached, bf16* __restrict__ all, int rows) {
+    const int per_head = HD / 8, per_row = 2 * nkv * per_head;
+    grid_dependents_launch();
+    // the step's tables were written before the kernel ahead of this one started
+    int seq = 0, base = 0;
+    grid_dependency_wait();
+    for (int i = 0; i < GATHER_ROWS; ++i) {
+        const int row = blockIdx.x * GATHER_ROWS + i;
+        if (row >= rows) return;
+        while (seq < n_seq && row >= base + seq_end[seq]) base += seq_end[seq++];
+        if (seq >= n_seq) return;
+        const int p = row - base, start = cached.seq_start[seq], slot = cached.seq_slot[seq];
+        if (p < first_seen(start, window) / BN * BN) continue;
+        const bool old = p < start;
+        const bf16* own = kv_src + (size_t)(seq_first_row[seq] + (old ? 0 : p - start)) * kv_row_elems + (size_t)kv_k_head0 * HD;
+        for (int j = threadIdx.x; j < per_row; j += 256) {
+            const int head = j / per_head, c = (j - head * per_head) * 8, kvh = head < nkv ? head : head - nkv;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (!old) v = *reinterpret_cast<const uint4*>(own + (size_t)head * HD + c);
+            else if (slot >= 0)
+                v = *reinterpret_cast<const uint4*>((const bf16*)(head < nkv ? cached.kpool : cached.vpool) +
+                                                    cached_row(cached, slot, p, nkv, kvh, HD) + c);
+            *reinterpret_cast<uint4*>(all + (size_t)row * 2 * nkv * HD + (size_t)head * HD + c) = v;
+        }
+    }
+}
+
 }  // namespace pf
 }  // namespace janis
 
@@ -411,13 +449,13 @@ JANIS_EXPORT void janis_attn_set_prefill_piece(int piece) { g_prefill_piece = pi
 // launch, plus 0.45 us per round of partial rows.  CTAs go to the SM that is free first, in the order of their
 // launch.  The step's lengths are on the device: the model takes n_seq sequences of equal length.
 static double prefill_model_us(int n_seq, int len, int nq, int window, int parts, int piece, int sms, double cta,
-                               double tile, int* longest) {
+                               double tile, int* longest, int start) {
     std::vector<std::pair<int, bool>> items;          // key tiles, leaves a partial result; in tile order
     long long split_parts = 0;
     *longest = 0;
     for (int q0 = 0; q0 < len; q0 += pf::BM) {
         int k_first, n;
-        pf::key_tiles(q0, len, window, k_first, n);
+        pf::key_tiles(q0, len, window, k_first, n, start);
         *longest = std::max(*longest, n);
         const int np = pf::parts_of(n, parts, piece);
         for (int p = 0; p < np; ++p) items.push_back({(int)((long long)n * (p + 1) / np - (long long)n * p / np), np > 1});
@@ -442,12 +480,14 @@ static double prefill_model_us(int n_seq, int len, int nq, int window, int parts
 // shape of step with the lengths rounded up to whole tiles of queries, so that few shapes are ever asked about.  The
 // candidates are multiples of an SM's even share of the key tiles (the best lay between 1.25 and 2 of it wherever it
 // was measured), a few small pieces, and "nothing shared": a piece as long as the longest tile's keys.
-static int prefill_piece_for(int n_tok, int n_seq, int nq, int window, int parts, bool tc05, int* longest) {
-    static std::map<std::tuple<int, int, int, int, int, bool>, std::pair<int, int>> known;
+// (sequences that go on: all from the same position, `start`, rounded up to a multiple of 512)
+static int prefill_piece_for(int n_tok, int n_seq, int nq, int window, int parts, bool tc05, int* longest, int start = 0) {
+    static std::map<std::tuple<int, int, int, int, int, bool, int>, std::pair<int, int>> known;
     static std::mutex mu;
     std::lock_guard<std::mutex> lock(mu);
     const int len = ((n_tok + n_seq - 1) / n_seq + pf::BM - 1) / pf::BM * pf::BM;
-    const auto key = std::make_tuple(len, n_seq, nq, abs(window) < len ? window : 0, parts, tc05);
+    start = (start + 511) / 512 * 512;
+    const auto key = std::make_tuple(len, n_seq, nq, abs(window) < start + len ? window : 0, parts, tc05, start);
     auto it = known.find(key);
     if (it == known.end()) {
         const int sms = sm_count();
@@ -455,11 +495,11 @@ static int prefill_piece_for(int n_tok, int n_seq, int nq, int window, int parts
         // kernel took 2.7 times as long per tile at head size 256 and has less to do around its tiles
         const double tile = tc05 ? 1.0 + 0.22 * pf::HD / 256.0 : 3.9 * pf::HD / 256.0, cta = tc05 ? 7.1 : 6.0;
         int most = 0, best = 4;
-        double best_us = prefill_model_us(n_seq, len, nq, window, parts, 4, sms, cta, tile, &most);
+        double best_us = prefill_model_us(n_seq, len, nq, window, parts, 4, sms, cta, tile, &most, start);
         long long key_tiles = 0;
         for (int q0 = 0; q0 < len; q0 += pf::BM) {
             int k_first, n;
-            pf::key_tiles(q0, len, window, k_first, n);
+            pf::key_tiles(q0, len, window, k_first, n, start);
             key_tiles += n;
         }
         const double share = (double)key_tiles * n_seq * nq / sms;
@@ -469,12 +509,12 @@ static int prefill_piece_for(int n_tok, int n_seq, int nq, int window, int parts
         for (int piece : tries) {
             if (piece <= 4 || piece >= most) continue;
             int unused;
-            const double us = prefill_model_us(n_seq, len, nq, window, parts, piece, sms, cta, tile, &unused);
+            const double us = prefill_model_us(n_seq, len, nq, window, parts, piece, sms, cta, tile, &unused, start);
             if (us <= best_us) { best_us = us; best = piece; }
         }
         if (most > 4) {                                // and nothing shared at all
             int unused;
-            if (prefill_model_us(n_seq, len, nq, window, 1, most, sms, cta, tile, &unused) <= best_us) best = most;
+            if (prefill_model_us(n_seq, len, nq, window, 1, most, sms, cta, tile, &unused, start) <= best_us) best = most;
         }
         if (known.size() > 4096) known.clear();
         it = known.emplace(key, std::make_pair(best, most)).first;
@@ -506,7 +546,9 @@ JANIS_EXPORT void janis_attn_set_prefill_kernel(int which) { g_prefill_kernel = 
 // With seq_start (int32 [n_seq], tokens of each sequence that earlier steps stored) the step continues sequences:
 // seq_len then holds the lengths after the step, seq_first_row the row of a sequence's first token of this step, and
 // keys and values of positions below seq_start come from the cache line (kpool, vpool, page_table, ring_len as in
-// janis_attn_decode); such a step runs on the mma.sync kernel.
+// janis_attn_decode).  Where the head size suits the tcgen05 kernel and `gathered` has room for all_rows >= the sum of seq_len
+// rows of 2 nkv heads, keys and values are first brought together there (all_rows is that sum as the host knows it, max_total
+// the longest of seq_len); otherwise such a step runs on the mma.sync kernel, which reads the pages itself.
 // q_row_elems, kv_row_elems: elements between neighbouring rows, where rows hold more than whole heads (0: the row heads
 // times the head size).  sinks ([nq] floats, or null): exp(sinks[h]) joins head h's denominator.
 JANIS_EXPORT int janis_attn_prefill_mma(const void* q_src, const void* kv_src, int n_tok, const int* seq_first_row,
@@ -515,7 +557,8 @@ JANIS_EXPORT int janis_attn_prefill_mma(const void* q_src, const void* kv_src, i
                                         float cap, int window, float* partial, long long partial_floats,
                                         const int* seq_start, const int* seq_slot, const void* kpool, const void* vpool,
                                         const int* page_table, int table_stride, int ring_len, int max_len,
-                                        int q_row_elems, int kv_row_elems, const float* sinks, cudaStream_t stream) {
+                                        int q_row_elems, int kv_row_elems, const float* sinks, void* gathered,
+                                        int all_rows, int max_total, cudaStream_t stream) {
     if (q_row_elems == 0) q_row_elems = q_row_heads * pf::HD;
     if (kv_row_elems == 0) kv_row_elems = kv_row_heads * pf::HD;
     if (q_row_elems % 8 || kv_row_elems % 8 || q_row_elems < nq * pf::HD || kv_row_elems < (kv_k_head0 + 2 * nkv) * pf::HD)
@@ -544,27 +587,38 @@ JANIS_EXPORT int janis_attn_prefill_mma(const void* q_src, const void* kv_src, i
     if (partial == nullptr || partial_floats < janis_attn_prefill_scratch(n_tiles_bound, nq)) parts = 1;
     // The pieces that shared tiles of queries are cut into: what a model of the step's time likes best.  When that
     // is "none shared", the step is launched without the places of the parts and without the merge.
-    const bool tc05 = g_prefill_kernel == 1 && !ext && pf::TC05_HEAD;
+    const bool gather = ext && g_prefill_kernel == 1 && pf::TC05_HEAD && gathered != nullptr && all_rows >= n_tok && max_total > 0 &&
+                        ((uintptr_t)gathered & 15) == 0;
+    const bool tc05 = g_prefill_kernel == 1 && (!ext || gather) && pf::TC05_HEAD;
     int piece = g_prefill_piece;
     if (piece <= 0 && parts > 1) {
         int longest = 0;
-        piece = prefill_piece_for(n_tok, n_seq, nq, window, parts, tc05, &longest);
+        piece = prefill_piece_for(n_tok, n_seq, nq, window, parts, tc05, &longest, gather ? (all_rows - n_tok) / n_seq : 0);
     }
     if (piece <= 0) piece = 4;
     // No tile of queries has more key tiles than the step's longest sequence has (when the sequences start with the
     // step): places for parts that no tile can have would be CTAs that only come and go (2 to 3 us each for a CTA of
     // this size), and a piece that no tile exceeds means that nothing is shared: no places for parts, no merge.
     // (max_len: the longest sequence's tokens in this step, when the host knows them; else the step's tokens bound it)
-    int most_tiles = ((max_len > 0 ? std::min(max_len, n_tok) : n_tok) + pf::BN - 1) / pf::BN;
+    // (sequences that go on through the gathered rows: their lengths after the step)
+    int most_tiles = ((gather ? max_total : max_len > 0 ? std::min(max_len, n_tok) : n_tok) + pf::BN - 1) / pf::BN;
     if (window != 0) most_tiles = std::min(most_tiles, (abs(window) + pf::BM) / pf::BN + 1);  // a window or chunk bounds a tile's keys
-    if (!ext && parts > 1) parts = std::max(1, std::min(parts, (most_tiles + piece - 1) / piece));
-    if (!ext && most_tiles <= 8) parts = 1;           // up to 512 keys a tile: sharing measured no faster (512 tokens: 17.0 against 16.5 us)
+    if ((!ext || gather) && parts > 1) parts = std::max(1, std::min(parts, (most_tiles + piece - 1) / piece));
+    if ((!ext || gather) && most_tiles <= 8) parts = 1;           // up to 512 keys a tile: sharing measured no faster (512 tokens: 17.0 against 16.5 us)
     if ((long long)n_tiles_bound * parts > 65535) return fail("attn_prefill_mma: %d tiles of queries exceed the grid", n_tiles_bound);
     int done = -1;
-    if (g_prefill_kernel == 1 && !ext)                // the tcgen05 kernel takes sequences that start at position 0
+    if (gather) {
+        if (launch_kernel("gather_keys_values", pf::gather_keys_values_kernel, dim3((all_rows + pf::GATHER_ROWS - 1) / pf::GATHER_ROWS), dim3(256),
+                          0, stream, 1, (const bf16*)kv_src, kv_row_elems, kv_k_head0, nkv, seq_first_row, seq_len, n_seq, window, cached,
+                          (bf16*)gathered, all_rows))
+            return 1;
+        done = launch_prefill_tc05(q_src, gathered, n_tok, seq_first_row, seq_len, n_seq, n_tiles_bound, out, nq, nkv, q_row_elems,
+                                   2 * nkv * pf::HD, 0, scale, cap, window, parts, piece, partial, sinks, seq_start, all_rows, stream);
+    } else if (g_prefill_kernel == 1 && !ext) {
         done = launch_prefill_tc05(q_src, kv_src, n_tok, seq_first_row, seq_len, n_seq, n_tiles_bound, out, nq, nkv,
                                    q_row_elems, kv_row_elems, kv_k_head0, scale, cap, window, parts, piece, partial,
-                                   sinks, stream);
+                                   sinks, nullptr, n_tok, stream);
+    }
     if (done > 0) return 1;
     if (done < 0) {
         dim3 grid(nq, n_tiles_bound * parts);
@@ -574,7 +628,7 @@ JANIS_EXPORT int janis_attn_prefill_mma(const void* q_src, const void* kv_src, i
                           kv_row_elems, kv_k_head0, scale, cap, window, parts, piece, partial, cached, sinks))
             return 1;
     }
-    g_prefill_kernels = parts == 1 ? 1 : 2;
+    g_prefill_kernels = (parts == 1 ? 1 : 2) + (gather ? 1 : 0);
     if (parts == 1) return 0;
     return launch_kernel("attn_prefill_merge", pf::attn_prefill_merge_kernel, dim3(n_tiles_bound, nq, pf::BM / pf::MERGE_ROWS), dim3(256), 0, stream, 1,
                          (const float*)partial, seq_first_row, seq_len, n_seq, (bf16*)out, nq, window, parts, piece,

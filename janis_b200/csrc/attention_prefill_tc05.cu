@@ -217,7 +217,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                          const int* __restrict__ seq_first_row, const int* __restrict__ seq_len, int n_seq,
                          bf16* __restrict__ out, int nq, int nkv, int kv_k_head0, float scale, float cap, int window,
-                         int parts, int piece, float* __restrict__ partial, const float* __restrict__ sinks) {
+                         int parts, int piece, float* __restrict__ partial, const float* __restrict__ sinks,
+                         const int* __restrict__ seq_start) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[N_BARS];
     __shared__ uint32_t tmem_slot;
@@ -232,12 +233,22 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const int item = (int)gridDim.y - 1 - (int)blockIdx.y;
     const int gtile = item / parts, part = item % parts;
     int seq = -1, q0 = 0, len = 0;
-    if (!pf::find_tile(gtile, seq_len, n_seq, seq, q0, len)) return;
+    if (!pf::find_tile(gtile, seq_len, n_seq, seq, q0, len, seq_start)) return;
     const int head = blockIdx.x;
     const int kvh = head / (nq / nkv);
-    const int first = seq_first_row[seq];
+    const int q_row = seq_first_row[seq] + q0;       // the tile's first row of queries and of the output
+    int first = q_row - q0;                          // the row of keys and values that position 0 has
     int k_first, n_tiles;
-    pf::key_tiles(q0, len, window, k_first, n_tiles);
+    if (seq_start != nullptr) {                      // the sequence goes on: q0 and len become positions
+        const int start = seq_start[seq];
+        pf::key_tiles(q0, len, window, k_first, n_tiles, start);
+        first = 0;
+        for (int s = 0; s < seq; ++s) first += seq_len[s];
+        q0 += start;
+        len += start;
+    } else {
+        pf::key_tiles(q0, len, window, k_first, n_tiles);
+    }
     const int np = pf::parts_of(n_tiles, parts, piece);
     const bool shared_tile = np > 1;
     if (part >= np) return;
@@ -282,7 +293,7 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     grid_dependency_wait();
     if (warp == LOADER_WARP && lane == 0) {           // Q and the first keys are on their way before the others are ready
         mbar_expect_tx(bar(Q_FULL), Q_BYTES);
-        for (int sl = 0; sl < SLABS; ++sl) tma_load_2d(sQ + sl * Q_SLAB, &map_q, head * HD + sl * 64, first + q0, bar(Q_FULL));
+        for (int sl = 0; sl < SLABS; ++sl) tma_load_2d(sQ + sl * Q_SLAB, &map_q, head * HD + sl * 64, q_row, bar(Q_FULL));
         for (int i = 0; i < 2 && i < n_tiles; ++i) {
             mbar_expect_tx(bar(K_FULL + i), KV_TILE);
             for (int sl = 0; sl < SLABS; ++sl)
@@ -591,7 +602,7 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
             } else {
                 constexpr int PIECES = HD / 8;        // pieces of 8 bfloat16 in a row
-                bf16* obase = out + (size_t)(first + q0) * nq * HD + (size_t)head * HD;
+                bf16* obase = out + (size_t)q_row * nq * HD + (size_t)head * HD;
                 for (int idx = threadIdx.x; idx < rows * PIECES; idx += SOFTMAX_WARPS * 32) {
                     const int rr = idx / PIECES, pc = idx % PIECES;
                     *reinterpret_cast<uint4*>(obase + (size_t)rr * nq * HD + pc * 8) =
@@ -620,7 +631,7 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 // before the second; a partial result (float) takes both stages, and the loader waits before the first.
 // ---------------------------------------------------------------------------------------------------------------
 struct Item {
-    int seq, q0, len, first, k_first, n_tiles, head, gtile, part, np;   // n_tiles < 0: there is no further item
+    int seq, q0, len, q_row, first, k_first, n_tiles, head, gtile, part, np;   // n_tiles < 0: there is no further item
 };
 
 enum { ITEM_FULL = N_BARS, ITEM_EMPTY = N_BARS + 2, Q_EMPTY = N_BARS + 4, EPI_DONE = N_BARS + 5, N_BARS_ITEMS = N_BARS + 6 };
@@ -633,10 +644,10 @@ __device__ int g_sched[SCHED_SLOTS][2];
 
 // find_tile by a whole warp: 32 sequences a round
 __device__ __forceinline__ bool find_tile_warp(int tile, const int* __restrict__ seq_len, int n_seq, int lane, int& seq,
-                                               int& q0, int& len) {
+                                               int& q0, int& len, const int* __restrict__ seq_start) {
     int before = 0;
     for (int s0 = 0; s0 < n_seq; s0 += 32) {
-        const int n = s0 + lane < n_seq ? seq_len[s0 + lane] : 0;
+        const int n = s0 + lane < n_seq ? seq_len[s0 + lane] - (seq_start ? seq_start[s0 + lane] : 0) : 0;
         const int nt = (n + BM - 1) / BM;
         int incl = nt;
 #pragma unroll
@@ -664,7 +675,7 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
                                const int* __restrict__ seq_first_row, const int* __restrict__ seq_len, int n_seq,
                                bf16* __restrict__ out, int nq, int nkv, int kv_k_head0, float scale, float cap, int window,
                                int parts, int piece, float* __restrict__ partial, int n_places, int sched_slot,
-                               const float* __restrict__ sinks) {
+                               const float* __restrict__ sinks, const int* __restrict__ seq_start) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[N_BARS_ITEMS];
     int* sched = g_sched[sched_slot];
@@ -715,7 +726,7 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
     auto fetch = [&]() -> Item {
         Item it;
         it.n_tiles = -1;
-        it.seq = it.q0 = it.len = it.first = it.k_first = it.head = it.gtile = it.part = it.np = 0;
+        it.seq = it.q0 = it.len = it.q_row = it.first = it.k_first = it.head = it.gtile = it.part = it.np = 0;
         for (;;) {
             int idx = 0;
             if (lane == 0) idx = atomicAdd(&sched[0], 1);
@@ -724,9 +735,10 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
             const int place = n_places - 1 - idx / nq;     // heads vary fastest; the last tile of queries comes first
             const int gtile = place / parts, part = place % parts;
             int seq = 0, q0 = 0, len = 0;
-            if (!find_tile_warp(gtile, seq_len, n_seq, lane, seq, q0, len)) continue;
+            if (!find_tile_warp(gtile, seq_len, n_seq, lane, seq, q0, len, seq_start)) continue;
+            const int start = seq_start ? seq_start[seq] : 0;
             int k_first, n_tiles;
-            pf::key_tiles(q0, len, window, k_first, n_tiles);
+            pf::key_tiles(q0, len, window, k_first, n_tiles, start);
             const int np = pf::parts_of(n_tiles, parts, piece);
             if (part >= np) continue;
             if (np > 1) {
@@ -734,7 +746,14 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 k_first += t0 * BN;
                 n_tiles = t1 - t0;
             }
-            it.seq = seq; it.q0 = q0; it.len = len; it.first = seq_first_row[seq]; it.k_first = k_first;
+            it.q_row = seq_first_row[seq] + q0;
+            it.first = seq_first_row[seq];
+            if (seq_start) {                         // the row of keys and values that position 0 has
+                int rows = 0;
+                for (int s = lane; s < seq; s += 32) rows += seq_len[s];
+                it.first = __reduce_add_sync(0xffffffffu, rows);
+            }
+            it.seq = seq; it.q0 = start + q0; it.len = start + len; it.k_first = k_first;
             it.n_tiles = n_tiles; it.head = idx % nq; it.gtile = gtile; it.part = part; it.np = np;
             return it;
         }
@@ -770,7 +789,7 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 // (Q is free: the item before was taken only after its last scores, below)
                 mbar_expect_tx(bar(Q_FULL), Q_BYTES);
                 for (int sl = 0; sl < SLABS; ++sl)
-                    tma_load_2d(sQ + sl * Q_SLAB, &map_q, cur.head * HD + sl * 64, cur.first + cur.q0, bar(Q_FULL));
+                    tma_load_2d(sQ + sl * Q_SLAB, &map_q, cur.head * HD + sl * 64, cur.q_row, bar(Q_FULL));
                 auto load_k = [&](int i) {
                     if (!ok || i >= n) return;
                     const int gi = g + i, s = gi & 1;
@@ -1087,7 +1106,7 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
                     }
                 } else {
                     constexpr int PIECES = HD / 8;
-                    bf16* obase = out + (size_t)(me.first + q0) * nq * HD + (size_t)me.head * HD;
+                    bf16* obase = out + (size_t)me.q_row * nq * HD + (size_t)me.head * HD;
                     for (int idx = threadIdx.x; idx < rows * PIECES; idx += SOFTMAX_WARPS * 32) {
                         const int rr = idx / PIECES, pc = idx % PIECES;
                         *reinterpret_cast<uint4*>(obase + (size_t)rr * nq * HD + pc * 8) =
@@ -1174,11 +1193,11 @@ static int tc05_sm_count() {
 int launch_prefill_tc05(const void* q_src, const void* kv_src, int n_tok, const int* seq_first_row, const int* seq_len,
                         int n_seq, int n_tiles_bound, void* out, int nq, int nkv, int q_row_elems, int kv_row_elems,
                         int kv_k_head0, float scale, float cap, int window, int parts, int piece, float* partial,
-                        const float* sinks, cudaStream_t stream) {
+                        const float* sinks, const int* seq_start, int kv_rows, cudaStream_t stream) {
     if (!pt::SUPPORTED) return -1;
     CUtensorMap mq, mkv;
     if (!pt::make_map(&mq, q_src, n_tok, q_row_elems, pt::BM) ||
-        !pt::make_map(&mkv, kv_src, n_tok, kv_row_elems, pt::BN))
+        !pt::make_map(&mkv, kv_src, kv_rows, kv_row_elems, pt::BN))
         return -1;                                    // no encoder, or operands it refuses: the other kernel runs
     static bool configured = false;
     if (!configured) {
@@ -1213,12 +1232,12 @@ int launch_prefill_tc05(const void* q_src, const void* kv_src, int n_tok, const 
         auto items = cap > 0.f ? pt::attn_prefill_tc05_items_kernel<true> : pt::attn_prefill_tc05_items_kernel<false>;
         return launch_kernel("attn_prefill_tc05", items, dim3(ctas), dim3(pt::THREADS), pt::SMEM_BYTES, stream, 1, mq, mkv,
                              seq_first_row, seq_len, n_seq, (bf16*)out, nq, nkv, kv_k_head0, scale, cap, window, parts,
-                             piece, partial, n_places, slot, sinks);
+                             piece, partial, n_places, slot, sinks, seq_start);
     }
     auto kernel = cap > 0.f ? pt::attn_prefill_tc05_kernel<true> : pt::attn_prefill_tc05_kernel<false>;
     return launch_kernel("attn_prefill_tc05", kernel, dim3(nq, n_tiles_bound * parts), dim3(pt::THREADS), pt::SMEM_BYTES,
                          stream, 1, mq, mkv, seq_first_row, seq_len, n_seq, (bf16*)out, nq, nkv, kv_k_head0, scale, cap,
-                         window, parts, piece, partial, sinks);
+                         window, parts, piece, partial, sinks, seq_start);
 }
 
 int prefill_tc05_timeouts_async(int* host, cudaStream_t stream) {

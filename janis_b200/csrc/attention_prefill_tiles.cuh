@@ -70,10 +70,12 @@ __host__ __device__ __forceinline__ int parts_of(int n_tiles, int parts, int pie
 }  // namespace pf
 
 // The tcgen05 kernel of the same step (attention_prefill_tc05.cu): 0 launched, 1 failed (message set),
-// -1 this head size or these operands are not for it.
+// -1 this head size or these operands are not for it.  Without seq_start, keys and values lie beside the queries (kv_rows =
+// n_tok).  With it, sequences go on: seq_len holds lengths after the step, and kv_src every position's keys and values, a
+// sequence's behind those of the sequences before it (position p of sequence s in row seq_len[0] + .. + seq_len[s - 1] + p).
 int launch_prefill_tc05(const void* q_src, const void* kv_src, int n_tok, const int* seq_first_row, const int* seq_len,
                         int n_seq, int n_tiles_bound, void* out, int nq, int nkv, int q_row_elems, int kv_row_elems,
                         int kv_k_head0, float scale, float cap, int window, int parts, int piece, float* partial,
-                        const float* sinks, cudaStream_t stream);
+                        const float* sinks, const int* seq_start, int kv_rows, cudaStream_t stream);
 
 }  // namespace janis

@@ -93,7 +93,7 @@ def attention_lib(head_dim: int):
         lib.janis_attn_prefill.argtypes = [P, P, I, P, P, P, P, I, I, I, I, I, I, F, F, I, P, P, P, P, P, I, I, P]
         lib.janis_attn_decode.argtypes = [P, P, P, I, P, I, P, P, P, c_longlong, P, I, I, I, I, F, F, I, I, I, I, P]
         lib.janis_attn_prefill_mma.argtypes = [P, P, I, P, P, I, I, P, I, I, I, I, I, F, F, I, P, c_longlong,
-                                               P, P, P, P, P, I, I, I, I, I, P, P]
+                                               P, P, P, P, P, I, I, I, I, I, P, P, I, I, P]
         lib.janis_attn_decode_sinks.argtypes = [P, P, P, I, P, I, P, P, P, c_longlong, P, I, I, I, I, F, F, I, I, I, I, P, P]
         lib.janis_attn_set_prefill_kernel.argtypes = [I]
         lib.janis_attn_set_prefill_kernel.restype = None
@@ -619,7 +619,7 @@ def _cached_args(name, seq_start, seq_slot, kpool, vpool, page_table, ring_len, 
 def attn_prefill(qkv, tok_pos, tok_seq, seq_first_row, out, nq: int, nkv: int, hd: int, scale: float, cap: float,
                  window: int, kv_src=None, kv_row_heads=None, kv_k_head0=None, seq_len=None, tensor_cores=True,
                  scratch=None, seq_start=None, seq_slot=None, kpool=None, vpool=None, page_table=None,
-                 ring_len: int = 0, host_lens=None):
+                 ring_len: int = 0, host_lens=None, gathered=None, all_rows: int = 0, max_total: int = 0):
     """Causal (and windowed when window > 0) attention over packed sequences.
     qkv: [T, nq + 2 nkv, hd], or [T, nq, hd] when keys and values come from `kv_src`, another layer's
     [T, kv_row_heads, hd] rows whose key heads start at head kv_k_head0 (values nkv heads later).
@@ -630,13 +630,17 @@ def attn_prefill(qkv, tok_pos, tok_seq, seq_first_row, out, nq: int, nkv: int, h
     ring_len), which must still hold what those steps left (this step's own keys are stored afterwards).
     `host_lens`: the tokens each sequence brings to this step, if the host knows them (a step replayed from a graph
     with other lengths does not): the grid then has no places to spare.
+    `gathered` (bfloat16, at least all_rows x 2 nkv x hd; all_rows = the sum of `seq_len`, max_total its largest, as the host
+    knows them): room in which a step that continues sequences brings all keys and values together, so that it can run on
+    the kernel of whole prompts; without it such a step reads the pages itself, more slowly.
     bfloat16 with `seq_len` (int32 [n_seq]) runs on the tensor cores; float32 runs the CUDA-core kernel, which is
     exact 32-bit."""
     T = qkv.shape[0]
     if qkv.dtype == torch.bfloat16 and seq_len is not None and tensor_cores:
         return _attn_prefill_mma(qkv, seq_first_row, seq_len, out, nq, nkv, hd, scale, cap, window, kv_src,
                                  kv_row_heads, kv_k_head0, scratch,
-                                 (seq_start, seq_slot, kpool, vpool, page_table, ring_len), host_lens)
+                                 (seq_start, seq_slot, kpool, vpool, page_table, ring_len), host_lens,
+                                 gathered, all_rows, max_total)
     if kv_src is None:
         _t(qkv, "qkv", _FLOATS, (T, nq + 2 * nkv, hd))
         kv_src, kv_row_heads, kv_k_head0 = qkv, nq + 2 * nkv, nq
@@ -660,8 +664,27 @@ def attn_prefill(qkv, tok_pos, tok_seq, seq_first_row, out, nq: int, nkv: int, h
     return out
 
 
+GATHER_BYTES = 512 << 20       # the most that a step's keys and values may take when they are brought together
+
+
+def attn_gathered_elems(all_rows: int, nkv: int, hd: int, dtype=torch.bfloat16) -> int:
+    """Elements of the room that a step of continued sequences with all_rows positions wants as `gathered` (0: none; the step
+    runs on the kernel that reads the pages)."""
+    n = (all_rows * 2 * nkv * hd + (1 << 22) - 1) >> 22 << 22      # (in steps of 8 MB: the rows grow with every piece)
+    return n if all_rows and dtype == torch.bfloat16 and hd % 64 == 0 and hd <= 256 and 2 * n <= GATHER_BYTES else 0
+
+
+def _gathered_args(name, gathered, all_rows, max_total, seq_start, nkv, hd):
+    if gathered is None or seq_start is None:
+        return (None, 0, 0)
+    _t(gathered, "gathered", torch.bfloat16)
+    if gathered.numel() < all_rows * 2 * nkv * hd or max_total > all_rows:
+        raise KernelError(f"{name}: room for {gathered.numel()} elements does not hold {all_rows} positions of 2 x {nkv} heads of {hd}")
+    return (gathered.data_ptr(), int(all_rows), int(max_total))
+
+
 def _attn_prefill_mma(qkv, seq_first_row, seq_len, out, nq, nkv, hd, scale, cap, window, kv_src, kv_row_heads,
-                      kv_k_head0, scratch=None, cached=(None,) * 5 + (0,), host_lens=None):
+                      kv_k_head0, scratch=None, cached=(None,) * 5 + (0,), host_lens=None, gathered=None, all_rows=0, max_total=0):
     T = qkv.shape[0]
     if kv_src is None:
         _t(qkv, "qkv", torch.bfloat16, (T, nq + 2 * nkv, hd))
@@ -677,6 +700,7 @@ def _attn_prefill_mma(qkv, seq_first_row, seq_len, out, nq, nkv, hd, scale, cap,
     n_seq = seq_len.numel()
     _t(seq_len, "seq_len", torch.int32, (n_seq,))
     _t(seq_first_row, "seq_first_row", torch.int32, (n_seq,))
+    together = _gathered_args("attn_prefill", gathered, all_rows, max_total, cached[0], nkv, hd)
     cached = _cached_args("attn_prefill", *cached, torch.bfloat16, n_seq, nkv, hd)
     lib = attention_lib(hd)
     bm = lib.janis_attn_prefill_tile()      # queries per CTA
@@ -694,7 +718,7 @@ def _attn_prefill_mma(qkv, seq_first_row, seq_len, out, nq, nkv, hd, scale, cap,
                                            qkv.shape[1], kv_row_heads, kv_k_head0, float(scale), float(cap),
                                            int(window), _t(scratch, "scratch", torch.float32) if scratch is not None else None,
                                            scratch.numel() if scratch is not None else 0, *cached,
-                                           max(int(n) for n in host_lens) if host_lens else 0, 0, 0, None, _stream()))
+                                           max(int(n) for n in host_lens) if host_lens else 0, 0, 0, None, *together, _stream()))
     global _launches
     _launches += int(lib.janis_attn_prefill_kernels()) - 1     # the merge, when tiles were shared
     return out
@@ -707,7 +731,7 @@ def attn_rows_sizes(dtype, H: int, G: int, d: int, dv: int) -> bool:
 
 def attn_prefill_rows(rows, seq_first_row, seq_len, out, H: int, G: int, hd: int, scale: float, window: int = 0, cap: float = 0.0,
                       sinks=None, scratch=None, host_lens=None, seq_start=None, seq_slot=None, kpool=None, vpool=None,
-                      page_table=None):
+                      page_table=None, gathered=None, all_rows: int = 0, max_total: int = 0):
     """`attn_prefill` (bfloat16, tensor cores) over rows that hold q (H heads), k and v (G heads each) first and anything
     behind them; sinks [H] float32: exp of head h's number joins its denominator.  window < 0: keys are seen
     inside the query's own chunk of -window positions, counted from the sequence's first.  The line of a step that continues
@@ -720,6 +744,7 @@ def attn_prefill_rows(rows, seq_first_row, seq_len, out, H: int, G: int, hd: int
     n_seq = seq_len.numel()
     _t(seq_len, "seq_len", torch.int32, (n_seq,))
     _t(seq_first_row, "seq_first_row", torch.int32, (n_seq,))
+    together = _gathered_args("attn_prefill_rows", gathered, all_rows, max_total, seq_start, G, hd)
     cached = _cached_args("attn_prefill_rows", seq_start, seq_slot, kpool, vpool, page_table, 0, torch.bfloat16, n_seq, G, hd)
     lib = attention_lib(hd)
     bm = lib.janis_attn_prefill_tile()
@@ -737,7 +762,7 @@ def attn_prefill_rows(rows, seq_first_row, seq_len, out, H: int, G: int, hd: int
                                            _t(scratch, "scratch", torch.float32) if scratch is not None else None,
                                            scratch.numel() if scratch is not None else 0, *cached,
                                            max(int(n) for n in host_lens) if host_lens else 0, width, width,
-                                           _t(sinks, "sinks", torch.float32, (H,)) if sinks is not None else None, _stream()))
+                                           _t(sinks, "sinks", torch.float32, (H,)) if sinks is not None else None, *together, _stream()))
     global _launches
     _launches += int(lib.janis_attn_prefill_kernels()) - 1
     return out

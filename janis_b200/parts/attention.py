@@ -77,6 +77,13 @@ def decode_geometry(ctx: StepContext, sm_count: int, head_dim: int, n_kv_heads: 
     return chunk, max_chunks
 
 
+def gathered_room(ctx: StepContext, n_kv_heads: int, head_dim: int) -> dict:
+    """The room in which a step that continues sequences brings its keys and values together, as arguments of the prompt
+    attention (nothing where the kernels have no use for it)."""
+    elems = getattr(ctx.rt.ops, "attn_gathered_elems", lambda *a: 0)(ctx.all_rows, n_kv_heads, head_dim, ctx.rt.dtype)
+    return dict(gathered=ctx.ws.buf("attn.gathered", (elems,), ctx.rt.dtype), all_rows=ctx.all_rows, max_total=ctx.len_bound) if elems else {}
+
+
 class SoftmaxAttention(Mixer):
     def __init__(self, hidden: int, n_heads: int, n_kv_heads: int, head_dim: int, scale: float,
                  position: PositionEncoding, names: dict[str, str], softcap: float = 0.0,
@@ -155,7 +162,7 @@ class SoftmaxAttention(Mixer):
             n_scratch = ops.attn_prefill_scratch_floats(T, ctx.n_seq, nq, hd, rt.dtype)
             scratch = ws.buf("attn.prefill_partial", (n_scratch,), torch.float32) if n_scratch else None
             before = dict(seq_start=ctx.seq_start, seq_slot=ctx.seq_slot, kpool=kv.k, vpool=kv.v, page_table=kv.table,
-                          ring_len=kv.ring_len) if extends else {}
+                          ring_len=kv.ring_len, **gathered_room(ctx, nkv, hd)) if extends else {}
             if own:
                 if line.has_readers:
                     ctx.shared[("kv", line.index)] = (qkv, heads, nq)

@@ -152,6 +152,7 @@ class StepContext:
     extends: bool = False           # a "prefill" step some of whose sequences have tokens in the cache already
                                     # (seq_start > 0): a mixer reads those from its cache line and stores this
                                     # step's own only after it has attended
+    all_rows: int = 0               # host-side: the sum of seq_end of such a step
     shared: dict = field(default_factory=dict)   # scratch that parts of one step hand to each other
 
 

@@ -48,7 +48,7 @@ import torch
 from ..cache.cache import KVNeed
 from ..weights.loader import TensorSpec
 from .base import Mixer, Runtime, StepContext
-from .attention import decode_geometry
+from .attention import decode_geometry, gathered_room
 from .position import RotaryEncoding
 
 
@@ -297,6 +297,7 @@ class TalkingHeadsAttention(Mixer):
                                         seen, chunk, max_chunks, cap=self.cap, sinks=self.sink_values)
         n_scratch = ops.attn_prefill_scratch_floats(ctx.n_tok, ctx.n_seq, H, d, rt.dtype)
         scratch = ws.buf("attn.prefill_partial", (n_scratch,), torch.float32) if n_scratch else None
-        before = dict(seq_start=ctx.seq_start, seq_slot=ctx.seq_slot, kpool=kv.k, vpool=kv.v, page_table=kv.table) if ctx.extends else {}
+        before = dict(seq_start=ctx.seq_start, seq_slot=ctx.seq_slot, kpool=kv.k, vpool=kv.v, page_table=kv.table,
+                      **gathered_room(ctx, G, d)) if ctx.extends else {}
         return ops.attn_prefill_rows(rows, ctx.seq_first_row, ctx.seq_end, att, H, G, d, self.scale, seen, cap=self.cap,
                                      sinks=self.sink_values, scratch=scratch, host_lens=ctx.step_lens, **before)

@@ -631,6 +631,51 @@ def test_attn_prefill_continues_from_the_cache(nq, nkv, hd, window, ring, cap):
         same(v2.cpu(), vr, "kv_store values")
 
 
+@pytest.mark.parametrize("hd,nq,nkv", [(64, 4, 2), (256, 2, 1)])
+@pytest.mark.parametrize("window,ring,cap", [(0, 0, 0.0), (0, 0, 20.0), (100, 128, 20.0), (64, 64, 0.0), (-100, 0, 0.0)])
+@pytest.mark.parametrize("form", [2, 3])
+def test_continued_prompt_through_gathered_rows(hd, nq, nkv, window, ring, cap, form):
+    """The tcgen05 kernel over keys and values brought together from the cache line and the step, in both of its forms, with
+    shared tiles of queries and without, against the mma.sync kernel that reads the pages (itself tested against the statement
+    above).  The room holds NaN before: what a window leaves out is not written, and must not count."""
+    starts, news, slots = [0, 5, 64, 700, 130, 63, 1], [70, 9, 1, 150, 260, 129, 1], [2, 0, 5, 1, 3, 4, 6]
+    n_seq, T = len(starts), sum(news)
+    pages_per_seq = ring // R.PAGE if ring else 14
+    n_pages = 7 * pages_per_seq + 3
+    perm = torch.randperm(n_pages, generator=torch.Generator().manual_seed(5))[:7 * pages_per_seq].view(7, pages_per_seq).int()
+    d = dev()
+    first = torch.tensor([0] + list(np.cumsum(news)[:-1]), dtype=torch.int32, device=d)
+    seq_start, seq_slot = torch.tensor(starts, dtype=torch.int32, device=d), torch.tensor(slots, dtype=torch.int32, device=d)
+    ends = [s + n for s, n in zip(starts, news)]
+    k, v = _paged(n_pages, nkv, hd, torch.bfloat16, 60)
+    qkv = rnd((T, nq + 2 * nkv, hd), torch.bfloat16, 62)
+    cached = dict(seq_start=seq_start, seq_slot=seq_slot, kpool=k, vpool=v, page_table=perm.to(d), ring_len=ring)
+    n = ops().attn_prefill_scratch_floats(T, n_seq, nq, hd)
+
+    def run(piece=0, **more):
+        out = torch.full((T, nq * hd), 9.0, dtype=torch.bfloat16, device=d)
+        ops().attn_set_prefill_piece(hd, piece)
+        try:
+            ops().attn_prefill(qkv, None, None, first, out, nq, nkv, hd, 1.0 / math.sqrt(hd), cap, window,
+                               seq_len=torch.tensor(ends, dtype=torch.int32, device=d),
+                               scratch=torch.full((n,), float("nan"), device=d) if n else None, host_lens=news, **cached, **more)
+        finally:
+            ops().attn_set_prefill_piece(hd, 0)
+        return out
+
+    want = run().double().cpu()
+    assert ops().attn_gathered_elems(sum(ends), nkv, hd) >= sum(ends) * 2 * nkv * hd
+    ops().attn_set_prefill_kernel(hd, form)
+    try:
+        for piece in (0, 4, 100):
+            room = torch.full((sum(ends) * 2 * nkv * hd + 64,), float("nan"), dtype=torch.bfloat16, device=d)
+            got = run(piece, gathered=room, all_rows=sum(ends), max_total=max(ends))
+            close(got, want, 2 * BF16_TOL, f"through gathered rows, pieces of {piece}")
+            assert room[-64:].isnan().all() and not room[:64].isnan().any()
+    finally:
+        ops().attn_set_prefill_kernel(hd, 1)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attn_prefill_reads_another_layers_keys(dtype):
     nq, nkv, hd = 4, 2, 32
