@@ -910,6 +910,327 @@ talk_attention_mma_kernel(const bf16* __restrict__ q_rows, int q_row_elems, cons
     }
 }
 
+// ---------------------------------------------------------------------------
+// Prompts whose heads are mixed before the softmax, 4 or 8 of them: sixteen rows and all heads a CTA.
+//
+// The kernel above keeps the sums of all heads in shared memory, which leaves it eight rows at 8 heads of 256 (half of every
+// 16-row operand idle), one buffer for keys and values in turn, and five barriers a tile of 32 keys.  Here a warp keeps what it
+// uses in every tile in registers: the queries of a pair of heads over a part of their features, and the pair's sums over a part
+// of the value features.  A tile of 32 keys, which lies in one page, takes three barriers:
+//   scores   a warp per (pair of heads, part of the features); every key is read from shared memory once, and the parts'
+//            sums meet in shared memory
+//   weights  a warp per row, a lane per key: parts added, scaled, capped, heads mixed, masked, online softmax, P as bfloat16
+//   sums     a warp per (pair of heads, part of the value features): O = O corr + P V; every value is read once
+// The values of a tile arrive while its scores and weights are formed, the keys of the next one during its weights and sums.
+// What bounds it is shared memory: some 430 KB a tile pass through it at 8 heads of 256, and 128 KB come from L2.
+// ---------------------------------------------------------------------------
+constexpr int TP_ROWS = 16, TP_BN = 32;
+
+struct TalkPromptShape {
+    int G, d, dv, block, window, sink;
+    float scale, cap;
+};
+
+// bytes: keys, values (the way out's sums in their place), parts of the scores, P, and per (head, row) m, l, corr; the matrix
+__host__ __device__ inline size_t talk_prompt_tiles_bytes(int H, int G, int d, int dv) {
+    const size_t tiles = (size_t)G * TP_BN * (d + 8 + dv + 8) * 2, sums = (size_t)H * TP_ROWS * (dv + 4) * 4;
+    return ((tiles > sums ? tiles : sums) + 15) & ~(size_t)15;
+}
+__host__ __device__ inline size_t talk_prompt_bytes(int H, int G, int d, int dv) {
+    return talk_prompt_tiles_bytes(H, G, d, dv) + (size_t)32 / H * H * TP_ROWS * TP_BN * 4 + (size_t)H * TP_ROWS * (TP_BN + 8) * 2 +
+           (size_t)3 * H * TP_ROWS * 4 + (size_t)H * H * 4 + 3 * TP_ROWS * 4;
+}
+
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+__device__ __forceinline__ float warp_max_redux(float v) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+template <int H, bool SHARED_KV>            // SHARED_KV: the heads of a pair read the same key/value head
+__global__ void __launch_bounds__(512, 1)
+talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
+                   const int* __restrict__ seq_slot, const bf16* __restrict__ kpool, const bf16* __restrict__ vpool,
+                   const int* __restrict__ page_table, int table_stride, const float* __restrict__ talk, const float* __restrict__ inv_v,
+                   bf16* __restrict__ out, const float* __restrict__ sink_vals, int n_tok, TalkPromptShape sh) {
+    constexpr int PARTS = 32 / H;           // warps that share a pair of heads: 4 or 8
+    constexpr int KS = 16 / PARTS;          // steps of 16 features a part has at 256 features: 4 or 2
+    constexpr int NT = 32 / PARTS;          // tiles of 8 value features a part has at 256: 8 or 4
+    extern __shared__ __align__(16) unsigned char talk_raw[];
+    const int G = sh.G, d = sh.d, dv = sh.dv, rep = H / G, ldk = d + 8, ldv = dv + 8;
+    bf16* k_s = reinterpret_cast<bf16*>(talk_raw);                         // [G][TP_BN][ldk]
+    bf16* v_s = k_s + (size_t)G * TP_BN * ldk;                             // [G][TP_BN][ldv]
+    float* part_s = reinterpret_cast<float*>(talk_raw + talk_prompt_tiles_bytes(H, G, d, dv));      // [PARTS][H][16][32], columns swizzled
+    bf16* p_s = reinterpret_cast<bf16*>(part_s + PARTS * H * TP_ROWS * TP_BN);                     // [H][16][TP_BN + 8]
+    float* m_s = reinterpret_cast<float*>(p_s + H * TP_ROWS * (TP_BN + 8));                        // [H][16]
+    float* l_s = m_s + H * TP_ROWS;
+    float* corr_s = l_s + H * TP_ROWS;
+    float* talk_s = corr_s + H * TP_ROWS;
+    int* pos_s = reinterpret_cast<int*>(talk_s + H * H);
+    int* seq_s = pos_s + TP_ROWS;
+    int* slot_s = seq_s + TP_ROWS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gr = lane >> 2, gc = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
+    const int pair = warp / PARTS, part = warp % PARTS;
+    const int ks = d / (16 * PARTS), nt2 = dv / (16 * PARTS);              // this warp's steps of features, its pairs of value tiles
+    // the last rows of a prompt see the most keys: they start first
+    const int r0 = (int)(gridDim.x - 1 - blockIdx.x) * TP_ROWS, n_rows = min(TP_ROWS, n_tok - r0);
+    grid_dependents_launch();
+    if (tid < TP_ROWS) {
+        const bool in = tid < n_rows;
+        const int sq = in ? tok_seq[r0 + tid] : -1;
+        pos_s[tid] = in ? tok_pos[r0 + tid] : 0;
+        seq_s[tid] = sq;
+        slot_s[tid] = in ? seq_slot[sq] : -1;
+    }
+    for (int u = tid; u < H * H; u += 512) talk_s[u] = talk[u];
+    for (int u = tid; u < H * TP_ROWS; u += 512) {
+        m_s[u] = sh.sink ? (sink_vals != nullptr ? sink_vals[u / TP_ROWS] : 0.f) : -CUDART_INF_F;
+        l_s[u] = sh.sink ? 1.f : 0.f;
+        corr_s[u] = 1.f;
+    }
+    grid_dependency_wait();
+    // the pair's queries over this warp's features, as first operands
+    uint32_t qa[2][KS][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int r = gr + (x & 1) * 8, c = (part * ks + k) * 16 + (x >> 1) * 8 + gc;
+                qa[e][k][x] = k < ks && r < n_rows
+                                  ? *reinterpret_cast<const uint32_t*>(q_rows + (size_t)(r0 + r) * q_row_elems + (size_t)(2 * pair + e) * d + c)
+                                  : 0u;
+            }
+    float o[2][NT][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) o[e][n][x] = 0.f;
+    __syncthreads();
+    const uint32_t k_a = smem_u32(k_s), v_a = smem_u32(v_s), p_a = smem_u32(p_s);
+
+    // rows of a tile from one page; what lies outside first .. last becomes zeros (0 x NaN is NaN)
+    auto load = [&](uint32_t dst, const bf16* pool, int width, int ld, const int* table, int j0, int first, int last) {
+        const size_t base = (size_t)table[j0 / JANIS_PAGE] * G * JANIS_PAGE + j0 % JANIS_PAGE;
+        for (int row = warp; row < G * TP_BN; row += 16) {
+            const int g = row / TP_BN, jj = row % TP_BN, j = j0 + jj;
+            const bool ok = j >= first && j <= last;
+            const bf16* src = pool + (base + (size_t)g * JANIS_PAGE + (ok ? jj : 0)) * width;
+            for (int c8 = lane; c8 < width / 8; c8 += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (row * ld + c8 * 8) * 2), "l"(src + c8 * 8), "r"(ok ? 16 : 0) : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    for (int a = 0; a < n_rows;) {
+        int b = a + 1;
+        while (b < n_rows && seq_s[b] == seq_s[a]) ++b;
+        const int slot = slot_s[a];
+        if (slot < 0) {
+            a = b;
+            continue;
+        }
+        int first = sh.block > 0 ? pos_s[a] / sh.block * sh.block : 0;
+        const int last = pos_s[b - 1];
+        if (sh.window > 0) first = max(first, pos_s[a] - sh.window + 1);
+        const int* table = page_table + (size_t)slot * table_stride;
+        int j0 = first / TP_BN * TP_BN;
+        load(k_a, kpool, d, ldk, table, j0, first, last);
+        for (; j0 <= last; j0 += TP_BN) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                                               // the keys are there; the values before have been read
+            load(v_a, vpool, dv, ldv, table, j0, first, last);
+            // ---- scores, 16 keys at a time
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                float acc[2][2][4];
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) acc[e][0][x] = acc[e][1][x] = 0.f;
+#pragma unroll
+                for (int k = 0; k < KS; ++k) {
+                    if (k >= ks) break;
+#pragma unroll
+                    for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
+                        uint32_t bq[4];
+                        ldsm_x4(bq, k_a + (((2 * pair + e) / rep * TP_BN + 16 * n + lr + (lm >> 1) * 8) * ldk + (part * ks + k) * 16 + (lm & 1) * 8) * 2);
+#pragma unroll
+                        for (int f = 0; f < 2; ++f) {
+                            if (!SHARED_KV && f != e) continue;
+                            const uint32_t b0[2] = {bq[0], bq[1]}, b1[2] = {bq[2], bq[3]};
+                            mma_bf16(acc[f][0], qa[f][k], b0);
+                            mma_bf16(acc[f][1], qa[f][k], b1);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+#pragma unroll
+                    for (int z = 0; z < 2; ++z)
+#pragma unroll
+                        for (int x = 0; x < 2; ++x) {
+                            const int r = gr + 8 * x;
+                            *reinterpret_cast<float2*>(part_s + ((part * H + 2 * pair + e) * TP_ROWS + r) * TP_BN + ((16 * n + 8 * z + gc) ^ ((r & 3) * 8))) =
+                                make_float2(acc[e][z][2 * x], acc[e][z][2 * x + 1]);
+                        }
+            }
+            __syncthreads();                                               // the scores are there; the keys have been read
+            const bool more = j0 + TP_BN <= last;
+            if (more) load(k_a, kpool, d, ldk, table, j0 + TP_BN, first, last);
+            // ---- weights: row `warp`, key j0 + lane
+            {
+                const int r = warp, j = j0 + lane, pos = pos_s[r];
+                bool seen = r >= a && r < b && j >= first && j <= pos;
+                if (sh.block > 0) seen = seen && j >= pos / sh.block * sh.block;
+                if (sh.window > 0) seen = seen && j > pos - sh.window;
+                float raw[H], p[H];
+#pragma unroll
+                for (int g = 0; g < H; ++g) {
+                    const float* src = part_s + (g * TP_ROWS + r) * TP_BN + (lane ^ ((r & 3) * 8));
+                    float z = 0.f;
+#pragma unroll
+                    for (int q = 0; q < PARTS; ++q) z += src[q * H * TP_ROWS * TP_BN];
+                    z *= sh.scale;
+                    if (sh.cap > 0.f) z = sh.cap * tanhf(z / sh.cap);
+                    raw[g] = z;
+                }
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int g = 0; g < H; g += 4) {
+                        const float4 t = *reinterpret_cast<const float4*>(talk_s + h * H + g);
+                        s = fmaf(t.x, raw[g], s);
+                        s = fmaf(t.y, raw[g + 1], s);
+                        s = fmaf(t.z, raw[g + 2], s);
+                        s = fmaf(t.w, raw[g + 3], s);
+                    }
+                    s = seen ? s : -CUDART_INF_F;
+                    const float m_old = m_s[h * TP_ROWS + r], m_new = fmaxf(m_old, warp_max_redux(s));
+                    p[h] = 0.f;
+                    float corr = 1.f;
+                    if (m_new != -CUDART_INF_F) {
+                        p[h] = expf(s - m_new);
+                        if (m_new != m_old) corr = m_old == -CUDART_INF_F ? 0.f : expf(m_old - m_new);
+                    }
+                    p_s[(h * TP_ROWS + r) * (TP_BN + 8) + lane] = __float2bfloat16_rn(p[h]);
+                    __syncwarp();                                          // every lane has read the old maximum
+                    if (lane == 0) {
+                        m_s[h * TP_ROWS + r] = m_new;
+                        corr_s[h * TP_ROWS + r] = corr;
+                    }
+                }
+                // the heads' sums over the lanes, each stage halving the heads a lane still carries
+                int h = 0, off = 16;
+#pragma unroll
+                for (int n = H / 2; n >= 1; n >>= 1, off >>= 1) {
+                    const bool upper = (lane & off) != 0;
+                    h += upper ? n : 0;
+#pragma unroll
+                    for (int i = 0; i < n; ++i) {
+                        const float mine = upper ? p[i + n] : p[i], theirs = upper ? p[i] : p[i + n];
+                        p[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, off);
+                    }
+                }
+                for (; off >= 1; off >>= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], off);
+                __syncwarp();
+                if ((lane & (32 / H - 1)) == 0) l_s[h * TP_ROWS + r] = l_s[h * TP_ROWS + r] * corr_s[h * TP_ROWS + r] + p[0];
+            }
+            if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                                               // the weights and the values are there
+            // ---- sums
+            {
+                uint32_t pa[2][2][4];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float c_lo = corr_s[(2 * pair + e) * TP_ROWS + gr], c_hi = corr_s[(2 * pair + e) * TP_ROWS + gr + 8];
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        o[e][n][0] *= c_lo;
+                        o[e][n][1] *= c_lo;
+                        o[e][n][2] *= c_hi;
+                        o[e][n][3] *= c_hi;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+                        ldsm_x4(pa[e][k], p_a + (((2 * pair + e) * TP_ROWS + (lane & 15)) * (TP_BN + 8) + 16 * k + (lane >> 4) * 8) * 2);
+                }
+#pragma unroll
+                for (int n = 0; n < NT / 2; ++n) {
+                    if (n >= nt2) break;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k)
+#pragma unroll
+                        for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
+                            uint32_t bv[4];
+                            ldsm_x4_trans(bv, v_a + (((2 * pair + e) / rep * TP_BN + 16 * k + lr + (lm & 1) * 8) * ldv + (part * nt2 + n) * 16 + (lm >> 1) * 8) * 2);
+#pragma unroll
+                            for (int f = 0; f < 2; ++f) {
+                                if (!SHARED_KV && f != e) continue;
+                                const uint32_t b0[2] = {bv[0], bv[1]}, b1[2] = {bv[2], bv[3]};
+                                mma_bf16(o[f][2 * n], pa[f][k], b0);
+                                mma_bf16(o[f][2 * n + 1], pa[f][k], b1);
+                            }
+                        }
+                }
+            }
+        }
+        __syncthreads();                                                   // the last values have been read
+        a = b;
+    }
+    // ---- the way out: the sums through shared memory, divided, turned back by the row's position, rounded
+    const int os = dv + 4;
+    float* o_s = reinterpret_cast<float*>(talk_raw);
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            if (n >= 2 * nt2) break;
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+                *reinterpret_cast<float2*>(o_s + ((2 * pair + e) * TP_ROWS + gr + 8 * x) * os + (part * 2 * nt2 + n) * 8 + gc) =
+                    make_float2(o[e][n][2 * x], o[e][n][2 * x + 1]);
+        }
+    __syncthreads();
+    const int hv = dv >> 1;
+    for (int u = tid; u < n_rows * H * hv; u += 512) {
+        const int m = u % hv, h = (u / hv) % H, r = u / (hv * H);
+        bf16* o_row = out + (size_t)(r0 + r) * H * dv + (size_t)h * dv;
+        float lo = 0.f, hi = 0.f;
+        if (slot_s[r] >= 0) {
+            const float inv_l = 1.f / l_s[h * TP_ROWS + r];
+            const float* src = o_s + (h * TP_ROWS + r) * os;
+            if (inv_v != nullptr) {
+                float s, c;
+                sincosf((float)pos_s[r] * inv_v[m], &s, &c);
+                rotate_pair(src[m] * inv_l, src[m + hv] * inv_l, -s, c, lo, hi);
+            } else {
+                lo = src[m] * inv_l;
+                hi = src[m + hv] * inv_l;
+            }
+        }
+        o_row[m] = __float2bfloat16_rn(lo);
+        o_row[m + hv] = __float2bfloat16_rn(hi);
+    }
+}
+
+// Whether talk_prompt_kernel takes the sizes: 4 or 8 heads, features in whole parts of whole steps up to 256, tiles that fit.
+static bool talk_prompt_takes(int H, int G, int d, int dv) {
+    if ((H != 4 && H != 8) || H % G || d > 256 || dv > 256) return false;
+    const int step = 16 * (32 / H);
+    return d % step == 0 && dv % step == 0 && talk_prompt_bytes(H, G, d, dv) <= (size_t)226 * 1024;
+}
+
 // The chunks of a decode row put together, in ascending order: per head the maximum over the chunks (and the
 // sink's 0), the weights exp(m_c - M), the denominators and sums added, divided, turned back, rounded.
 __global__ void __launch_bounds__(128)
@@ -1048,7 +1369,7 @@ static int talk_plain_tile(int H, int G, int d, int dv, size_t* bytes) {
     return 0;
 }
 
-static int talk_kernel_choice = 1;        // 1: the tensor-core kernel where it fits; 0: the plain kernel always
+static int talk_kernel_choice = 1;        // 1: the tensor-core kernels where they fit; 2: without the prompt kernel; 0: the plain kernel always
 
 JANIS_EXPORT void janis_talk_attention_set_kernel(int which) { talk_kernel_choice = which; }
 
@@ -1143,7 +1464,24 @@ JANIS_EXPORT int janis_talk_attention(const void* q_rows, int dtype, int q_row_e
     if (two_pass && (stats == nullptr || stats_floats < (long long)T * 2 * H))
         return fail("talk_attention: heads mixed after the softmax need %lld floats for the rows' maxima and denominators", (long long)T * 2 * H);
     if (v_in_keys) vpool = kpool;
-    if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && q_row_elems % 8 == 0 &&
+    // Prompts of 4 or 8 heads mixed before the softmax: 8 heads of 256 over 4, one prompt of 2,048 tokens 441 us a layer against
+    // 743 in the kernel below, 300 tokens 86 against 131, eight of 512 210 against 470, 16 tokens 32 = 32.  The kernel below takes the
+    // other sizes, decode steps and what this one leaves out.
+    if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && talk != nullptr && !mix_after && !one_row && !v_in_keys &&
+        keep_first == 0 && q_row_elems % 2 == 0 && talk_prompt_takes(H, G, d, dv) &&
+        (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0 && ((uintptr_t)q_rows & 3) == 0) {
+        const TalkPromptShape ps = {G, d, dv, block, window, sink ? 1 : 0, scale, cap};
+        const size_t bytes = talk_prompt_bytes(H, G, d, dv);
+        const bool pairs = (H / G) % 2 == 0;
+        auto kernel = H == 8 ? (pairs ? talk_prompt_kernel<8, true> : talk_prompt_kernel<8, false>)
+                             : (pairs ? talk_prompt_kernel<4, true> : talk_prompt_kernel<4, false>);
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        if (e != cudaSuccess) return fail("talk_attention: shared memory of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+        return launch_kernel("talk_attention", kernel, dim3((T + TP_ROWS - 1) / TP_ROWS), dim3(512), bytes, stream, 1, (const bf16*)q_rows,
+                             q_row_elems, tok_pos, tok_seq, seq_slot, (const bf16*)kpool, (const bf16*)vpool, page_table, table_stride,
+                             talk, inv_v, (bf16*)out, sink_vals, T, ps);
+    }
+    if (dtype == JANIS_BF16 && talk_kernel_choice != 0 && q_row_elems % 8 == 0 &&
         (((uintptr_t)q_rows | (uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0) {
         size_t mma_bytes = 0;
         TalkMmaShape ms = talk_mma_shape(H, G, d, dv, one_row, &mma_bytes);

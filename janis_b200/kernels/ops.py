@@ -1049,7 +1049,8 @@ def talk_attention_scratch_floats(T: int, n_chunks: int, H: int, dv: int) -> int
 
 
 def talk_attention_set_kernel(which: int = 1) -> None:
-    """1: the tensor-core kernel where the sizes allow it (the default); 0: the plain kernel always.  For tests."""
+    """1: the tensor-core kernels where the sizes allow it (the default); 2: the same without the kernel for prompts of 4 or 8
+    mixed heads; 0: the plain kernel always.  For tests."""
     mixers().janis_talk_attention_set_kernel(int(which))
 
 

@@ -286,6 +286,48 @@ def test_attention_kernel_against_its_statement(dtype, H, G, d, dv, block, sink,
 
 
 @GPU
+@pytest.mark.parametrize("H,G,d,dv", [(8, 4, 256, 256), (8, 2, 64, 128), (8, 8, 128, 64), (4, 2, 128, 256), (4, 4, 256, 128)])
+@pytest.mark.parametrize("block,window,sink,cap,turn", [(0, 0, True, 0.0, True), (40, 0, True, 5.0, False), (0, 33, False, 0.0, True)])
+def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, turn):
+    """Whole runs of rows through the kernel that keeps sixteen rows and all heads a CTA: sequences of unequal lengths side by
+    side in a CTA, some from later positions, one without a slot, tiles that begin before a block or a window, learnt sinks,
+    and pages whose unseen places hold NaN."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    lens, starts = [1, 21, 97, 40, 5], [0, 30, 0, 64, 0]
+    ends = [n + s for n, s in zip(lens, starts)]
+    kp, vp, table, slots = _paged(len(lens), ends, G, d, dv, torch.bfloat16, 3)
+    for s, n in enumerate(ends):                   # behind a sequence's end
+        page = int(table[int(slots[s]), (n - 1) // ops.PAGE])
+        kp[page, :, (n - 1) % ops.PAGE + 1:] = float("nan")
+        vp[page, :, (n - 1) % ops.PAGE + 1:] = float("nan")
+    slots[4] = -1
+    tok_pos = torch.cat([torch.arange(s, s + n) for s, n in zip(starts, lens)]).int()
+    tok_seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int()
+    T = len(tok_pos)
+    g = torch.Generator().manual_seed(H * d + block)
+    q = torch.randn(T, H * d + 8, generator=g).bfloat16()
+    M = (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).float()
+    inv_v = torch.tensor([10000.0 ** (-2.0 * m / dv) for m in range(dv // 2)], dtype=torch.float32) if turn else None
+    sinks = torch.randn(H, generator=g) if sink and cap else None
+    want = torch.zeros(T, H * dv, dtype=torch.bfloat16)
+    R.talk_attention(q, tok_pos, tok_seq, slots, kp, vp, table, M, inv_v, want, H, G, d, dv, d ** -0.5, block, sink, window=window, cap=cap,
+                     sink_values=sinks)
+    dev = lambda x: x.cuda() if x is not None else None
+    off = {}
+    for which in (1, 2):
+        ops.talk_attention_set_kernel(which)
+        try:
+            got = torch.full((T, H * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+            ops.talk_attention(dev(q), dev(tok_pos), dev(tok_seq), dev(slots), dev(kp), dev(vp), dev(table), dev(M), dev(inv_v), got,
+                               H, G, d, dv, d ** -0.5, block, sink, window=window, cap=cap, sink_values=dev(sinks))
+        finally:
+            ops.talk_attention_set_kernel(1)
+        off[which] = (got.cpu().double() - want.double()).abs().max().item()
+        assert off[which] <= 2e-2 * max(1.0, want.double().abs().max().item()), (which, off)
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,d,dv,rot,turn", [(4, 2, 32, 16, 16, True), (3, 3, 16, 32, 16, False), (2, 1, 48, 40, 0, True)])
 def test_rotation_and_cache_write_against_their_statement(dtype, H, G, d, dv, rot, turn):
