@@ -928,6 +928,7 @@ constexpr int TP_ROWS = 16, TP_BN = 32;
 
 struct TalkPromptShape {
     int G, d, dv, block, window, sink;
+    int chunk_tiles;    // > 0: a row's tiles of keys are cut over gridDim.y CTAs, so many each, which leave partial results
     float scale, cap;
 };
 
@@ -957,7 +958,7 @@ __global__ void __launch_bounds__(512, 1)
 talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
                    const int* __restrict__ seq_slot, const bf16* __restrict__ kpool, const bf16* __restrict__ vpool,
                    const int* __restrict__ page_table, int table_stride, const float* __restrict__ talk, const float* __restrict__ inv_v,
-                   bf16* __restrict__ out, const float* __restrict__ sink_vals, int n_tok, TalkPromptShape sh) {
+                   bf16* __restrict__ out, const float* __restrict__ sink_vals, int n_tok, TalkPromptShape sh, float* __restrict__ partial) {
     constexpr int PARTS = 32 / H;           // warps that share a pair of heads: 4 or 8
     constexpr int KS = 16 / PARTS;          // steps of 16 features a part has at 256 features: 4 or 2
     constexpr int NT = 32 / PARTS;          // tiles of 8 value features a part has at 256: 8 or 4
@@ -988,9 +989,10 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
         slot_s[tid] = in ? seq_slot[sq] : -1;
     }
     for (int u = tid; u < H * H; u += 512) talk_s[u] = talk[u];
+    const bool split = sh.chunk_tiles > 0;                                 // (the sink joins at the merge)
     for (int u = tid; u < H * TP_ROWS; u += 512) {
-        m_s[u] = sh.sink ? (sink_vals != nullptr ? sink_vals[u / TP_ROWS] : 0.f) : -CUDART_INF_F;
-        l_s[u] = sh.sink ? 1.f : 0.f;
+        m_s[u] = sh.sink && !split ? (sink_vals != nullptr ? sink_vals[u / TP_ROWS] : 0.f) : -CUDART_INF_F;
+        l_s[u] = sh.sink && !split ? 1.f : 0.f;
         corr_s[u] = 1.f;
     }
     grid_dependency_wait();
@@ -1039,10 +1041,18 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
             continue;
         }
         int first = sh.block > 0 ? pos_s[a] / sh.block * sh.block : 0;
-        const int last = pos_s[b - 1];
+        int last = pos_s[b - 1];
         if (sh.window > 0) first = max(first, pos_s[a] - sh.window + 1);
         const int* table = page_table + (size_t)slot * table_stride;
         int j0 = first / TP_BN * TP_BN;
+        if (split) {                                                       // this CTA's share of the run's tiles
+            j0 += (int)blockIdx.y * sh.chunk_tiles * TP_BN;
+            if (blockIdx.y + 1 < gridDim.y) last = min(last, j0 + sh.chunk_tiles * TP_BN - 1);
+            if (j0 > last) {
+                a = b;
+                continue;
+            }
+        }
         load(k_a, kpool, d, ldk, table, j0, first, last);
         for (; j0 <= last; j0 += TP_BN) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1089,7 +1099,7 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
             // ---- weights: row `warp`, key j0 + lane
             {
                 const int r = warp, j = j0 + lane, pos = pos_s[r];
-                bool seen = r >= a && r < b && j >= first && j <= pos;
+                bool seen = r >= a && r < b && j >= first && j <= pos && j <= last;
                 if (sh.block > 0) seen = seen && j >= pos / sh.block * sh.block;
                 if (sh.window > 0) seen = seen && j > pos - sh.window;
                 float raw[H], p[H];
@@ -1202,6 +1212,20 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
                     make_float2(o[e][n][2 * x], o[e][n][2 * x + 1]);
         }
     __syncthreads();
+    if (split) {
+        // per row and head the unnormalised sums, then the maximum and the denominator (no key seen: -inf, and no sums)
+        float* base = partial + ((size_t)r0 * gridDim.y + blockIdx.y) * H * (dv + 2);
+        for (int hr = warp; hr < n_rows * H; hr += 16) {
+            const int r = hr / H, h = hr % H;
+            const float m = m_s[h * TP_ROWS + r];
+            float* dst = base + ((size_t)r * gridDim.y * H + h) * (dv + 2);
+            if (m != -CUDART_INF_F)
+                for (int c = 2 * lane; c < dv; c += 64)
+                    *reinterpret_cast<float2*>(dst + c) = *reinterpret_cast<const float2*>(o_s + (h * TP_ROWS + r) * os + c);
+            if (lane == 0) *reinterpret_cast<float2*>(dst + dv) = make_float2(m, l_s[h * TP_ROWS + r]);
+        }
+        return;
+    }
     const int hv = dv >> 1;
     for (int u = tid; u < n_rows * H * hv; u += 512) {
         const int m = u % hv, h = (u / hv) % H, r = u / (hv * H);
@@ -1373,6 +1397,21 @@ static int talk_kernel_choice = 1;        // 1: the tensor-core kernels where th
 
 JANIS_EXPORT void janis_talk_attention_set_kernel(int which) { talk_kernel_choice = which; }
 
+// Over how many CTAs a prompt's rows should have their keys cut (1: not).  The last of a prompt's blocks of rows see the most keys,
+// and the other SMs wait for them; in shares of a third of an SM's even part of the tiles (four tiles at least) they come out
+// even.  A prompt whose longest block is small against that part does so by itself.  (8 heads of 256: 1,024 tokens 233 us a layer
+// uncut, 95 in four; the shares' sums pass through memory, 8 KB a row and share, which bounds their number to eight and 256 MB.)
+JANIS_EXPORT int janis_talk_prompt_chunks(int T, int H, int G, int d, int dv, int max_keys) {
+    if (T <= 0 || max_keys <= 0 || G <= 0 || !talk_prompt_takes(H, G, d, dv)) return 1;
+    const double tiles = (max_keys + TP_BN - 1) / TP_BN, blocks = (T + TP_ROWS - 1) / TP_ROWS, part = blocks * tiles / 2 / 148;
+    if (tiles <= 0.4 * part) return 1;
+    const double share = part / 3 > 4 ? part / 3 : 4;
+    int n = (int)((tiles + share - 1) / share);
+    const long long most = (64LL << 20) / ((long long)T * H * (dv + 2));
+    if (n > most) n = (int)most;
+    return n > 8 ? 8 : (n > 1 ? n : 1);
+}
+
 // The shape the tensor-core kernel runs a step with, or qr = 0 when it does not take the sizes.
 static TalkMmaShape talk_mma_shape(int H, int G, int d, int dv, int one_row, size_t* bytes) {
     TalkMmaShape sh = {};
@@ -1470,16 +1509,29 @@ JANIS_EXPORT int janis_talk_attention(const void* q_rows, int dtype, int q_row_e
     if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && talk != nullptr && !mix_after && !one_row && !v_in_keys &&
         keep_first == 0 && q_row_elems % 2 == 0 && talk_prompt_takes(H, G, d, dv) &&
         (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0 && ((uintptr_t)q_rows & 3) == 0) {
-        const TalkPromptShape ps = {G, d, dv, block, window, sink ? 1 : 0, scale, cap};
+        TalkPromptShape ps = {G, d, dv, block, window, sink ? 1 : 0, 0, scale, cap};
+        int chunks = 1;
+        if (n_chunks > 1 && max_keys > 0 && partial != nullptr && ((uintptr_t)partial & 7) == 0) {
+            if (partial_floats < (long long)T * n_chunks * H * (dv + 2))
+                return fail("talk_attention: scratch of %lld floats is too small for %d rows in %d chunks", partial_floats, T, n_chunks);
+            // (rows of a CTA may begin in different tiles of a block or window: their first row's tiles are what is cut)
+            const int tiles = (max_keys + TP_ROWS - 1 + TP_BN - 1) / TP_BN + 1;
+            chunks = n_chunks;
+            ps.chunk_tiles = (tiles + chunks - 1) / chunks;
+        }
         const size_t bytes = talk_prompt_bytes(H, G, d, dv);
         const bool pairs = (H / G) % 2 == 0;
         auto kernel = H == 8 ? (pairs ? talk_prompt_kernel<8, true> : talk_prompt_kernel<8, false>)
                              : (pairs ? talk_prompt_kernel<4, true> : talk_prompt_kernel<4, false>);
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return fail("talk_attention: shared memory of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-        return launch_kernel("talk_attention", kernel, dim3((T + TP_ROWS - 1) / TP_ROWS), dim3(512), bytes, stream, 1, (const bf16*)q_rows,
-                             q_row_elems, tok_pos, tok_seq, seq_slot, (const bf16*)kpool, (const bf16*)vpool, page_table, table_stride,
-                             talk, inv_v, (bf16*)out, sink_vals, T, ps);
+        if (launch_kernel("talk_attention", kernel, dim3((T + TP_ROWS - 1) / TP_ROWS, chunks), dim3(512), bytes, stream, 1, (const bf16*)q_rows,
+                          q_row_elems, tok_pos, tok_seq, seq_slot, (const bf16*)kpool, (const bf16*)vpool, page_table, table_stride,
+                          talk, inv_v, (bf16*)out, sink_vals, T, ps, partial))
+            return 1;
+        if (chunks == 1) return 0;
+        return launch_kernel("talk_attention_merge", talk_attention_merge_kernel, dim3(T), dim3(128), 0, stream, 1, (const float*)partial, chunks,
+                             tok_pos, tok_seq, seq_slot, inv_v, (bf16*)out, H, dv, sink ? 1 : 0, sink_vals);
     }
     if (dtype == JANIS_BF16 && talk_kernel_choice != 0 && q_row_elems % 8 == 0 &&
         (((uintptr_t)q_rows | (uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0) {

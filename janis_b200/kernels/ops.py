@@ -146,6 +146,8 @@ def mixers():
         lib.janis_talk_attention_rows_floats.argtypes = [I, I, I, I, I, I, I]
         lib.janis_talk_attention_rows_floats.restype = c_longlong
         lib.janis_talk_attention_rows.argtypes = [P, I, I, P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, I, I, I, F, P, I, P, c_longlong, I, P]
+        lib.janis_talk_prompt_chunks.argtypes = [I, I, I, I, I, I]
+        lib.janis_talk_prompt_chunks.restype = I
         lib.janis_gla_scan.argtypes = [P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P]
         lib.janis_head_norm_gate.argtypes = [P, P, I, I, I, P, F, P, I, I, I, I, I, P]
         lib.janis_mlstm_scan.argtypes = [P, I, I, I, I, I, P, P, F, P, I, P, P, P, P, P, P, P, P, I, I, I, I, F, P]
@@ -959,7 +961,8 @@ def talk_attention(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table,
     or 8 rows of the step; one_row=True, for decode steps, gives every row a CTA of its own); everything else
     runs the plain kernel, which is exact 32-bit for float32.  A decode step on the tensor cores may cut every row's
     keys over n_chunks CTAs (max_keys: a bound on the keys a row sees; scratch: float32, at least
-    `talk_attention_scratch_floats`) whose shares a second kernel puts together.
+    `talk_attention_scratch_floats`) whose shares a second kernel puts together; so may a prompt step of 4 or 8 mixed heads
+    (`talk_prompt_chunks`).
     cap > 0: every scaled score becomes cap tanh(score / cap) first.  sink_values [H] float32 (with sink): exp of
     head h's value joins its denominator instead of 1.  mix_after: talk mixes the heads' weights after the softmax
     instead of their scores before it, which takes two passes over the keys and `stats`, float32 of at least
@@ -995,8 +998,14 @@ def talk_attention(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table,
         _t(stats, "stats", torch.float32) if stats is not None else None, stats.numel() if stats is not None else 0,
         int(keep_first), _stream()),
         kernels=(2 if two_pass else 1) *
-                (2 if (one_row and n_chunks > 1 and scratch is not None and q_rows.dtype == torch.bfloat16) else 1))
+                (2 if (n_chunks > 1 and scratch is not None and q_rows.dtype == torch.bfloat16) else 1))
     return out
+
+
+def talk_prompt_chunks(T: int, H: int, G: int, d: int, dv: int, max_keys: int) -> int:
+    """Over how many CTAs a prompt step of mixed heads should have its rows' keys cut (`n_chunks` of `talk_attention`, with
+    scratch and max_keys; 1: not, or not by the kernel that can)."""
+    return int(mixers().janis_talk_prompt_chunks(int(T), int(H), int(G), int(d), int(dv), int(max_keys)))
 
 
 def talk_attention_rows_floats(dtype, T: int, H: int, G: int, d: int, dv: int, max_keys: int) -> int:
@@ -1054,18 +1063,26 @@ def talk_attention_set_kernel(which: int = 1) -> None:
     mixers().janis_talk_attention_set_kernel(int(which))
 
 
-def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_first_row, seq_start, seq_end, state,
-             o_out, n_seq: int, H: int, d: int, dv: int, q_scale: float, tau: float, decay=None):
-    """The recurrence of gated linear attention over the tokens each sequence brings to the step, in order:
-    a = sigmoid(z + z_bias)^(1/tau) per key channel, S = diag(a) S + k v^T, o = S^T (q q_scale).
-    rows [T, width] holds the projections (q [H, d] at q_off, k at k_off, v [H, dv] at v_off), z [T, H d] the
-    projected decay logits; state float32 [slots, H, dv, d] (a column's key channels side by side) is read and written back for sequences whose slot is
-    >= 0; o_out float32 [T, H dv]; decay float32 [T, H d] receives the decays (a kernel of its own forms them once
-    for all the CTAs of a head; allocated here when not given)."""
-    T, width = rows.shape
-    if decay is None:
-        decay = torch.empty((T, H * d), dtype=torch.float32, device=rows.device)
-    _t(decay, "decay", torch.float32, (T, H * d))
+GLA_CHUNK_FLOATS = 64 << 20    # the most scratch that a chunked prompt may take (256 MB)
+GLA_CHUNK_TOKENS, GLA_CHUNK_STEP = 16, 128
+
+
+def gla_chunks_floats(dtype, T: int, n_seq: int, H: int, d: int, dv: int) -> int:
+    """Floats of scratch with which `gla_scan` runs a step of T tokens in n_seq sequences in chunks, or 0 where it does not: other
+    sizes or types, fewer than GLA_CHUNK_TOKENS tokens a sequence (a chunk costs the same however few it holds) or GLA_CHUNK_STEP in
+    all (one of 64 tokens takes 24 us in chunks and 21 one by one, one of 300 47 and 60), or more scratch than GLA_CHUNK_FLOATS."""
+    if dtype != torch.bfloat16 or T < max(GLA_CHUNK_TOKENS * n_seq, GLA_CHUNK_STEP):
+        return 0
+    n = int(mixers().janis_gla_chunks_floats(int(T), int(n_seq), int(H), int(d), int(dv)))
+    return n if n <= GLA_CHUNK_FLOATS else 0
+
+
+def _gla_chunked(rows, v_off, T, n_seq, H, d, dv, chunks) -> bool:
+    need = gla_chunks_floats(rows.dtype, T, n_seq, H, d, dv)
+    return 0 < need <= chunks.numel() and rows.shape[1] % 8 == 0 and v_off % 8 == 0 and rows.data_ptr() % 16 == 0 and chunks.data_ptr() % 16 == 0
+
+
+def _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv) -> None:
     _t(rows, "rows", _FLOATS, (T, None))
     _t(z, "z", rows.dtype, (T, H * d))
     _t(z_bias, "z_bias", rows.dtype, (H * d,))
@@ -1075,6 +1092,32 @@ def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_
         _t(tab, name, torch.int32)
         if tab.numel() < n_seq:
             raise KernelError(f"gla_scan: {name} shorter than the step's sequences")
+
+
+def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_first_row, seq_start, seq_end, state,
+             o_out, n_seq: int, H: int, d: int, dv: int, q_scale: float, tau: float, decay=None, chunks=None):
+    """The recurrence of gated linear attention over the tokens each sequence brings to the step, in order:
+    a = sigmoid(z + z_bias)^(1/tau) per key channel, S = diag(a) S + k v^T, o = S^T (q q_scale).
+    rows [T, width] holds the projections (q [H, d] at q_off, k at k_off, v [H, dv] at v_off), z [T, H d] the
+    projected decay logits; state float32 [slots, H, dv, d] (a column's key channels side by side) is read and written back for sequences whose slot is
+    >= 0; o_out float32 [T, H dv]; decay float32 [T, H d] receives the decays (a kernel of its own forms them once
+    for all the CTAs of a head; allocated here when not given).  `chunks` (float32 of at least `gla_chunks_floats`): scratch
+    with which a prompt runs 16 tokens at a time on the tensor cores; the decays are then not left in `decay`."""
+    T, width = rows.shape
+    if chunks is not None:
+        _t(chunks, "chunks", torch.float32)
+        decay = None
+        if _gla_chunked(rows, v_off, T, n_seq, H, d, dv, chunks):
+            _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv)
+            lib = mixers()
+            _check(lib, lib.janis_gla_chunks(rows.data_ptr(), width, q_off, k_off, v_off, z.data_ptr(), z_bias.data_ptr(), T, seq_slot.data_ptr(),
+                                             seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(),
+                                             n_seq, H, d, dv, float(q_scale), float(tau), chunks.data_ptr(), chunks.numel(), _stream()), kernels=2)
+            return o_out
+    if decay is None:
+        decay = torch.empty((T, H * d), dtype=torch.float32, device=rows.device)
+    _t(decay, "decay", torch.float32, (T, H * d))
+    _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv)
     lib = mixers()
     _check(lib, lib.janis_gla_scan(rows.data_ptr(), _DT[rows.dtype], width, q_off, k_off, v_off, z.data_ptr(),
                                    z_bias.data_ptr(), decay.data_ptr(), T, seq_slot.data_ptr(), seq_first_row.data_ptr(),

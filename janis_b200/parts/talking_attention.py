@@ -276,6 +276,12 @@ class TalkingHeadsAttention(Mixer):
             n_chunks = max(1, min(rt.sm_count // max(T, 1), -(-max_keys // 128), 64))
             n = ops.talk_attention_scratch_floats(T, n_chunks, H, dv)
             scratch = ws.buf("tattn.partial", (n,), torch.float32) if n else None
+        elif self.talk is not None and rt.dtype == torch.bfloat16 and not self.keep_first and hasattr(ops, "talk_prompt_chunks"):
+            # a prompt of a few blocks of rows: the keys of a row over several CTAs, where that kernel takes the heads
+            max_keys = min([ctx.len_bound] + [n for n in (self.block, self.window) if n])
+            n_chunks = ops.talk_prompt_chunks(T, H, G, d, dv, max_keys)
+            n = ops.talk_attention_scratch_floats(T, n_chunks, H, dv)
+            scratch = ws.buf("tattn.partial", (n,), torch.float32) if n else None
         return ops.talk_attention(rows, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, kv.k, kv.v, kv.table, self.talk, inv_v, att,
                                   H, G, d, dv, self.scale, self.block, self.sink, one_row=decode, max_keys=max_keys,
                                   n_chunks=n_chunks, scratch=scratch, window=self.window, **more)

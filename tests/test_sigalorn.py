@@ -314,17 +314,19 @@ def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, 
     R.talk_attention(q, tok_pos, tok_seq, slots, kp, vp, table, M, inv_v, want, H, G, d, dv, d ** -0.5, block, sink, window=window, cap=cap,
                      sink_values=sinks)
     dev = lambda x: x.cuda() if x is not None else None
-    off = {}
-    for which in (1, 2):
+    for which, chunks in ((1, 1), (1, 3), (2, 1)):
         ops.talk_attention_set_kernel(which)
         try:
             got = torch.full((T, H * dv), float("nan"), dtype=torch.bfloat16, device="cuda")
+            n = ops.talk_attention_scratch_floats(T, chunks, H, dv)
             ops.talk_attention(dev(q), dev(tok_pos), dev(tok_seq), dev(slots), dev(kp), dev(vp), dev(table), dev(M), dev(inv_v), got,
-                               H, G, d, dv, d ** -0.5, block, sink, window=window, cap=cap, sink_values=dev(sinks))
+                               H, G, d, dv, d ** -0.5, block, sink, window=window, cap=cap, sink_values=dev(sinks), n_chunks=chunks,
+                               max_keys=min([n for n in (block, window, max(ends)) if n]),
+                               scratch=torch.full((n,), float("nan"), device="cuda") if n else None)
         finally:
             ops.talk_attention_set_kernel(1)
-        off[which] = (got.cpu().double() - want.double()).abs().max().item()
-        assert off[which] <= 2e-2 * max(1.0, want.double().abs().max().item()), (which, off)
+        err = (got.cpu().double() - want.double()).abs().max().item()
+        assert err <= 2e-2 * max(1.0, want.double().abs().max().item()), (which, chunks, err)
 
 
 @GPU
