@@ -1,0 +1,337 @@
+// Gated linear attention's recurrence in prompts, 16 tokens at a time on the tensor cores (bfloat16 inputs):
+//
+//   S_t = diag(a_t) S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t,   a_t = sigmoid(z_t + b)^(1/tau) per key channel
+//
+// With b_t[i] the sum of log a[i] from the chunk's start up to t, the tokens of a chunk are three products:
+//
+//   o_t   = S_0^T (q_t e^(b_t))  +  sum_(s <= t) A[t, s] v_s,      A[t, s] = sum_i q_t[i] k_s[i] e^(b_t[i] - b_s[i])
+//   S_end = diag(e^(b_end)) S_0 + sum_s (k_s e^(b_end - b_s)) v_s^T
+//
+// A first kernel forms, for all chunks at the same time, the weighted queries and keys, A and e^(b_end) - 1.  No exponent in
+// them is positive, so nothing overflows however strong a decay is; b is summed in double and kept as two floats, so that a difference is
+// as exact as one logarithm.  The second kernel is the chain over the chunks.  What the recurrence keeps as floats enters
+// its products as sums of three bfloat16 numbers (both operands where both are floats: the six products that reach a float's
+// last bits), the large and the small parts in accumulators of their own, and S takes a chunk's sum by one rounded addition.
+//
+// A CTA owns 32 value columns of a sequence's head, four warps to 16 of them: each keeps S for a quarter of the key channels in
+// registers (as the accumulators of the last product, which are at the same time second operands of the first), and the
+// four sums of a result meet in shared memory.  The chain bounds it: some 250 instructions a warp and two barriers a chunk.
+//
+// 8 heads of 128 x 256, against gla_scan_kernel (bound by shared memory: three 16-byte reads for 16 multiply-adds a lane) with its
+// kernel for the decays: one sequence of 2,048 tokens 374 -> 215 us, 300 tokens 60 -> 47, eight of 512 666 -> 233.  Errors
+// against 64 bits over 2,048 tokens: results 3.3e-7 -> 1.4e-7, states 3.2e-7 -> 0.7e-7; where the states remember a thousand tokens
+// 5.3e-6 -> 1.9e-7 and 7.3e-6 -> 2.1e-7.
+#include "mma_bf16.cuh"
+
+namespace janis {
+
+constexpr int GQ = 16;                       // tokens a chunk
+constexpr int GC_COLS = 32;                  // value columns a CTA
+constexpr int GC_STAGES = 3;
+
+struct GlaChunkShape {
+    int row_elems, q_off, k_off, v_off, H, d, dv, n_tok;
+    float q_scale, inv_tau;
+};
+
+// What the first kernel leaves: weighted queries and keys [2][3][n_tok][H d], A [n_tok][H][3][16] (bfloat16 parts), and
+// e^(b_end) - 1 [chunk][H d] floats; chunk c of sequence s in place first_row / 16 + s + c.
+struct GlaChunkScratch {
+    bf16 *qk, *a;
+    float* grow;
+};
+__host__ __device__ inline GlaChunkScratch gla_chunk_scratch(void* p, const GlaChunkShape& g) {
+    GlaChunkScratch s;
+    s.qk = reinterpret_cast<bf16*>(p);
+    s.a = s.qk + (size_t)6 * g.n_tok * g.H * g.d;
+    s.grow = reinterpret_cast<float*>(s.a + (size_t)g.n_tok * g.H * 48);
+    return s;
+}
+
+__device__ __forceinline__ void split3_one(float x, bf16& hi, bf16& mid, bf16& lo) {
+    hi = __float2bfloat16_rn(x);
+    x -= __bfloat162float(hi);
+    mid = __float2bfloat16_rn(x);
+    lo = __float2bfloat16_rn(x - __bfloat162float(mid));
+}
+
+// A CTA per (sequence, chunk, head): first a thread per key channel, then a thread per pair of tokens
+__global__ void __launch_bounds__(256)
+gla_chunk_terms_kernel(const bf16* __restrict__ rows, const bf16* __restrict__ z_rows, const bf16* __restrict__ bias, GlaChunkShape g,
+                       const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                       GlaChunkScratch out) {
+    extern __shared__ float gla_terms[];
+    const int d = g.d, ld = d + 1, seq = blockIdx.z, chunk = blockIdx.x, h = blockIdx.y;
+    float *q_s = gla_terms, *k_s = q_s + GQ * ld, *hi_s = k_s + GQ * ld, *lo_s = hi_s + GQ * ld;      // [16][ld]
+    grid_dependents_launch();
+    const int first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq], row0 = first + chunk * GQ;
+    const int n = min(GQ, n_all - chunk * GQ);
+    if (n <= 0) return;
+    grid_dependency_wait();
+    const size_t plane = (size_t)g.n_tok * g.H * d;
+    for (int i = threadIdx.x; i < d; i += 256) {
+        const float bi = __bfloat162float(bias[h * d + i]);
+        double b = 0.0;
+        for (int t = 0; t < n; ++t) {
+            const bf16* row = rows + (size_t)(row0 + t) * g.row_elems;
+            const float z = __bfloat162float(z_rows[(size_t)(row0 + t) * g.H * d + h * d + i]) + bi;
+            float la = (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) * g.inv_tau;
+            la = la < -1e5f ? -1e5f : la;                               // (e^-1e5 is 0 already)
+            b += (double)la;
+            const float hi = (float)b, q = __bfloat162float(row[g.q_off + h * d + i]) * g.q_scale;
+            q_s[t * ld + i] = q;
+            k_s[t * ld + i] = __bfloat162float(row[g.k_off + h * d + i]);
+            hi_s[t * ld + i] = hi;
+            lo_s[t * ld + i] = (float)(b - (double)hi);
+            const size_t at = (size_t)(row0 + t) * g.H * d + h * d + i;
+            split3_one(q * expf(hi), out.qk[at], out.qk[plane + at], out.qk[2 * plane + at]);
+        }
+        for (int t = 0; t < n; ++t) {
+            const size_t at = 3 * plane + (size_t)(row0 + t) * g.H * d + h * d + i;
+            const float left = (float)(b - ((double)hi_s[t * ld + i] + (double)lo_s[t * ld + i]));
+            split3_one(k_s[t * ld + i] * expf(left), out.qk[at], out.qk[plane + at], out.qk[2 * plane + at]);
+        }
+        out.grow[((size_t)(first / GQ + seq + chunk) * g.H + h) * d + i] = expm1f((float)b);
+    }
+    __syncthreads();
+    const int t = threadIdx.x >> 4, s = threadIdx.x & 15;
+    if (t >= n) return;
+    float acc[2] = {0.f, 0.f};
+    if (s <= t) {
+        for (int i = 0; i < d; i += 2)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float x = (hi_s[t * ld + i + e] - hi_s[s * ld + i + e]) + (lo_s[t * ld + i + e] - lo_s[s * ld + i + e]);
+                acc[e] = fmaf(q_s[t * ld + i + e] * k_s[s * ld + i + e], expf(x), acc[e]);
+            }
+    }
+    bf16* dst = out.a + ((size_t)(row0 + t) * g.H + h) * 48 + s;
+    split3_one(acc[0] + acc[1], dst[0], dst[16], dst[32]);
+}
+
+__host__ __device__ constexpr int gla_stage_bytes(int d) {
+    return (6 * GQ * (d + 8) + 3 * GQ * (GQ + 8) + GQ * (GC_COLS + 8)) * 2 + d * 4;
+}
+__host__ __device__ constexpr int gla_chain_bytes(int d) { return GC_STAGES * gla_stage_bytes(d) + 8 * GQ * 20 * 4; }
+
+template <int NK>                            // d = 64 NK key channels: 16 NK a warp
+__global__ void __launch_bounds__(256)
+gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch in, const int* __restrict__ seq_slot,
+                 const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                 float* __restrict__ state, float* __restrict__ o_out) {
+    constexpr int D = 64 * NK, LDK = D + 8, LDA = GQ + 8, LDV = GC_COLS + 8, STAGE = gla_stage_bytes(D);
+    constexpr int Q_AT = 0, K_AT = 3 * GQ * LDK * 2, A_AT = 2 * K_AT, V_AT = A_AT + 3 * GQ * LDA * 2, G_AT = V_AT + GQ * LDV * 2;
+    extern __shared__ __align__(16) unsigned char gla_raw[];
+    float* sum_s = reinterpret_cast<float*>(gla_raw + GC_STAGES * STAGE);            // [8 warps][16 tokens][20]
+    const int seq = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * GC_COLS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, pt = warp >> 2, quarter = warp & 3;
+    const int gr = lane >> 2, gc = (lane & 3) * 2, lr = lane & 7, lm = lane >> 3;
+    grid_dependents_launch();
+    const int slot = seq_slot[seq], row0 = seq_first_row[seq], n_tok = seq_end[seq] - seq_start[seq];
+    if (n_tok <= 0) return;
+    grid_dependency_wait();
+    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(gla_raw);
+    const size_t plane = (size_t)g.n_tok * g.H * D;
+    const int chunks = (n_tok + GQ - 1) / GQ;
+    const size_t place0 = (size_t)(row0 / GQ + seq);
+    auto fetch = [&](int c) {                                              // (a group for every chunk, an empty one past the last)
+        if (c < chunks) {
+            const uint32_t to = raw + (c % GC_STAGES) * STAGE;
+            const int n = min(GQ, n_tok - c * GQ);
+            const size_t r = (size_t)row0 + (size_t)c * GQ;
+            for (int p = tid; p < 6 * GQ * (D / 8); p += 256) {
+                const int x = p / (D / 8), i = p % (D / 8), t = x % GQ, part = x / GQ;
+                const bool ok = t < n;
+                copy16_or_zero(to + Q_AT + (x * LDK + i * 8) * 2, in.qk + part * plane + (r + (ok ? t : 0)) * g.H * D + h * D + i * 8, ok);
+            }
+            for (int p = tid; p < GQ * 6; p += 256) {
+                const int t = p / 6, i = p % 6;
+                const bool ok = t < n;
+                copy16_or_zero(to + A_AT + (((i >> 1) * GQ + t) * LDA + (i & 1) * 8) * 2, in.a + ((r + (ok ? t : 0)) * g.H + h) * 48 + i * 8, ok);
+            }
+            for (int p = tid; p < GQ * (GC_COLS / 8); p += 256) {
+                const int t = p / (GC_COLS / 8), i = p % (GC_COLS / 8);
+                const bool ok = t < n;
+                copy16_or_zero(to + V_AT + (t * LDV + i * 8) * 2, rows + (r + (ok ? t : 0)) * g.row_elems + g.v_off + h * g.dv + col0 + i * 8, ok);
+            }
+            for (int p = tid; p < D / 4; p += 256) copy16_or_zero(to + G_AT + p * 16, in.grow + ((place0 + c) * g.H + h) * D + p * 4, true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    // S[col][channel]: tile j holds channels n0 + 8 j + gc, + 1 of columns col0 + 16 pt + gr (0, 1) and + 8 (2, 3)
+    const int n0 = quarter * 16 * NK;
+    float S[2 * NK][4];
+    float* st = slot >= 0 ? state + (((size_t)slot * g.H + h) * g.dv + col0 + 16 * pt) * D + n0 : nullptr;
+#pragma unroll
+    for (int j = 0; j < 2 * NK; ++j) {
+        float2 a = make_float2(0.f, 0.f), b = a;
+        if (st != nullptr) {
+            a = *reinterpret_cast<const float2*>(st + (size_t)gr * D + 8 * j + gc);
+            b = *reinterpret_cast<const float2*>(st + (size_t)(gr + 8) * D + 8 * j + gc);
+        }
+        S[j][0] = a.x; S[j][1] = a.y; S[j][2] = b.x; S[j][3] = b.y;
+    }
+    for (int c = 0; c < GC_STAGES - 1; ++c) fetch(c);
+    for (int c = 0; c < chunks; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GC_STAGES - 2) : "memory");
+        __syncthreads();                                                   // chunk c is there; chunk c - 1 and the sums have been read
+        fetch(c + GC_STAGES - 1);
+        const uint32_t at = raw + (c % GC_STAGES) * STAGE;
+        const float* grow = reinterpret_cast<const float*>(gla_raw + (c % GC_STAGES) * STAGE + G_AT);
+        // o: this quarter's channels of the state; the first quarter adds the chunk's own tokens
+        float hi[2][4], rest[2][4];
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) hi[p][e] = rest[p][e] = 0.f;
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            uint32_t a[3][4], b[3][2][2];                                  // b: [part][columns 0..7, 8..15][channels 0..7, 8..15]
+#pragma unroll
+            for (int z = 0; z < 3; ++z)
+                ldmatrix4(a[z], at + Q_AT + ((z * GQ + lr + (lm & 1) * 8) * LDK + n0 + 16 * k + (lm >> 1) * 8) * 2);
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int e = 0; e < 2; ++e)
+                    split3(S[2 * k + e][2 * p], S[2 * k + e][2 * p + 1], b[0][p][e], b[1][p][e], b[2][p][e]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(rest[p], a[2], b[0][p][0], b[0][p][1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(hi[p], a[0], b[0][p][0], b[0][p][1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(rest[p], a[1], b[1][p][0], b[1][p][1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(rest[p], a[0], b[2][p][0], b[2][p][1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(rest[p], a[1], b[0][p][0], b[0][p][1]);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) mma_16816(rest[p], a[0], b[1][p][0], b[1][p][1]);
+        }
+        if (quarter == 0) {
+            uint32_t b[4];
+            ldmatrix4_trans(b, at + V_AT + ((lr + (lm & 1) * 8) * LDV + 16 * pt + (lm >> 1) * 8) * 2);
+            float own[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) own[p][e] = 0.f;
+#pragma unroll
+            for (int z = 2; z >= 0; --z) {
+                uint32_t a[4];
+                ldmatrix4(a, at + A_AT + ((z * GQ + lr + (lm & 1) * 8) * LDA + (lm >> 1) * 8) * 2);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) mma_16816(z ? rest[p] : own[p], a, b[2 * p], b[2 * p + 1]);
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) hi[p][e] += own[p][e];
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                *reinterpret_cast<float2*>(sum_s + (warp * GQ + gr + 8 * e) * 20 + 8 * p + gc) =
+                    make_float2(hi[p][2 * e] + rest[p][2 * e], hi[p][2 * e + 1] + rest[p][2 * e + 1]);
+        // the state at the chunk's end
+        {
+            uint32_t v[4];
+            ldmatrix4_trans(v, at + V_AT + ((lr + (lm >> 1) * 8) * LDV + 16 * pt + (lm & 1) * 8) * 2);
+#pragma unroll
+            for (int j = 0; j < NK; ++j) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int z = 0; z < 3; ++z)
+                    ldmatrix4_trans(b[z], at + K_AT + ((z * GQ + lr + (lm & 1) * 8) * LDK + n0 + 16 * j + (lm >> 1) * 8) * 2);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_16816(y, v, b[2][2 * e], b[2][2 * e + 1]);
+                    mma_16816(x, v, b[0][2 * e], b[0][2 * e + 1]);
+                    mma_16816(y, v, b[1][2 * e], b[1][2 * e + 1]);
+                    const float2 gw = *reinterpret_cast<const float2*>(grow + n0 + 16 * j + 8 * e + gc);
+                    float(&s)[4] = S[2 * j + e];
+                    s[0] += fmaf(s[0], gw.x, x[0] + y[0]);
+                    s[1] += fmaf(s[1], gw.y, x[1] + y[1]);
+                    s[2] += fmaf(s[2], gw.x, x[2] + y[2]);
+                    s[3] += fmaf(s[3], gw.y, x[3] + y[3]);
+                }
+            }
+        }
+        __syncthreads();                                                   // the quarters' sums are there
+        {
+            const int t = tid >> 4, col = (tid & 15) * 2, p = col >> 4;
+            if (c * GQ + t < n_tok) {
+                const float* src = sum_s + (p * 4 * GQ + t) * 20 + (col & 15);
+                float2 y = *reinterpret_cast<const float2*>(src);
+#pragma unroll
+                for (int q = 1; q < 4; ++q) {
+                    const float2 w = *reinterpret_cast<const float2*>(src + q * GQ * 20);
+                    y.x += w.x;
+                    y.y += w.y;
+                }
+                *reinterpret_cast<float2*>(o_out + ((size_t)(row0 + c * GQ + t) * g.H + h) * g.dv + col0 + col) = y;
+            }
+        }
+    }
+    if (st != nullptr) {
+#pragma unroll
+        for (int j = 0; j < 2 * NK; ++j) {
+            *reinterpret_cast<float2*>(st + (size_t)gr * D + 8 * j + gc) = make_float2(S[j][0], S[j][1]);
+            *reinterpret_cast<float2*>(st + (size_t)(gr + 8) * D + 8 * j + gc) = make_float2(S[j][2], S[j][3]);
+        }
+    }
+}
+
+template <int NK>
+static int gla_chain_launch(const bf16* rows, const GlaChunkShape& g, const GlaChunkScratch& in, const int* seq_slot, const int* seq_first_row,
+                            const int* seq_start, const int* seq_end, int n_seq, float* state, float* o_out, cudaStream_t stream) {
+    constexpr int bytes = gla_chain_bytes(64 * NK);
+    const cudaError_t e = cudaFuncSetAttribute(gla_chain_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return fail("gla_chunks: shared memory of %d bytes refused: %s", bytes, cudaGetErrorString(e));
+    // (launched once its predecessor is over: its few CTAs run long and have to lie on SMs of their own)
+    return launch_kernel_after("gla_chain", gla_chain_kernel<NK>, dim3(n_seq, g.H, g.dv / GC_COLS), dim3(256), bytes, stream, 1, rows, g, in,
+                               seq_slot, seq_first_row, seq_start, seq_end, state, o_out);
+}
+
+}  // namespace janis
+
+using namespace janis;
+
+// Floats of scratch for a step of n_tok tokens in n_seq sequences; 0 where the chunked form does not take the sizes.
+JANIS_EXPORT long long janis_gla_chunks_floats(int n_tok, int n_seq, int H, int d, int dv) {
+    if (n_tok <= 0 || n_seq <= 0 || H <= 0 || !(d == 64 || d == 128 || d == 256) || dv <= 0 || dv % GC_COLS) return 0;
+    return 3LL * n_tok * H * d + 24LL * n_tok * H + ((long long)n_tok / GQ + n_seq) * H * d;
+}
+
+JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, int k_off, int v_off, const void* z, const void* bias, int n_tok,
+                                  const int* seq_slot, const int* seq_first_row, const int* seq_start, const int* seq_end, float* state,
+                                  float* o_out, int n_seq, int H, int d, int dv, float q_scale, float tau, void* scratch,
+                                  long long scratch_floats, cudaStream_t stream) {
+    if (n_seq <= 0 || n_tok <= 0) return 0;
+    const long long need = janis_gla_chunks_floats(n_tok, n_seq, H, d, dv);
+    if (need == 0 || scratch == nullptr || scratch_floats < need)
+        return fail("gla_chunks: %d heads of %d x %d (or a scratch of %lld floats) are not taken", H, d, dv, scratch_floats);
+    if (!(tau > 0.f)) return fail("gla_chunks: tau must be positive");
+    if (row_elems % 8 || v_off % 8 || (((uintptr_t)rows | (uintptr_t)scratch) & 15) || (((uintptr_t)state | (uintptr_t)o_out) & 7))
+        return fail("gla_chunks: rows of %d elements, values at %d: not in whole pieces of 16 bytes", row_elems, v_off);
+    if (n_seq > 65535 || H > 65535) return fail("gla_chunks: too many sequences or heads (%d, %d)", n_seq, H);
+    GlaChunkShape g;
+    g.row_elems = row_elems; g.q_off = q_off; g.k_off = k_off; g.v_off = v_off; g.H = H; g.d = d; g.dv = dv; g.n_tok = n_tok;
+    g.q_scale = q_scale; g.inv_tau = 1.0f / tau;
+    const GlaChunkScratch s = gla_chunk_scratch(scratch, g);
+    const size_t bytes = (size_t)4 * GQ * (d + 1) * sizeof(float);
+    const cudaError_t e = cudaFuncSetAttribute(gla_chunk_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return fail("gla_chunks: shared memory of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
+    if (launch_kernel("gla_chunk_terms", gla_chunk_terms_kernel, dim3((n_tok + GQ - 1) / GQ, H, n_seq), dim3(256), bytes, stream, 1, (const bf16*)rows,
+                      (const bf16*)z, (const bf16*)bias, g, seq_first_row, seq_start, seq_end, s))
+        return 1;
+#define JANIS_GLA_CHAIN(NK)                                                                                                       \
+    return gla_chain_launch<NK>((const bf16*)rows, g, s, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, o_out, stream);
+    if (d == 64) { JANIS_GLA_CHAIN(1) }
+    if (d == 128) { JANIS_GLA_CHAIN(2) }
+    JANIS_GLA_CHAIN(4)
+#undef JANIS_GLA_CHAIN
+}

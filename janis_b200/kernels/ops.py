@@ -148,6 +148,9 @@ def mixers():
         lib.janis_talk_attention_rows.argtypes = [P, I, I, P, P, P, P, P, P, I, P, P, I, I, I, I, I, F, I, I, I, F, P, I, P, c_longlong, I, P]
         lib.janis_talk_prompt_chunks.argtypes = [I, I, I, I, I, I]
         lib.janis_talk_prompt_chunks.restype = I
+        lib.janis_gla_chunks_floats.argtypes = [I, I, I, I, I]
+        lib.janis_gla_chunks_floats.restype = c_longlong
+        lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P, c_longlong, P]
         lib.janis_gla_scan.argtypes = [P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P]
         lib.janis_head_norm_gate.argtypes = [P, P, I, I, I, P, F, P, I, I, I, I, I, P]
         lib.janis_mlstm_scan.argtypes = [P, I, I, I, I, I, P, P, F, P, I, P, P, P, P, P, P, P, P, I, I, I, I, F, P]

@@ -363,6 +363,42 @@ def test_rotation_and_cache_write_against_their_statement(dtype, H, G, d, dv, ro
 
 
 @GPU
+@pytest.mark.parametrize("H,d,dv,tau", [(2, 64, 32, 8.0), (2, 128, 64, 16.0), (1, 256, 96, 0.05)])
+def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau):
+    """16 tokens at a time: sequences on a chunk's border and beside it (one without a slot), the second step going on from the
+    states of the first; tau = 0.05 makes decays of e^-100 and less beside ones near 1; scratch of NaN, not a float more than asked for."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    g = torch.Generator().manual_seed(6)
+    lens = [1, 16, 17, 111, 5]
+    T, n_seq = sum(lens), len(lens)
+    b2 = (1.0 + torch.randn(H * d, generator=g)).bfloat16()
+    state = torch.zeros(6, H, dv, d)
+    got_state = state.clone().cuda()
+    slots, first = torch.tensor([2, 5, 0, 3, -1], dtype=torch.int32), torch.tensor([0, 1, 17, 34, 145], dtype=torch.int32)
+    start = torch.zeros(n_seq, dtype=torch.int32)
+    offs = (8, 8 + H * d, 8 + 2 * H * d)
+    floats = ops.gla_chunks_floats(torch.bfloat16, T, n_seq, H, d, dv)
+    assert floats
+    for _ in range(2):
+        rows = torch.randn(T, 8 + 2 * H * d + H * dv, generator=g).bfloat16()
+        z = (2.0 * torch.randn(T, H * d, generator=g)).bfloat16()
+        end = start + torch.tensor(lens, dtype=torch.int32)
+        want, want_state = torch.zeros(T, H * dv), state.clone()
+        R.gla_scan(rows, *offs, z, b2, slots, first, start, end, want_state, want, n_seq, H, d, dv, d ** -0.5, tau)
+        scratch = torch.full((floats + 16,), float("nan"), device="cuda")
+        got = torch.full((T, H * dv), float("nan"), device="cuda")
+        ops.gla_scan(rows.cuda(), *offs, z.cuda(), b2.cuda(), slots.cuda(), first.cuda(), start.cuda(), end.cuda(), got_state, got, n_seq,
+                     H, d, dv, d ** -0.5, tau, chunks=scratch[:floats])
+        assert scratch[floats:].isnan().all() and not scratch[:4].isnan().any()
+        for name, x, y in (("results", got, want), ("states", got_state, want_state)):
+            err = (x.cpu().double() - y.double()).abs().max().item()
+            assert err <= 5e-5 * max(1.0, y.double().abs().max().item()), (name, err)
+        assert torch.equal(got_state[[1, 4]].cpu(), state[[1, 4]]), "a slot that is not in the step keeps its state"
+        state, start = want_state, end
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,d,dv,tau", [(2, 16, 24, 8.0), (1, 40, 48, 32.0), (3, 8, 8, 1.0), (2, 128, 72, 16.0), (1, 200, 32, 4.0)])
 def test_recurrence_kernel_against_its_statement(dtype, H, d, dv, tau):
