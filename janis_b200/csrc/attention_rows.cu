@@ -33,6 +33,7 @@ struct RowsShape {
     int n_chunks;       // CTAs a row
     int sink;           // 0 none; 1 a key of score 0 without a value; 2 learnt values
     int lanes;          // lanes of the scores' kernel that share a key's row
+    int shared_floats;  // rows_mixed_kernel: floats of the queries or of the partial sums, whichever are more
     float scale, cap;
 };
 
@@ -331,6 +332,236 @@ rows_sum_kernel(const float* __restrict__ o_part, const int* __restrict__ tok_po
     for (int e = 0; e < 4; ++e) out[(size_t)t * n + i + e] = from_float<T>(s[e]);
 }
 
+// Heads mixed before the softmax: a chunk needs no other chunk's numbers, so one kernel takes it all the way: scores, the heads'
+// scores mixed, the chunk's own maximum, sum and unnormalised o; a second kernel brings the chunks to one maximum, adds
+// them, divides, and turns the result back by the row's position where the values were turned by theirs.  Keys and values are
+// read once, 16 bytes a lane, which bounds it.
+template <typename T, int VB>
+__global__ void __launch_bounds__(ROWS_THREADS, VB <= 2 ? 3 : 2)
+rows_mixed_kernel(const T* __restrict__ q_rows, int q_row_elems, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
+                  const int* __restrict__ seq_slot, const T* __restrict__ kpool, const T* __restrict__ vpool,
+                  const int* __restrict__ page_table, int table_stride, const float* __restrict__ talk, RowsShape sh,
+                  float* __restrict__ part, float* __restrict__ o_part) {
+    constexpr int V = Vec16<T>::N;
+    extern __shared__ float rows_smem[];
+    const int H = sh.H, G = sh.G, d = sh.d, dv = sh.dv, rep = H / G, chunk = sh.chunk, qs = d + 8;
+    float* s_s = rows_smem;                         // the chunk's scores, head by head
+    float* p_s = s_s + (size_t)H * chunk;           // mixed, then the weights
+    float* q_s = p_s + (size_t)H * chunk;           // the row's queries; later VB x V x ROWS_THREADS partial sums
+    float* red = q_s;
+    int* base_s = reinterpret_cast<int*>(q_s + sh.shared_floats);      // where a key's row starts, in rows
+    const int t = blockIdx.y, c = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    grid_dependents_launch();
+    const int pos = tok_pos[t], slot = seq_slot[tok_seq[t]];
+    int j0, j1;
+    const RowsKeys keys = rows_range(sh, pos, c, j0, j1);
+    grid_dependency_wait();
+    if (slot < 0 || j0 > j1) return;                // (the merge leaves such chunks out)
+    for (int i = tid * V; i < H * d; i += ROWS_THREADS * V) {
+        float x[V];
+        rows_unpack<T>(*reinterpret_cast<const uint4*>(q_rows + (size_t)t * q_row_elems + i), x);
+#pragma unroll
+        for (int e = 0; e < V; e += 4) Vec16<float>::store(q_s + (size_t)(i / d) * qs + i % d + e, x + e);
+    }
+    const int n_keys = j1 - j0 + 1, n_pairs = n_keys * G;
+    const int* table = page_table + (size_t)slot * table_stride;
+    for (int jj = tid; jj < n_keys; jj += ROWS_THREADS) {
+        const int j = rows_key(keys, j0 + jj);
+        base_s[jj] = table[j / JANIS_PAGE] * G * JANIS_PAGE + j % JANIS_PAGE;
+    }
+    __syncthreads();
+    // (the scores as in rows_scores_kernel)
+    const int P = sh.lanes, sub = tid % P, n_slots = ROWS_THREADS / P, n_pieces = d / V;
+    for (int pair0 = 0; pair0 < n_pairs; pair0 += n_slots) {
+        const int mine = pair0 + tid / P, pair = mine < n_pairs ? mine : n_pairs - 1;
+        const int jj = pair / G, g = pair % G;
+        const T* krow = kpool + ((size_t)base_s[jj] + (size_t)g * JANIS_PAGE) * d;
+        for (int hb = 0; hb < rep; hb += VB) {
+            float acc[VB];
+#pragma unroll
+            for (int r = 0; r < VB; ++r) acc[r] = 0.f;
+            for (int i0 = sub; i0 < n_pieces; i0 += ROWS_FLIGHT * P) {
+                uint4 raw[ROWS_FLIGHT];
+#pragma unroll
+                for (int u = 0; u < ROWS_FLIGHT; ++u)
+                    if (i0 + u * P < n_pieces) raw[u] = *reinterpret_cast<const uint4*>(krow + (size_t)(i0 + u * P) * V);
+#pragma unroll
+                for (int u = 0; u < ROWS_FLIGHT; ++u) {
+                    if (i0 + u * P < n_pieces) {
+                        float x[V];
+                        rows_unpack<T>(raw[u], x);
+#pragma unroll
+                        for (int r = 0; r < VB; ++r) {
+                            if (hb + r < rep) {
+                                const float* qh = q_s + (size_t)(g * rep + hb + r) * qs + (size_t)(i0 + u * P) * V;
+#pragma unroll
+                                for (int e = 0; e < V; e += 4) {
+                                    const float4 q4 = *reinterpret_cast<const float4*>(qh + e);
+                                    acc[r] = fmaf(q4.x, x[e], acc[r]);
+                                    acc[r] = fmaf(q4.y, x[e + 1], acc[r]);
+                                    acc[r] = fmaf(q4.z, x[e + 2], acc[r]);
+                                    acc[r] = fmaf(q4.w, x[e + 3], acc[r]);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < VB; ++r) {
+                if (hb + r < rep) {
+                    float v = acc[r];
+                    for (int o = P >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    v *= sh.scale;
+                    if (sh.cap > 0.f) v = sh.cap * tanhf(v / sh.cap);
+                    if (sub == 0 && mine < n_pairs) s_s[(size_t)(g * rep + hb + r) * chunk + jj] = v;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // mixed; a warp per head brings them to the chunk's maximum
+    for (int h = warp; h < H; h += ROWS_WARPS) {
+        float m = -CUDART_INF_F, l = 0.f;
+        for (int jj = lane; jj < n_keys; jj += 32) {
+            float x = 0.f;
+            for (int g = 0; g < H; ++g) x = fmaf(talk[h * H + g], s_s[(size_t)g * chunk + jj], x);
+            p_s[(size_t)h * chunk + jj] = x;
+            m = fmaxf(m, x);
+        }
+        m = warp_max(m);
+        for (int jj = lane; jj < n_keys; jj += 32) {
+            const float w = m == -CUDART_INF_F ? 0.f : expf(p_s[(size_t)h * chunk + jj] - m);
+            p_s[(size_t)h * chunk + jj] = w;
+            l += w;
+        }
+        l = warp_sum(l);
+        float* prt = part + (((size_t)t * sh.n_chunks + c) * H + h) * 2;
+        if (lane == 0) prt[0] = m, prt[1] = l;
+    }
+    __syncthreads();
+    // (the sums as in rows_values_kernel)
+    const int per_head = dv / V, n_units = G * per_head;
+    const int share = n_units >= ROWS_THREADS ? 1 : ROWS_THREADS / n_units;
+    float* out = o_part + ((size_t)t * sh.n_chunks + c) * H * dv;
+    for (int u0 = 0; u0 < n_units; u0 += ROWS_THREADS / share) {
+        const int u = u0 + tid % (ROWS_THREADS / share), s1 = tid / (ROWS_THREADS / share);
+        const bool live = u < n_units && s1 < share;
+        const int g = live ? u / per_head : 0, c0 = live ? (u % per_head) * V : 0;
+        for (int hb = 0; hb < rep; hb += VB) {
+            float acc[VB][V];
+#pragma unroll
+            for (int r = 0; r < VB; ++r)
+#pragma unroll
+                for (int e = 0; e < V; ++e) acc[r][e] = 0.f;
+            if (live) {
+                for (int jj = s1; jj < n_keys; jj += ROWS_FLIGHT * share) {
+                    uint4 raw[ROWS_FLIGHT];
+#pragma unroll
+                    for (int k = 0; k < ROWS_FLIGHT; ++k)
+                        if (jj + k * share < n_keys)
+                            raw[k] = *reinterpret_cast<const uint4*>(vpool + ((size_t)base_s[jj + k * share] + (size_t)g * JANIS_PAGE) * sh.v_stride + c0);
+#pragma unroll
+                    for (int k = 0; k < ROWS_FLIGHT; ++k) {
+                        if (jj + k * share < n_keys) {
+                            float x[V];
+                            rows_unpack<T>(raw[k], x);
+#pragma unroll
+                            for (int r = 0; r < VB; ++r) {
+                                if (hb + r < rep) {
+                                    const float p = p_s[(size_t)(g * rep + hb + r) * chunk + jj + k * share];
+#pragma unroll
+                                    for (int e = 0; e < V; ++e) acc[r][e] = fmaf(p, x[e], acc[r][e]);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+            if (share == 1) {
+                if (live)
+                    for (int r = 0; r < VB && hb + r < rep; ++r)
+#pragma unroll
+                        for (int e = 0; e < V; e += 4) Vec16<float>::store(out + (size_t)(g * rep + hb + r) * dv + c0 + e, acc[r] + e);
+                continue;
+            }
+            __syncthreads();                        // (red may still be read from the pass before)
+#pragma unroll
+            for (int r = 0; r < VB; ++r)
+#pragma unroll
+                for (int e = 0; e < V; ++e) red[(size_t)(r * V + e) * ROWS_THREADS + tid] = acc[r][e];
+            __syncthreads();
+            if (live && s1 == 0) {
+                for (int r = 0; r < VB; ++r) {
+                    if (hb + r >= rep) break;
+                    float sum[V];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) sum[e] = 0.f;
+                    for (int s2 = 0; s2 < share; ++s2) {
+                        const int other = s2 * (ROWS_THREADS / share) + tid;
+#pragma unroll
+                        for (int e = 0; e < V; ++e) sum[e] += red[(size_t)(r * V + e) * ROWS_THREADS + other];
+                    }
+#pragma unroll
+                    for (int e = 0; e < V; e += 4) Vec16<float>::store(out + (size_t)(g * rep + hb + r) * dv + c0 + e, sum + e);
+                }
+            }
+        }
+    }
+}
+
+constexpr int ROWS_MERGE_CHUNKS = 128;
+
+// A CTA per (head, row), a thread per pair of features half a head apart
+template <typename T>
+__global__ void __launch_bounds__(128)
+rows_mixed_merge_kernel(const float* __restrict__ part, const float* __restrict__ o_part, const int* __restrict__ tok_pos,
+                        const int* __restrict__ tok_seq, const int* __restrict__ seq_slot, const float* __restrict__ inv_v,
+                        const float* __restrict__ sink_values, RowsShape sh, T* __restrict__ out) {
+    __shared__ float w_s[ROWS_MERGE_CHUNKS];
+    const int h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, H = sh.H, dv = sh.dv, hv = dv >> 1;
+    grid_dependents_launch();
+    const int pos = tok_pos[t], slot = seq_slot[tok_seq[t]];
+    const int first = first_seen(pos, sh.window), kept = sh.window > 0 ? min(sh.keep_first, first) : 0;
+    const int n_valid = slot < 0 ? 0 : min(sh.n_chunks, (kept + pos - first) / sh.chunk + 1);
+    grid_dependency_wait();
+    // every warp forms the row's maximum and denominator for itself; the first one leaves the chunks' weights
+    const float* prt = part + ((size_t)t * sh.n_chunks * H + h) * 2;
+    const float z = sh.sink == 2 ? sink_values[h] : 0.f;
+    float M = sh.sink ? z : -CUDART_INF_F;
+    for (int c = lane; c < n_valid; c += 32) M = fmaxf(M, prt[(size_t)c * H * 2]);
+    M = warp_max(M);
+    float L = 0.f;
+    for (int c = lane; c < n_valid; c += 32) {
+        const float m = prt[(size_t)c * H * 2], w = m == -CUDART_INF_F ? 0.f : expf(m - M);
+        L = fmaf(w, prt[(size_t)c * H * 2 + 1], L);
+        if (tid < 32) w_s[c] = w;
+    }
+    L = warp_sum(L);
+    if (sh.sink) L += expf(z - M);
+    __syncthreads();
+    const float inv_l = n_valid > 0 ? 1.f / L : 0.f;
+    const float* src = o_part + ((size_t)t * sh.n_chunks * H + h) * dv;
+    T* o_row = out + ((size_t)t * H + h) * dv;
+    for (int i = tid; i < hv; i += 128) {
+        float a = 0.f, b = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < n_valid; ++c) {
+            const float w = w_s[c];
+            a = fmaf(w, src[(size_t)c * H * dv + i], a);
+            b = fmaf(w, src[(size_t)c * H * dv + i + hv], b);
+        }
+        float lo = a * inv_l, hi = b * inv_l;
+        if (inv_v != nullptr) {
+            float s, c;
+            sincosf((float)pos * inv_v[i], &s, &c);
+            rotate_pair(a * inv_l, b * inv_l, -s, c, lo, hi);
+        }
+        o_row[i] = from_float<T>(lo);
+        o_row[i + hv] = from_float<T>(hi);
+    }
+}
+
 struct RowsPlan {
     RowsShape sh;
     size_t scores, part, fin, o_part, total;        // offsets into the scratch, in floats
@@ -436,4 +667,50 @@ JANIS_EXPORT int janis_talk_attention_rows(const void* q_rows, int dtype, int q_
     if (dtype == JANIS_BF16) JANIS_ROWS(bf16)
 #undef JANIS_ROWS
     return fail("talk_attention_rows: unknown dtype %d", dtype);
+}
+
+// The same for heads mixed by `talk` before the softmax, with values that were turned by their own positions where inv_v is given.
+// Scratch as for janis_talk_attention_rows.
+JANIS_EXPORT int janis_talk_attention_rows_mixed(const void* q_rows, int dtype, int q_row_elems, const int* tok_pos, const int* tok_seq,
+                                                 const int* seq_slot, const void* kpool, const void* vpool, const int* page_table,
+                                                 int table_stride, const float* talk, const float* inv_v, void* out, int T, int H, int G,
+                                                 int d, int dv, float scale, int sink, int max_keys, int window, float cap,
+                                                 const float* sink_values, float* scratch, long long scratch_floats, int keep_first,
+                                                 cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (keep_first < 0 || (keep_first > 0 && window <= 0)) return fail("talk_attention_rows_mixed: %d kept first positions need a window", keep_first);
+    const long long want = janis_talk_attention_rows_floats(dtype, T, H, G, d, dv, max_keys);
+    const int vec = dtype == JANIS_F32 ? 4 : 8;
+    if (want <= 0 || dv % 2 || talk == nullptr || T > 65535 || q_row_elems % vec) return fail("talk_attention_rows_mixed: sizes not taken (%d heads over %d, %d and %d features)", H, G, d, dv);
+    if (scratch == nullptr || scratch_floats < want) return fail("talk_attention_rows_mixed: scratch of %lld floats, %lld wanted", scratch_floats, want);
+    if ((reinterpret_cast<uintptr_t>(q_rows) | reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool) | reinterpret_cast<uintptr_t>(scratch)) & 15)
+        return fail("talk_attention_rows_mixed: rows, pools and scratch start on 16-byte borders");
+    RowsPlan p = rows_plan(T, H, G, d, dv, max_keys, vec);
+    RowsShape& sh = p.sh;
+    if (sh.n_chunks > ROWS_MERGE_CHUNKS) return fail("talk_attention_rows_mixed: %d chunks", sh.n_chunks);
+    sh.H = H; sh.G = G; sh.d = d; sh.dv = dv; sh.v_stride = dv; sh.window = window; sh.keep_first = keep_first;
+    sh.sink = sink ? (sink_values != nullptr ? 2 : 1) : 0;
+    sh.scale = scale;
+    sh.cap = cap;
+    const int vb = H / G <= 2 ? 2 : ROWS_VB, sums = ROWS_THREADS * vb * vec;
+    sh.shared_floats = H * (d + 8) > sums ? H * (d + 8) : sums;
+    const size_t bytes = ((size_t)2 * H * sh.chunk + sh.shared_floats + sh.chunk) * sizeof(float);
+    if (bytes > 200 * 1024) return fail("talk_attention_rows_mixed: %zu bytes of shared memory", bytes);
+#define JANIS_ROWS_MIXED(TT)                                                                                                          \
+    {                                                                                                                                 \
+        auto kernel = H / G <= 2 ? rows_mixed_kernel<TT, 2> : rows_mixed_kernel<TT, ROWS_VB>;                                        \
+        if (bytes > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) \
+            return fail("talk_attention_rows_mixed: shared memory of %zu bytes refused", bytes);                                     \
+        if (launch_kernel("talk_attention_rows_mixed", kernel, dim3(sh.n_chunks, T), dim3(ROWS_THREADS), bytes, stream, 1, (const TT*)q_rows, \
+                          q_row_elems, tok_pos, tok_seq, seq_slot, (const TT*)kpool, (const TT*)vpool, page_table, table_stride, talk, \
+                          sh, scratch + p.part, scratch + p.o_part))                                                                 \
+            return 1;                                                                                                                 \
+        return launch_kernel("talk_attention_rows_mixed (merge)", rows_mixed_merge_kernel<TT>, dim3(H, T), dim3(128), 0, stream, 1,    \
+                             (const float*)(scratch + p.part), (const float*)(scratch + p.o_part), tok_pos, tok_seq, seq_slot, inv_v, \
+                             sink_values, sh, (TT*)out);                                                                              \
+    }
+    if (dtype == JANIS_F32) JANIS_ROWS_MIXED(float)
+    if (dtype == JANIS_BF16) JANIS_ROWS_MIXED(bf16)
+#undef JANIS_ROWS_MIXED
+    return fail("talk_attention_rows_mixed: unknown dtype %d", dtype);
 }

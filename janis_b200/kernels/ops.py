@@ -151,6 +151,7 @@ def mixers():
         lib.janis_gla_chunks_floats.argtypes = [I, I, I, I, I]
         lib.janis_gla_chunks_floats.restype = c_longlong
         lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P, c_longlong, P]
+        lib.janis_talk_attention_rows_mixed.argtypes = [P, I, I, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, F, I, I, I, F, P, P, c_longlong, I, P]
         lib.janis_gla_scan.argtypes = [P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P]
         lib.janis_head_norm_gate.argtypes = [P, P, I, I, I, P, F, P, I, I, I, I, I, P]
         lib.janis_mlstm_scan.argtypes = [P, I, I, I, I, I, P, P, F, P, I, P, P, P, P, P, P, P, P, I, I, I, I, F, P]
@@ -1048,6 +1049,34 @@ def talk_attention_rows(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_t
         float(scale), 1 if sink else 0, int(max_keys), int(window), float(cap),
         _t(sink_values, "sink_values", torch.float32, (H,)) if sink_values is not None else None,
         1 if values_in_keys else 0, _t(scratch, "scratch", torch.float32), scratch.numel(), int(keep_first), _stream()), kernels=4)
+    return out
+
+
+def talk_attention_rows_mixed(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table, talk, inv_v, out, H: int, G: int, d: int,
+                              dv: int, scale: float, scratch, max_keys: int, sink: bool = False, window: int = 0, cap: float = 0.0,
+                              sink_values=None, keep_first: int = 0):
+    """`talk_attention_rows` for heads whose scores talk [H, H] float32 mixes before the softmax, in two launches; with inv_v
+    [dv / 2] each head's output is turned back by the row's position.  Sizes and scratch as `talk_attention_rows_floats` says, with
+    an even dv and rows of whole 16-byte pieces."""
+    T = q_rows.shape[0]
+    _t(q_rows, "q_rows", _FLOATS, (T, None))
+    n_pages = kpool.shape[0]
+    _t(kpool, "kpool", q_rows.dtype, (n_pages, G, PAGE, d))
+    _t(vpool, "vpool", q_rows.dtype, (n_pages, G, PAGE, dv))
+    if sink_values is not None and not sink:
+        raise KernelError("talk_attention_rows_mixed: sink values without a sink")
+    _t(page_table, "page_table", torch.int32, (None, None))
+    _t(out, "out", q_rows.dtype, (T, H * dv))
+    if tok_pos.numel() < T or tok_seq.numel() < T:
+        raise KernelError("talk_attention_rows_mixed: position tables shorter than the step")
+    lib = mixers()
+    _check(lib, lib.janis_talk_attention_rows_mixed(
+        q_rows.data_ptr(), _DT[q_rows.dtype], q_rows.shape[1], _t(tok_pos, "tok_pos", torch.int32), _t(tok_seq, "tok_seq", torch.int32),
+        _t(seq_slot, "seq_slot", torch.int32), kpool.data_ptr(), vpool.data_ptr(), page_table.data_ptr(), page_table.shape[1],
+        _t(talk, "talk", torch.float32, (H, H)), _t(inv_v, "inv_v", torch.float32, (dv // 2,)) if inv_v is not None else None,
+        out.data_ptr(), T, H, G, d, dv, float(scale), 1 if sink else 0, int(max_keys), int(window), float(cap),
+        _t(sink_values, "sink_values", torch.float32, (H,)) if sink_values is not None else None,
+        _t(scratch, "scratch", torch.float32), scratch.numel(), int(keep_first), _stream()), kernels=2)
     return out
 
 

@@ -267,6 +267,15 @@ class TalkingHeadsAttention(Mixer):
             return ops.talk_attention_rows(rows, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, kv.k, kv.v, kv.table, None, att, H, G, d, dv,
                                            self.scale, ws.buf("tattn.rows_scratch", (rows_floats,), torch.float32), max_keys,
                                            sink=self.sink, window=self.window or -self.block, **more)
+        if (decode and rt.dtype == torch.bfloat16 and self.talk is not None and not (self.block and self.window) and not self.values_from_keys
+                and dv % 2 == 0 and rows.shape[1] % 8 == 0 and hasattr(ops, "talk_attention_rows_mixed")):
+            # heads mixed before the softmax: keys and values read once, 16 bytes a lane, and a merge
+            max_keys = min(ctx.len_bound, (self.window or self.block) + self.keep_first) if self.window or self.block else ctx.len_bound
+            rows_floats = ops.talk_attention_rows_floats(rt.dtype, T, H, G, d, dv, max_keys)
+            if rows_floats:
+                return ops.talk_attention_rows_mixed(rows, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, kv.k, kv.v, kv.table, self.talk, inv_v, att,
+                                                     H, G, d, dv, self.scale, ws.buf("tattn.rows_scratch", (rows_floats,), torch.float32),
+                                                     max_keys, sink=self.sink, window=self.window or -self.block, **more)
         if decode:
             # a decode row's keys over several CTAs when the rows alone would leave most of the GPU idle: about a
             # CTA an SM in all, none with fewer than 128 keys (the bound on the lengths is the host's)

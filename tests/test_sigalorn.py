@@ -286,6 +286,40 @@ def test_attention_kernel_against_its_statement(dtype, H, G, d, dv, block, sink,
 
 
 @GPU
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,d,dv", [(8, 4, 256, 256), (3, 1, 24, 40), (16, 8, 64, 48), (6, 6, 8, 8)])
+@pytest.mark.parametrize("window,keep_first,sink,cap,turn", [(0, 0, True, 0.0, True), (-100, 0, True, 5.0, False), (90, 4, False, 0.0, True)])
+def test_single_rows_of_mixed_heads(dtype, H, G, d, dv, window, keep_first, sink, cap, turn):
+    """Decode rows whose heads are mixed before the softmax: one key, a page's border, a chunk of keys and one more, far into the
+    sequence; a row without a slot; learnt sinks; scratch of NaN."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    pos = [0, 63, 64, 299, 120, 5]
+    kp, vp, table, slots = _paged(len(pos), [p + 1 for p in pos], G, d, dv, dtype, 3)
+    slots[5] = -1
+    T = len(pos)
+    g = torch.Generator().manual_seed(H * d)
+    q = torch.randn(T, H * d + 8, generator=g).to(dtype)
+    M = (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).float()
+    inv_v = torch.tensor([10000.0 ** (-2.0 * m / dv) for m in range(dv // 2)], dtype=torch.float32) if turn else None
+    sinks = torch.randn(H, generator=g) if sink and cap else None
+    tok_pos, tok_seq = torch.tensor(pos, dtype=torch.int32), torch.arange(T, dtype=torch.int32)
+    want = torch.zeros(T, H * dv, dtype=dtype)
+    R.talk_attention(q, tok_pos, tok_seq, slots, kp, vp, table, M, inv_v, want, H, G, d, dv, d ** -0.5, 0, sink, window=window, cap=cap,
+                     sink_values=sinks, keep_first=keep_first)
+    dev = lambda x: x.cuda() if x is not None else None
+    max_keys = abs(window) + keep_first if window else 300
+    n = ops.talk_attention_rows_floats(dtype, T, H, G, d, dv, max_keys)
+    assert n > 0
+    got = torch.full((T, H * dv), float("nan"), dtype=dtype, device="cuda")
+    ops.talk_attention_rows_mixed(dev(q), dev(tok_pos), dev(tok_seq), dev(slots), dev(kp), dev(vp), dev(table), dev(M), dev(inv_v), got, H, G,
+                                  d, dv, d ** -0.5, torch.full((n,), float("nan"), device="cuda"), max_keys, sink=sink, window=window,
+                                  cap=cap, sink_values=dev(sinks), keep_first=keep_first)
+    err = (got.cpu().double() - want.double()).abs().max().item()
+    assert err <= (2e-5 if dtype == torch.float32 else 2e-2) * max(1.0, want.double().abs().max().item()), err
+
+
+@GPU
 @pytest.mark.parametrize("H,G,d,dv", [(8, 4, 256, 256), (8, 2, 64, 128), (8, 8, 128, 64), (4, 2, 128, 256), (4, 4, 256, 128)])
 @pytest.mark.parametrize("block,window,sink,cap,turn", [(0, 0, True, 0.0, True), (40, 0, True, 5.0, False), (0, 33, False, 0.0, True)])
 def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, turn):
