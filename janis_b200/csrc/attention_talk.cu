@@ -996,6 +996,24 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
         corr_s[u] = 1.f;
     }
     grid_dependency_wait();
+    __syncthreads();
+    if (split && blockIdx.y > 0) {                                         // a share that no run reaches
+        bool any = false;
+        for (int a = 0; a < n_rows;) {
+            int b = a + 1;
+            while (b < n_rows && seq_s[b] == seq_s[a]) ++b;
+            int first = sh.block > 0 ? pos_s[a] / sh.block * sh.block : 0;
+            if (sh.window > 0) first = max(first, pos_s[a] - sh.window + 1);
+            any = any || (slot_s[a] >= 0 && first / TP_BN * TP_BN + (int)blockIdx.y * sh.chunk_tiles * TP_BN <= pos_s[b - 1]);
+            a = b;
+        }
+        if (!any) {
+            float* base = partial + ((size_t)r0 * gridDim.y + blockIdx.y) * H * (dv + 2) + dv;
+            for (int hr = tid; hr < n_rows * H; hr += 512)
+                *reinterpret_cast<float2*>(base + ((size_t)(hr / H) * gridDim.y * H + hr % H) * (dv + 2)) = make_float2(-CUDART_INF_F, 0.f);
+            return;
+        }
+    }
     // the pair's queries over this warp's features, as first operands
     uint32_t qa[2][KS][4];
 #pragma unroll
@@ -1113,38 +1131,39 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
                     if (sh.cap > 0.f) z = sh.cap * tanhf(z / sh.cap);
                     raw[g] = z;
                 }
+                float m_new[H];
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
-                    float s = 0.f;
+                    float x = 0.f;
 #pragma unroll
                     for (int g = 0; g < H; g += 4) {
                         const float4 t = *reinterpret_cast<const float4*>(talk_s + h * H + g);
-                        s = fmaf(t.x, raw[g], s);
-                        s = fmaf(t.y, raw[g + 1], s);
-                        s = fmaf(t.z, raw[g + 2], s);
-                        s = fmaf(t.w, raw[g + 3], s);
+                        x = fmaf(t.x, raw[g], x);
+                        x = fmaf(t.y, raw[g + 1], x);
+                        x = fmaf(t.z, raw[g + 2], x);
+                        x = fmaf(t.w, raw[g + 3], x);
                     }
-                    s = seen ? s : -CUDART_INF_F;
-                    const float m_old = m_s[h * TP_ROWS + r], m_new = fmaxf(m_old, warp_max_redux(s));
-                    p[h] = 0.f;
-                    float corr = 1.f;
-                    if (m_new != -CUDART_INF_F) {
-                        p[h] = expf(s - m_new);
-                        if (m_new != m_old) corr = m_old == -CUDART_INF_F ? 0.f : expf(m_old - m_new);
-                    }
+                    p[h] = seen ? x : -CUDART_INF_F;
+                    m_new[h] = fmaxf(m_s[h * TP_ROWS + r], warp_max_redux(p[h]));
+                }
+                // 32 / H lanes stand for a head: they bring its sums to the new maximum
+                constexpr int LANES = 32 / H;
+                const int mine_h = lane / LANES;
+                const float m_old = m_s[mine_h * TP_ROWS + r];
+                float m_mine = m_new[0];
+#pragma unroll
+                for (int h = 1; h < H; ++h) m_mine = mine_h == h ? m_new[h] : m_mine;
+                const float corr = m_mine == m_old ? 1.f : (m_old == -CUDART_INF_F ? 0.f : expf(m_old - m_mine));
+#pragma unroll
+                for (int h = 0; h < H; ++h) {
+                    p[h] = m_new[h] != -CUDART_INF_F ? expf(p[h] - m_new[h]) : 0.f;
                     p_s[(h * TP_ROWS + r) * (TP_BN + 8) + lane] = __float2bfloat16_rn(p[h]);
-                    __syncwarp();                                          // every lane has read the old maximum
-                    if (lane == 0) {
-                        m_s[h * TP_ROWS + r] = m_new;
-                        corr_s[h * TP_ROWS + r] = corr;
-                    }
                 }
                 // the heads' sums over the lanes, each stage halving the heads a lane still carries
-                int h = 0, off = 16;
+                int off = 16;
 #pragma unroll
                 for (int n = H / 2; n >= 1; n >>= 1, off >>= 1) {
                     const bool upper = (lane & off) != 0;
-                    h += upper ? n : 0;
 #pragma unroll
                     for (int i = 0; i < n; ++i) {
                         const float mine = upper ? p[i + n] : p[i], theirs = upper ? p[i] : p[i + n];
@@ -1152,8 +1171,11 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
                     }
                 }
                 for (; off >= 1; off >>= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], off);
-                __syncwarp();
-                if ((lane & (32 / H - 1)) == 0) l_s[h * TP_ROWS + r] = l_s[h * TP_ROWS + r] * corr_s[h * TP_ROWS + r] + p[0];
+                if (lane % LANES == 0) {                                   // (the shuffles: every lane has read the old maxima)
+                    m_s[mine_h * TP_ROWS + r] = m_mine;
+                    corr_s[mine_h * TP_ROWS + r] = corr;
+                    l_s[mine_h * TP_ROWS + r] = l_s[mine_h * TP_ROWS + r] * corr + p[0];
+                }
             }
             if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -1398,18 +1420,31 @@ static int talk_kernel_choice = 1;        // 1: the tensor-core kernels where th
 JANIS_EXPORT void janis_talk_attention_set_kernel(int which) { talk_kernel_choice = which; }
 
 // Over how many CTAs a prompt's rows should have their keys cut (1: not).  The last of a prompt's blocks of rows see the most keys,
-// and the other SMs wait for them; in shares of a third of an SM's even part of the tiles (four tiles at least) they come out
-// even.  A prompt whose longest block is small against that part does so by itself.  (8 heads of 256: 1,024 tokens 233 us a layer
-// uncut, 95 in four; the shares' sums pass through memory, 8 KB a row and share, which bounds their number to eight and 256 MB.)
+// and the other SMs wait for them; but a CTA costs about a tile and a half besides its tiles, and the shares' sums pass through
+// memory, 8 KB a row and share at 8 heads of 256.  The number with the least of: an SM's part of the tiles and of the CTAs, half a share
+// (what the last CTA stands out on average), and the sums' traffic in tiles.
 JANIS_EXPORT int janis_talk_prompt_chunks(int T, int H, int G, int d, int dv, int max_keys) {
     if (T <= 0 || max_keys <= 0 || G <= 0 || !talk_prompt_takes(H, G, d, dv)) return 1;
-    const double tiles = (max_keys + TP_BN - 1) / TP_BN, blocks = (T + TP_ROWS - 1) / TP_ROWS, part = blocks * tiles / 2 / 148;
-    if (tiles <= 0.4 * part) return 1;
-    const double share = part / 3 > 4 ? part / 3 : 4;
-    int n = (int)((tiles + share - 1) / share);
-    const long long most = (64LL << 20) / ((long long)T * H * (dv + 2));
-    if (n > most) n = (int)most;
-    return n > 8 ? 8 : (n > 1 ? n : 1);
+    const int tiles = (max_keys + TP_BN - 1) / TP_BN, blocks = (T + TP_ROWS - 1) / TP_ROWS;
+    const int per_seq = (max_keys + TP_ROWS - 1) / TP_ROWS < blocks ? (max_keys + TP_ROWS - 1) / TP_ROWS : blocks;
+    int best = 1;
+    double least = 0.0;
+    for (int n = 1; n <= 6 && tiles >= 3 * n; ++n) {
+        if ((long long)T * n * H * (dv + 2) > (64LL << 20) && n > 1) break;
+        const double share = (double)((tiles + n - 1) / n), seqs = (double)blocks / per_seq;
+        double items = 0.0;
+        for (int c = 0; c < n; ++c) {
+            const double reach = per_seq - c * share * TP_BN / TP_ROWS;      // blocks of rows whose keys reach the share
+            if (reach > 0) items += seqs * (per_seq == blocks && T < max_keys ? blocks : reach);
+        }
+        const double traffic = n > 1 ? (double)T * n * H * dv * 8.0 / 5e12 / 5e-6 : 0.0;
+        const double cost = (blocks * (double)tiles / 2 + 1.5 * items) / 148 + share / 2 + traffic;
+        if (n == 1 || cost < least) {
+            least = cost;
+            best = n;
+        }
+    }
+    return best;
 }
 
 // The shape the tensor-core kernel runs a step with, or qr = 0 when it does not take the sizes.
