@@ -11,6 +11,8 @@
 //            p_h = sum_g M[h, g] w_g, and o_h = sum_j p_h[j] v_kv(h)[j] over the chunk's keys, as floats;
 //   sum      per row: the chunks' o added in ascending order and rounded.
 //
+// (Heads mixed before the softmax: rows_mixed_kernel below, two launches.)
+//
 // Keys are read once and values once, 16 bytes a lane; the scores cross global memory as floats (a few megabytes).  A
 // chunk's borders depend on the row's own first seen key and the chunk length, and every sum's order on the sizes, so a
 // row's result does not depend on the rows beside it.  Scores, weights and sums are float whatever is stored.

@@ -21,7 +21,7 @@
 // Every kernel here reads keys and values from the cache line only, so a step stores first and attends
 // afterwards, and a prompt that continues, a decode step and a layer that reads another layer's line are the
 // same launch.  Sizes are run-time numbers.  Scores, weights and sums are float whatever is stored.
-#include "common.cuh"
+#include "mma_bf16.cuh"
 
 #include <math_constants.h>
 
@@ -1039,16 +1039,19 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
 
     // rows of a tile from one page; what lies outside first .. last becomes zeros (0 x NaN is NaN)
     auto load = [&](uint32_t dst, const bf16* pool, int width, int ld, const int* table, int j0, int first, int last) {
-        const size_t base = (size_t)table[j0 / JANIS_PAGE] * G * JANIS_PAGE + j0 % JANIS_PAGE;
-        for (int row = warp; row < G * TP_BN; row += 16) {
-            const int g = row / TP_BN, jj = row % TP_BN, j = j0 + jj;
-            const bool ok = j >= first && j <= last;
-            const bf16* src = pool + (base + (size_t)g * JANIS_PAGE + (ok ? jj : 0)) * width;
-            for (int c8 = lane; c8 < width / 8; c8 += 32)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (row * ld + c8 * 8) * 2), "l"(src + c8 * 8), "r"(ok ? 16 : 0) : "memory");
+        if (lane * 8 < width) {
+            const bf16* src = pool + ((size_t)table[j0 / JANIS_PAGE] * G * JANIS_PAGE + j0 % JANIS_PAGE) * width + lane * 8;
+            const uint32_t to = dst + (warp * ld + lane * 8) * 2;
+#pragma unroll 4
+            for (int i = 0; i < 2 * G; ++i) {                              // rows warp, warp + 16, ...: two of a head
+                const int jj = warp + 16 * (i & 1), j = j0 + jj;
+                const bool ok = j >= first && j <= last;
+                copy16_or_zero(to + i * 32 * ld, src + (ok ? ((i >> 1) * JANIS_PAGE + jj) * width : 0), ok);
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    const int kv0 = 2 * pair / rep * TP_BN, kv1 = (2 * pair + 1) / rep * TP_BN;                   // the pair's first rows in a tile
 
     for (int a = 0; a < n_rows;) {
         int b = a + 1;
@@ -1090,7 +1093,7 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
 #pragma unroll
                     for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
                         uint32_t bq[4];
-                        ldsm_x4(bq, k_a + (((2 * pair + e) / rep * TP_BN + 16 * n + lr + (lm >> 1) * 8) * ldk + (part * ks + k) * 16 + (lm & 1) * 8) * 2);
+                        ldsm_x4(bq, k_a + (((e ? kv1 : kv0) + 16 * n + lr + (lm >> 1) * 8) * ldk + (part * ks + k) * 16 + (lm & 1) * 8) * 2);
 #pragma unroll
                         for (int f = 0; f < 2; ++f) {
                             if (!SHARED_KV && f != e) continue;
@@ -1205,7 +1208,7 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
 #pragma unroll
                         for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
                             uint32_t bv[4];
-                            ldsm_x4_trans(bv, v_a + (((2 * pair + e) / rep * TP_BN + 16 * k + lr + (lm & 1) * 8) * ldv + (part * nt2 + n) * 16 + (lm >> 1) * 8) * 2);
+                            ldsm_x4_trans(bv, v_a + (((e ? kv1 : kv0) + 16 * k + lr + (lm & 1) * 8) * ldv + (part * nt2 + n) * 16 + (lm >> 1) * 8) * 2);
 #pragma unroll
                             for (int f = 0; f < 2; ++f) {
                                 if (!SHARED_KV && f != e) continue;

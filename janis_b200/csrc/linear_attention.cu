@@ -8,7 +8,8 @@
 // followed, in a second kernel, by an RMS norm of each head's o over dv, a gate silu(g) and the rounding to the
 // activation type.  Decays, their logarithms, the state and o are float whatever the projections are stored in.
 // The state lives in the cache (one [H, d, dv] block per slot and line): a step loads it, runs its tokens in
-// order and writes it back, so a prompt, a prompt that continues and a decode step are the same launch.
+// order and writes it back, so a prompt, a prompt that continues and a decode step are the same launch.  (Longer prompts in
+// bfloat16 at key sizes of 64, 128 and 256 run in chunks: gla_chunks.cu.)
 #include "common.cuh"
 
 #include <math_constants.h>

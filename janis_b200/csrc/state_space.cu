@@ -12,7 +12,8 @@
 //
 // delta, the decays, the state and o are float whatever the projections are stored in.  The state lives in the
 // cache, [slots, C, N] floats per line: a step loads it, runs its tokens in order and writes it back; sequences
-// without a slot (padding) start from zero and store nothing.
+// without a slot (padding) start from zero and store nothing.  (The duality form of a bfloat16 prompt runs in chunks where its
+// sizes allow it: duality_scan.cu.)
 #include <type_traits>
 
 #include "common.cuh"
