@@ -1541,8 +1541,8 @@ JANIS_EXPORT int janis_talk_attention(const void* q_rows, int dtype, int q_row_e
     if (two_pass && (stats == nullptr || stats_floats < (long long)T * 2 * H))
         return fail("talk_attention: heads mixed after the softmax need %lld floats for the rows' maxima and denominators", (long long)T * 2 * H);
     if (v_in_keys) vpool = kpool;
-    // Prompts of 4 or 8 heads mixed before the softmax: 8 heads of 256 over 4, one prompt of 2,048 tokens 441 us a layer against
-    // 743 in the kernel below, 300 tokens 86 against 131, eight of 512 210 against 470, 16 tokens 32 = 32.  The kernel below takes the
+    // Prompts of 4 or 8 heads mixed before the softmax: 8 heads of 256 over 4, one prompt of 2,048 tokens 248 us a layer against
+    // 743 in the kernel below, 1,024 tokens 87 against 382, 300 tokens 55 against 130, eight of 512 186 against 471, 16 tokens 32 = 32.  The kernel below takes the
     // other sizes, decode steps and what this one leaves out.
     if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && talk != nullptr && !mix_after && !one_row && !v_in_keys &&
         keep_first == 0 && q_row_elems % 2 == 0 && talk_prompt_takes(H, G, d, dv) &&

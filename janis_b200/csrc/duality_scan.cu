@@ -23,8 +23,8 @@
 // tile instead of one hide each other's waits (328 us -> 218).
 //
 // 72 heads of 64 channels, 128 states, with the scan of selective_scan_staged_kernel (an issue slot in two, 263 instructions
-// a token and warp) and its kernel for the step sizes: one sequence of 2,048 tokens 954 -> 220 us, 300 tokens 149 -> 39, eight
-// of 512 1,400 -> 240, eight of 8 49 -> 31, one of 4 27 -> 23.  Errors against 64 bits over 2,048 tokens: results 1.1e-7 for
+// a token and warp) and its kernel for the step sizes: one sequence of 2,048 tokens 954 -> 209 us, 300 tokens 148 -> 39, eight
+// of 512 1,400 -> 229, eight of 8 49 -> 29, one of 4 27 -> 23.  Errors against 64 bits over 2,048 tokens: results 1.1e-7 for
 // 1.0e-7, states 0.8e-7 for 0.7e-7; where the states remember a thousand tokens 1.5e-7 for 5.5e-7 and 1.2e-7 for 6.6e-7.
 #include "mma_bf16.cuh"
 
@@ -75,19 +75,25 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
     const uint32_t m_a = (uint32_t)__cvta_generic_to_shared(m_s);
     const bf16* bsrc = bc_rows + (size_t)row0 * g.bc_stride + g.b_off + (size_t)group * N;
     const int c_from_b = g.c_off - g.b_off;
-    const bf16* usrc = u_rows + (size_t)row0 * g.u_stride + g.u_off + c0;
+    // this thread's pieces: one column of the rows of B and C side by side, one of the inputs'
+    const int bq = tid % (4 * NK), bt = tid / (4 * NK), b_step = blockDim.x / (4 * NK), which = bq >= 2 * NK, bi = (bq - which * 2 * NK) * 8;
+    const int ut = tid / (2 * npt), ui = tid % (2 * npt) * 8;              // (64 npt threads: 32 rows at a time)
+    bsrc += (which ? c_from_b : 0) + bi;
+    const bf16* usrc = u_rows + (size_t)row0 * g.u_stride + g.u_off + c0 + ui;
     auto fetch = [&](int t0, int buf) {
-        const uint32_t to = stage_a + buf * STAGE * 2;
-        for (int p = tid; p < DQ * 4 * NK; p += blockDim.x) {              // rows of B, then C: 2 NK pieces each
-            const int t = p / (4 * NK), q = p - t * 4 * NK, which = q >= 2 * NK, i = q - which * 2 * NK;
-            const bool ok = t0 + t < n_tok;
-            copy16_or_zero(to + ((which * DQ + t) * LDN + i * 8) * 2,
-                           bsrc + (ok ? (size_t)(t0 + t) * g.bc_stride + (which ? c_from_b : 0) + i * 8 : 0), ok);
+        const uint32_t to = stage_a + buf * STAGE * 2, b_to = to + (which * DQ * LDN + bi) * 2;
+        const int n = n_tok - t0;
+        const bf16* b0 = bsrc + (size_t)t0 * g.bc_stride;
+#pragma unroll 4
+        for (int t = bt; t < DQ; t += b_step) {
+            const bool ok = t < n;
+            copy16_or_zero(b_to + t * LDN * 2, b0 + (ok ? (size_t)t * g.bc_stride : 0), ok);
         }
-        for (int p = tid; p < DQ * 2 * npt; p += blockDim.x) {
-            const int t = p / (2 * npt), i = p - t * 2 * npt;
-            const bool ok = t0 + t < n_tok;
-            copy16_or_zero(to + (2 * DQ * LDN + t * DUP + i * 8) * 2, usrc + (ok ? (size_t)(t0 + t) * g.u_stride + i * 8 : 0), ok);
+        const bf16* u0 = usrc + (size_t)t0 * g.u_stride;
+#pragma unroll
+        for (int t = ut; t < DQ; t += 32) {
+            const bool ok = t < n;
+            copy16_or_zero(to + (2 * DQ * LDN + t * DUP + ui) * 2, u0 + (ok ? (size_t)t * g.u_stride : 0), ok);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };

@@ -18,7 +18,7 @@
 // four sums of a result meet in shared memory.  The chain bounds it: some 250 instructions a warp and two barriers a chunk.
 //
 // 8 heads of 128 x 256, against gla_scan_kernel (bound by shared memory: three 16-byte reads for 16 multiply-adds a lane) with its
-// kernel for the decays: one sequence of 2,048 tokens 374 -> 215 us, 300 tokens 60 -> 47, eight of 512 666 -> 233.  Errors
+// kernel for the decays: one sequence of 2,048 tokens 374 -> 195 us, 300 tokens 60 -> 43, eight of 512 666 -> 228.  Errors
 // against 64 bits over 2,048 tokens: results 3.3e-7 -> 1.4e-7, states 3.2e-7 -> 0.7e-7; where the states remember a thousand tokens
 // 5.3e-6 -> 1.9e-7 and 7.3e-6 -> 2.1e-7.
 #include "mma_bf16.cuh"
@@ -134,27 +134,30 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
     const size_t plane = (size_t)g.n_tok * g.H * D;
     const int chunks = (n_tok + GQ - 1) / GQ;
     const size_t place0 = (size_t)(row0 / GQ + seq);
+    // this thread's pieces: column qi of rows qx, qx + STEP, ... of the weighted queries and keys; one piece of A, of the values
+    // and of the decays (fewer threads bring those)
+    constexpr int STEP = 256 / (D / 8);
+    const int qi = tid % (D / 8) * 8, qx = tid / (D / 8), at_ = tid / 6, ai = tid % 6, vt = tid / (GC_COLS / 8), vi = tid % (GC_COLS / 8) * 8;
+    const size_t hd = (size_t)g.H * D;
+    const bf16* qk0 = in.qk + (size_t)row0 * hd + h * D + qi;
+    const bf16* a0 = in.a + ((size_t)(row0 + at_) * g.H + h) * 48 + ai * 8;
+    const bf16* v0 = rows + (size_t)(row0 + vt) * g.row_elems + g.v_off + h * g.dv + col0 + vi;
+    const float* g0 = in.grow + (place0 * g.H + h) * D + tid * 4;
     auto fetch = [&](int c) {                                              // (a group for every chunk, an empty one past the last)
         if (c < chunks) {
             const uint32_t to = raw + (c % GC_STAGES) * STAGE;
-            const int n = min(GQ, n_tok - c * GQ);
-            const size_t r = (size_t)row0 + (size_t)c * GQ;
-            for (int p = tid; p < 6 * GQ * (D / 8); p += 256) {
-                const int x = p / (D / 8), i = p % (D / 8), t = x % GQ, part = x / GQ;
+            const int n = n_tok - c * GQ;                                  // tokens from the chunk's first on
+            const bf16* q = qk0 + (size_t)c * GQ * hd;
+            const uint32_t q_to = to + Q_AT + (qx * LDK + qi) * 2;
+#pragma unroll
+            for (int it = 0; it < 6 * GQ / STEP; ++it) {
+                const int x = qx + it * STEP, t = x % GQ;
                 const bool ok = t < n;
-                copy16_or_zero(to + Q_AT + (x * LDK + i * 8) * 2, in.qk + part * plane + (r + (ok ? t : 0)) * g.H * D + h * D + i * 8, ok);
+                copy16_or_zero(q_to + it * STEP * LDK * 2, q + (x / GQ) * plane + (ok ? t : 0) * hd, ok);
             }
-            for (int p = tid; p < GQ * 6; p += 256) {
-                const int t = p / 6, i = p % 6;
-                const bool ok = t < n;
-                copy16_or_zero(to + A_AT + (((i >> 1) * GQ + t) * LDA + (i & 1) * 8) * 2, in.a + ((r + (ok ? t : 0)) * g.H + h) * 48 + i * 8, ok);
-            }
-            for (int p = tid; p < GQ * (GC_COLS / 8); p += 256) {
-                const int t = p / (GC_COLS / 8), i = p % (GC_COLS / 8);
-                const bool ok = t < n;
-                copy16_or_zero(to + V_AT + (t * LDV + i * 8) * 2, rows + (r + (ok ? t : 0)) * g.row_elems + g.v_off + h * g.dv + col0 + i * 8, ok);
-            }
-            for (int p = tid; p < D / 4; p += 256) copy16_or_zero(to + G_AT + p * 16, in.grow + ((place0 + c) * g.H + h) * D + p * 4, true);
+            if (tid < GQ * 6) copy16_or_zero(to + A_AT + (((ai >> 1) * GQ + at_) * LDA + (ai & 1) * 8) * 2, at_ < n ? a0 + (size_t)c * GQ * g.H * 48 : in.a, at_ < n);
+            if (tid < GQ * (GC_COLS / 8)) copy16_or_zero(to + V_AT + (vt * LDV + vi) * 2, vt < n ? v0 + (size_t)c * GQ * g.row_elems : rows, vt < n);
+            if (tid < D / 4) copy16_or_zero(to + G_AT + tid * 16, g0 + (size_t)c * hd, true);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };

@@ -1102,7 +1102,7 @@ GLA_CHUNK_TOKENS, GLA_CHUNK_STEP = 16, 128
 def gla_chunks_floats(dtype, T: int, n_seq: int, H: int, d: int, dv: int) -> int:
     """Floats of scratch with which `gla_scan` runs a step of T tokens in n_seq sequences in chunks, or 0 where it does not: other
     sizes or types, fewer than GLA_CHUNK_TOKENS tokens a sequence (a chunk costs the same however few it holds) or GLA_CHUNK_STEP in
-    all (one of 64 tokens takes 24 us in chunks and 21 one by one, one of 300 47 and 60), or more scratch than GLA_CHUNK_FLOATS."""
+    all (one of 64 tokens takes 26 us in chunks and 22 one by one, one of 300 43 and 60), or more scratch than GLA_CHUNK_FLOATS."""
     if dtype != torch.bfloat16 or T < max(GLA_CHUNK_TOKENS * n_seq, GLA_CHUNK_STEP):
         return 0
     n = int(mixers().janis_gla_chunks_floats(int(T), int(n_seq), int(H), int(d), int(dv)))

@@ -96,8 +96,8 @@ class SelectiveScanMixer(Mixer):
         xp = rt.linear(u, self.w_x, ws.buf("ssm.x", (T, R + 2 * N), rt.dtype))          # lo | B | C
         dt = rt.linear(xp, self.w_dt, ws.buf("ssm.dt", (T, C), rt.dtype))
         y = ws.buf("ssm.y", (T, C), rt.dtype)
-        # room for the step sizes and, in prompts, for two dozen pieces of a sequence beside one for each sequence
-        rows = T if ctx.mode == "decode" else T + (24 + ctx.n_seq) * (N + 1) // 2 + 1
+        # room for the step sizes and, in prompts whose states run in pieces, for two dozen pieces beside one for each sequence
+        rows = T + (24 + ctx.n_seq) * (N + 1) // 2 + 1 if ctx.mode == "prefill" and N in (8, 16) else T
         ops.selective_scan(u, 0, dt, 0, self.b_dt, self.A, True, xp, R, R + N, self.D, uz, C, ctx.seq_slot,
                            ctx.seq_first_row, ctx.seq_start, ctx.seq_end, ctx.n_seq, st.data, y, C, N, 1, C,
                            scratch=ws.buf("scan.steps", (ops.selective_scan_scratch_floats(rows, C),), torch.float32))
