@@ -561,6 +561,9 @@ selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ 
     grid_dependents_launch();
     const int slot = seq_slot[seq], first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq];
     const int t0 = p * piece, n_tok = min(piece, n_all - t0);
+    // (every CTA waits, those with nothing to do too: where no sequence has a second piece nobody else would, and the kernels
+    // behind this one, which wait for it alone, could pass the one before it)
+    grid_dependency_wait();
     if (n_tok <= 0 || (LOCAL && t0 + piece >= n_all)) return;
     const int row0 = first + t0;
     const size_t place = (size_t)(first / piece + seq + p);
@@ -568,7 +571,6 @@ selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ 
 #pragma unroll
     for (int k = 0; k < N; k += 4) Vec16<float>::load(A + (size_t)head * N + k, Ar + k);
     const float Dh = LOCAL ? 0.f : D[head];
-    grid_dependency_wait();
     const float* from = LOCAL ? nullptr : ends + (place * C + c) * N;
 #pragma unroll
     for (int k = 0; k < N; k += 4) {
