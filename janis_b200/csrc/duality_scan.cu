@@ -15,6 +15,10 @@
 // double and kept as two floats, so that the difference of two of them is as exact as one x; the decay of a whole chunk
 // is applied as S + S (e^c - 1).
 //
+// Two things the products cannot take: an infinite or NaN input u_s, which the zeros of M above the diagonal would carry to the
+// tokens before it (0 x inf), and an A above 0, whose e^(c_t) may overflow where S_0 is 0.  A chunk that meets either runs as
+// the recurrence is written, one token after another, from the same registers.
+//
 // A CTA owns up to 64 channels of a sequence's head, two warps to 16 of them: each keeps S for half of the states in registers (as
 // the accumulators of the last product, which are at the same time the second operands of the first one), adds up
 // e^(c_t) S_0 C_t over its states, and gives its partner the sums of those 32 tokens of a chunk whose results the partner
@@ -148,6 +152,43 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         S[j][0] = a.x; S[j][1] = a.y; S[j][2] = b.x; S[j][3] = b.y;
     }
 
+    // Tokens one after another: for the chunks that the products cannot take
+    auto plain = [&](int t0, int n_here, int buf) {
+        const bf16 *B_s = stage_s + (size_t)buf * STAGE + n0, *C_s = B_s + DQ * LDN, *u_s = stage_s + (size_t)buf * STAGE + 2 * DQ * LDN + pt * 16;
+        const float* delta_s = scal_s + buf * SCAL + 2 * DQ;
+        for (int t = 0; t < n_here; ++t) {
+            const float dl = delta_s[t], grown = expm1f(dl * Ah), ua = __bfloat162float(u_s[t * DUP + gr]), ub = __bfloat162float(u_s[t * DUP + gr + 8]);
+            float ya = 0.f, yb = 0.f;
+#pragma unroll
+            for (int j = 0; j < 2 * NH; ++j)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float b = __bfloat162float(B_s[t * LDN + 8 * j + gc + e]), c = __bfloat162float(C_s[t * LDN + 8 * j + gc + e]);
+                    S[j][e] += fmaf(S[j][e], grown, dl * ua * b);
+                    S[j][2 + e] += fmaf(S[j][2 + e], grown, dl * ub * b);
+                    ya = fmaf(S[j][e], c, ya);
+                    yb = fmaf(S[j][2 + e], c, yb);
+                }
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                ya += __shfl_xor_sync(0xffffffffu, ya, o);
+                yb += __shfl_xor_sync(0xffffffffu, yb, o);
+            }
+            if ((lane & 3) == 0 && half) swap_s[t * DXP + pt * 16 + gr] = ya, swap_s[t * DXP + pt * 16 + gr + 8] = yb;
+            if ((lane & 3) == 0 && !half) {
+                float* y = out + (size_t)(row0 + t0 + t) * g.C + cw + gr;
+                y[0] = fmaf(Dh, ua, ya), y[8] = fmaf(Dh, ub, yb);
+            }
+        }
+        __syncthreads();
+        for (int i = lane; i < 16 * n_here && !half; i += 32) {
+            // (a lane's own warp wrote what it adds to, before the barrier)
+            const int t = i >> 4, ch = i & 15;
+            out[(size_t)(row0 + t0 + t) * g.C + cw + ch] += swap_s[t * DXP + pt * 16 + ch];
+        }
+    };
+    const bool shrinks = Ah <= 0.f;
+
     fetch(0, 0);
     if (warp == nwarp - 1) decays(0, scal_s);
     int buf = 0;
@@ -160,7 +201,18 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        __syncthreads();
+        bool good = shrinks;                                               // the inputs that this thread brought are finite
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            const uint4 v = *reinterpret_cast<const uint4*>(stage_s + (size_t)buf * STAGE + 2 * DQ * LDN + (ut + 32 * t) * DUP + ui);
+            good = good && all_finite(v.x, v.y, v.z, v.w);
+        }
+        if (!__syncthreads_and(good)) {
+            if (more && warp == nwarp - 1) decays(t0 + DQ, scal_s + (buf ^ 1) * SCAL);
+            plain(t0, n_here, buf);
+            __syncthreads();                                               // the buffers have been read
+            continue;
+        }
         const uint32_t b_a = stage_a + buf * STAGE * 2, c_a = b_a + DQ * LDN * 2, u_a = c_a + DQ * LDN * 2;
         const float* hi_s = scal_s + buf * SCAL;
         const float *lo_s = hi_s + DQ, *delta_s = lo_s + DQ, *grow_s = delta_s + DQ, *left_s = grow_s + DQ;

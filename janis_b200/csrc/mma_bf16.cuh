@@ -37,6 +37,12 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+// Whether four pairs of bfloat16 numbers hold no infinity and no NaN: an exponent of ones carries into the sign's place
+__device__ __forceinline__ bool all_finite(uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    const uint32_t m = 0x7f807f80u, one = 0x00800080u;
+    return ((((a & m) + one) | ((b & m) + one) | ((c & m) + one) | ((d & m) + one)) & 0x80008000u) == 0;
+}
+
 // 16 bytes from global to shared memory; zeros where !ok
 __device__ __forceinline__ void copy16_or_zero(uint32_t shared, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(shared), "l"(src), "r"(ok ? 16 : 0) : "memory");

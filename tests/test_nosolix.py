@@ -390,6 +390,56 @@ def test_chunked_duality_scan_against_its_statement(C, N, cph, cpg, lens):
 
 
 @GPU
+@pytest.mark.parametrize("C,N,cph,cpg", [(128, 128, 64, 128), (64, 32, 16, 32)])
+@pytest.mark.parametrize("bad", ["input", "B", "C", "step", "growth"])
+def test_chunked_duality_scan_of_inputs_beyond_numbers(C, N, cph, cpg, bad):
+    """An infinity or a NaN at one token reaches that token's results and later ones, never an earlier token of its chunk; and heads
+    whose states grow: a state of zeros stays zeros however much it would have grown, a small one grows."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    lens, starts, slots = [100, 70], [0, 30], [1, 0]
+    _, seq_slot, first, seq_start, seq_end, T = _tables(lens, starts, slots)
+    heads, groups = C // cph, C // cpg
+    g = torch.Generator().manual_seed(C + len(bad))
+    u = torch.randn(T, C, generator=g).bfloat16()
+    dt = torch.randn(T, heads, generator=g).bfloat16()
+    bc = torch.randn(T, 2 * groups * N, generator=g).bfloat16()
+    dt_bias, D = torch.randn(heads, generator=g) - 1.0, torch.randn(heads, generator=g)
+    A = -torch.exp(torch.randn(heads, generator=g))
+    state = torch.randn(2, C, N, generator=g)
+    if bad == "input":
+        u[37, 5], u[90, C - 1], u[110, 17] = float("inf"), float("nan"), float("-inf")
+    elif bad == "B":
+        bc[37, 3] = float("inf")
+    elif bad == "C":
+        bc[37, groups * N + 3] = float("nan")
+    elif bad == "step":
+        dt[37, 0] = float("nan")
+    else:
+        A[0], state[1], state[0] = 2.0, 0.0, 1e-30 * state[0]      # 64 steps of about 0.5: e^64 and more
+        u[:96], u[100:168] = 0.0, 0.0
+    want, want_state = torch.zeros(T, C), state.clone()
+    args = lambda dev, st, out: (dev(u), 0, dev(dt), 0, dev(dt_bias), dev(A), False, dev(bc), 0, groups * N, dev(D), None, 0,
+                                 dev(seq_slot), dev(first), dev(seq_start), dev(seq_end), len(lens), st, out, C, N, cph, cpg)
+    R.selective_scan(*args(lambda x: x, want_state, want))
+    assert bad == "growth" or not want.isfinite().all()
+    for form in (3, 2):
+        ops.selective_scan_set_form(form)
+        try:
+            got, got_state = torch.full((T, C), 7.0, device="cuda"), state.clone().cuda()
+            ops.selective_scan(*args(lambda x: x.cuda(), got_state, got))
+        finally:
+            ops.selective_scan_set_form(0)
+        for name, x, y in (("results", got.cpu(), want), ("states", got_state.cpu(), want_state)):
+            fine = y.isfinite()
+            assert torch.equal(x.isfinite(), fine), (form, name)
+            # (growth: an error of 6e-8 in each of 100 step sizes, each times an exponent's sum of up to 100)
+            tol = 5e-4 if bad == "growth" else 5e-5
+            err = (x[fine].double() - y[fine].double()).abs().max().item()
+            assert err <= tol * max(1e-12, y[fine].double().abs().max().item()), (form, name, err)
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("C,N,cph,cpg,gated", [(260, 16, 1, 260, True), (128, 8, 1, 64, True), (64, 16, 4, 64, False)])
 @pytest.mark.parametrize("pieces", [2, 7, 300])
