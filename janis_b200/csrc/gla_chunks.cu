@@ -12,6 +12,8 @@
 // as exact as one logarithm.  The second kernel is the chain over the chunks.  What the recurrence keeps as floats enters
 // its products as sums of three bfloat16 numbers (both operands where both are floats: the six products that reach a float's
 // last bits), the large and the small parts in accumulators of their own, and S takes a chunk's sum by one rounded addition.
+// A chunk with an infinite or NaN value adds up A v one token after another: the zeros of A above the diagonal would
+// carry it to the tokens before it (0 x inf).
 //
 // A CTA owns 32 value columns of a sequence's head, four warps to 16 of them: each keeps S for a quarter of the key channels in
 // registers (as the accumulators of the last product, which are at the same time second operands of the first), and the
@@ -220,12 +222,27 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
             for (int p = 0; p < 2; ++p)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) own[p][e] = 0.f;
+            if (__all_sync(0xffffffffu, all_finite(b[0], b[1], b[2], b[3]))) {
 #pragma unroll
-            for (int z = 2; z >= 0; --z) {
-                uint32_t a[4];
-                ldmatrix4(a, at + A_AT + ((z * GQ + lr + (lm & 1) * 8) * LDA + (lm >> 1) * 8) * 2);
+                for (int z = 2; z >= 0; --z) {
+                    uint32_t a[4];
+                    ldmatrix4(a, at + A_AT + ((z * GQ + lr + (lm & 1) * 8) * LDA + (lm >> 1) * 8) * 2);
 #pragma unroll
-                for (int p = 0; p < 2; ++p) mma_16816(z ? rest[p] : own[p], a, b[2 * p], b[2 * p + 1]);
+                    for (int p = 0; p < 2; ++p) mma_16816(z ? rest[p] : own[p], a, b[2 * p], b[2 * p + 1]);
+                }
+            } else {
+                // an infinite or NaN value counts from its token on: the products' zeros would carry it to the tokens before
+                const bf16* stage = reinterpret_cast<const bf16*>(gla_raw + (c % GC_STAGES) * STAGE);
+                const bf16 *a_s = stage + A_AT / 2, *v_s = stage + V_AT / 2 + 16 * pt + gc;
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        for (int s = 0; s <= gr + 8 * (e >> 1); ++s) {
+                            const bf16* as = a_s + (gr + 8 * (e >> 1)) * LDA + s;
+                            const float w = __bfloat162float(as[0]) + (__bfloat162float(as[GQ * LDA]) + __bfloat162float(as[2 * GQ * LDA]));
+                            own[p][e] = fmaf(w, __bfloat162float(v_s[s * LDV + 8 * p + (e & 1)]), own[p][e]);
+                        }
             }
 #pragma unroll
             for (int p = 0; p < 2; ++p)

@@ -433,6 +433,40 @@ def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau):
 
 
 @GPU
+@pytest.mark.parametrize("bad", ["q", "k", "v", "decay"])
+def test_recurrence_in_chunks_of_inputs_beyond_numbers(bad):
+    """An infinity or a NaN at one token reaches that token's results and later ones, never an earlier token of its chunk."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    H, d, dv, lens = 2, 64, 64, [100, 60]
+    g = torch.Generator().manual_seed(len(bad))
+    T, offs = sum(lens), (0, H * d, 2 * H * d)
+    rows = torch.randn(T, 2 * H * d + H * dv, generator=g).bfloat16()
+    z, b2 = torch.randn(T, H * d, generator=g).bfloat16(), torch.randn(H * d, generator=g).bfloat16()
+    if bad == "decay":
+        z[37, 3] = float("nan")
+    else:
+        for t, c, x in ((37, 5, "inf"), (94, 33, "nan"), (111, 2, "-inf")):
+            rows[t, offs["qkv".index(bad)] + c] = float(x)
+    state = torch.randn(2, H, dv, d, generator=g)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32)
+    slots, first, start, end = i32([1, 0]), i32([0, 100]), i32([0, 0]), i32(lens)
+    want, want_state = torch.zeros(T, H * dv), state.clone()
+    R.gla_scan(rows, *offs, z, b2, slots, first, start, end, want_state, want, 2, H, d, dv, d ** -0.5, 8.0)
+    assert not want.isfinite().all()
+    for chunked in (True, False):
+        n = ops.gla_chunks_floats(torch.bfloat16, T, 2, H, d, dv)
+        got, got_state = torch.full((T, H * dv), 7.0, device="cuda"), state.clone().cuda()
+        ops.gla_scan(rows.cuda(), *offs, z.cuda(), b2.cuda(), slots.cuda(), first.cuda(), start.cuda(), end.cuda(), got_state, got, 2,
+                     H, d, dv, d ** -0.5, 8.0, chunks=torch.full((n,), float("nan"), device="cuda") if chunked else None)
+        for name, x, y in (("results", got.cpu(), want), ("states", got_state.cpu(), want_state)):
+            fine = y.isfinite()
+            assert torch.equal(x.isfinite(), fine), (chunked, name)
+            err = (x[fine].double() - y[fine].double()).abs().max().item()
+            assert err <= 5e-5 * max(1.0, y[fine].double().abs().max().item()), (chunked, name, err)
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,d,dv,tau", [(2, 16, 24, 8.0), (1, 40, 48, 32.0), (3, 8, 8, 1.0), (2, 128, 72, 16.0), (1, 200, 32, 4.0)])
 def test_recurrence_kernel_against_its_statement(dtype, H, d, dv, tau):
