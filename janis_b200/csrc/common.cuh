@@ -157,6 +157,46 @@ __device__ __forceinline__ size_t cached_row(const CachedPrefix& c, int slot, in
     return (((size_t)page * nkv + kvh) * JANIS_PAGE + idx % JANIS_PAGE) * (size_t)hd;
 }
 
+// The pieces of `size` tokens that a step's sequences are cut into, counted through in the order of the sequences (which
+// need not be that of their rows).  Both by a whole warp, 32 sequences at a time.
+__device__ __forceinline__ int pieces_of(const int* __restrict__ seq_start, const int* __restrict__ seq_end, int s, int n_seq, int size) {
+    const int n = s < n_seq ? seq_end[s] - seq_start[s] : 0;
+    return n > 0 ? (n + size - 1) / size : 0;
+}
+// the pieces before sequence `seq`'s first one
+__device__ __forceinline__ int pieces_before(const int* __restrict__ seq_start, const int* __restrict__ seq_end, int seq, int size) {
+    int n = 0;
+    for (int s = threadIdx.x & 31; s < seq; s += 32) n += pieces_of(seq_start, seq_end, s, seq, size);
+    return __reduce_add_sync(0xffffffffu, n);
+}
+// whose piece `place` is, and which one of that sequence; false: there are no more than `place` pieces
+__device__ __forceinline__ bool find_piece(int place, const int* __restrict__ seq_start, const int* __restrict__ seq_end, int n_seq, int size,
+                                           int& seq, int& piece) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    seq = 0;
+    piece = place;
+    if (place < pieces_of(seq_start, seq_end, 0, n_seq, size)) return true;
+    for (int s0 = 0; s0 < n_seq; s0 += 32) {
+        const int n = pieces_of(seq_start, seq_end, s0 + lane, n_seq, size);
+        int upto = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, before + upto > place);
+        if (past != 0) {
+            const int l = __ffs(past) - 1;
+            seq = s0 + l;
+            piece = place - before - __shfl_sync(0xffffffffu, upto - n, l);
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(bf16 v) { return __bfloat162float(v); }
 

@@ -37,7 +37,7 @@ struct GlaChunkShape {
 };
 
 // What the first kernel leaves: weighted queries and keys [2][3][n_tok][H d], A [n_tok][H][3][16] (bfloat16 parts), and
-// e^(b_end) - 1 [chunk][H d] floats; chunk c of sequence s in place first_row / 16 + s + c.
+// e^(b_end) - 1 [chunk][H d] floats, the sequences' chunks one after another.
 struct GlaChunkScratch {
     bf16 *qk, *a;
     float* grow;
@@ -57,18 +57,20 @@ __device__ __forceinline__ void split3_one(float x, bf16& hi, bf16& mid, bf16& l
     lo = __float2bfloat16_rn(x - __bfloat162float(mid));
 }
 
-// A CTA per (sequence, chunk, head): first a thread per key channel, then a thread per pair of tokens
+// A CTA per (chunk, head), the sequences' chunks counted through: first a thread per key channel, then a thread per pair of tokens.
+// (The step's n_tok / 16 + n_seq bound the chunks' number; a place for every chunk of the step in every sequence would be
+// 2 million CTAs for 256 prompts of 64 tokens.)
 __global__ void __launch_bounds__(256)
 gla_chunk_terms_kernel(const bf16* __restrict__ rows, const bf16* __restrict__ z_rows, const bf16* __restrict__ bias, GlaChunkShape g,
-                       const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                       int n_seq, const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
                        GlaChunkScratch out) {
     extern __shared__ float gla_terms[];
-    const int d = g.d, ld = d + 1, seq = blockIdx.z, chunk = blockIdx.x, h = blockIdx.y;
+    const int d = g.d, ld = d + 1, place = blockIdx.x, h = blockIdx.y;
     float *q_s = gla_terms, *k_s = q_s + GQ * ld, *hi_s = k_s + GQ * ld, *lo_s = hi_s + GQ * ld;      // [16][ld]
     grid_dependents_launch();
-    const int first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq], row0 = first + chunk * GQ;
-    const int n = min(GQ, n_all - chunk * GQ);
-    if (n <= 0) return;
+    int seq = 0, chunk = 0;
+    if (!find_piece(place, seq_start, seq_end, n_seq, GQ, seq, chunk)) return;
+    const int row0 = seq_first_row[seq] + chunk * GQ, n = min(GQ, seq_end[seq] - seq_start[seq] - chunk * GQ);
     grid_dependency_wait();
     const size_t plane = (size_t)g.n_tok * g.H * d;
     for (int i = threadIdx.x; i < d; i += 256) {
@@ -93,7 +95,7 @@ gla_chunk_terms_kernel(const bf16* __restrict__ rows, const bf16* __restrict__ z
             const float left = (float)(b - ((double)hi_s[t * ld + i] + (double)lo_s[t * ld + i]));
             split3_one(k_s[t * ld + i] * expf(left), out.qk[at], out.qk[plane + at], out.qk[2 * plane + at]);
         }
-        out.grow[((size_t)(first / GQ + seq + chunk) * g.H + h) * d + i] = expm1f((float)b);
+        out.grow[((size_t)place * g.H + h) * d + i] = expm1f((float)b);
     }
     __syncthreads();
     const int t = threadIdx.x >> 4, s = threadIdx.x & 15;
@@ -135,7 +137,7 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(gla_raw);
     const size_t plane = (size_t)g.n_tok * g.H * D;
     const int chunks = (n_tok + GQ - 1) / GQ;
-    const size_t place0 = (size_t)(row0 / GQ + seq);
+    const size_t place0 = (size_t)pieces_before(seq_start, seq_end, seq, GQ);
     // this thread's pieces: column qi of rows qx, qx + STEP, ... of the weighted queries and keys; one piece of A, of the values
     // and of the decays (fewer threads bring those)
     constexpr int STEP = 256 / (D / 8);
@@ -337,7 +339,7 @@ JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, in
     if (!(tau > 0.f)) return fail("gla_chunks: tau must be positive");
     if (row_elems % 8 || v_off % 8 || (((uintptr_t)rows | (uintptr_t)scratch) & 15) || (((uintptr_t)state | (uintptr_t)o_out) & 7))
         return fail("gla_chunks: rows of %d elements, values at %d: not in whole pieces of 16 bytes", row_elems, v_off);
-    if (n_seq > 65535 || H > 65535) return fail("gla_chunks: too many sequences or heads (%d, %d)", n_seq, H);
+    if (H > 65535) return fail("gla_chunks: too many heads (%d)", H);
     GlaChunkShape g;
     g.row_elems = row_elems; g.q_off = q_off; g.k_off = k_off; g.v_off = v_off; g.H = H; g.d = d; g.dv = dv; g.n_tok = n_tok;
     g.q_scale = q_scale; g.inv_tau = 1.0f / tau;
@@ -345,8 +347,8 @@ JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, in
     const size_t bytes = (size_t)4 * GQ * (d + 1) * sizeof(float);
     const cudaError_t e = cudaFuncSetAttribute(gla_chunk_terms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail("gla_chunks: shared memory of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-    if (launch_kernel("gla_chunk_terms", gla_chunk_terms_kernel, dim3((n_tok + GQ - 1) / GQ, H, n_seq), dim3(256), bytes, stream, 1, (const bf16*)rows,
-                      (const bf16*)z, (const bf16*)bias, g, seq_first_row, seq_start, seq_end, s))
+    if (launch_kernel("gla_chunk_terms", gla_chunk_terms_kernel, dim3(n_tok / GQ + n_seq, H), dim3(256), bytes, stream, 1, (const bf16*)rows,
+                      (const bf16*)z, (const bf16*)bias, g, n_seq, seq_first_row, seq_start, seq_end, s))
         return 1;
 #define JANIS_GLA_CHAIN(NK)                                                                                                       \
     return gla_chain_launch<NK>((const bf16*)rows, g, s, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, o_out, stream);

@@ -398,7 +398,8 @@ def test_rotation_and_cache_write_against_their_statement(dtype, H, G, d, dv, ro
 
 @GPU
 @pytest.mark.parametrize("H,d,dv,tau", [(2, 64, 32, 8.0), (2, 128, 64, 16.0), (1, 256, 96, 0.05)])
-def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau):
+@pytest.mark.parametrize("order", ["forwards", "backwards"])
+def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau, order):
     """16 tokens at a time: sequences on a chunk's border and beside it (one without a slot), the second step going on from the
     states of the first; tau = 0.05 makes decays of e^-100 and less beside ones near 1; scratch of NaN, not a float more than asked for."""
     from janis_b200.kernels import ops
@@ -410,6 +411,8 @@ def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau):
     state = torch.zeros(6, H, dv, d)
     got_state = state.clone().cuda()
     slots, first = torch.tensor([2, 5, 0, 3, -1], dtype=torch.int32), torch.tensor([0, 1, 17, 34, 145], dtype=torch.int32)
+    if order == "backwards":                       # the last sequence's rows come first
+        first = T - first - torch.tensor(lens, dtype=torch.int32)
     start = torch.zeros(n_seq, dtype=torch.int32)
     offs = (8, 8 + H * d, 8 + 2 * H * d)
     floats = ops.gla_chunks_floats(torch.bfloat16, T, n_seq, H, d, dv)
