@@ -234,12 +234,29 @@ constexpr int SCAN_THREADS = 128;
 
 // Step sizes once per (token, head), as floats: delta = softplus(dt + bias) and, where a head has one decay,
 // exp(delta A) - 1.  (Left to the scan, every lane of a channel and every channel of a head would form them again.)
+// For a prompt that runs in pieces (selective_scan_piece_kernel) the first warp also counts the sequences' pieces through, in
+// whatever order their rows lie: where[s] is the number before sequence s's first one.
 template <typename T>
 __global__ void __launch_bounds__(256)
 scan_steps_kernel(const T* __restrict__ dt_rows, int dt_stride, int dt_off, const float* __restrict__ dt_bias,
-                  const float* __restrict__ A_head, float* __restrict__ delta, float* __restrict__ grow, int heads, size_t n) {
+                  const float* __restrict__ A_head, float* __restrict__ delta, float* __restrict__ grow, int heads, size_t n,
+                  int* __restrict__ where, int piece, int n_seq, const int* __restrict__ seq_start, const int* __restrict__ seq_end) {
     grid_dependents_launch();
     grid_dependency_wait();
+    if (where != nullptr && blockIdx.x == 0 && threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        for (int s0 = 0, before = 0; s0 < n_seq; s0 += 32) {
+            const int n = pieces_of(seq_start, seq_end, s0 + lane, n_seq, piece);
+            int upto = before + n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v - before;
+            }
+            if (s0 + lane < n_seq) where[s0 + lane] = upto - n;
+            before = __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t t = i / heads;
         const int h = (int)(i % heads);
@@ -548,11 +565,14 @@ selective_scan_staged_kernel(const T* __restrict__ u_rows, const T* __restrict__
 // what a token costs beside its states is paid once, and there are pieces enough to fill the SMs' issue slots, which bound it.
 // 4,608 channels, 16 states, against selective_scan_kernel: one sequence of 2,048 tokens 1,105 -> 390 us, 300 tokens 148 -> 74,
 // 128 tokens 66 -> 47 (64 tokens 39 -> 46: the launcher leaves short steps to the other kernel); eight of 512 1,200 -> 677.
+// The grid has a place for every piece of the step in every sequence.  Those that nothing is left for cost little: 256 sequences of 64
+// tokens 4,220 -> 1,800, 512 of 32 4,300 -> 2,150; a flat grid whose CTAs look for their sequence took 1,730 and 2,300 there, and
+// 437 for 402 at one sequence of 2,048.
 template <typename T, int N, bool LOCAL>
 __global__ void __launch_bounds__(128)
 selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ bc_rows, const T* __restrict__ z_rows,
                             const float* __restrict__ delta, const float* __restrict__ A, const float* __restrict__ D, ScanShape g,
-                            int piece, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
+                            int piece, const int* __restrict__ where, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
                             const int* __restrict__ seq_start, const int* __restrict__ seq_end, float* __restrict__ state,
                             float* __restrict__ ends, float* __restrict__ sums, void* __restrict__ out_raw) {
     const int seq = blockIdx.z, p = blockIdx.y, c_raw = blockIdx.x * 128 + threadIdx.x, C = g.C;
@@ -566,7 +586,7 @@ selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ 
     grid_dependency_wait();
     if (n_tok <= 0 || (LOCAL && t0 + piece >= n_all)) return;
     const int row0 = first + t0;
-    const size_t place = (size_t)(first / piece + seq + p);
+    const size_t place = (size_t)(where[seq] + p);
     float Ar[N], S[N];
 #pragma unroll
     for (int k = 0; k < N; k += 4) Vec16<float>::load(A + (size_t)head * N + k, Ar + k);
@@ -656,17 +676,17 @@ selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ 
 // A thread per (sequence, channel, state)
 template <int N>
 __global__ void __launch_bounds__(256)
-selective_scan_carry_kernel(const float* __restrict__ A, int C, int cph, int piece, const int* __restrict__ seq_slot,
-                            const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+selective_scan_carry_kernel(const float* __restrict__ A, int C, int cph, int piece, const int* __restrict__ where,
+                            const int* __restrict__ seq_slot, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
                             const float* __restrict__ state, float* __restrict__ ends, const float* __restrict__ sums) {
     const int seq = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, c = i / N, k = i - c * N;
     grid_dependents_launch();
-    const int slot = seq_slot[seq], first = seq_first_row[seq], n_all = seq_end[seq] - seq_start[seq];
+    const int slot = seq_slot[seq], n_all = seq_end[seq] - seq_start[seq];
     if (c >= C || n_all <= 0) return;
     const float a = A[(size_t)(c / cph) * N + k];
     grid_dependency_wait();
     float S = slot >= 0 ? state[((size_t)slot * C + c) * N + k] : 0.f;
-    const size_t place = (size_t)(first / piece + seq);
+    const size_t place = (size_t)where[seq];
     const int pieces = (n_all + piece - 1) / piece;
     for (int p = 0; p < pieces; ++p) {
         float* e = ends + ((place + p) * C + c) * N + k;
@@ -830,18 +850,18 @@ static long long scan_piece_floats(int C, int N) { return (long long)C * (N + 1)
 
 template <typename T, int N>
 static int scan_pieces_launch(const void* u, const void* bc, const void* z, const float* delta, const float* A, const float* D, ScanShape g,
-                              int piece, int n_tok, const int* seq_slot, const int* seq_first_row, const int* seq_start,
+                              int piece, const int* where, int n_tok, const int* seq_slot, const int* seq_first_row, const int* seq_start,
                               const int* seq_end, int n_seq, float* state, float* ends, float* sums, void* out, cudaStream_t stream) {
     const int pieces = (n_tok + piece - 1) / piece;
     const dim3 grid((g.C + 127) / 128, pieces, n_seq), block(128);
     if (launch_kernel("selective_scan", selective_scan_piece_kernel<T, N, true>, grid, block, 0, stream, 1, (const T*)u, (const T*)bc,
-                      (const T*)z, delta, A, D, g, piece, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out))
+                      (const T*)z, delta, A, D, g, piece, where, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out))
         return 1;
     if (launch_kernel("selective_scan_carry", selective_scan_carry_kernel<N>, dim3((g.C * N + 255) / 256, n_seq), dim3(256), 0, stream, 1,
-                      A, g.C, g.cph, piece, seq_slot, seq_first_row, seq_start, seq_end, (const float*)state, ends, (const float*)sums))
+                      A, g.C, g.cph, piece, where, seq_slot, seq_start, seq_end, (const float*)state, ends, (const float*)sums))
         return 1;
     return launch_kernel("selective_scan", selective_scan_piece_kernel<T, N, false>, grid, block, 0, stream, 1, (const T*)u, (const T*)bc,
-                         (const T*)z, delta, A, D, g, piece, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out);
+                         (const T*)z, delta, A, D, g, piece, where, seq_slot, seq_first_row, seq_start, seq_end, state, ends, sums, out);
 }
 
 JANIS_EXPORT long long janis_selective_scan_scratch(int n_tok, int heads) { return 2LL * n_tok * heads; }
@@ -936,7 +956,7 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
         const bool aligned = (((uintptr_t)bc | (uintptr_t)A | (uintptr_t)state | (uintptr_t)scratch) & 15) == 0 && bc_stride % epp == 0 &&
                              b_off % epp == 0 && c_off % epp == 0 && (size_t)n_tok * g.heads % 2 == 0 && C % 4 == 0;
         const long long room = (scratch_floats - 2LL * n_tok * g.heads) / scan_piece_floats(C, N) - n_seq;
-        if (aligned && room >= 2) {
+        if (aligned && room >= 2 && n_seq <= (long long)n_tok * g.heads) {
             long long want = (148LL * 16 * 32 + C - 1) / C;
             if (want > room) want = room;
             if (want < 2) want = 2;
@@ -947,17 +967,18 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
             piece = length < 8 ? 8 : (int)length;
         }
     }
+    int* where = piece > 0 ? (int*)grow : nullptr;           // (in the place of the heads' decays, which this form does not keep)
     float* ends = scratch + 2 * (size_t)n_tok * g.heads;
     float* sums = piece > 0 ? ends + ((size_t)(n_tok / piece) + n_seq) * C * N : nullptr;
 #define JANIS_SCAN_PIECES(T)                                                                                                  \
     if (piece > 0)                                                                                                             \
-        return N == 8 ? scan_pieces_launch<T, 8>(u, bc, z, delta, A, D, g, piece, n_tok, seq_slot, seq_first_row, seq_start,     \
+        return N == 8 ? scan_pieces_launch<T, 8>(u, bc, z, delta, A, D, g, piece, where, n_tok, seq_slot, seq_first_row, seq_start,     \
                                                  seq_end, n_seq, state, ends, sums, out, stream)                                 \
-                      : scan_pieces_launch<T, 16>(u, bc, z, delta, A, D, g, piece, n_tok, seq_slot, seq_first_row, seq_start,    \
+                      : scan_pieces_launch<T, 16>(u, bc, z, delta, A, D, g, piece, where, n_tok, seq_slot, seq_first_row, seq_start,    \
                                                   seq_end, n_seq, state, ends, sums, out, stream);
     if (dtype == JANIS_F32) {
         if (launch_kernel("scan_steps", scan_steps_kernel<float>, sgrid, sblock, 0, stream, 1, (const float*)dt, dt_stride, dt_off,
-                          dt_bias, A_head, delta, grow, g.heads, n))
+                          dt_bias, A_head, delta, grow, g.heads, n, where, piece, n_seq, seq_start, seq_end))
             return 1;
         JANIS_SCAN_PIECES(float)
         return a_per_state ? scan_launch<float, true>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream)
@@ -965,7 +986,7 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
     }
     if (dtype == JANIS_BF16) {
         if (launch_kernel("scan_steps", scan_steps_kernel<bf16>, sgrid, sblock, 0, stream, 1, (const bf16*)dt, dt_stride, dt_off,
-                          dt_bias, A_head, delta, grow, g.heads, n))
+                          dt_bias, A_head, delta, grow, g.heads, n, where, piece, n_seq, seq_start, seq_end))
             return 1;
         JANIS_SCAN_PIECES(bf16)
         return a_per_state ? scan_launch<bf16, true>(u, bc, z, delta, grow, A, D, g, best_spl, vec, staged_bytes, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, out, stream)

@@ -442,14 +442,16 @@ def test_chunked_duality_scan_of_inputs_beyond_numbers(C, N, cph, cpg, bad):
 @GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("C,N,cph,cpg,gated", [(260, 16, 1, 260, True), (128, 8, 1, 64, True), (64, 16, 4, 64, False)])
-@pytest.mark.parametrize("pieces", [2, 7, 300])
-def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, pieces):
+@pytest.mark.parametrize("pieces,order", [(2, "forwards"), (7, "forwards"), (300, "forwards"), (7, "backwards"), (300, "backwards")])
+def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, pieces, order):
     """Room for 2, 7 and 300 pieces of 220 tokens (the last one: pieces of 8 tokens): sequences of one piece and of many, on a
     border of pieces and beside it, from zero and from stored states, with a padding sequence."""
     from janis_b200.kernels import ops
     from tests import kernel_refs as R
     lens, starts, slots = [120, 1, 8, 81, 10], [0, 30, 5, 0, 0], [3, 0, 1, 4, -1]
     _, seq_slot, first, seq_start, seq_end, T = _tables(lens, starts, slots)
+    if order == "backwards":                                 # the last sequence's rows come first
+        first = T - first - torch.tensor(lens, dtype=torch.int32)
     heads, groups = C // cph, C // cpg
     g = torch.Generator().manual_seed(C + N + pieces)
     u, z = torch.randn(T, C + 8, generator=g).to(dtype), torch.randn(T, C, generator=g).to(dtype)
