@@ -673,6 +673,14 @@ selective_scan_piece_kernel(const T* __restrict__ u_rows, const T* __restrict__ 
     }
 }
 
+// S e^x + end, as the steps that x sums up would have given it: a state of 0 stays 0 and a small one grows step by step where e^x
+// alone is beyond the largest float
+__device__ __forceinline__ float carried(float S, float x, float end) {
+    if (S == 0.f) return end;
+    for (x = x > 512.f ? 512.f : x; x > 64.f; x -= 64.f) S *= 6.2351491e27f;       // e^64 (512: nothing but 0 is left finite)
+    return decayed(S, decay_minus_one(x), end);
+}
+
 // A thread per (sequence, channel, state)
 template <int N>
 __global__ void __launch_bounds__(256)
@@ -693,7 +701,7 @@ selective_scan_carry_kernel(const float* __restrict__ A, int C, int cph, int pie
         const bool last = p + 1 == pieces;                       // (the last piece leaves nothing here)
         const float end = last ? 0.f : *e, sum = last ? 0.f : sums[(place + p) * C + c];
         *e = S;
-        if (!last) S = decayed(S, decay_minus_one(sum * a), end);
+        if (!last) S = carried(S, sum * a, end);
     }
 }
 

@@ -482,6 +482,44 @@ def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, piec
 
 
 @GPU
+@pytest.mark.parametrize("N", [8, 16])
+def test_scan_in_pieces_of_growing_states(N):
+    """Decays above 1 over pieces that would multiply by more than the largest float: a state of zeros stays zeros, a small one
+    grows."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    C, lens, starts, slots = 64, [150, 60], [0, 30], [1, 0]
+    _, seq_slot, first, seq_start, seq_end, T = _tables(lens, starts, slots)
+    g = torch.Generator().manual_seed(N)
+    u, dt = torch.randn(T, C, generator=g).bfloat16(), torch.zeros(T, C).bfloat16()
+    u[:140], u[150:205] = 0.0, 0.0
+    bc = torch.randn(T, 2 * N, generator=g).bfloat16()
+    bc[:, N:] = torch.eye(N)[0].bfloat16()                                                    # results: the first state
+    dt_bias, D = torch.full((C,), math.log(math.e - 1.0)), torch.zeros(C)                    # steps of 1
+    A = torch.linspace(0.5, 2.0, C)[:, None] * torch.ones(1, N)
+    state = 1e-30 * torch.randn(2, C, N, generator=g)                                         # over 60 steps up to e^120
+    state[1] = 0.0
+    want, want_state = torch.zeros(T, C), state.clone()
+    args = lambda dev, st, out: (dev(u), 0, dev(dt), 0, dev(dt_bias), dev(A), True, dev(bc), 0, N, dev(D), None, 0, dev(seq_slot),
+                                 dev(first), dev(seq_start), dev(seq_end), len(lens), st, out, C, N, 1, C)
+    R.selective_scan(*args(lambda x: x, want_state, want))
+    for form, pieces in ((4, 2), (4, 7), (1, 0)):
+        floats = ops.selective_scan_scratch_floats(T, C) + (pieces + len(lens)) * C * (N + 1)
+        ops.selective_scan_set_form(form)
+        try:
+            got, got_state = torch.full((T, C), 7.0, device="cuda"), state.clone().cuda()
+            ops.selective_scan(*args(lambda x: x.cuda(), got_state, got), scratch=torch.full((floats,), float("nan"), device="cuda"))
+        finally:
+            ops.selective_scan_set_form(0)
+        for name, x, y in (("results", got.cpu(), want), ("states", got_state.cpu(), want_state)):
+            # 60 steps that grow by up to e^2: an error of 6e-8 in a step's size, exponential and sum makes 2.4e-7 a step
+            assert x.isfinite().all() and y.isfinite().all(), (form, pieces, name)
+            err = ((x.double() - y.double()).abs() / y.double().abs())[y != 0].max().item()
+            assert err <= 1e-4, (form, pieces, name, err)
+            assert (x[y == 0] == 0).all(), (form, pieces, name)
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_small_kernels_against_their_statements(dtype):
     from janis_b200.kernels import ops
