@@ -570,14 +570,15 @@ struct RowsPlan {
     size_t smem_scores, smem_values;
 };
 
-static RowsPlan rows_plan(int T, int H, int G, int d, int dv, int max_keys, int vec) {
+// (with_scores: the scores cross memory; rows_mixed_kernel keeps them)
+static RowsPlan rows_plan(int T, int H, int G, int d, int dv, int max_keys, int vec, bool with_scores = true) {
     RowsPlan p = {};
     const int pages = (max_keys + 63) / 64;
     p.sh.chunk = 64 * ((pages + 63) / 64);
     p.sh.n_chunks = (max_keys + p.sh.chunk - 1) / p.sh.chunk;
     if (p.sh.n_chunks < 1) p.sh.n_chunks = 1;
     size_t at = 0;
-    p.scores = at; at += (size_t)T * H * p.sh.n_chunks * p.sh.chunk;
+    p.scores = at; at += with_scores ? (size_t)T * H * p.sh.n_chunks * p.sh.chunk : 0;
     p.part = at;   at += (size_t)T * p.sh.n_chunks * H * 2;
     p.fin = at;    at += (size_t)T * H * 2;
     at = (at + 3) & ~(size_t)3;
@@ -671,8 +672,25 @@ JANIS_EXPORT int janis_talk_attention_rows(const void* q_rows, int dtype, int q_
     return fail("talk_attention_rows: unknown dtype %d", dtype);
 }
 
+// What rows_mixed_kernel runs a step with; p.total = 0 where it does not take the sizes.
+static RowsPlan rows_mixed_plan(int dtype, int T, int H, int G, int d, int dv, int max_keys, size_t* bytes) {
+    const int vec = dtype == JANIS_F32 ? 4 : 8;
+    if (T <= 0 || T > 65535 || H <= 0 || G <= 0 || H % G || d <= 0 || dv <= 0 || max_keys <= 0 || d % vec || dv % vec || dv % 2 || H > 128) return RowsPlan{};
+    RowsPlan p = rows_plan(T, H, G, d, dv, max_keys, vec, false);
+    const int vb = H / G <= 2 ? 2 : ROWS_VB, sums = ROWS_THREADS * vb * vec;
+    p.sh.shared_floats = H * (d + 8) > sums ? H * (d + 8) : sums;
+    *bytes = ((size_t)2 * H * p.sh.chunk + p.sh.shared_floats + p.sh.chunk) * sizeof(float);
+    if (*bytes > 200 * 1024 || p.smem_scores > 160 * 1024 || p.smem_values > 160 * 1024 || p.sh.n_chunks > ROWS_MERGE_CHUNKS) p.total = 0;
+    return p;
+}
+
+// Floats of scratch that `janis_talk_attention_rows_mixed` wants for such a step, or 0 when it does not take the sizes.
+JANIS_EXPORT long long janis_talk_attention_rows_mixed_floats(int dtype, int T, int H, int G, int d, int dv, int max_keys) {
+    size_t bytes = 0;
+    return (long long)rows_mixed_plan(dtype, T, H, G, d, dv, max_keys, &bytes).total;
+}
+
 // The same for heads mixed by `talk` before the softmax, with values that were turned by their own positions where inv_v is given.
-// Scratch as for janis_talk_attention_rows.
 JANIS_EXPORT int janis_talk_attention_rows_mixed(const void* q_rows, int dtype, int q_row_elems, const int* tok_pos, const int* tok_seq,
                                                  const int* seq_slot, const void* kpool, const void* vpool, const int* page_table,
                                                  int table_stride, const float* talk, const float* inv_v, void* out, int T, int H, int G,
@@ -681,23 +699,18 @@ JANIS_EXPORT int janis_talk_attention_rows_mixed(const void* q_rows, int dtype, 
                                                  cudaStream_t stream) {
     if (T <= 0) return 0;
     if (keep_first < 0 || (keep_first > 0 && window <= 0)) return fail("talk_attention_rows_mixed: %d kept first positions need a window", keep_first);
-    const long long want = janis_talk_attention_rows_floats(dtype, T, H, G, d, dv, max_keys);
-    const int vec = dtype == JANIS_F32 ? 4 : 8;
-    if (want <= 0 || dv % 2 || talk == nullptr || T > 65535 || q_row_elems % vec) return fail("talk_attention_rows_mixed: sizes not taken (%d heads over %d, %d and %d features)", H, G, d, dv);
+    size_t bytes = 0;
+    RowsPlan p = rows_mixed_plan(dtype, T, H, G, d, dv, max_keys, &bytes);
+    const long long want = (long long)p.total;
+    if (want <= 0 || talk == nullptr || q_row_elems % (dtype == JANIS_F32 ? 4 : 8)) return fail("talk_attention_rows_mixed: sizes not taken (%d heads over %d, %d and %d features)", H, G, d, dv);
     if (scratch == nullptr || scratch_floats < want) return fail("talk_attention_rows_mixed: scratch of %lld floats, %lld wanted", scratch_floats, want);
     if ((reinterpret_cast<uintptr_t>(q_rows) | reinterpret_cast<uintptr_t>(kpool) | reinterpret_cast<uintptr_t>(vpool) | reinterpret_cast<uintptr_t>(scratch)) & 15)
         return fail("talk_attention_rows_mixed: rows, pools and scratch start on 16-byte borders");
-    RowsPlan p = rows_plan(T, H, G, d, dv, max_keys, vec);
     RowsShape& sh = p.sh;
-    if (sh.n_chunks > ROWS_MERGE_CHUNKS) return fail("talk_attention_rows_mixed: %d chunks", sh.n_chunks);
     sh.H = H; sh.G = G; sh.d = d; sh.dv = dv; sh.v_stride = dv; sh.window = window; sh.keep_first = keep_first;
     sh.sink = sink ? (sink_values != nullptr ? 2 : 1) : 0;
     sh.scale = scale;
     sh.cap = cap;
-    const int vb = H / G <= 2 ? 2 : ROWS_VB, sums = ROWS_THREADS * vb * vec;
-    sh.shared_floats = H * (d + 8) > sums ? H * (d + 8) : sums;
-    const size_t bytes = ((size_t)2 * H * sh.chunk + sh.shared_floats + sh.chunk) * sizeof(float);
-    if (bytes > 200 * 1024) return fail("talk_attention_rows_mixed: %zu bytes of shared memory", bytes);
 #define JANIS_ROWS_MIXED(TT)                                                                                                          \
     {                                                                                                                                 \
         auto kernel = H / G <= 2 ? rows_mixed_kernel<TT, 2> : rows_mixed_kernel<TT, ROWS_VB>;                                        \

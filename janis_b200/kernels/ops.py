@@ -151,6 +151,8 @@ def mixers():
         lib.janis_gla_chunks_floats.argtypes = [I, I, I, I, I]
         lib.janis_gla_chunks_floats.restype = c_longlong
         lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P, c_longlong, P]
+        lib.janis_talk_attention_rows_mixed_floats.argtypes = [I, I, I, I, I, I, I]
+        lib.janis_talk_attention_rows_mixed_floats.restype = c_longlong
         lib.janis_talk_attention_rows_mixed.argtypes = [P, I, I, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, F, I, I, I, F, P, P, c_longlong, I, P]
         lib.janis_gla_scan.argtypes = [P, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P]
         lib.janis_head_norm_gate.argtypes = [P, P, I, I, I, P, F, P, I, I, I, I, I, P]
@@ -1052,12 +1054,19 @@ def talk_attention_rows(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_t
     return out
 
 
+def talk_attention_rows_mixed_floats(dtype, T: int, H: int, G: int, d: int, dv: int, max_keys: int) -> int:
+    """Floats of scratch that `talk_attention_rows_mixed` wants for a step of T rows that see up to max_keys keys each, or 0
+    where it does not take the sizes (it holds a chunk's scores twice beside the queries, so that fewer fit than
+    `talk_attention_rows` takes)."""
+    return int(mixers().janis_talk_attention_rows_mixed_floats(_DT[dtype], int(T), int(H), int(G), int(d), int(dv), int(max_keys)))
+
+
 def talk_attention_rows_mixed(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table, talk, inv_v, out, H: int, G: int, d: int,
                               dv: int, scale: float, scratch, max_keys: int, sink: bool = False, window: int = 0, cap: float = 0.0,
                               sink_values=None, keep_first: int = 0):
     """`talk_attention_rows` for heads whose scores talk [H, H] float32 mixes before the softmax, in two launches; with inv_v
-    [dv / 2] each head's output is turned back by the row's position.  Sizes and scratch as `talk_attention_rows_floats` says, with
-    an even dv and rows of whole 16-byte pieces."""
+    [dv / 2] each head's output is turned back by the row's position.  Sizes and scratch as `talk_attention_rows_mixed_floats`
+    says, with rows of whole 16-byte pieces."""
     T = q_rows.shape[0]
     _t(q_rows, "q_rows", _FLOATS, (T, None))
     n_pages = kpool.shape[0]

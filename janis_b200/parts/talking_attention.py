@@ -268,10 +268,10 @@ class TalkingHeadsAttention(Mixer):
                                            self.scale, ws.buf("tattn.rows_scratch", (rows_floats,), torch.float32), max_keys,
                                            sink=self.sink, window=self.window or -self.block, **more)
         if (decode and rt.dtype == torch.bfloat16 and self.talk is not None and not (self.block and self.window) and not self.values_from_keys
-                and dv % 2 == 0 and rows.shape[1] % 8 == 0 and hasattr(ops, "talk_attention_rows_mixed")):
+                and rows.shape[1] % 8 == 0 and hasattr(ops, "talk_attention_rows_mixed")):
             # heads mixed before the softmax: keys and values read once, 16 bytes a lane, and a merge
             max_keys = min(ctx.len_bound, (self.window or self.block) + self.keep_first) if self.window or self.block else ctx.len_bound
-            rows_floats = ops.talk_attention_rows_floats(rt.dtype, T, H, G, d, dv, max_keys)
+            rows_floats = ops.talk_attention_rows_mixed_floats(rt.dtype, T, H, G, d, dv, max_keys)
             if rows_floats:
                 return ops.talk_attention_rows_mixed(rows, ctx.tok_pos, ctx.tok_seq, ctx.seq_slot, kv.k, kv.v, kv.table, self.talk, inv_v, att,
                                                      H, G, d, dv, self.scale, ws.buf("tattn.rows_scratch", (rows_floats,), torch.float32),

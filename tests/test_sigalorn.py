@@ -320,6 +320,35 @@ def test_single_rows_of_mixed_heads(dtype, H, G, d, dv, window, keep_first, sink
 
 
 @GPU
+@pytest.mark.parametrize("H,fits", [(100, True), (120, False)])
+def test_single_rows_of_mixed_heads_at_the_limit_of_shared_memory(H, fits):
+    """100 heads of 192 over 5,000 keys fit the kernel that mixes heads in single rows; with 120, which the kernels without
+    mixing take, it says that they do not, and the kernels of before run the step.  The part asks the same function."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    G, d, dv, pos, max_keys = 4, 192, 16, [70, 3], 5000
+    kp, vp, table, slots = _paged(2, [p + 1 for p in pos], G, d, dv, torch.bfloat16, 3)
+    g = torch.Generator().manual_seed(H)
+    q = torch.randn(2, H * d, generator=g).bfloat16()
+    M = (torch.eye(H) + 0.1 * torch.randn(H, H, generator=g)).float()
+    tok_pos, tok_seq = torch.tensor(pos, dtype=torch.int32), torch.arange(2, dtype=torch.int32)
+    want = torch.zeros(2, H * dv, dtype=torch.bfloat16)
+    R.talk_attention(q, tok_pos, tok_seq, slots, kp, vp, table, M, None, want, H, G, d, dv, d ** -0.5, 0, True)
+    assert ops.talk_attention_rows_floats(torch.bfloat16, 2, H, G, d, dv, max_keys) > 0
+    n = ops.talk_attention_rows_mixed_floats(torch.bfloat16, 2, H, G, d, dv, max_keys)
+    assert (n > 0) == fits
+    args = [t.cuda() for t in (q, tok_pos, tok_seq, slots, kp, vp, table, M)] + [None, torch.zeros(2, H * dv, dtype=torch.bfloat16, device="cuda")]
+    if fits:
+        ops.talk_attention_rows_mixed(*args, H, G, d, dv, d ** -0.5, torch.full((n,), float("nan"), device="cuda"), max_keys, sink=True)
+    else:
+        with pytest.raises(ops.KernelError):
+            ops.talk_attention_rows_mixed(*args, H, G, d, dv, d ** -0.5, torch.zeros(1 << 22, device="cuda"), max_keys, sink=True)
+        ops.talk_attention(*args, H, G, d, dv, d ** -0.5, 0, True, one_row=True)
+    err = (args[-1].cpu().double() - want.double()).abs().max().item()
+    assert err <= 2e-2 * max(1.0, want.double().abs().max().item()), err
+
+
+@GPU
 @pytest.mark.parametrize("H,G,d,dv", [(8, 4, 256, 256), (8, 2, 64, 128), (8, 8, 128, 64), (4, 2, 128, 256), (4, 4, 256, 128)])
 @pytest.mark.parametrize("block,window,sink,cap,turn", [(0, 0, True, 0.0, True), (40, 0, True, 5.0, False), (0, 33, False, 0.0, True)])
 def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, turn):
