@@ -85,6 +85,12 @@ inline int& overlap_launches() {
     return on;
 }
 
+// Kernels that this thread has launched through the library; what a call launched is the difference around it.
+inline int& launches_made() {
+    static thread_local int n = 0;
+    return n;
+}
+
 // Launch with the attribute above, and as thread-block clusters of `cluster` CTAs when cluster > 1.
 template <typename... KArgs, typename... Args>
 inline int launch_kernel_as(bool early, const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
@@ -112,6 +118,7 @@ inline int launch_kernel_as(bool early, const char* what, void (*kernel)(KArgs..
     cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     if (e != cudaSuccess) return fail("%s: launch failed: %s", what, cudaGetErrorString(e));
+    ++launches_made();
     return 0;
 }
 

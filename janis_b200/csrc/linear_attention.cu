@@ -496,6 +496,7 @@ using namespace janis;
 JANIS_EXPORT void janis_mixers_set_overlap(int on) { overlap_launches() = on ? 1 : 0; }
 
 JANIS_EXPORT const char* janis_last_error() { return error_buffer(); }
+JANIS_EXPORT int janis_launches_made() { return launches_made(); }
 
 template <typename T>
 static int gla_scan_launch(const void* rows, const GlaRows& g, const float* decay, const int* seq_slot,

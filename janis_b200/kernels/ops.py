@@ -240,6 +240,13 @@ def _check(lib, rc: int, kernels: int = 1) -> None:
     _launches += kernels
 
 
+def _check_counted(lib, entry, *args) -> None:
+    """A call whose sizes decide how many kernels it launches: the library counts them."""
+    before = lib.janis_launches_made()
+    rc = entry(*args)
+    _check(lib, rc, lib.janis_launches_made() - before)
+
+
 def _t(x: torch.Tensor, name: str, dtype=None, shape=None) -> int:
     """The address of a tensor an entry point is given, after the checks the C side cannot make: on the device,
     contiguous, of an accepted dtype (one, or a tuple), of the wanted shape (None: any extent)."""
@@ -990,7 +997,7 @@ def talk_attention(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table,
     if tok_pos.numel() < T or tok_seq.numel() < T:
         raise KernelError("talk_attention: position tables shorter than the step")
     lib = mixers()
-    _check(lib, lib.janis_talk_attention(
+    _check_counted(lib, lib.janis_talk_attention,
         q_rows.data_ptr(), _DT[q_rows.dtype], q_rows.shape[1], _t(tok_pos, "tok_pos", torch.int32),
         _t(tok_seq, "tok_seq", torch.int32), _t(seq_slot, "seq_slot", torch.int32), kpool.data_ptr(),
         None if values_in_keys else vpool.data_ptr(), page_table.data_ptr(), page_table.shape[1],
@@ -1002,9 +1009,7 @@ def talk_attention(q_rows, tok_pos, tok_seq, seq_slot, kpool, vpool, page_table,
         _t(sink_values, "sink_values", torch.float32, (H,)) if sink_values is not None else None,
         1 if mix_after else 0, 1 if values_in_keys else 0,
         _t(stats, "stats", torch.float32) if stats is not None else None, stats.numel() if stats is not None else 0,
-        int(keep_first), _stream()),
-        kernels=(2 if two_pass else 1) *
-                (2 if (n_chunks > 1 and scratch is not None and q_rows.dtype == torch.bfloat16) else 1))
+        int(keep_first), _stream())
     return out
 
 
@@ -1360,12 +1365,12 @@ def selective_scan(u, u_off: int, dt, dt_off: int, dt_bias, A, a_per_state: bool
             seq_start.data_ptr(), seq_end.data_ptr(), n_seq, state.data_ptr(), out.data_ptr(), C, N, int(ch_per_head),
             int(ch_per_group), _stream()))
         return out
-    _check(lib, lib.janis_selective_scan(
+    _check_counted(lib, lib.janis_selective_scan,
         u.data_ptr(), _DT[dtype], u.shape[1], int(u_off), dt.data_ptr(), dt.shape[1], int(dt_off), dt_bias.data_ptr(),
         A.data_ptr(), 1 if a_per_state else 0, bc.data_ptr(), bc.shape[1], int(b_off), int(c_off), D.data_ptr(),
         z.data_ptr() if z is not None else None, z.shape[1] if z is not None else 0, int(z_off), seq_slot.data_ptr(),
         seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), n_seq, state.data_ptr(), out.data_ptr(),
-        C, N, int(ch_per_head), int(ch_per_group), T, scratch.data_ptr(), scratch.numel(), _stream()), kernels=2)
+        C, N, int(ch_per_head), int(ch_per_group), T, scratch.data_ptr(), scratch.numel(), _stream())
     return out
 
 

@@ -482,6 +482,22 @@ def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, piec
 
 
 @GPU
+def test_a_scan_counts_the_kernels_it_launches():
+    """Step sizes and one scan; in pieces step sizes, two runs and the carry between them."""
+    from janis_b200.kernels import ops
+    T, C, N = 200, 64, 16
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    u, bc, A = torch.ones(T, C, device="cuda"), torch.ones(T, 2 * N, device="cuda"), -torch.ones(C, N, device="cuda")
+    ones, state, out = torch.ones(C, device="cuda"), torch.zeros(1, C, N, device="cuda"), torch.empty(T, C, device="cuda")
+    for room, kernels in ((0, 2), (9, 4)):
+        scratch = torch.empty(ops.selective_scan_scratch_floats(T, C) + room * C * (N + 1), device="cuda")
+        before = ops.launch_count()
+        ops.selective_scan(u, 0, u, 0, ones, A, True, bc, 0, N, ones, None, 0, i32([0]), i32([0]), i32([0]), i32([T]), 1, state, out,
+                           C, N, 1, C, scratch=scratch)
+        assert ops.launch_count() - before == kernels
+
+
+@GPU
 @pytest.mark.parametrize("N", [8, 16])
 def test_scan_in_pieces_of_growing_states(N):
     """Decays above 1 over pieces that would multiply by more than the largest float: a state of zeros stays zeros, a small one
