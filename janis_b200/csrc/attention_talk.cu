@@ -1549,9 +1549,8 @@ JANIS_EXPORT int janis_talk_attention(const void* q_rows, int dtype, int q_row_e
         (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0 && ((uintptr_t)q_rows & 3) == 0) {
         TalkPromptShape ps = {G, d, dv, block, window, sink ? 1 : 0, 0, scale, cap};
         int chunks = 1;
-        if (n_chunks > 1 && max_keys > 0 && partial != nullptr && ((uintptr_t)partial & 7) == 0) {
-            if (partial_floats < (long long)T * n_chunks * H * (dv + 2))
-                return fail("talk_attention: scratch of %lld floats is too small for %d rows in %d chunks", partial_floats, T, n_chunks);
+        if (n_chunks > 1 && max_keys > 0 && partial != nullptr && ((uintptr_t)partial & 7) == 0 &&
+            partial_floats >= (long long)T * n_chunks * H * (dv + 2)) {       // (a prompt's keys need not be cut)
             // (rows of a CTA may begin in different tiles of a block or window: their first row's tiles are what is cut)
             const int tiles = (max_keys + TP_ROWS - 1 + TP_BN - 1) / TP_BN + 1;
             chunks = n_chunks;

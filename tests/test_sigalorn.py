@@ -393,6 +393,25 @@ def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, 
 
 
 @GPU
+def test_a_prompt_of_mixed_heads_runs_without_room_for_chunks():
+    """A prompt's keys are cut over several CTAs where the scratch has room, and left whole where it has none."""
+    from janis_b200.kernels import ops
+    H, G, d, dv, T = 8, 4, 64, 64, 40
+    kp, vp, table, slots = _paged(1, [T], G, d, dv, torch.bfloat16, 3)
+    g = torch.Generator().manual_seed(2)
+    q, M = torch.randn(T, H * d, generator=g).bfloat16(), torch.eye(H)
+    args = [t.cuda() for t in (q, torch.arange(T).int(), torch.zeros(T).int(), slots, kp, vp, table, M)] + [None]
+    outs = []
+    for floats, kernels in ((ops.talk_attention_scratch_floats(T, 3, H, dv), 2), (10, 1), (0, 1)):
+        before = ops.launch_count()
+        outs.append(ops.talk_attention(*args, torch.zeros(T, H * dv, dtype=torch.bfloat16, device="cuda"), H, G, d, dv, d ** -0.5, 0, True,
+                                       n_chunks=3, max_keys=T, scratch=torch.empty(floats, device="cuda") if floats else None))
+        assert ops.launch_count() - before == kernels
+    assert torch.equal(outs[1], outs[2])
+    assert (outs[0].double() - outs[1].double()).abs().max() <= 2e-2 * outs[1].double().abs().max()
+
+
+@GPU
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,G,d,dv,rot,turn", [(4, 2, 32, 16, 16, True), (3, 3, 16, 32, 16, False), (2, 1, 48, 40, 0, True)])
 def test_rotation_and_cache_write_against_their_statement(dtype, H, G, d, dv, rot, turn):
