@@ -432,14 +432,15 @@ rows_mixed_kernel(const T* __restrict__ q_rows, int q_row_elems, const int* __re
             m = fmaxf(m, x);
         }
         m = warp_max(m);
+        const float from = m != -CUDART_INF_F ? m : 0.f;
         for (int jj = lane; jj < n_keys; jj += 32) {
-            const float w = m == -CUDART_INF_F ? 0.f : expf(p_s[(size_t)h * chunk + jj] - m);
+            const float w = expf(p_s[(size_t)h * chunk + jj] - from);
             p_s[(size_t)h * chunk + jj] = w;
             l += w;
         }
         l = warp_sum(l);
         float* prt = part + (((size_t)t * sh.n_chunks + c) * H + h) * 2;
-        if (lane == 0) prt[0] = m, prt[1] = l;
+        if (lane == 0) prt[0] = m == -CUDART_INF_F && l != 0.f ? 0.f : m, prt[1] = l;      // (all NaN: the merge must see them)
     }
     __syncthreads();
     // (the sums as in rows_values_kernel)

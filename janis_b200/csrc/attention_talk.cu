@@ -1159,7 +1159,7 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
                 const float corr = m_mine == m_old ? 1.f : (m_old == -CUDART_INF_F ? 0.f : expf(m_old - m_mine));
 #pragma unroll
                 for (int h = 0; h < H; ++h) {
-                    p[h] = m_new[h] != -CUDART_INF_F ? expf(p[h] - m_new[h]) : 0.f;
+                    p[h] = expf(p[h] - (m_new[h] != -CUDART_INF_F ? m_new[h] : 0.f));      // (a NaN stays one; nothing seen: 0)
                     p_s[(h * TP_ROWS + r) * (TP_BN + 8) + lane] = __float2bfloat16_rn(p[h]);
                 }
                 // the heads' sums over the lanes, each stage halving the heads a lane still carries
@@ -1242,12 +1242,12 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
         float* base = partial + ((size_t)r0 * gridDim.y + blockIdx.y) * H * (dv + 2);
         for (int hr = warp; hr < n_rows * H; hr += 16) {
             const int r = hr / H, h = hr % H;
-            const float m = m_s[h * TP_ROWS + r];
+            const float l = l_s[h * TP_ROWS + r], m = m_s[h * TP_ROWS + r] == -CUDART_INF_F && l != 0.f ? 0.f : m_s[h * TP_ROWS + r];   // (all NaN)
             float* dst = base + ((size_t)r * gridDim.y * H + h) * (dv + 2);
             if (m != -CUDART_INF_F)
                 for (int c = 2 * lane; c < dv; c += 64)
                     *reinterpret_cast<float2*>(dst + c) = *reinterpret_cast<const float2*>(o_s + (h * TP_ROWS + r) * os + c);
-            if (lane == 0) *reinterpret_cast<float2*>(dst + dv) = make_float2(m, l_s[h * TP_ROWS + r]);
+            if (lane == 0) *reinterpret_cast<float2*>(dst + dv) = make_float2(m, l);
         }
         return;
     }

@@ -393,6 +393,42 @@ def test_prompt_attention_of_mixed_heads(H, G, d, dv, block, window, sink, cap, 
 
 
 @GPU
+@pytest.mark.parametrize("H,G,d,dv", [(8, 4, 256, 256), (4, 4, 128, 128)])
+def test_keys_of_nan_reach_every_row_of_mixed_heads_that_sees_them(H, G, d, dv):
+    """A whole tile or chunk of NaN keys at a sequence's beginning makes the rows behind it NaN and not averages of the other
+    keys: in prompts, with the keys cut and whole, and in single rows.  Another sequence of the step stays as it is."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    lens = [200, 50]
+    kp, vp, table, slots = _paged(2, lens, G, d, dv, torch.bfloat16, 3)
+    kp[int(table[int(slots[0]), 0])] = float("nan")
+    tok_pos, tok_seq = torch.cat([torch.arange(n) for n in lens]).int(), torch.repeat_interleave(torch.arange(2), torch.tensor(lens)).int()
+    g = torch.Generator().manual_seed(H)
+    q = torch.randn(sum(lens), H * d, generator=g).bfloat16()
+    M = (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).float()
+
+    def check(rows, got):
+        want = torch.zeros(len(rows), H * dv, dtype=torch.bfloat16)
+        R.talk_attention(q[rows], tok_pos[rows], tok_seq[rows], slots, kp, vp, table, M, None, want, H, G, d, dv, d ** -0.5, 0, False)
+        got = got.cpu()
+        assert want[tok_seq[rows] == 0].isnan().all() and got[tok_seq[rows] == 0].isnan().all()
+        other = tok_seq[rows] == 1
+        assert (got[other].double() - want[other].double()).abs().max() <= 2e-2 * max(1.0, want[other].double().abs().max().item())
+
+    def args(rows):
+        return [t.cuda() for t in (q[rows], tok_pos[rows], tok_seq[rows], slots, kp, vp, table, M)] + [None,
+                torch.zeros(len(rows), H * dv, dtype=torch.bfloat16, device="cuda"), H, G, d, dv, d ** -0.5]
+    all_rows = torch.arange(sum(lens))
+    for chunks in (1, 3):
+        n = ops.talk_attention_scratch_floats(len(all_rows), chunks, H, dv)
+        check(all_rows, ops.talk_attention(*args(all_rows), 0, False, n_chunks=chunks, max_keys=200,
+                                           scratch=torch.full((n,), float("nan"), device="cuda") if n else None))
+    ends = torch.tensor([199, 249])
+    n = ops.talk_attention_rows_mixed_floats(torch.bfloat16, 2, H, G, d, dv, 200)
+    check(ends, ops.talk_attention_rows_mixed(*args(ends), torch.full((n,), float("nan"), device="cuda"), 200))
+
+
+@GPU
 def test_a_prompt_of_mixed_heads_runs_without_room_for_chunks():
     """A prompt's keys are cut over several CTAs where the scratch has room, and left whole where it has none."""
     from janis_b200.kernels import ops
