@@ -66,17 +66,17 @@ constexpr int THREADS = (SOFTMAX_WARPS + 3) * 32;
 constexpr int OCOLS = HD / SPLIT;                     // accumulator columns a softmax thread looks after
 constexpr float RESCALE_STEP = 8.0f;                  // in units of log2: P stays below 2^8
 // The softmax's work per score is what bounds this kernel, most of it on the special-function unit (16 results a
-// cycle and SM, against 128 fused multiply-adds).  Two switches take work off it:
-//   JANIS_PT_TANH_APPROX: the cap's tanh as one tanh.approx (relative error 2^-11, on scores that the product with V
-//     weighs by P rounded to bfloat16, relative error 2^-9) instead of 2^x and 1/x;
+// cycle and SM, against 128 fused multiply-adds).  Two things take work off it:
+//   CAP_APPROX: the cap's tanh as one tanh.approx (relative error 2^-11, on scores that the product with V
+//     weighs by P rounded to bfloat16, relative error 2^-9) instead of 2^x and 1/x.  Sequences that go on have CAP_EXACT, 2^x and
+//     1/x (an error of 2^-23 of the cap), as in the mma.sync kernel that ran them before: on a score near a cap of 50
+//     2^-11 is 0.02 in the exponent;
 //   JANIS_PT_POLY_EX2: every second exponential of the softmax as a cubic on the fused multiply-add pipe (relative
 //     error 9e-5: the integer part goes into the exponent field, the fraction through the polynomial).
 // Measured on a B200 at head size 256 (4 x 4,096 tokens, one launch): both off 425 us, tanh.approx alone 372 us,
 // the cubic alone 444 us: the softmax warps are short of issue slots as much as of special-function results, and
-// the cubic costs seven instructions for the one it saves.  So the first is on and the second stays a switch.
-#ifndef JANIS_PT_TANH_APPROX
-#define JANIS_PT_TANH_APPROX 1
-#endif
+// the cubic costs seven instructions for the one it saves.  So whole prompts take the first and the second stays a switch.
+enum { CAP_NONE = 0, CAP_APPROX = 1, CAP_EXACT = 2 };
 #ifndef JANIS_PT_POLY_EX2
 #define JANIS_PT_POLY_EX2 0
 #endif
@@ -212,7 +212,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 
-template <bool CAPPED>                                // CAPPED: scores go through cap * tanh(s / cap)
+template <int CAP>                                    // unless CAP_NONE, scores go through cap * tanh(s / cap)
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                          const int* __restrict__ seq_first_row, const int* __restrict__ seq_len, int n_seq,
@@ -394,7 +394,7 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const float LOG2E = 1.4426950408889634f;
         // scores in units of log2(e): cap2 tanh(s scale / cap) = cap2 - 2 cap2 / (2^(s k_tanh) + 1), or s scale2
         const float cap2 = cap * LOG2E, scale2 = scale * LOG2E;
-        const float k_tanh = CAPPED ? scale / cap * (JANIS_PT_TANH_APPROX ? 1.0f : 2.0f * LOG2E) : 0.f;
+        const float k_tanh = CAP ? scale / cap * (CAP == CAP_APPROX ? 1.0f : 2.0f * LOG2E) : 0.f;
         float m_ref = -INFINITY, l_run = 0.f;         // reference of the exponentials (log2 units); sum over this thread's keys
         // Two tiles are in flight in every thread: stage one of tile it + 1 (scores out of tensor memory, scale,
         // cap, masks, this thread's maximum told to the row's other threads) runs before stage two of tile it (the
@@ -410,21 +410,19 @@ attn_prefill_tc05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             fence_before();
             warp_arrive(bar(S_EMPTY + b), lane);      // the scores are in registers
             base = m_ref == -INFINITY ? 0.f : m_ref;
-            const float c0 = CAPPED ? cap2 - base : -base, c1 = -2.0f * cap2;
+            const float c0 = CAP ? cap2 - base : -base, c1 = -2.0f * cap2;
             const bool inner = k0 + BN - 1 <= q0 && k0 + BN <= len && k0 >= last_from;
             float mx = -INFINITY;
 #pragma unroll
             for (int j = 0; j < CPT; ++j) {
                 const float s = __uint_as_float(sv[j]);
                 float v;
-                if (CAPPED) {
-#if JANIS_PT_TANH_APPROX
+                if (CAP == CAP_APPROX) {
                     v = fmaf(tanh_approx(s * k_tanh), cap2, -base);
-#else
+                } else if (CAP == CAP_EXACT) {
                     float rc;
                     asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(rc) : "f"(pf::ex2(s * k_tanh) + 1.0f));
                     v = fmaf(rc, c1, c0);              // exact limits: 2^x = inf gives cap2, 2^x = 0 gives -cap2
-#endif
                 } else {
                     v = fmaf(s, scale2, c0);
                 }
@@ -669,7 +667,7 @@ __device__ __forceinline__ bool find_tile_warp(int tile, const int* __restrict__
     return false;
 }
 
-template <bool CAPPED>
+template <int CAP>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
                                const int* __restrict__ seq_first_row, const int* __restrict__ seq_len, int n_seq,
@@ -908,7 +906,7 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const float LOG2E = 1.4426950408889634f;
         const float cap2 = cap * LOG2E, scale2 = scale * LOG2E;
-        const float k_tanh = CAPPED ? scale / cap * (JANIS_PT_TANH_APPROX ? 1.0f : 2.0f * LOG2E) : 0.f;
+        const float k_tanh = CAP ? scale / cap * (CAP == CAP_APPROX ? 1.0f : 2.0f * LOG2E) : 0.f;
         bool ok = true;
         int g = 0, gx = 0;                           // tiles, and exchanges through ROW_X, before this item
         for (int k = 0; ok; ++k) {
@@ -931,21 +929,19 @@ attn_prefill_tc05_items_kernel(const __grid_constant__ CUtensorMap map_q, const 
                 fence_before();
                 warp_arrive(bar(S_EMPTY + b), lane);
                 base = m_ref == -INFINITY ? 0.f : m_ref;
-                const float c0 = CAPPED ? cap2 - base : -base, c1 = -2.0f * cap2;
+                const float c0 = CAP ? cap2 - base : -base, c1 = -2.0f * cap2;
                 const bool inner = k0 + BN - 1 <= q0 && k0 + BN <= len && k0 >= last_from;
                 float mx = -INFINITY;
 #pragma unroll
                 for (int j = 0; j < CPT; ++j) {
                     const float s = __uint_as_float(sv[j]);
                     float v;
-                    if (CAPPED) {
-#if JANIS_PT_TANH_APPROX
+                    if (CAP == CAP_APPROX) {
                         v = fmaf(tanh_approx(s * k_tanh), cap2, -base);
-#else
+                    } else if (CAP == CAP_EXACT) {
                         float rc;
                         asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(rc) : "f"(pf::ex2(s * k_tanh) + 1.0f));
                         v = fmaf(rc, c1, c0);
-#endif
                     } else {
                         v = fmaf(s, scale2, c0);
                     }
@@ -1201,40 +1197,33 @@ int launch_prefill_tc05(const void* q_src, const void* kv_src, int n_tok, const 
         return -1;                                    // no encoder, or operands it refuses: the other kernel runs
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(pt::attn_prefill_tc05_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             pt::SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(pt::attn_prefill_tc05_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     pt::SMEM_BYTES);
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {pt::attn_prefill_tc05_kernel<pt::CAP_NONE>, pt::attn_prefill_tc05_kernel<pt::CAP_APPROX>, pt::attn_prefill_tc05_kernel<pt::CAP_EXACT>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pt::SMEM_BYTES);
+        for (auto kernel : {pt::attn_prefill_tc05_items_kernel<pt::CAP_NONE>, pt::attn_prefill_tc05_items_kernel<pt::CAP_APPROX>,
+                            pt::attn_prefill_tc05_items_kernel<pt::CAP_EXACT>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pt::SMEM_BYTES);
         if (e != cudaSuccess) return fail("attn_prefill_tc05: shared memory of %d bytes refused: %s", pt::SMEM_BYTES,
                                           cudaGetErrorString(e));
         configured = true;
     }
+    const int how_capped = cap > 0.f ? (seq_start ? pt::CAP_EXACT : pt::CAP_APPROX) : pt::CAP_NONE;
     const bool many = (long long)n_tiles_bound * parts * nq >= (long long)tc05_sm_count();
     if (g_tc05_items == 2 || (g_tc05_items == 1 && many)) {
-        static bool items_configured = false;
-        if (!items_configured) {
-            cudaError_t e = cudaFuncSetAttribute(pt::attn_prefill_tc05_items_kernel<true>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, pt::SMEM_BYTES);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(pt::attn_prefill_tc05_items_kernel<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, pt::SMEM_BYTES);
-            if (e != cudaSuccess) return fail("attn_prefill_tc05: shared memory of %d bytes refused: %s", pt::SMEM_BYTES,
-                                              cudaGetErrorString(e));
-            items_configured = true;
-        }
         static int next_slot = 0;
         const int slot = next_slot;
         next_slot = (next_slot + 1) % pt::SCHED_SLOTS;
         const int n_places = n_tiles_bound * parts;
         const long long total = (long long)n_places * nq;
         const int ctas = (int)std::min<long long>(total, tc05_sm_count());
-        auto items = cap > 0.f ? pt::attn_prefill_tc05_items_kernel<true> : pt::attn_prefill_tc05_items_kernel<false>;
+        auto items = how_capped == pt::CAP_NONE ? pt::attn_prefill_tc05_items_kernel<pt::CAP_NONE>
+                     : how_capped == pt::CAP_APPROX ? pt::attn_prefill_tc05_items_kernel<pt::CAP_APPROX> : pt::attn_prefill_tc05_items_kernel<pt::CAP_EXACT>;
         return launch_kernel("attn_prefill_tc05", items, dim3(ctas), dim3(pt::THREADS), pt::SMEM_BYTES, stream, 1, mq, mkv,
                              seq_first_row, seq_len, n_seq, (bf16*)out, nq, nkv, kv_k_head0, scale, cap, window, parts,
                              piece, partial, n_places, slot, sinks, seq_start);
     }
-    auto kernel = cap > 0.f ? pt::attn_prefill_tc05_kernel<true> : pt::attn_prefill_tc05_kernel<false>;
+    auto kernel = how_capped == pt::CAP_NONE ? pt::attn_prefill_tc05_kernel<pt::CAP_NONE>
+                  : how_capped == pt::CAP_APPROX ? pt::attn_prefill_tc05_kernel<pt::CAP_APPROX> : pt::attn_prefill_tc05_kernel<pt::CAP_EXACT>;
     return launch_kernel("attn_prefill_tc05", kernel, dim3(nq, n_tiles_bound * parts), dim3(pt::THREADS), pt::SMEM_BYTES,
                          stream, 1, mq, mkv, seq_first_row, seq_len, n_seq, (bf16*)out, nq, nkv, kv_k_head0, scale, cap,
                          window, parts, piece, partial, sinks, seq_start);

@@ -676,6 +676,42 @@ def test_continued_prompt_through_gathered_rows(hd, nq, nkv, window, ring, cap, 
         ops().attn_set_prefill_kernel(hd, 1)
 
 
+@pytest.mark.parametrize("form", [2, 3])
+def test_continued_prompts_keep_the_caps_bits(form):
+    """Scores near a cap of 50, where an error of 2^-11 in the cap's tanh would move a weight by 2 %: two keys share a row's weight, with
+    values 1 and -1, so that the result tells the difference of their capped scores."""
+    hd, T, cap = 64, 128, 50.0
+    g = torch.Generator().manual_seed(9)
+    d = dev()
+    # every row sees its sequence's first two positions alone with scores that count: the others' keys point away
+    k = torch.zeros(T + 2, 1, hd)
+    k[:2, 0, 0], k[2:, 0, 0] = 1.0, -4.0
+    k[1, 0, 1] = 1.0
+    q = torch.zeros(T, 1, hd)
+    q[:, 0, 0] = 40.0 + 60.0 * torch.rand(T, generator=g)          # scores 40 .. 100, capped to 33 .. 48
+    q[:, 0, 1] = 4.0 * torch.rand(T, generator=g) - 2.0
+    v = torch.zeros(T + 2, 1, hd)
+    v[0], v[1] = 1.0, -1.0
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    s = torch.einsum("thd,jhd->tj", q.double(), k.double())[:, :2]
+    want = torch.softmax(cap * torch.tanh(s / cap), 1) @ torch.tensor([1.0, -1.0], dtype=torch.float64)
+    qkv = torch.cat([q, k[2:], v[2:]], 1).contiguous().to(d)
+    kp, vp = torch.zeros(1, 1, R.PAGE, hd, dtype=torch.bfloat16, device=d), torch.zeros(1, 1, R.PAGE, hd, dtype=torch.bfloat16, device=d)
+    kp[0, 0, :2], vp[0, 0, :2] = k[:2, 0].to(d), v[:2, 0].to(d)
+    i32 = lambda x: torch.tensor([x], dtype=torch.int32, device=d)
+    ops().attn_set_prefill_kernel(hd, form)
+    try:
+        out = torch.empty(T, hd, dtype=torch.bfloat16, device=d)
+        ops().attn_prefill(qkv, None, None, i32(0), out, 1, 1, hd, 1.0, cap, 0, seq_len=i32(T + 2), host_lens=[T], seq_start=i32(2),
+                           seq_slot=i32(0), kpool=kp, vpool=vp, page_table=torch.zeros(1, 1, dtype=torch.int32, device=d),
+                           gathered=torch.empty((T + 2) * 2 * hd, dtype=torch.bfloat16, device=d), all_rows=T + 2, max_total=T + 2)
+    finally:
+        ops().attn_set_prefill_kernel(hd, 1)
+    # weights and results rounded to bfloat16: 2^-9 of 1 each, and of the weights' sum
+    err = (out.double().cpu().mean(1) - want).abs().max().item()
+    assert err <= 3 * 2.0 ** -9, err
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attn_prefill_reads_another_layers_keys(dtype):
     nq, nkv, hd = 4, 2, 32
