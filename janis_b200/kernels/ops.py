@@ -684,9 +684,11 @@ GATHER_BYTES = 512 << 20       # the most that a step's keys and values may take
 
 def attn_gathered_elems(all_rows: int, nkv: int, hd: int, dtype=torch.bfloat16) -> int:
     """Elements of the room that a step of continued sequences with all_rows positions wants as `gathered` (0: none; the step
-    runs on the kernel that reads the pages)."""
-    n = (all_rows * 2 * nkv * hd + (1 << 22) - 1) >> 22 << 22      # (in steps of 8 MB: the rows grow with every piece)
-    return n if all_rows and dtype == torch.bfloat16 and hd % 64 == 0 and hd <= 256 and 2 * n <= GATHER_BYTES else 0
+    runs on the kernel that reads the pages).  The next power of two from 8 MB on: the rows grow with every piece of a prompt,
+    and a workspace that grew with them would leave the sizes it had behind in the allocator."""
+    if not all_rows or dtype != torch.bfloat16 or hd % 64 or hd > 256 or 4 * all_rows * nkv * hd > GATHER_BYTES:
+        return 0
+    return 1 << max(22, (2 * all_rows * nkv * hd - 1).bit_length())
 
 
 def _gathered_args(name, gathered, all_rows, max_total, seq_start, nkv, hd):

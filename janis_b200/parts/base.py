@@ -101,6 +101,10 @@ class Workspace:
             if cur is not None and name in self._in_graph:
                 self._retired.append(cur)         # keep its memory valid for the graphs that recorded it
                 self._in_graph.discard(name)
+            # the old one goes before the new one comes (work that still reads it lies ahead on the same stream)
+            cur = last = None
+            self._bufs.pop(name, None)
+            self._views.pop(name, None)
             # zeros, not whatever the allocator hands out: a kernel that reads a row nobody wrote (a tile that runs
             # past the step's rows) must find numbers there
             cur = torch.zeros(max(n, 1), dtype=dtype, device=self.device)

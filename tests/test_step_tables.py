@@ -56,3 +56,37 @@ def test_tables_of_a_step_that_fills_its_shape():
     assert (host[2 * 512:2 * 512 + 16] == 0).all() and not host[2 * 512 + 16:3 * 512].any()
     o = 3 * 512
     assert host[o + 2 * 32:o + 2 * 32 + 2].tolist() == [16, 0]       # no padding token: the padding sequence is empty
+
+
+def test_the_room_for_continued_prompts_takes_few_sizes():
+    """A prompt of 65,536 tokens in pieces of 500 asks for more room at every piece; what it gets changes at few of them, never
+    holds less than asked for or more than twice that, and stays within the bound."""
+    import torch
+    from janis_b200.kernels import ops
+    sizes = set()
+    for rows in range(500, 65537, 500):
+        n = ops.attn_gathered_elems(rows, 8, 256)
+        want = rows * 2 * 8 * 256
+        if 2 * want > ops.GATHER_BYTES:
+            assert n == 0
+            continue
+        assert want <= n <= max(2 * want, 1 << 22) and 2 * n <= ops.GATHER_BYTES
+        sizes.add(n)
+    assert len(sizes) <= 7
+    assert ops.attn_gathered_elems(100, 8, 256, torch.float32) == ops.attn_gathered_elems(100, 8, 80) == ops.attn_gathered_elems(0, 8, 256) == 0
+
+
+def test_a_workspace_buffer_that_grows_lets_its_old_memory_go_first():
+    import weakref
+    import torch
+    from janis_b200.parts.base import Workspace
+    ws = Workspace("cpu")
+    old = weakref.ref(ws.buf("x", (10,), torch.float32).untyped_storage())
+    seen = []
+    zeros = torch.zeros
+    try:
+        torch.zeros = lambda *a, **k: seen.append(old() is None) or zeros(*a, **k)
+        assert ws.buf("x", (1000,), torch.float32).shape == (1000,)
+    finally:
+        torch.zeros = zeros
+    assert seen == [True] and ws.buf("x", (10,), torch.float32).shape == (10,)
