@@ -324,7 +324,7 @@ using namespace janis;
 
 // Floats of scratch for a step of n_tok tokens in n_seq sequences; 0 where the chunked form does not take the sizes.
 JANIS_EXPORT long long janis_gla_chunks_floats(int n_tok, int n_seq, int H, int d, int dv) {
-    if (n_tok <= 0 || n_seq <= 0 || H <= 0 || !(d == 64 || d == 128 || d == 256) || dv <= 0 || dv % GC_COLS) return 0;
+    if (n_tok <= 0 || n_seq <= 0 || H <= 0 || H > 65535 || !(d == 64 || d == 128 || d == 256) || dv <= 0 || dv % GC_COLS) return 0;
     return 3LL * n_tok * H * d + 24LL * n_tok * H + ((long long)n_tok / GQ + n_seq) * H * d;
 }
 
@@ -339,7 +339,6 @@ JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, in
     if (!(tau > 0.f)) return fail("gla_chunks: tau must be positive");
     if (row_elems % 8 || v_off % 8 || (((uintptr_t)rows | (uintptr_t)scratch) & 15) || (((uintptr_t)state | (uintptr_t)o_out) & 7))
         return fail("gla_chunks: rows of %d elements, values at %d: not in whole pieces of 16 bytes", row_elems, v_off);
-    if (H > 65535) return fail("gla_chunks: too many heads (%d)", H);
     GlaChunkShape g;
     g.row_elems = row_elems; g.q_off = q_off; g.k_off = k_off; g.v_off = v_off; g.H = H; g.d = d; g.dv = dv; g.n_tok = n_tok;
     g.q_scale = q_scale; g.inv_tau = 1.0f / tau;

@@ -1125,9 +1125,10 @@ def gla_chunks_floats(dtype, T: int, n_seq: int, H: int, d: int, dv: int) -> int
     return n if n <= GLA_CHUNK_FLOATS else 0
 
 
-def _gla_chunked(rows, v_off, T, n_seq, H, d, dv, chunks) -> bool:
+def _gla_chunked(rows, v_off, state, o_out, T, n_seq, H, d, dv, chunks) -> bool:
     need = gla_chunks_floats(rows.dtype, T, n_seq, H, d, dv)
-    return 0 < need <= chunks.numel() and rows.shape[1] % 8 == 0 and v_off % 8 == 0 and rows.data_ptr() % 16 == 0 and chunks.data_ptr() % 16 == 0
+    return (0 < need <= chunks.numel() and rows.shape[1] % 8 == 0 and v_off % 8 == 0 and (rows.data_ptr() | chunks.data_ptr()) % 16 == 0
+            and (state.data_ptr() | o_out.data_ptr()) % 8 == 0)
 
 
 def _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv) -> None:
@@ -1155,7 +1156,7 @@ def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_
     if chunks is not None:
         _t(chunks, "chunks", torch.float32)
         decay = None
-        if _gla_chunked(rows, v_off, T, n_seq, H, d, dv, chunks):
+        if _gla_chunked(rows, v_off, state, o_out, T, n_seq, H, d, dv, chunks):
             _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv)
             lib = mixers()
             _check(lib, lib.janis_gla_chunks(rows.data_ptr(), width, q_off, k_off, v_off, z.data_ptr(), z_bias.data_ptr(), T, seq_slot.data_ptr(),

@@ -520,6 +520,28 @@ def test_recurrence_in_chunks_against_its_statement(H, d, dv, tau, order):
 
 
 @GPU
+def test_recurrence_of_states_off_the_chunks_alignment():
+    """States or results that start between two 8-byte borders are not for the kernels that run in chunks; such a call runs
+    token by token, as it does without scratch."""
+    from janis_b200.kernels import ops
+    H, d, dv, T = 1, 64, 32, 200
+    g = torch.Generator().manual_seed(1)
+    rows, z, b = (torch.randn(*n, generator=g).bfloat16().cuda() for n in ((T, 2 * H * d + H * dv), (T, H * d), (H * d,)))
+    i32 = lambda v: torch.tensor([v], dtype=torch.int32, device="cuda")
+    n = ops.gla_chunks_floats(torch.bfloat16, T, 1, H, d, dv)
+    assert n > 0
+    outs = []
+    for off_state, off_out, chunks in ((1, 0, True), (0, 1, True), (0, 0, False)):
+        state = torch.zeros(1 + H * dv * d, device="cuda")[off_state:off_state + H * dv * d].view(1, H, dv, d)
+        out = torch.zeros(1 + T * H * dv, device="cuda")[off_out:off_out + T * H * dv].view(T, H * dv)
+        ops.gla_scan(rows, 0, H * d, 2 * H * d, z, b, i32(0), i32(0), i32(0), i32(T), state, out, 1, H, d, dv, d ** -0.5, 8.0,
+                     chunks=torch.empty(n, device="cuda") if chunks else None)
+        outs.append((out.clone(), state.clone()))
+    for out, state in outs[:2]:
+        assert torch.equal(out, outs[2][0]) and torch.equal(state, outs[2][1])
+
+
+@GPU
 @pytest.mark.parametrize("bad", ["q", "k", "v", "decay"])
 def test_recurrence_in_chunks_of_inputs_beyond_numbers(bad):
     """An infinity or a NaN at one token reaches that token's results and later ones, never an earlier token of its chunk."""
