@@ -14,6 +14,7 @@
 // cache, [slots, C, N] floats per line: a step loads it, runs its tokens in order and writes it back; sequences
 // without a slot (padding) start from zero and store nothing.  (The duality form of a bfloat16 prompt runs in chunks where its
 // sizes allow it: duality_scan.cu.)
+#include <cstring>
 #include <type_traits>
 
 #include "common.cuh"
@@ -31,9 +32,9 @@ __device__ __forceinline__ float decay_minus_one(float x) { return expm1f(x); }
 
 // The same for x <= 0 without a branch, for the selective scan's prompts, which form one per state and token and do little else.
 // x = j ln 2 + f with a whole j (Cody and Waite's reduction: ln 2 in two floats), e^f - 1 is its Taylor series up to f^8 (the
-// next term is 6e-10 of the sum at |f| = ln 2 / 2), and 2^j (e^f - 1) + (2^j - 1) has one rounding: within 0.87 units in the
-// last place of exp(x) - 1, as compared with 64 bits over all negative floats' exponents.
-__device__ __forceinline__ float shrink_minus_one(float x) {
+// next term is 6e-10 of the sum at |f| = ln 2 / 2), and 2^j (e^f - 1) + (2^j - 1) has one rounding: within 0.881 units in the
+// last place of exp(x) - 1, as compared with 64 bits at every negative float.
+__host__ __device__ __forceinline__ float shrink_minus_one(float x) {
     x = x < -30.f ? -30.f : x;                            // (-1 there already; a NaN stays one)
     const float t = fmaf(x, 1.44269504f, 12582912.f), j = t - 12582912.f;      // x / ln 2 rounded, and in the low bits of t
     const float f = fmaf(j, -1.42860682e-6f, fmaf(j, -0.693145751953125f, x));
@@ -43,7 +44,16 @@ __device__ __forceinline__ float shrink_minus_one(float x) {
     p = fmaf(p, f, 1.f / 24.f);
     p = fmaf(p, f, 1.f / 6.f);
     p = fmaf(p, f, 0.5f);
-    const float q = fmaf(f * f, p, f), s = __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
+#ifdef __CUDA_ARCH__
+    const float s = __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
+#else
+    uint32_t bits;
+    float s;
+    memcpy(&bits, &t, 4);
+    bits = (bits << 23) + 0x3f800000u;
+    memcpy(&s, &bits, 4);
+#endif
+    const float q = fmaf(f * f, p, f);
     return fmaf(s, q, s - 1.f);
 }
 __device__ __forceinline__ float decayed(float S, float grow, float input) { return S + fmaf(S, grow, input); }
@@ -873,6 +883,11 @@ static int scan_pieces_launch(const void* u, const void* bc, const void* z, cons
 }
 
 JANIS_EXPORT long long janis_selective_scan_scratch(int n_tok, int heads) { return 2LL * n_tok * heads; }
+
+// shrink_minus_one of n numbers on the host (the same arithmetic; for tests)
+JANIS_EXPORT void janis_shrink_minus_one(const float* x, float* y, int n) {
+    for (int i = 0; i < n; ++i) y[i] = shrink_minus_one(x[i]);
+}
 
 constexpr int SCAN_PIECES_FROM = 128;  // tokens of a step
 

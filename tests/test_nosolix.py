@@ -481,6 +481,34 @@ def test_scan_in_pieces_against_its_statement(dtype, C, N, cph, cpg, gated, piec
     assert torch.equal(got_state[[2, 5]].cpu(), state[[2, 5]]), "a slot that is not in the step keeps its state"
 
 
+def test_the_scans_exponential_keeps_its_bound():
+    """exp(x) - 1 for x <= 0 as the selective scan's prompts form it (its arithmetic run on the host) against 64 bits: every exponent, both
+    sides of every border of its reduction and of its clamp, numbers near 0 and subnormal ones.  0.8805 units in the last place at
+    -0.34739450 is the largest error there is (all negative floats were compared)."""
+    import ctypes
+    import numpy as np
+    from janis_b200.csrc.build import mixers_library
+    form = mixers_library().janis_shrink_minus_one
+    form.argtypes, form.restype = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int], None
+    rng = np.random.default_rng(1)
+    exponents = np.repeat(np.arange(1, 255, dtype=np.uint32), 4000)
+    x = (0x80000000 | (exponents << 23) | rng.integers(0, 1 << 23, exponents.size, dtype=np.uint32)).astype(np.uint32).view(np.float32)
+    near = np.concatenate([-(np.arange(0, 46) + 0.5) * np.log(2.0), [-30.0, -0.34739450, -1.0, -87.3, -104.0]]).astype(np.float32)
+    near = (near.view(np.uint32)[:, None] + np.arange(-50, 51)).astype(np.uint32).view(np.float32).ravel()
+    subnormal = (0x80000000 + rng.integers(0, 1 << 23, 5000)).astype(np.uint32).view(np.float32)
+    dense = -rng.uniform(0.0, 32.0, 2_000_000).astype(np.float32)
+    x = np.concatenate([x, near, subnormal, dense, np.array([0.0, -0.0, -np.inf], np.float32)])
+    y = np.empty_like(x)
+    form(x.ctypes.data, y.ctypes.data, x.size)
+    want = np.expm1(x.astype(np.float64))
+    ulp = np.maximum(2.0 ** (np.frexp(want)[1] - 24.0), 2.0 ** -149)
+    err = np.abs(y - want) / ulp
+    assert err.max() <= 0.881, (x[err.argmax()], err.max())
+    nan = np.array([np.nan], np.float32)
+    form(nan.ctypes.data, nan.ctypes.data, 1)
+    assert np.isnan(nan[0])
+
+
 @GPU
 def test_a_scan_counts_the_kernels_it_launches():
     """Step sizes and one scan; in pieces step sizes, two runs and the carry between them."""
