@@ -504,22 +504,12 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
 __device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm_x2_trans(uint32_t (&r)[2], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
 }
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
 constexpr int TALK_MMA_WARPS = 16, TALK_MMA_THREADS = TALK_MMA_WARPS * 32;
 
 struct TalkMmaShape {
@@ -692,13 +682,13 @@ talk_attention_mma_kernel(const bf16* __restrict__ q_rows, int q_row_elems, cons
                         const uint32_t b_step = (uint32_t)(8 * L.kvs * 2);
                         for (int kk = 0; kk < d / 16; ++kk) {
                             uint32_t af[4];
-                            ldsm_x4(af, a_base + kk * 32);
+                            ldmatrix4(af, a_base + kk * 32);
 #pragma unroll
                             for (int t = 0; t < 4; ++t)
                                 if (t < n_here) {
                                     uint32_t bfr[2];
                                     ldsm_x2(bfr, b_base + t * b_step + kk * 32);
-                                    mma_bf16(acc[t], af, bfr);
+                                    mma_16816(acc[t], af, bfr[0], bfr[1]);
                                 }
                         }
                         const int r = lane >> 2;
@@ -833,13 +823,13 @@ talk_attention_mma_kernel(const bf16* __restrict__ q_rows, int q_row_elems, cons
                         const uint32_t b_base = smem_u32(kv_s + ((size_t)kvh * BN + (lane & 15)) * L.kvs + nt0 * 8);
                         for (int kk = 0; kk < BN / 16; ++kk) {
                             uint32_t af[4];
-                            ldsm_x4(af, a_base + kk * 32);
+                            ldmatrix4(af, a_base + kk * 32);
 #pragma unroll
                             for (int t = 0; t < 4; ++t)
                                 if (t < n_here) {
                                     uint32_t bfr[2];
                                     ldsm_x2_trans(bfr, b_base + (uint32_t)(kk * 16 * L.kvs * 2) + t * 16);
-                                    mma_bf16(acc[t], af, bfr);
+                                    mma_16816(acc[t], af, bfr[0], bfr[1]);
                                 }
                         }
 #pragma unroll
@@ -940,11 +930,6 @@ __host__ __device__ inline size_t talk_prompt_tiles_bytes(int H, int G, int d, i
 __host__ __device__ inline size_t talk_prompt_bytes(int H, int G, int d, int dv) {
     return talk_prompt_tiles_bytes(H, G, d, dv) + (size_t)32 / H * H * TP_ROWS * TP_BN * 4 + (size_t)H * TP_ROWS * (TP_BN + 8) * 2 +
            (size_t)3 * H * TP_ROWS * 4 + (size_t)H * H * 4 + 3 * TP_ROWS * 4;
-}
-
-__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
 __device__ __forceinline__ float warp_max_redux(float v) {
@@ -1093,13 +1078,12 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
 #pragma unroll
                     for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
                         uint32_t bq[4];
-                        ldsm_x4(bq, k_a + (((e ? kv1 : kv0) + 16 * n + lr + (lm >> 1) * 8) * ldk + (part * ks + k) * 16 + (lm & 1) * 8) * 2);
+                        ldmatrix4(bq, k_a + (((e ? kv1 : kv0) + 16 * n + lr + (lm >> 1) * 8) * ldk + (part * ks + k) * 16 + (lm & 1) * 8) * 2);
 #pragma unroll
                         for (int f = 0; f < 2; ++f) {
                             if (!SHARED_KV && f != e) continue;
-                            const uint32_t b0[2] = {bq[0], bq[1]}, b1[2] = {bq[2], bq[3]};
-                            mma_bf16(acc[f][0], qa[f][k], b0);
-                            mma_bf16(acc[f][1], qa[f][k], b1);
+                            mma_16816(acc[f][0], qa[f][k], bq[0], bq[1]);
+                            mma_16816(acc[f][1], qa[f][k], bq[2], bq[3]);
                         }
                     }
                 }
@@ -1198,7 +1182,7 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
                     }
 #pragma unroll
                     for (int k = 0; k < 2; ++k)
-                        ldsm_x4(pa[e][k], p_a + (((2 * pair + e) * TP_ROWS + (lane & 15)) * (TP_BN + 8) + 16 * k + (lane >> 4) * 8) * 2);
+                        ldmatrix4(pa[e][k], p_a + (((2 * pair + e) * TP_ROWS + (lane & 15)) * (TP_BN + 8) + 16 * k + (lane >> 4) * 8) * 2);
                 }
 #pragma unroll
                 for (int n = 0; n < NT / 2; ++n) {
@@ -1208,13 +1192,12 @@ talk_prompt_kernel(const bf16* __restrict__ q_rows, int q_row_elems, const int* 
 #pragma unroll
                         for (int e = 0; e < (SHARED_KV ? 1 : 2); ++e) {
                             uint32_t bv[4];
-                            ldsm_x4_trans(bv, v_a + (((e ? kv1 : kv0) + 16 * k + lr + (lm & 1) * 8) * ldv + (part * nt2 + n) * 16 + (lm >> 1) * 8) * 2);
+                            ldmatrix4_trans(bv, v_a + (((e ? kv1 : kv0) + 16 * k + lr + (lm & 1) * 8) * ldv + (part * nt2 + n) * 16 + (lm >> 1) * 8) * 2);
 #pragma unroll
                             for (int f = 0; f < 2; ++f) {
                                 if (!SHARED_KV && f != e) continue;
-                                const uint32_t b0[2] = {bv[0], bv[1]}, b1[2] = {bv[2], bv[3]};
-                                mma_bf16(o[f][2 * n], pa[f][k], b0);
-                                mma_bf16(o[f][2 * n + 1], pa[f][k], b1);
+                                mma_16816(o[f][2 * n], pa[f][k], bv[0], bv[1]);
+                                mma_16816(o[f][2 * n + 1], pa[f][k], bv[2], bv[3]);
                             }
                         }
                 }
