@@ -80,7 +80,8 @@ def decode_geometry(ctx: StepContext, sm_count: int, head_dim: int, n_kv_heads: 
 def gathered_room(ctx: StepContext, n_kv_heads: int, head_dim: int) -> dict:
     """The room in which a step that continues sequences brings its keys and values together, as arguments of the prompt
     attention (nothing where the kernels have no use for it)."""
-    elems = getattr(ctx.rt.ops, "attn_gathered_elems", lambda *a: 0)(ctx.all_rows, n_kv_heads, head_dim, ctx.rt.dtype)
+    elems = getattr(ctx.rt.ops, "attn_gathered_elems", lambda *a: 0)(ctx.all_rows, n_kv_heads, head_dim, ctx.rt.dtype, ctx.len_bound,
+                                                                  max(ctx.step_lens or (0,)))
     return dict(gathered=ctx.ws.buf("attn.gathered", (elems,), ctx.rt.dtype), all_rows=ctx.all_rows, max_total=ctx.len_bound) if elems else {}
 
 

@@ -76,6 +76,18 @@ def test_the_room_for_continued_prompts_takes_few_sizes():
     assert ops.attn_gathered_elems(100, 8, 256, torch.float32) == ops.attn_gathered_elems(100, 8, 80) == ops.attn_gathered_elems(0, 8, 256) == 0
 
 
+def test_short_continuations_read_the_pages():
+    """Gathering is for steps whose attention would make the device wait: long sequences, many of them, or many new tokens."""
+    from janis_b200.kernels import ops
+    import torch
+    gathers = lambda ends, new: ops.attn_gathered_elems(sum(ends), 4, 256, torch.bfloat16, max(ends), max(new)) > 0
+    for ends, new in (([1502], [2]), ([702] * 3, [2] * 3), ([400], [200]), ([251] * 8, [1] * 8), ([511], [300])):
+        assert not gathers(ends, new), ends
+    for ends, new in (([2502], [2]), ([900], [200]), ([512], [64]), ([501] * 30, [1] * 30), ([101] * 63, [1] * 63), ([2048], [2])):
+        assert gathers(ends, new), ends
+    assert ops.attn_gathered_elems(100, 4, 256) > 0          # (lengths unknown)
+
+
 def test_a_workspace_buffer_that_grows_lets_its_old_memory_go_first():
     import weakref
     import torch
