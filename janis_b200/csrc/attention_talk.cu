@@ -1524,10 +1524,13 @@ JANIS_EXPORT int janis_talk_attention(const void* q_rows, int dtype, int q_row_e
     if (two_pass && (stats == nullptr || stats_floats < (long long)T * 2 * H))
         return fail("talk_attention: heads mixed after the softmax need %lld floats for the rows' maxima and denominators", (long long)T * 2 * H);
     if (v_in_keys) vpool = kpool;
-    // Prompts of 4 or 8 heads mixed before the softmax: 8 heads of 256 over 4, one prompt of 2,048 tokens 248 us a layer against
-    // 743 in the kernel below, 1,024 tokens 87 against 382, 300 tokens 55 against 130, eight of 512 186 against 471, 16 tokens 32 = 32.  The kernel below takes the
-    // other sizes, decode steps and what this one leaves out.
-    if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && talk != nullptr && !mix_after && !one_row && !v_in_keys &&
+    // Prompts of 4 or 8 heads mixed before the softmax: 8 heads of 256 over 4, one prompt of 2,048 tokens 243 us a layer against
+    // 743 in the kernel below, 1,024 tokens 85 against 381, 300 tokens 53 against 130, eight of 512 181 against 471, 48 tokens 33
+    // against 36.  Where no row sees more than one tile of keys there is nothing to win by keeping queries and sums: 16 tokens 28
+    // against 25, 32 tokens 28 against 25, sixteen of 16 28 against 25 (but 8 tokens, one block of rows there, 19 against 25).  The
+    // kernel below takes those, the other sizes, decode steps and what this one leaves out.
+    const bool one_tile = max_keys > 0 && max_keys <= TP_BN && T > 8;
+    if (dtype == JANIS_BF16 && talk_kernel_choice == 1 && !one_tile && talk != nullptr && !mix_after && !one_row && !v_in_keys &&
         keep_first == 0 && q_row_elems % 2 == 0 && talk_prompt_takes(H, G, d, dv) &&
         (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0 && ((uintptr_t)q_rows & 3) == 0) {
         TalkPromptShape ps = {G, d, dv, block, window, sink ? 1 : 0, 0, scale, cap};

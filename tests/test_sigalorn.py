@@ -429,6 +429,24 @@ def test_keys_of_nan_reach_every_row_of_mixed_heads_that_sees_them(H, G, d, dv):
 
 
 @GPU
+@pytest.mark.parametrize("T", [8, 9, 32, 33])
+def test_prompts_of_mixed_heads_about_one_tile_of_keys(T):
+    """Both sides of the sizes at which another kernel takes a prompt of 8 mixed heads."""
+    from janis_b200.kernels import ops
+    from tests import kernel_refs as R
+    H, G, d, dv = 8, 4, 64, 64
+    kp, vp, table, slots = _paged(1, [T], G, d, dv, torch.bfloat16, 3)
+    g = torch.Generator().manual_seed(T)
+    q, M = torch.randn(T, H * d, generator=g).bfloat16(), (torch.eye(H) + 0.3 * torch.randn(H, H, generator=g)).float()
+    tables = [torch.arange(T).int(), torch.zeros(T).int(), slots, kp, vp, table, M]
+    want = torch.zeros(T, H * dv, dtype=torch.bfloat16)
+    R.talk_attention(q, *tables, None, want, H, G, d, dv, d ** -0.5, 0, True)
+    got = ops.talk_attention(q.cuda(), *[t.cuda() for t in tables], None, torch.zeros(T, H * dv, dtype=torch.bfloat16, device="cuda"),
+                             H, G, d, dv, d ** -0.5, 0, True, max_keys=T)
+    assert (got.cpu().double() - want.double()).abs().max() <= 2e-2 * max(1.0, want.double().abs().max().item())
+
+
+@GPU
 def test_a_prompt_of_mixed_heads_runs_without_room_for_chunks():
     """A prompt's keys are cut over several CTAs where the scratch has room, and left whole where it has none."""
     from janis_b200.kernels import ops
