@@ -37,7 +37,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompil
 CORE_SOURCES = ["elementwise.cu", "gemm_f32.cu", "gemv_bf16.cu", "gemm_tc05.cu", "sampling.cu"]
 ATTENTION_SOURCES = ["attention.cu", "attention_prefill_mma.cu", "attention_prefill_tc05.cu", "attention_no_alloc.cu"]
 MIXER_SOURCES = ["attention_talk.cu", "attention_rows.cu", "attention_prep.cu", "linear_attention.cu", "gla_chunks.cu", "delta_rule.cu", "state_space.cu", "duality_scan.cu", "gated_recurrence.cu", "branch_ops.cu", "hyper_streams.cu"]
-HEADERS = ["common.cuh", "attention_no_alloc.h", "attention_prefill_tiles.cuh", "mma_bf16.cuh"]
+HEADERS = ["common.cuh", "attention_no_alloc.h", "attention_prefill_tiles.cuh", "mma_bf16.cuh", "tcgen05.cuh"]
 
 
 class BuildError(RuntimeError):

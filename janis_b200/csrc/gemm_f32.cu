@@ -1,155 +1,417 @@
-// out[M, N] = x[M, K] * W[N, K]^T in true 32-bit: float operands, fused
-// multiply-adds on the CUDA cores, no tensor-core mode of any kind.  Each output
-// element is accumulated by one thread, the even and the odd k each in ascending
-// order and the two sums added at the end, so its value
-// depends on its own row of x and row of W only: not on M, not on the tiling of
-// other rows.  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
+// out[M, N] = x[M, K] * W[N, K]^T of float operands at float precision, on the tensor cores.
 //
-// The multiply-adds bound it (74 TFLOP/s of them), so everything else has to stay out of their issue slots.
-// `fma.rn.f32x2` multiplies the pairs (k, k + 1) of a row of x and a row of W as they lie in memory, so nothing is
-// transposed or duplicated: tiles of 16 k come by `cp.async` into a ring of shared memory and 16-byte reads take
-// four k of a row.  A CTA owns 64 x 64 outputs, a thread 8 rows of them and TN = 8 or 4 columns.
-// 683 x 18432 outputs over 2304 k: 1.32 ms, 44 TFLOP/s (1.92 ms with 4 x 4 outputs a thread, scalar multiply-adds and
-// tiles stored transposed); 683 x 2304 over 9216: 0.84 ms against 1.09.  The error against 64 bits is 6.1e-7 of the
-// result against 8.6e-7, as two sums of half the length round less.
+// A float is the sum of three bfloat16 numbers to its last bit (hi, mid, lo: 8 bits each of 24), products of bfloat16
+// numbers are exact in float, and the tensor cores add them up in float: x w = (xh + xm + xl)(wh + wm + wl), of which
+// xm wl, xl wm and xl wl (2^-25 of the product and less) are left out.  Where a block of W holds nothing but bfloat16 numbers
+// (a bfloat16 checkpoint run in 32 bits) wm and wl are zero and three products are left; the kernel looks at every block it
+// splits, so nothing is remembered about a matrix.
+//
+// The tensor cores cut the sum's last bits off each time they add to it, which would show after thousands of additions
+// of the same sign; so they only add up CHUNK blocks of 32 k at a time, and registers add the chunks, rounding to nearest.
+// Every output is formed from its own row of x and row of W in one order, whatever M, N and the tiling are.  An output
+// that does not come out finite (an infinity or NaN among the operands, or beyond the range) is formed again as a plain sum of
+// float products, so infinities and NaN go where they go in such a sum.  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
+//
+// x is split once, by a kernel of its own, into three planes of bfloat16.  A CTA owns 128 rows of W (the lanes of tensor memory)
+// and up to 192 rows of x (its columns).  Some warps read a block of 32 k of W into registers, ahead, split it, and write it
+// into a ring of three stages as the tensor cores read it (rows of 64 bytes, 64-byte swizzle); one thread brings x's planes by
+// TMA; two warps issue the products into two accumulators in tensor memory, while others add the chunk before to their
+// registers.
+//
+// Against pairs of multiply-adds on the CUDA cores (the form before, 74 TFLOP/s at best), one B200, W of bfloat16 numbers (of any floats):
+// 683 x 18432 over 2304 1,309 -> 274 (356) us, 683 x 2304 over 9216 831 -> 156 (191), over 2048 187 -> 42 (52), 3 x 256000 over 2304
+// 1,650 -> 505 (568), 1 x 2304 over 9216 356 -> 175; errors against 64 bits over 2,304 k 6.1e-7 -> 2.1e-7 (3.4e-7) of the result, of
+// operands of one sign 3.3e-7 -> 2.5e-7.  What bounds it: an issuer's waits and commits, 1,100 cycles a block of which the products are
+// 300 to 550, two issuers beside each other; for few rows of x, W's way from memory.  Chunks of 32 x 2 k are as long as the cut-off
+// bits allow: 32 x 4 has an error of 3.9e-7 (7.5e-7).
 #include "common.cuh"
+#include "mma_bf16.cuh"
+#include "tcgen05.cuh"
 
 namespace janis {
 
-constexpr int BM = 64, BN = 64, BK = 16, LD = BK + 4, STAGES = 4;      // rows of 80 bytes: eight of them lie in different banks
+int* tc05_timeout_counter();          // gemm_tc05.cu
+namespace tc { bool make_planes_map(CUtensorMap* map, const void* ptr, int rows, int K, int planes, int box_k, int box_rows); }
 
-typedef unsigned long long f32x2;
+namespace f32 {
 
-__device__ __forceinline__ void fma_pair(f32x2& c, f32x2 a, f32x2 b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-}
+using namespace tc;
 
-__device__ __forceinline__ void load_pairs(f32x2 (&v)[2], uint32_t shared) {
-    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[0]), "=l"(v[1]) : "r"(shared));
-}
+constexpr int BK = 32, STAGES = 3;
+#ifndef JANIS_F32_CHUNK
+#define JANIS_F32_CHUNK 2             // blocks of 32 k between additions in registers (a tuning switch)
+#endif
+constexpr int CHUNK = JANIS_F32_CHUNK;
+constexpr int W_ROWS = 128, W_PLANE = W_ROWS * 64;     // a plane: one of hi, mid, lo
+__host__ __device__ constexpr int stage_bytes(int cols) { return 3 * (W_PLANE + cols * 64); }
+__host__ __device__ constexpr int smem_bytes(int cols) { return STAGES * stage_bytes(cols) + 1024; }
 
-// Bytes [0, n) of BYTES from global memory, zeros behind them
-template <int BYTES>
-__device__ __forceinline__ void copy_async(uint32_t shared, const void* src, int n) {
-    if (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(shared), "l"(src), "r"(n) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(shared), "l"(src), "r"(n) : "memory");
-}
-
-// TN = 8: 2 warps of 64 x 32 outputs; TN = 4: 4 warps of 64 x 16.  VEC: rows are 16-byte aligned, K a multiple of 4.
-template <int TN, bool VEC>
-__global__ void __launch_bounds__(512 / TN)
-gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ W, float* __restrict__ out, int M, int N,
-                int K, float cap) {
-    constexpr int NT = 512 / TN, STAGE_BYTES = (BM + BN) * LD * 4;
-    __shared__ __align__(16) float tile[STAGES][BM + BN][LD];          // rows of x, then rows of W
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // neighbouring CTAs take the rows of x above one strip of W, so that the strip is fetched from memory once
-    const int m_tiles = (M + BM - 1) / BM;
-    const int m0 = (int)(blockIdx.x % m_tiles) * BM, n0 = (int)(blockIdx.x / m_tiles) * BN;
-    const int tm = lane & 7, tn = warp * 4 * TN + (lane >> 3);         // rows tm + 8 i, columns tn + 4 j
-    const int n_tiles = (K + BK - 1) / BK;
-    grid_dependents_launch();
-    grid_dependency_wait();                                            // x is the kernel before's result
-
-    // The pieces this thread brings: column kp of rows first, first + STEP, ...  Nobody stores the products of rows past the end;
-    // in the place of such a row of x stands the tile's row of W, which comes anyway.  (The last row of x over and over is a few
-    // lines of L2 for which all CTAs wait: one row against 18,432 x 2,304 took 375 us.  Reading nothing and writing zeros costs
-    // instructions in every tile: 1,370 us for 1,332 at 683 rows.)
-    constexpr int PER = BK / (VEC ? 4 : 1), STEP = NT / PER, PIECES = (BM + BN) / STEP;
-    const int first = tid / PER, kp = tid % PER * (VEC ? 4 : 1);
-    const float* src[PIECES];
+// Four floats from k on; zeros past the row's end and where !ok.  The loads are volatile so that they stay where they stand: the
+// compiler may move others down to the block that uses them.
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* row, int k, int K, bool ok) {
+    float4 v;
+    if (VEC) {
+        asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n"
+                     "@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n}\n"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "l"(row + k), "r"((int)(ok && k < K)));
+    } else {
+        float e[4];
 #pragma unroll
-    for (int e = 0; e < PIECES; ++e) {
-        const int r = first + e * STEP;
-        const bool of_x = e < PIECES / 2 && (!VEC || m0 + r < M);          // (without VEC the 32 addresses have no registers to spare)
-        const int row = of_x ? min(m0 + r, M - 1) : min(n0 + r % BM, N - 1);
-        src[e] = (of_x ? x : W) + (size_t)row * K + kp;
+        for (int j = 0; j < 4; ++j)
+            asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.b32 %0, 0;\n@p ld.global.nc.f32 %0, [%1];\n}\n"
+                         : "=f"(e[j])
+                         : "l"(row + k + j), "r"((int)(ok && k + j < K)));
+        v = make_float4(e[0], e[1], e[2], e[3]);
     }
-    const uint32_t base = (uint32_t)__cvta_generic_to_shared(&tile[0][0][0]);
-    auto fetch = [&](int t) {                                          // (a group for every tile, an empty one past the last)
-        if (t < n_tiles) {
-            const uint32_t to = base + (t % STAGES) * STAGE_BYTES + (first * LD + kp) * 4;
-            const int n = t * BK + kp < K ? (VEC ? 16 : 4) : 0;
-#pragma unroll
-            for (int e = 0; e < PIECES; ++e) copy_async<VEC ? 16 : 4>(to + e * STEP * LD * 4, n ? src[e] + t * BK : src[e] - kp, n);
+    return v;
+}
+
+__device__ __forceinline__ void store8(uint32_t shared, uint32_t a, uint32_t b) {
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(shared), "r"(a), "r"(b) : "memory");
+}
+
+// Whether `mine` holds for any thread of four warps that split W together (group `turn`)
+__device__ __forceinline__ bool any_of_group(int turn, bool mine) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbarrier.cta.red.or.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(any) : "r"((int)mine), "r"(1 + turn) : "memory");
+    return any != 0;
+}
+
+// x [M, K] as three planes [3][M][Kp] of bfloat16 numbers that add up to it; Kp: K rounded up to 8, zeros behind K
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+split_rows_kernel(const float* x, bf16* __restrict__ planes, int M, int K, int Kp) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    const int per_row = Kp / 8;
+    const size_t n = (size_t)M * per_row, plane = (size_t)M * Kp;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        const size_t m = i / per_row;
+        const int k = (int)(i - m * per_row) * 8;
+        const float4 a = load4<VEC>(x + m * K, k, K, true), b = load4<VEC>(x + m * K, k + 4, K, true);
+        uint4 hi, mid, lo;
+        split3(a.x, a.y, hi.x, mid.x, lo.x);
+        split3(a.z, a.w, hi.y, mid.y, lo.y);
+        split3(b.x, b.y, hi.z, mid.z, lo.z);
+        split3(b.z, b.w, hi.w, mid.w, lo.w);
+        bf16* to = planes + m * Kp + k;
+        *reinterpret_cast<uint4*>(to) = hi;
+        *reinterpret_cast<uint4*>(to + plane) = mid;
+        *reinterpret_cast<uint4*>(to + 2 * plane) = lo;
+    }
+}
+
+// SUMS warps that add up, SPLITS warps that split W (groups of four take blocks in turn), and four warps of which two issue the
+// products and one brings x.  VEC: rows of W are 16-byte aligned, K a multiple of 4.
+template <int SUMS, int SPLITS, int MOST_COLS, bool VEC>
+__global__ void __launch_bounds__((SUMS + SPLITS + 4) * 32, SUMS == 8 ? 1 : 2)
+gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restrict__ x, const float* W, float* __restrict__ out,
+                int M, int N, int K, int cols, float cap, int* __restrict__ timeouts) {
+    constexpr int GROUPS = SUMS / 4, UNITS = MOST_COLS / 16 / GROUPS;       // units of 16 columns of sums in a thread
+    constexpr int TURNS = SPLITS / 4, NW = W_ROWS / 16, AHEAD = 2;          // 16 rows of W a pass of four warps, 8 threads a row
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) unsigned long long bars[2 * STAGES + 5];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int low_bits[STAGES];                      // 1 + the last block whose W was not all bfloat16 numbers
+    __shared__ int failed;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t stage0 = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023) & ~1023u;
+    const uint32_t full = (uint32_t)__cvta_generic_to_shared(bars), empty = full + 8 * STAGES;
+    const uint32_t sums_there = empty + 8 * STAGES, sums_taken = sums_there + 16, all_done = sums_taken + 16;
+    const int stage_size = stage_bytes(cols), x_plane = cols * 64;
+    const int m_tiles = (M + cols - 1) / cols;            // neighbouring CTAs take the rows of x of one strip of W
+    const int m0 = (int)(blockIdx.x % m_tiles) * cols, n0 = (int)(blockIdx.x / m_tiles) * W_ROWS;
+    const int n_blocks = (K + BK - 1) / BK, n_chunks = (n_blocks + CHUNK - 1) / CHUNK;
+    const int tmem_cols = 2 * cols <= 32 ? 32 : (2 * cols <= 64 ? 64 : (2 * cols <= 128 ? 128 : (2 * cols <= 256 ? 256 : 512)));
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) {
+            mbar_init(full + 8 * i, 5);          // four warps of W, the copies of x
+            mbar_init(empty + 8 * i, 1);
+            low_bits[i] = 0;
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(sums_there + 8 * i, 1);
+            mbar_init(sums_taken + 8 * i, SUMS);
+        }
+        mbar_init(all_done, 2);
+        failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == SUMS + SPLITS) tmem_alloc((uint32_t)__cvta_generic_to_shared(&tmem_slot), tmem_cols);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+    grid_dependents_launch();
+    grid_dependency_wait();                               // the planes are the kernel before's result
 
-    f32x2 acc[8][TN];                                                  // (sum over even k, sum over odd k)
+    // Registers go to the warps that hold sums: of 640 x 96 at launch 256 x 128 + 256 x 96 + 128 x 32 are in use, of 384 x 80 (two
+    // CTAs an SM) 128 x 96 + 128 x 104 + 128 x 32.
+    if (warp >= SUMS + SPLITS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        const int issuer = warp - SUMS - SPLITS;
+        if (issuer < 2) {
+            // Two warps issue products, a chunk each in turn and into an accumulator each: what a block costs an issuer besides (waits,
+            // commits: 1,100 cycles in all) lies beside the other's.  The whole warp runs the loop, so that descriptors stay in the uniform
+            // registers that the products take them from, and the elected lane issues (a thread of the programmer's choice under a branch
+            // took twice as long).
+            const uint32_t idesc = instr_desc(W_ROWS, cols);
+            const uint32_t plane16 = (uint32_t)x_plane >> 4;                    // (an address in a descriptor counts 16 bytes)
+            const uint32_t d = tmem + issuer * cols;
+            bool ok = true;
+            for (int c = issuer; c < n_chunks && ok; c += 2) {
+                if (c >= 2 && !__all_sync(0xffffffffu, mbar_wait(sums_taken + 8 * issuer, (c / 2 - 1) & 1))) { ok = false; break; }
+                const int first = c * CHUNK, last = min(first + CHUNK, n_blocks) - 1;
+                for (int b = first; b <= last; ++b) {
+                    const int s = b % STAGES;
+                    if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (b / STAGES) & 1))) { ok = false; break; }
+                    // The splitters' writes are fenced for the tensor cores here, behind the barrier that orders them.
+                    fence_async_shared();
+                    fence_after_sync();
+                    const uint64_t w = smem_desc_64(stage0 + s * stage_size), xs = w + (3 * W_PLANE >> 4);
+                    const bool whole = *(volatile int*)&low_bits[s] == b + 1;
+                    uint32_t add = b != first;            // the chunk's first product replaces what the accumulator held
+                    if (elect_one()) {
+                        if (whole) {                      // small ones first
+                            umma(d, w + (2 * W_PLANE >> 4), xs, idesc, add);
+                            umma(d, w + (2 * W_PLANE >> 4) + 2, xs + 2, idesc, 1);
+                            umma(d, w + (W_PLANE >> 4), xs + plane16, idesc, 1);
+                            umma(d, w + (W_PLANE >> 4) + 2, xs + plane16 + 2, idesc, 1);
+                            umma(d, w + (W_PLANE >> 4), xs, idesc, 1);
+                            umma(d, w + (W_PLANE >> 4) + 2, xs + 2, idesc, 1);
+                            add = 1;
+                        }
+                        umma(d, w, xs + 2 * plane16, idesc, add);
+                        umma(d, w + 2, xs + 2 * plane16 + 2, idesc, 1);
+                        umma(d, w, xs + plane16, idesc, 1);
+                        umma(d, w + 2, xs + plane16 + 2, idesc, 1);
+                        umma(d, w, xs, idesc, 1);
+                        umma(d, w + 2, xs + 2, idesc, 1);
+                        umma_commit(empty + 8 * s);
+                        if (b == last) umma_commit(sums_there + 8 * issuer);
+                    }
+                    __syncwarp();
+                }
+            }
+            if (!ok) atomicExch(&failed, 1);
+            if (elect_one()) umma_commit(all_done);
+            __syncwarp();
+            mbar_wait(all_done, 0);
+        } else if (issuer == 2 && lane == 0) {            // brings the planes of x
+            for (int b = 0; b < n_blocks; ++b) {
+                const int s = b % STAGES;
+                if (b >= STAGES && !mbar_wait_parked(empty + 8 * s, (b / STAGES - 1) & 1, &failed)) { atomicExch(&failed, 1); break; }
+                mbar_expect_tx(full + 8 * s, 3 * x_plane);
+                tma_load_3d(stage0 + s * stage_size + 3 * W_PLANE, &map_x, b * BK, m0, 0, full + 8 * s);
+            }
+        }
+        __syncwarp();
+        asm volatile("bar.sync 0;" ::: "memory");         // the last sums have been read
+        if (warp == SUMS + SPLITS) {
+            tmem_free(tmem, tmem_cols);
+            if (failed && lane == 0) atomicAdd(timeouts, 1);
+        }
+    } else if (warp >= SUMS) {
+        if (SUMS == 4) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        const int thread = threadIdx.x - SUMS * 32, turn = thread >> 7;
+        const int quad = thread & 7, r = (thread & 127) >> 3;                    // 4 k of rows r, r + 16, ...
+        const uint32_t place = r * 64 + (((quad >> 1) ^ ((r >> 1) & 3)) << 4) + (quad & 1) * 8;
+        const float* wr = W + (size_t)min(n0 + r, N - 1) * K;
+        const int rows = N - n0 - r;                      // a pass of this thread's is within W where 16 i < rows
+        float4 wv[AHEAD][NW];
+        auto fetch = [&](int b, int a) {
+            const int k = b * BK + quad * 4;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+            for (int i = 0; i < NW; ++i) wv[a][i] = load4<VEC>(wr + (size_t)(i * 16) * K, k, K, i * 16 < rows);
+        };
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+        for (int a = 0; a < AHEAD; ++a) fetch(turn + a * TURNS, a);
+        bool ok = true;
+        for (int b0 = turn; b0 < n_blocks; b0 += AHEAD * TURNS) {
+#pragma unroll
+            for (int a = 0; a < AHEAD; ++a) {
+                const int b = b0 + a * TURNS;
+                if (b >= n_blocks) break;
+                const int s = b % STAGES, round = b / STAGES;
+                // (who gives up goes on without waiting: the other warps of the group count on its arrivals)
+                if (ok && round > 0) ok = mbar_wait_parked(empty + 8 * s, (round - 1) & 1, &failed);
+                const uint32_t to = stage0 + s * stage_size + place;
+                uint32_t low = 0;
+#pragma unroll
+                for (int i = 0; i < NW; ++i)
+                    low |= __float_as_uint(wv[a][i].x) | __float_as_uint(wv[a][i].y) | __float_as_uint(wv[a][i].z) | __float_as_uint(wv[a][i].w);
+                // Whether mid and lo have to be written is asked of all four warps: the stage may hold what another group left there.
+                if (any_of_group(turn, (low & 0xffffu) != 0)) {
+#pragma unroll
+                    for (int i = 0; i < NW; ++i) {
+                        uint32_t h0, h1, m0_, m1, l0, l1;
+                        split3(wv[a][i].x, wv[a][i].y, h0, m0_, l0);
+                        split3(wv[a][i].z, wv[a][i].w, h1, m1, l1);
+                        const uint32_t at = to + i * 16 * 64;
+                        store8(at, h0, h1);
+                        store8(at + W_PLANE, m0_, m1);
+                        store8(at + 2 * W_PLANE, l0, l1);
+                    }
+                    if ((thread & 127) == 0) *(volatile int*)&low_bits[s] = b + 1;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NW; ++i)
+                        store8(to + i * 16 * 64, __byte_perm(__float_as_uint(wv[a][i].x), __float_as_uint(wv[a][i].y), 0x7632),
+                               __byte_perm(__float_as_uint(wv[a][i].z), __float_as_uint(wv[a][i].w), 0x7632));
+                }
+                if (b + AHEAD * TURNS < n_blocks) fetch(b + AHEAD * TURNS, a);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full + 8 * s);
+            }
+        }
+        if (!ok) atomicExch(&failed, 1);
+        asm volatile("bar.sync 0;" ::: "memory");
+    } else {
+        if (SUMS == 8) asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
+        float acc[UNITS][16];
+        const int quarter = warp & 3, group = warp >> 2;
+        const uint32_t mine = tmem + ((uint32_t)(quarter * 32) << 16);
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) acc[u][j] = 0.f;
+        bool ok = true;
+        for (int c = 0; c < n_chunks; ++c) {              // add the chunk in tensor memory to the registers
+            if (!mbar_wait_parked(sums_there + 8 * (c & 1), (c / 2) & 1, &failed)) { ok = false; break; }
+            fence_after_sync();
+#pragma unroll
+            for (int u = 0; u < UNITS; ++u) {
+                const int col = (group + u * GROUPS) * 16;
+                if (col >= cols) break;
+                uint32_t v[16];
+                tmem_load16(v, mine + (c & 1) * cols + col);
+                tmem_wait_load();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[u][j] += __uint_as_float(v[j]);
+            }
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(sums_taken + 8 * (c & 1));
+        }
+        if (!ok) atomicExch(&failed, 1);
+        fence_before_sync();
+        asm volatile("bar.sync 0;" ::: "memory");
+        if (failed) return;
 
-    for (int t = 0; t < STAGES - 1; ++t) fetch(t);
-    for (int t = 0; t < n_tiles; ++t) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncthreads();                                               // tile t is there; tile t - 1 has been read by all
-        fetch(t + STAGES - 1);
-        const uint32_t xa = base + (t % STAGES) * STAGE_BYTES + tm * (LD * 4);
-        const uint32_t wa = base + (t % STAGES) * STAGE_BYTES + (BM + tn) * (LD * 4);
+        const int n = n0 + quarter * 32 + lane;           // neighbouring lanes hold neighbouring columns of out
 #pragma unroll
-        for (int kk = 0; kk < BK; kk += 4) {
-            f32x2 a[8][2];
+        for (int u = 0; u < UNITS; ++u) {
+            const int col = (group + u * GROUPS) * 16;
+            if (col >= cols) break;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) load_pairs(a[i], xa + (8 * i * LD + kk) * 4);
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                f32x2 w[2];
-                load_pairs(w, wa + (4 * j * LD + kk) * 4);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) fma_pair(acc[i][j], a[i][0], w[0]);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) fma_pair(acc[i][j], a[i][1], w[1]);
+            for (int j = 0; j < 16; ++j) {
+                const int m = m0 + col + j;
+                if (m >= M) break;
+                float v = acc[u][j];
+                uint32_t odd = __ballot_sync(0xffffffffu, n < N && !(fabsf(v) <= 3.402823466e38f));
+                while (odd) {                             // (hardly ever) the warp forms such a sum of plain products
+                    const int l = __ffs(odd) - 1;
+                    odd &= odd - 1;
+                    const float *xp = x + (size_t)m * K, *wp = W + (size_t)(n - lane + l) * K;
+                    float plain = 0.f;
+                    for (int k = lane; k < K; k += 32) plain = fmaf(xp[k], wp[k], plain);
+                    plain = warp_sum(plain);
+                    if (lane == l) v = plain;
+                }
+                if (n < N) {
+                    if (cap > 0.f) v = cap * tanhf(v / cap);
+                    out[(size_t)m * N + n] = v;
+                }
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = m0 + tm + 8 * i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int n = n0 + tn + 4 * j;
-            if (n >= N) continue;
-            float even, odd;
-            asm("mov.b64 {%0, %1}, %2;" : "=f"(even), "=f"(odd) : "l"(acc[i][j]));
-            float v = even + odd;
-            if (cap > 0.f) v = cap * tanhf(v / cap);
-            out[(size_t)m * N + n] = v;
-        }
-    }
 }
 
+template <int SUMS, int SPLITS, int MOST_COLS, bool VEC>
+static int launch(const CUtensorMap& map_x, const float* x, const float* W, float* out, int M, int N, int K, int cols, float cap,
+                  long long tiles, int* timeouts, cudaStream_t stream) {
+    auto kernel = gemm_f32_kernel<SUMS, SPLITS, MOST_COLS, VEC>;
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(MOST_COLS));
+        if (e != cudaSuccess) return fail("gemm_f32: shared memory of %d bytes refused: %s", smem_bytes(MOST_COLS), cudaGetErrorString(e));
+        configured = true;
+    }
+    return launch_kernel("gemm_f32", kernel, dim3((unsigned)tiles), dim3((SUMS + SPLITS + 4) * 32), smem_bytes(cols), stream, 1, map_x, x, W,
+                         out, M, N, K, cols, cap, timeouts);
+}
+
+}  // namespace f32
 }  // namespace janis
 
 using namespace janis;
 
-JANIS_EXPORT int janis_gemm_f32(const float* x, const float* W, float* out, int M, int N, int K, float cap,
+JANIS_EXPORT int janis_launches_made() { return launches_made(); }
+
+// rows of x whose planes take no more than 64 MB (256 at least): a product of more rows is made in parts
+static int f32_part_rows(int M, int K) {
+    const long long rows = (64ll << 20) / (6ll * ((K + 7) / 8 * 8)) / 256 * 256;
+    const long long most = rows < 256 ? 256 : rows;
+    return (int)(M < most ? M : most);
+}
+
+// bfloat16 numbers of room for the planes of x that janis_gemm_f32 wants
+JANIS_EXPORT long long janis_gemm_f32_room(int M, int K) {
+    return M <= 0 || K <= 0 ? 0 : 3ll * f32_part_rows(M, K) * ((K + 7) / 8 * 8);
+}
+
+// planes: 16-byte aligned room of janis_gemm_f32_room(M, K) bfloat16 numbers
+JANIS_EXPORT int janis_gemm_f32(const float* x, const float* W, float* out, int M, int N, int K, float cap, void* planes,
                                 cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return fail("gemm_f32: K must be positive, found %d", K);
-    if ((M + BM - 1) / BM > 65535) return fail("gemm_f32: too many rows (%d)", M);
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-    if (tiles > 0x7fffffff) return fail("gemm_f32: %d x %d outputs are too many", M, N);
-    const dim3 grid((unsigned)tiles);
+    if ((M + 63) / 64 > 65535) return fail("gemm_f32: too many rows (%d)", M);
+    if (planes == nullptr || ((uintptr_t)planes & 15)) return fail("gemm_f32: the planes of x need 16-byte aligned room");
     static thread_local int sms = 0;
     if (sms == 0) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return fail("gemm_f32: the device does not say how many SMs it has");
     }
-    // The time is what the busiest quarter of an SM has to do.  Warps of 64 x 32 outputs read less from shared memory an
-    // instruction (44 TFLOP/s against 37 when the SMs are full); warps of half the size leave less undone in the last round.
-    const long long quarters = 4ll * sms;
-    const long long large = (2 * tiles + quarters - 1) / quarters * 20, small = (4 * tiles + quarters - 1) / quarters * 12;
-    const bool vec = K % 4 == 0 && ((uintptr_t)x | (uintptr_t)W) % 16 == 0;
-    if (large <= small)
-        return vec ? launch_kernel("gemm_f32", gemm_f32_kernel<8, true>, grid, dim3(64), 0, stream, 1, x, W, out, M, N, K, cap)
-                   : launch_kernel("gemm_f32", gemm_f32_kernel<8, false>, grid, dim3(64), 0, stream, 1, x, W, out, M, N, K, cap);
-    return vec ? launch_kernel("gemm_f32", gemm_f32_kernel<4, true>, grid, dim3(128), 0, stream, 1, x, W, out, M, N, K, cap)
-               : launch_kernel("gemm_f32", gemm_f32_kernel<4, false>, grid, dim3(128), 0, stream, 1, x, W, out, M, N, K, cap);
+    int* timeouts = tc05_timeout_counter();
+    if (timeouts == nullptr) return fail("gemm_f32: the counter of timeouts has no address");
+    const long long strips = (N + f32::W_ROWS - 1) / f32::W_ROWS;
+    const bool w_vec = K % 4 == 0 && (uintptr_t)W % 16 == 0;
+    const int part = f32_part_rows(M, K), Kp = (K + 7) / 8 * 8;
+    for (int first = 0; first < M; first += part, x += (size_t)part * K, out += (size_t)part * N) {
+        const int rows = M - first < part ? M - first : part;
+        // Up to 64 rows of x: two CTAs an SM.  More: as many rows a CTA as make the last round of CTAs full; a block costs its
+        // products (in proportion to the rows) and the splitting of W.
+        const bool small = rows <= 64;
+        int cols = (rows + 15) / 16 * 16;
+        if (!small) {
+            long long best = -1;
+            for (int c = 64; c <= 192; c += 16) {
+                const long long cost = (strips * ((rows + c - 1) / c) + sms - 1) / sms * (c + 48);
+                if (best < 0 || cost <= best) { best = cost; cols = c; }
+            }
+        }
+        const long long tiles = strips * ((rows + cols - 1) / cols);
+        if (tiles > 0x7fffffff) return fail("gemm_f32: %d x %d outputs are too many", rows, N);
+        CUtensorMap map_x;
+        if (!tc::make_planes_map(&map_x, planes, rows, Kp, 3, f32::BK, cols))
+            return fail("gemm_f32: cuTensorMapEncodeTiled is not available or refused the operands");
+        const long long pieces = (long long)rows * (Kp / 8);
+        const dim3 grid((unsigned)(pieces > 256ll * 8 * sms ? 8 * sms : (pieces + 255) / 256));
+        const bool x_vec = K % 4 == 0 && (uintptr_t)x % 16 == 0;
+        if (launch_kernel("gemm_f32", x_vec ? f32::split_rows_kernel<true> : f32::split_rows_kernel<false>, grid, dim3(256), 0, stream, 1, x,
+                          (bf16*)planes, rows, K, Kp))
+            return 1;
+        const int failed = small ? (w_vec ? f32::launch<4, 4, 64, true>(map_x, x, W, out, rows, N, K, cols, cap, tiles, timeouts, stream)
+                                          : f32::launch<4, 4, 64, false>(map_x, x, W, out, rows, N, K, cols, cap, tiles, timeouts, stream))
+                                 : (w_vec ? f32::launch<8, 8, 192, true>(map_x, x, W, out, rows, N, K, cols, cap, tiles, timeouts, stream)
+                                          : f32::launch<8, 8, 192, false>(map_x, x, W, out, rows, N, K, cols, cap, tiles, timeouts, stream));
+        if (failed) return 1;
+    }
+    return 0;
 }

@@ -24,6 +24,7 @@
 #include <tuple>
 
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -45,56 +46,6 @@ static_assert(sizeof(float) * BLOCK_N * MAX_M <= MIN_STAGES * STAGE_BYTES, "the 
 enum { EPI_NONE = 0, EPI_GATED_GELU = 1, EPI_SOFTCAP = 2, EPI_GATED_SILU = 3 };
 
 __device__ int g_timeouts = 0;
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, int bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    // test_wait polls without suspending the thread (try_wait may park it for a while, which costs a stage's
-    // worth of latency at every hand-over); about a second's worth of polls, then give up
-    for (int it = 0; it < (1 << 26); ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-        "l"(map), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-// shared-memory operand: K-major rows of 128 bytes, 128-byte swizzle, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);            // start address
-    d |= (uint64_t)1 << 16;                             // leading byte offset (unused with a swizzle)
-    d |= (uint64_t)(1024 >> 4) << 32;                   // stride byte offset: next group of 8 rows
-    d |= (uint64_t)1 << 46;                             // descriptor version of sm_100
-    d |= (uint64_t)2 << 61;                             // SWIZZLE_128B
-    return d;
-}
-// kind::f16, bfloat16 operands both K-major, float accumulator, shape M x N x 16
-__device__ __forceinline__ uint32_t instr_desc(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
-}
 
 template <typename TO>
 __global__ void __launch_bounds__(THREADS)
@@ -324,6 +275,20 @@ static bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, int box
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// [planes, rows, K] bfloat16, K contiguous and a multiple of 8, in boxes of box_k (rows of 64 bytes) x box_rows x all planes with
+// the 64-byte swizzle
+bool make_planes_map(CUtensorMap* map, const void* ptr, int rows, int K, int planes, int box_k, int box_rows) {
+    EncodeTiled enc = encoder();
+    if (!enc) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)planes};
+    const cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)K * 2 * rows};
+    const cuuint32_t box[3] = {(cuuint32_t)box_k, (cuuint32_t)box_rows, (cuuint32_t)planes};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, elem,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 static const CUtensorMap* cached_map(const void* ptr, int rows, int K, int box_rows) {
     static std::map<std::tuple<const void*, int, int, int>, CUtensorMap> cache;
     static std::mutex lock;
@@ -360,7 +325,15 @@ JANIS_EXPORT void janis_tc05_set_stages(int stages) {
     g_tc05_stages = stages <= 0 ? 0 : (stages < tc::MIN_STAGES ? tc::MIN_STAGES : (stages > tc::MAX_STAGES ? tc::MAX_STAGES : stages));
 }
 
-namespace janis { int gemv_push_timeouts_async(int* host, cudaStream_t stream); }      // gemv_bf16.cu
+namespace janis {
+int gemv_push_timeouts_async(int* host, cudaStream_t stream);      // gemv_bf16.cu
+
+// where this library's kernels count the waits they gave up, on the current device
+int* tc05_timeout_counter() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, tc::g_timeouts) == cudaSuccess ? (int*)p : nullptr;
+}
+}  // namespace janis
 
 // The same count copied into `host` (pinned memory, two ints: this kernel's count, then that of the skinny products'
 // clusters) in the order of `stream`, without waiting for it: a caller that waits for the stream anyway (for its

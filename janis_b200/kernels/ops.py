@@ -59,7 +59,9 @@ def core():
         lib.janis_bias_act.argtypes = [P, P, I, I, I, I, F, F, P]
         lib.janis_rope_store.argtypes = [P, I, P, P, P, P, P, I, I, I, I, I, I, P, P, P, I, I, I, P]
         lib.janis_kv_store.argtypes = [P, I, P, P, P, P, I, I, I, I, I, P, P, P, I, I, P]
-        lib.janis_gemm_f32.argtypes = [P, P, P, I, I, I, F, P]
+        lib.janis_gemm_f32.argtypes = [P, P, P, I, I, I, F, P, P]
+        lib.janis_gemm_f32_room.argtypes = [I, I]
+        lib.janis_gemm_f32_room.restype = c_longlong
         lib.janis_gemv_bf16.argtypes = [P, P, P, I, I, I, I, I, F, I, F, F, P]
         lib.janis_gemv_bf16_bias_act.argtypes = [P, P, P, I, I, I, P, I, F, F, P]
         lib.janis_gemv_rope_store.argtypes = [P, P, P, I, I, P, P, P, P, P, I, I, I, I, P, P, P, I, I, P]
@@ -419,12 +421,14 @@ def kv_store(qkv, tok_pos, tok_seq, seq_slot, seq_end, nq: int, nkv: int, hd: in
 # ---------------------------------------------------------------------------
 
 def gemm_f32(x, w, out, cap: float = 0.0):
-    """out[M, N] = x[M, K] w[N, K]^T in true float32 (CUDA cores); optional cap * tanh(v / cap)."""
+    """out[M, N] = x[M, K] w[N, K]^T at float32's precision (floats as sums of bfloat16 numbers on the tensor cores);
+    optional cap * tanh(v / cap)."""
     M, K = x.shape
     N = w.shape[0]
     lib = core()
-    _check(lib, lib.janis_gemm_f32(_t(x, "x", torch.float32, (M, K)), _t(w, "w", torch.float32, (N, K)),
-                                   _t(out, "out", torch.float32, (M, N)), M, N, K, float(cap), _stream()))
+    xp, wp, op = _t(x, "x", torch.float32, (M, K)), _t(w, "w", torch.float32, (N, K)), _t(out, "out", torch.float32, (M, N))
+    planes = torch.empty(max(lib.janis_gemm_f32_room(M, K), 1), dtype=torch.bfloat16, device=x.device)
+    _check_counted(lib, lib.janis_gemm_f32, xp, wp, op, M, N, K, float(cap), planes.data_ptr(), _stream())
     return out
 
 

@@ -285,6 +285,45 @@ def test_gemm_f32_row_does_not_depend_on_batch():
     assert torch.equal(full[20:21], one)
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 129, 33), (65, 128, 64), (193, 127, 100), (16, 300, 31), (130, 260, 2051), (1500, 40, 9216)])
+def test_gemm_f32_blocks(M, N, K):
+    """The edges of the tiles (128 rows of W, 16 to 192 of x, 32 k; 1,500 rows over 9,216 come in two parts), rows that are not
+    16-byte aligned, and W whose blocks of 32 k are bfloat16 numbers here and floats there.  2,048 products of size 1 add up with
+    an error of some 3e-7 of the root of their number; the largest of 260 x 130 such errors stays below 5e-6 of it."""
+    x = rnd((M, K), torch.float32, 60)
+    w = rnd((N, K), torch.float32, 61)
+    w[:, : K // 2] = w[:, : K // 2].bfloat16().float()
+    w[N // 2:, K // 3:] = w[N // 2:, K // 3:].bfloat16().float()
+    out = torch.empty((M, N), dtype=torch.float32, device=dev())
+    ops().gemm_f32(x, w, out)
+    want = x.cpu().double() @ w.cpu().double().T
+    assert ((out.cpu().double() - want).abs().max() / K ** 0.5).item() <= 5e-6
+    one = torch.empty((1, N), dtype=torch.float32, device=dev())
+    ops().gemm_f32(x[M - 1:].contiguous(), w, one)
+    assert torch.equal(out[M - 1:], one)
+
+
+def test_gemm_f32_infinities_and_nan():
+    """An infinity or NaN reaches the outputs that a sum of float products takes it to, and no others."""
+    x = rnd((70, 96), torch.float32, 62)
+    w = rnd((140, 96), torch.float32, 63).bfloat16().float()
+    x[3, 5], x[9, 95], x[20, 0], w[7, 40], w[129, 2] = math.inf, math.nan, -math.inf, math.inf, math.nan
+    x[33, 40] = 0.0                                          # 0 x inf
+    x[50] = 3e38                                             # hi rounds to infinity; the sums pass the largest float
+    w[100] = 0.0
+    out = torch.empty((70, 140), dtype=torch.float32, device=dev())
+    ops().gemm_f32(x, w, out)
+    want = (x.cpu()[:, None, :] * w.cpu()[None]).double().sum(-1)
+    got = out.cpu().double()
+    rest = torch.ones(70, dtype=torch.bool)
+    rest[50] = False                                         # (where a partial sum passes the range turns on the order of the sum)
+    assert torch.equal(got[rest].isnan(), want[rest].isnan())
+    assert torch.equal(got[rest].isposinf(), want[rest].isposinf()) and torch.equal(got[rest].isneginf(), want[rest].isneginf())
+    ok = want[rest].isfinite()
+    assert (got[rest][ok] - want[rest][ok]).abs().max().item() <= 1e-4
+    assert got[50, 100].item() == 0.0                        # finite operands, a finite result
+
+
 @pytest.mark.parametrize("dout", DTYPES)
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 33, 64])
 @pytest.mark.parametrize("N,K", [(16, 32), (40, 72), (384, 96), (2304, 2048), (1000, 328)])
