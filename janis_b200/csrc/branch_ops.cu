@@ -29,6 +29,37 @@ dyt_norm_kernel(float* __restrict__ h, const TR* __restrict__ res, const int* __
     }
 }
 
+// The same, eight values a thread (H a multiple of 8, rows on 16 bytes): no row is one CTA's, so few rows still fill SMs, and w and b are
+// there before the kernel waits.  8 rows of 2,304: 1.5 us of a decode step against 7.3 (a CTA a row, a value a turn); 2,048 rows 9.4 against 14.6.
+template <typename TR, typename TO>
+__global__ void __launch_bounds__(128)
+dyt_norm_vec_kernel(float* __restrict__ h, const TR* __restrict__ res, const int* __restrict__ rows, float alpha,
+                    const float* __restrict__ w, const float* __restrict__ b, TO* __restrict__ y, int R, int H) {
+    const size_t at = ((size_t)blockIdx.x * 128 + threadIdx.x) * 8;
+    const size_t r = at / H;
+    const int i = (int)(at - r * H);
+    float wv[8], bv[8], v[8];
+    grid_dependents_launch();
+    if (r < (size_t)R) {
+        load_eight(w + i, wv);
+        load_eight(b + i, bv);
+    }
+    grid_dependency_wait();
+    if (r >= (size_t)R) return;
+    float* hr = h + (size_t)(rows != nullptr ? rows[r] : (int)r) * H + i;
+    load_eight(hr, v);
+    if (res != nullptr) {
+        float x[8];
+        load_eight(res + r * H + i, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] += x[e];
+        store_eight(hr, v);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = fmaf(tanhf(alpha * v[e]), wv[e], bv[e]);
+    store_eight(y + r * H + i, v);
+}
+
 // acc[r] = (first ? 0 : acc[r]) + share * x[r] / sqrt(mean(x[r]^2) + eps) * w
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -50,6 +81,47 @@ rmsnorm_accumulate_kernel(const T* __restrict__ x, const float* __restrict__ w, 
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         const float v = to_float(xr[i]) * inv * w[i];
         ar[i] = first ? v : ar[i] + v;
+    }
+}
+
+// The same with the row in registers: NV times eight values a thread (H a multiple of 8, rows on 16 bytes), read once.  8 rows of
+// 2,304: 2.2 us of a decode step against 7.2; 2,048 rows 9.2 against 15.4.
+template <typename T, int NV>
+__global__ void __launch_bounds__(128)
+rmsnorm_accumulate_vec_kernel(const T* __restrict__ x, const float* __restrict__ w, float eps, float share, float* __restrict__ acc, int first, int H) {
+    __shared__ float scratch[32];
+    const size_t r = blockIdx.x;
+    float v[NV][8], a[NV][8], ww[NV][8];
+    grid_dependents_launch();
+    grid_dependency_wait();
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * 128 + threadIdx.x) * 8;
+        if (i < H) {
+            load_eight(x + r * H + i, v[n]);
+            load_eight(w + i, ww[n]);
+            if (!first) load_eight(acc + r * H + i, a[n]);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+        if ((n * 128 + threadIdx.x) * 8 < H)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ss = fmaf(v[n][e], v[n][e], ss);
+    ss = block_sum(ss, scratch);
+    const float inv = share / sqrtf(ss / (float)H + eps);
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * 128 + threadIdx.x) * 8;
+        if (i < H) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const float y = v[n][e] * inv * ww[n][e];
+                v[n][e] = first ? y : a[n][e] + y;
+            }
+            store_eight(acc + r * H + i, v[n]);
+        }
     }
 }
 
@@ -650,9 +722,13 @@ JANIS_EXPORT int janis_dyt_norm(float* h, const void* res, int res_dtype, const 
     if (R <= 0) return 0;
     if (res != nullptr && rows != nullptr) return fail("dyt_norm: a residual is added to all rows, not to chosen ones");
     const dim3 grid(R), block(H >= 1024 ? 256 : 128);
+    const long long pieces = (long long)R * H / 8;
+    const bool vec = H % 8 == 0 && (((uintptr_t)h | (uintptr_t)res | (uintptr_t)w | (uintptr_t)b | (uintptr_t)y) & 15) == 0 && pieces / 128 < 0x7fffffff;
 #define JANIS_DYT(TR, TO)                                                                                              \
-    return launch_kernel("dyt_norm", dyt_norm_kernel<TR, TO>, grid, block, 0, stream, 1, h, (const TR*)res, rows, alpha, w, \
-                         b, (TO*)y, H);
+    return vec ? launch_kernel("dyt_norm", dyt_norm_vec_kernel<TR, TO>, dim3((unsigned)((pieces + 127) / 128)), dim3(128), 0, stream, 1, h, \
+                               (const TR*)res, rows, alpha, w, b, (TO*)y, R, H)                                          \
+               : launch_kernel("dyt_norm", dyt_norm_kernel<TR, TO>, grid, block, 0, stream, 1, h, (const TR*)res, rows, alpha, w, \
+                               b, (TO*)y, H);
     const int rd = res != nullptr ? res_dtype : JANIS_F32;
     if (rd == JANIS_F32 && y_dtype == JANIS_F32) { JANIS_DYT(float, float) }
     if (rd == JANIS_F32 && y_dtype == JANIS_BF16) { JANIS_DYT(float, bf16) }
@@ -666,6 +742,15 @@ JANIS_EXPORT int janis_rmsnorm_accumulate(const void* x, int dtype, const float*
                                           int first, int R, int H, cudaStream_t stream) {
     if (R <= 0) return 0;
     const dim3 grid(R), block(H >= 1024 ? 256 : 128);
+    if (H % 8 == 0 && H <= 4 * 1024 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)acc) & 15) == 0) {
+#define JANIS_ACC(T, NV)                                                                                               \
+    if (H <= NV * 1024)                                                                                                \
+        return launch_kernel("rmsnorm_accumulate", rmsnorm_accumulate_vec_kernel<T, NV>, grid, dim3(128), 0, stream, 1, (const T*)x, w, eps, share, \
+                             acc, first, H);
+        if (dtype == JANIS_F32) { JANIS_ACC(float, 1) JANIS_ACC(float, 2) JANIS_ACC(float, 3) JANIS_ACC(float, 4) }
+        if (dtype == JANIS_BF16) { JANIS_ACC(bf16, 1) JANIS_ACC(bf16, 2) JANIS_ACC(bf16, 3) JANIS_ACC(bf16, 4) }
+#undef JANIS_ACC
+    }
     if (dtype == JANIS_F32)
         return launch_kernel("rmsnorm_accumulate", rmsnorm_accumulate_kernel<float>, grid, block, 0, stream, 1,
                              (const float*)x, w, eps, share, acc, first, H);

@@ -245,6 +245,18 @@ template <> struct Vec16<bf16> {
     }
 };
 
+// eight consecutive values, on 16 bytes
+template <typename T>
+__device__ __forceinline__ void load_eight(const T* p, float* out) {
+    Vec16<T>::load(p, out);
+    if (Vec16<T>::N == 4) Vec16<T>::load(p + 4, out + 4);
+}
+template <typename T>
+__device__ __forceinline__ void store_eight(T* p, const float* in) {
+    Vec16<T>::store(p, in);
+    if (Vec16<T>::N == 4) Vec16<T>::store(p + 4, in + 4);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -214,6 +214,103 @@ gla_scan_kernel(const T* __restrict__ rows, GlaRows g, const float* __restrict__
     }
 }
 
+__device__ __forceinline__ void load_four(const float* p, float* o) { Vec16<float>::load(p, o); }
+__device__ __forceinline__ void load_four(const bf16* p, float* o) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
+    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+
+// One token a sequence (a decode step): the state comes and goes once.  A warp takes four columns of a head's state (two for more than
+// 128 key channels), a lane four channels of each, so that its accesses are whole lines; q, k and the decays, which are formed
+// here, lie in registers for all of them.  The state is asked for (into L2) before the kernel waits for the one that makes
+// its inputs.  Eight sequences, 8 heads of 128 x 256: 4.8 us with the decays against 21.6 in the scan above, which runs a tile of
+// 16 tokens of which one is there.  Sequences of more tokens run through them in turn.
+template <typename T, int NV>
+__global__ void __launch_bounds__(256)
+gla_step_kernel(const T* __restrict__ rows, GlaRows g, const T* __restrict__ z, const T* __restrict__ bias, const int* __restrict__ seq_slot,
+                const int* __restrict__ seq_first_row, const int* __restrict__ seq_start, const int* __restrict__ seq_end,
+                float* __restrict__ state, float* __restrict__ o_out, float* __restrict__ decay) {
+    constexpr int J = NV == 1 ? 4 : 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.x, h = blockIdx.y;
+    const int d = g.d, dv = g.dv, H = g.H, col0 = (blockIdx.z * 8 + warp) * J;
+    grid_dependents_launch();
+    const int slot = seq_slot[seq], row0 = seq_first_row[seq], n_tok = seq_end[seq] - seq_start[seq];
+    float* st = slot >= 0 ? state + ((size_t)slot * H + h) * d * dv : nullptr;
+    if (st != nullptr && n_tok > 0) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                if (col0 + j < dv && v * 128 + lane * 4 < d)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(st + (size_t)(col0 + j) * d + v * 128 + lane * 4));
+    }
+    grid_dependency_wait();
+    if (n_tok <= 0 || col0 >= dv) return;
+    float4 S[J][NV];
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = v * 128 + lane * 4;
+            S[j][v] = st != nullptr && col0 + j < dv && i < d ? *reinterpret_cast<const float4*>(st + (size_t)(col0 + j) * d + i)
+                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    for (int t = 0; t < n_tok; ++t) {
+        const size_t r = (size_t)(row0 + t);
+        const T* row = rows + r * g.row_elems;
+        float q[NV][4], k[NV][4], a[NV][4];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const int i = v * 128 + lane * 4, c = h * d + i;
+            if (i < d) {                                     // (d is a multiple of 4)
+                float b[4];
+                load_four(row + g.q_off + c, q[v]);
+                load_four(row + g.k_off + c, k[v]);
+                load_four(z + r * H * d + c, a[v]);
+                load_four(bias + c, b);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    q[v][e] *= g.q_scale;
+                    a[v][e] = expf(log_sigmoid(a[v][e] + b[e]) * g.inv_tau);
+                }
+                if (col0 == 0) Vec16<float>::store(decay + r * H * d + c, a[v]);       // (the caller may want them)
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) q[v][e] = k[v][e] = a[v][e] = 0.f;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int col = min(col0 + j, dv - 1);
+            const float x = to_float(row[g.v_off + h * dv + col]);
+            float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                S[j][v].x = fmaf(a[v][0], S[j][v].x, k[v][0] * x);
+                S[j][v].y = fmaf(a[v][1], S[j][v].y, k[v][1] * x);
+                S[j][v].z = fmaf(a[v][2], S[j][v].z, k[v][2] * x);
+                S[j][v].w = fmaf(a[v][3], S[j][v].w, k[v][3] * x);
+                part[0] = fmaf(S[j][v].x, q[v][0], part[0]);
+                part[1] = fmaf(S[j][v].y, q[v][1], part[1]);
+                part[2] = fmaf(S[j][v].z, q[v][2], part[2]);
+                part[3] = fmaf(S[j][v].w, q[v][3], part[3]);
+            }
+            const float o = warp_sum((part[0] + part[1]) + (part[2] + part[3]));
+            if (lane == 0 && col0 + j < dv) o_out[r * H * dv + h * dv + col0 + j] = o;
+        }
+    }
+    if (st != nullptr) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const int i = v * 128 + lane * 4;
+                if (col0 + j < dv && i < d) *reinterpret_cast<float4*>(st + (size_t)(col0 + j) * d + i) = S[j][v];
+            }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Matrix memory with exponential gates (mLSTM): per head and sequence a matrix C [d, dv], a vector n [d] and a
 // running maximum m, all float:
@@ -514,6 +611,18 @@ static int gla_scan_launch(const void* rows, const GlaRows& g, const float* deca
     return fail("gla_scan: key size %d is above %d", g.d, GLA_KS * 16);
 }
 
+template <typename T>
+static int gla_step_launch(const void* rows, const GlaRows& g, const void* z, const void* bias, const int* seq_slot, const int* seq_first_row,
+                           const int* seq_start, const int* seq_end, float* state, float* o_out, float* decay, int n_seq, cudaStream_t stream) {
+    const int per_cta = g.d <= 128 ? 32 : 16;
+    const dim3 grid(n_seq, g.H, (g.dv + per_cta - 1) / per_cta), block(256);
+    if (g.d <= 128)
+        return launch_kernel("gla_scan", gla_step_kernel<T, 1>, grid, block, 0, stream, 1, (const T*)rows, g, (const T*)z, (const T*)bias, seq_slot,
+                             seq_first_row, seq_start, seq_end, state, o_out, decay);
+    return launch_kernel("gla_scan", gla_step_kernel<T, 2>, grid, block, 0, stream, 1, (const T*)rows, g, (const T*)z, (const T*)bias, seq_slot,
+                         seq_first_row, seq_start, seq_end, state, o_out, decay);
+}
+
 JANIS_EXPORT int janis_gla_scan(const void* rows, int dtype, int row_elems, int q_off, int k_off, int v_off,
                                 const void* z_rows, const void* z_bias, float* decay, int n_tok, const int* seq_slot,
                                 const int* seq_first_row, const int* seq_start, const int* seq_end, float* state,
@@ -525,6 +634,13 @@ JANIS_EXPORT int janis_gla_scan(const void* rows, int dtype, int row_elems, int 
     GlaRows g;
     g.row_elems = row_elems; g.q_off = q_off; g.k_off = k_off; g.v_off = v_off;
     g.H = H; g.d = d; g.dv = dv; g.q_scale = q_scale; g.inv_tau = 1.0f / tau;
+    // a token a sequence, whole runs of four key channels on their alignment, up to 256 of them: the form that only loads and stores the state
+    const uintptr_t run = dtype == JANIS_F32 ? 16 : 8;
+    if (n_tok <= n_seq && d % 4 == 0 && d <= 256 && (((uintptr_t)state | (uintptr_t)decay) & 15) == 0 && (dv + 15) / 16 <= 65535 && row_elems % 4 == 0 && q_off % 4 == 0 &&
+        k_off % 4 == 0 && ((uintptr_t)rows | (uintptr_t)z_rows | (uintptr_t)z_bias) % run == 0) {
+        if (dtype == JANIS_F32) return gla_step_launch<float>(rows, g, z_rows, z_bias, seq_slot, seq_first_row, seq_start, seq_end, state, o_out, decay, n_seq, stream);
+        if (dtype == JANIS_BF16) return gla_step_launch<bf16>(rows, g, z_rows, z_bias, seq_slot, seq_first_row, seq_start, seq_end, state, o_out, decay, n_seq, stream);
+    }
     const size_t n = (size_t)n_tok * H * d, want = (n + 255) / 256;
     const dim3 dgrid((unsigned)(want < 148 * 16 ? want : 148 * 16)), dblock(256);
     if (dtype == JANIS_F32) {

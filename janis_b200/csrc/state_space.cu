@@ -242,40 +242,6 @@ struct ScanShape {
 
 constexpr int SCAN_THREADS = 128;
 
-// Step sizes once per (token, head), as floats: delta = softplus(dt + bias) and, where a head has one decay,
-// exp(delta A) - 1.  (Left to the scan, every lane of a channel and every channel of a head would form them again.)
-// For a prompt that runs in pieces (selective_scan_piece_kernel) the first warp also counts the sequences' pieces through, in
-// whatever order their rows lie: where[s] is the number before sequence s's first one.
-template <typename T>
-__global__ void __launch_bounds__(256)
-scan_steps_kernel(const T* __restrict__ dt_rows, int dt_stride, int dt_off, const float* __restrict__ dt_bias,
-                  const float* __restrict__ A_head, float* __restrict__ delta, float* __restrict__ grow, int heads, size_t n,
-                  int* __restrict__ where, int piece, int n_seq, const int* __restrict__ seq_start, const int* __restrict__ seq_end) {
-    grid_dependents_launch();
-    grid_dependency_wait();
-    if (where != nullptr && blockIdx.x == 0 && threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        for (int s0 = 0, before = 0; s0 < n_seq; s0 += 32) {
-            const int n = pieces_of(seq_start, seq_end, s0 + lane, n_seq, piece);
-            int upto = before + n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, upto, o);
-                if (lane >= o) upto += v - before;
-            }
-            if (s0 + lane < n_seq) where[s0 + lane] = upto - n;
-            before = __shfl_sync(0xffffffffu, upto, 31);
-        }
-    }
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t t = i / heads;
-        const int h = (int)(i % heads);
-        const float d = softplus_f(to_float(dt_rows[t * dt_stride + dt_off + h]) + dt_bias[h]);
-        delta[i] = d;
-        if (A_head != nullptr) grow[i] = decay_minus_one(d * A_head[h]);
-    }
-}
-
 // SPL consecutive values as floats; VEC: loads of min(16, SPL * sizeof(T)) bytes (the address is aligned to that)
 template <typename T, int SPL, bool VEC>
 __device__ __forceinline__ void load_run(const T* __restrict__ p, float (&out)[SPL]) {
@@ -309,6 +275,63 @@ __device__ __forceinline__ void load_run(const T* __restrict__ p, float (&out)[S
     } else {
 #pragma unroll
         for (int k = 0; k < SPL; ++k) out[k] = to_float(p[k]);
+    }
+}
+
+// Step sizes once per (token, head), as floats: delta = softplus(dt + bias) and, where a head has one decay,
+// exp(delta A) - 1.  (Left to the scan, every lane of a channel and every channel of a head would form them again.)
+// For a prompt that runs in pieces (selective_scan_piece_kernel) the first warp also counts the sequences' pieces through, in
+// whatever order their rows lie: where[s] is the number before sequence s's first one.
+template <typename T>
+__global__ void __launch_bounds__(256)
+scan_steps_kernel(const T* __restrict__ dt_rows, int dt_stride, int dt_off, const float* __restrict__ dt_bias,
+                  const float* __restrict__ A_head, float* __restrict__ delta, float* __restrict__ grow, int heads, size_t n,
+                  int* __restrict__ where, int piece, int n_seq, const int* __restrict__ seq_start, const int* __restrict__ seq_end) {
+    grid_dependents_launch();
+    grid_dependency_wait();
+    if (where != nullptr && blockIdx.x == 0 && threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        for (int s0 = 0, before = 0; s0 < n_seq; s0 += 32) {
+            const int n = pieces_of(seq_start, seq_end, s0 + lane, n_seq, piece);
+            int upto = before + n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v - before;
+            }
+            if (s0 + lane < n_seq) where[s0 + lane] = upto - n;
+            before = __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    // Four heads a thread where they lie on their alignment, and places of 32 bits (a place's token by a 64-bit division for every
+    // head, and one head a thread: 2,048 tokens of 4,608 heads 35 us; so 18.9)
+    const bool four = heads % 4 == 0 && dt_stride % 4 == 0 && dt_off % 4 == 0 && n <= 0x7fffffffu &&
+                      ((uintptr_t)dt_rows % (4 * sizeof(T)) | (((uintptr_t)delta | (uintptr_t)grow | (uintptr_t)dt_bias | (uintptr_t)A_head) & 15)) == 0;
+    if (four) {
+        const unsigned per_row = (unsigned)heads / 4, pieces = (unsigned)(n / 4);
+        for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += gridDim.x * blockDim.x) {
+            const unsigned t = i / per_row, h = (i - t * per_row) * 4;
+            float dt[4], bias[4];
+            load_run<T, 4, true>(dt_rows + (size_t)t * dt_stride + dt_off + h, dt);
+            Vec16<float>::load(dt_bias + h, bias);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) dt[e] = softplus_f(dt[e] + bias[e]);
+            Vec16<float>::store(delta + (size_t)i * 4, dt);
+            if (A_head != nullptr) {
+                Vec16<float>::load(A_head + h, bias);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) dt[e] = decay_minus_one(dt[e] * bias[e]);
+                Vec16<float>::store(grow + (size_t)i * 4, dt);
+            }
+        }
+        return;
+    }
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t t = i / heads;
+        const int h = (int)(i % heads);
+        const float d = softplus_f(to_float(dt_rows[t * dt_stride + dt_off + h]) + dt_bias[h]);
+        delta[i] = d;
+        if (A_head != nullptr) grow[i] = decay_minus_one(d * A_head[h]);
     }
 }
 
@@ -419,6 +442,79 @@ selective_scan_kernel(const T* __restrict__ u_rows, const T* __restrict__ bc_row
 #pragma unroll
         for (int k = 0; k < SPL; ++k)
             if (n0 + k < N) st[n0 + k] = S[k];
+    }
+}
+
+// One token a sequence (a decode step): the state comes and goes once, and nothing else costs.  Four states a lane, LN lanes a channel
+// (16-byte accesses that are whole lines across a warp), J channels a lane in flight; the state is asked for (into L2) before the
+// kernel waits for the one that makes its inputs, and the step sizes are formed here.  Sequences of more tokens run through them in
+// turn.  Eight sequences, 4,608 channels of 128 states, one decay a head: 25.1 us with its step sizes' kernel -> 14.2; of
+// 16 states: 25.7 -> 3.5 (the form above computes a tile of 8 or 2 tokens of which one is there).
+template <typename T, int LN, bool PER_STATE>
+__global__ void __launch_bounds__(256)
+scan_step_kernel(const T* __restrict__ u_rows, const T* __restrict__ bc_rows, const T* __restrict__ z_rows, const T* __restrict__ dt_rows,
+                 int dt_stride, int dt_off, const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
+                 ScanShape g, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
+                 const int* __restrict__ seq_end, float* __restrict__ state, void* __restrict__ out_raw) {
+    constexpr int N = 4 * LN, CH = 32 / LN, J = LN >= 16 ? 4 : 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, seq = blockIdx.x, n0 = (lane % LN) * 4;
+    grid_dependents_launch();
+    const int slot = seq_slot[seq], row0 = seq_first_row[seq], n_tok = seq_end[seq] - seq_start[seq];
+    int c[J];
+    float4 S[J], a4[J];
+    float Dh[J], Ah[J], bias[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const int raw = ((blockIdx.y * 8 + warp) * J + j) * CH + lane / LN;
+        c[j] = raw < g.C ? raw : -1;
+        if (c[j] < 0 || n_tok <= 0) continue;
+        if (slot >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(state + ((size_t)slot * g.C + c[j]) * N + n0));
+        const int head = c[j] / g.cph;
+        Dh[j] = D[head];
+        bias[j] = dt_bias[head];
+        if (PER_STATE) a4[j] = *reinterpret_cast<const float4*>(A + (size_t)head * N + n0);
+        else Ah[j] = A[head];
+    }
+    grid_dependency_wait();
+    if (n_tok <= 0) return;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+        S[j] = c[j] >= 0 && slot >= 0 ? *reinterpret_cast<const float4*>(state + ((size_t)slot * g.C + c[j]) * N + n0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t = 0; t < n_tok; ++t) {
+        const size_t row = (size_t)(row0 + t);
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int ch = c[j] >= 0 ? c[j] : 0, head = ch / g.cph;
+            float B[4], Cc[4];
+            const T* b = bc_rows + row * g.bc_stride + g.b_off + ch / g.cpg * N + n0;
+            load_run<T, 4, true>(b, B);
+            load_run<T, 4, true>(b + g.c_off - g.b_off, Cc);
+            const float u = to_float(u_rows[row * g.u_stride + g.u_off + ch]);
+            const float d = softplus_f(to_float(dt_rows[row * dt_stride + dt_off + head]) + bias[j]), du = d * u;
+            float gr[4];
+            if (PER_STATE) {
+                gr[0] = decay_minus_one(d * a4[j].x); gr[1] = decay_minus_one(d * a4[j].y);
+                gr[2] = decay_minus_one(d * a4[j].z); gr[3] = decay_minus_one(d * a4[j].w);
+            } else gr[0] = gr[1] = gr[2] = gr[3] = decay_minus_one(d * Ah[j]);
+            S[j].x = decayed(S[j].x, gr[0], du * B[0]);
+            S[j].y = decayed(S[j].y, gr[1], du * B[1]);
+            S[j].z = decayed(S[j].z, gr[2], du * B[2]);
+            S[j].w = decayed(S[j].w, gr[3], du * B[3]);
+            float acc = fmaf(S[j].z, Cc[2], S[j].x * Cc[0]) + fmaf(S[j].w, Cc[3], S[j].y * Cc[1]);
+#pragma unroll
+            for (int off = LN >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+            if (lane % LN == 0 && c[j] >= 0) {
+                const float y = fmaf(Dh[j], u, acc);
+                const size_t at = row * g.C + ch;
+                if (g.gated) reinterpret_cast<T*>(out_raw)[at] = from_float<T>(y * silu_f(to_float(z_rows[row * g.z_stride + g.z_off + ch])));
+                else reinterpret_cast<float*>(out_raw)[at] = y;
+            }
+        }
+    }
+    if (slot >= 0) {
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+            if (c[j] >= 0) *reinterpret_cast<float4*>(state + ((size_t)slot * g.C + c[j]) * N + n0) = S[j];
     }
 }
 
@@ -738,6 +834,49 @@ gate_group_norm_kernel(const float* __restrict__ o, const T* __restrict__ rows, 
         dst[i] = from_float<T>(src[i] * silu_f(to_float(z[i])) * inv * w[c0 + i]);
 }
 
+// The same with the part in registers: NV times eight values a thread (runs on 16 bytes), read once, the gate formed once.  8 tokens of
+// one part of 4,608: 4.7 us of a decode step against 15.3; 2,048 tokens 20.2 against 39.5.
+template <typename T, int NV>
+__global__ void __launch_bounds__(256)
+gate_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ rows, int row_elems, int z_off,
+                           const float* __restrict__ w, float eps, T* __restrict__ out, int C, int per) {
+    __shared__ float scratch[32];
+    const size_t t = blockIdx.x;
+    const int c0 = blockIdx.y * per;
+    const float* src = o + t * C + c0;
+    const T* z = rows + t * row_elems + z_off + c0;
+    float v[NV][8], ww[NV][8];
+    grid_dependents_launch();
+    grid_dependency_wait();
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * 256 + threadIdx.x) * 8;
+        if (i < per) {
+            float gate[8];
+            load_eight(w + c0 + i, ww[n]);
+            load_eight(src + i, v[n]);
+            load_eight(z + i, gate);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                v[n][e] *= silu_f(gate[e]);
+                ss = fmaf(v[n][e], v[n][e], ss);
+            }
+        }
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.0f / sqrtf(ss / (float)per + eps);
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * 256 + threadIdx.x) * 8;
+        if (i < per) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[n][e] = v[n][e] * inv * ww[n][e];
+            store_eight(out + t * C + c0 + i, v[n]);
+        }
+    }
+}
+
 }  // namespace janis
 
 using namespace janis;
@@ -866,6 +1005,27 @@ static int scan_launch(const void* u, const void* bc, const void* z, const float
 // Floats of scratch for a sequence's pieces beside the 2 n_tok heads of the step sizes, a piece.
 static long long scan_piece_floats(int C, int N) { return (long long)C * (N + 1); }
 
+template <typename T, bool PER_STATE>
+static int scan_step_launch(const void* u, const void* bc, const void* z, const void* dt, int dt_stride, int dt_off, const float* dt_bias,
+                            const float* A, const float* D, const ScanShape& g, const int* seq_slot, const int* seq_first_row,
+                            const int* seq_start, const int* seq_end, int n_seq, float* state, void* out, cudaStream_t stream) {
+#define JANIS_SCAN_STEP(LN)                                                                                                        \
+    if (g.N == 4 * LN) {                                                                                                           \
+        const int per_cta = 8 * (32 / LN) * (LN >= 16 ? 4 : 1);                                                                    \
+        return launch_kernel("selective_scan", scan_step_kernel<T, LN, PER_STATE>, dim3(n_seq, (g.C + per_cta - 1) / per_cta), dim3(256), 0, stream, 1, \
+                             (const T*)u, (const T*)bc, (const T*)z, (const T*)dt, dt_stride, dt_off, dt_bias, A, D, g, seq_slot, seq_first_row,       \
+                             seq_start, seq_end, state, out);                                                                      \
+    }
+    JANIS_SCAN_STEP(1)
+    JANIS_SCAN_STEP(2)
+    JANIS_SCAN_STEP(4)
+    JANIS_SCAN_STEP(8)
+    JANIS_SCAN_STEP(16)
+    JANIS_SCAN_STEP(32)
+#undef JANIS_SCAN_STEP
+    return fail("selective_scan: no one-token form for %d states", g.N);
+}
+
 template <typename T, int N>
 static int scan_pieces_launch(const void* u, const void* bc, const void* z, const float* delta, const float* A, const float* D, ScanShape g,
                               int piece, const int* where, int n_tok, const int* seq_slot, const int* seq_first_row, const int* seq_start,
@@ -913,6 +1073,21 @@ JANIS_EXPORT int janis_selective_scan(const void* u, int dtype, int u_stride, in
     g.u_stride = u_stride; g.u_off = u_off; g.bc_stride = bc_stride; g.b_off = b_off; g.c_off = c_off;
     g.z_stride = z_stride; g.z_off = z_off; g.gated = z != nullptr ? 1 : 0;
     g.C = C; g.N = N; g.cph = cph; g.cpg = cpg; g.heads = C / cph;
+    // A token a sequence, a power of two of states from 4 to 128, runs of four states aligned: the form that only loads and stores them.
+    if (n_tok <= n_seq && N >= 4 && N <= 128 && (N & (N - 1)) == 0 && !scan_lanes_forced && !scan_form_forced && (C + 7) / 8 <= 65535 &&
+        (dtype == JANIS_BF16 || dtype == JANIS_F32)) {
+        const size_t run4 = dtype == JANIS_F32 ? 16 : 8;
+        if ((((uintptr_t)state | (uintptr_t)A) & 15) == 0 && (uintptr_t)bc % run4 == 0 && bc_stride % 4 == 0 && b_off % 4 == 0 && c_off % 4 == 0) {
+#define JANIS_STEP(T, PER)                                                                                                                 \
+    return scan_step_launch<T, PER>(u, bc, z, dt, dt_stride, dt_off, dt_bias, A, D, g, seq_slot, seq_first_row, seq_start, seq_end, n_seq, state, \
+                                    out, stream);
+            if (dtype == JANIS_F32 && a_per_state) { JANIS_STEP(float, true) }
+            if (dtype == JANIS_F32) { JANIS_STEP(float, false) }
+            if (a_per_state) { JANIS_STEP(bf16, true) }
+            JANIS_STEP(bf16, false)
+#undef JANIS_STEP
+        }
+    }
     // Lanes a channel and states a lane.  What a token costs beside its states is shared by the states of a lane, so a
     // prompt takes the fewest lanes that still give the launch some 256 CTAs, among the pairs that waste the fewest
     // places (else the most lanes among them).  A step of one token a sequence only loads and stores the state: it
@@ -1024,6 +1199,17 @@ JANIS_EXPORT int janis_gate_group_norm(const float* o, const void* rows, int dty
     if (T <= 0) return 0;
     if (n_groups <= 0 || C % n_groups || n_groups > 65535) return fail("gate_group_norm: %d channels in %d parts", C, n_groups);
     const dim3 grid(T, n_groups), block(256);
+    const int per = C / n_groups;
+    const int epp = dtype == JANIS_F32 ? 4 : 8;                 // (a row's places on 16 bytes)
+    if (per % 8 == 0 && per <= 8192 && z_off % epp == 0 && row_elems % epp == 0 && (((uintptr_t)o | (uintptr_t)rows | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
+#define JANIS_GGN(TT, NV)                                                                                              \
+    if (per <= NV * 2048)                                                                                              \
+        return launch_kernel("gate_group_norm", gate_group_norm_vec_kernel<TT, NV>, grid, block, 0, stream, 1, o, (const TT*)rows, row_elems, z_off, \
+                             w, eps, (TT*)out, C, per);
+        if (dtype == JANIS_F32) { JANIS_GGN(float, 1) JANIS_GGN(float, 2) JANIS_GGN(float, 3) JANIS_GGN(float, 4) }
+        if (dtype == JANIS_BF16) { JANIS_GGN(bf16, 1) JANIS_GGN(bf16, 2) JANIS_GGN(bf16, 3) JANIS_GGN(bf16, 4) }
+#undef JANIS_GGN
+    }
     if (dtype == JANIS_F32)
         return launch_kernel("gate_group_norm", gate_group_norm_kernel<float>, grid, block, 0, stream, 1, o, (const float*)rows,
                              row_elems, z_off, w, eps, (float*)out, C, C / n_groups);

@@ -1180,10 +1180,10 @@ def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_
     _t(decay, "decay", torch.float32, (T, H * d))
     _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv)
     lib = mixers()
-    _check(lib, lib.janis_gla_scan(rows.data_ptr(), _DT[rows.dtype], width, q_off, k_off, v_off, z.data_ptr(),
-                                   z_bias.data_ptr(), decay.data_ptr(), T, seq_slot.data_ptr(), seq_first_row.data_ptr(),
-                                   seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(), n_seq,
-                                   H, d, dv, float(q_scale), float(tau), _stream()), kernels=2)
+    _check_counted(lib, lib.janis_gla_scan, rows.data_ptr(), _DT[rows.dtype], width, q_off, k_off, v_off, z.data_ptr(),
+                   z_bias.data_ptr(), decay.data_ptr(), T, seq_slot.data_ptr(), seq_first_row.data_ptr(),
+                   seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(), n_seq,
+                   H, d, dv, float(q_scale), float(tau), _stream())
     return o_out
 
 

@@ -1155,3 +1155,62 @@ def test_repeat_penalty_and_mask():
     ops().mask_tokens(logits, ids.to(dev()))
     assert torch.isinf(logits[:, 1]).all() and torch.isinf(logits[:, 50]).all()
     assert torch.isfinite(logits[:, 2]).all()
+
+
+# ---------------------------------------------------------------------------
+# one token a sequence: the states' own forms
+# ---------------------------------------------------------------------------
+
+def _step_tables(lens, slots):
+    lens = torch.tensor(lens, dtype=torch.int32)
+    first = (lens.cumsum(0) - lens).int()
+    start = torch.tensor([7 * i for i in range(len(lens))], dtype=torch.int32)
+    return torch.tensor(slots, dtype=torch.int32), first, start, (start + lens).int()
+
+
+# one token each, a padding sequence among them; an empty sequence beside one of two tokens (as many tokens as sequences)
+STEP_BATCHES = [([1, 1, 1, 1, 1], [3, 0, -1, 5, 1]), ([1, 0, 2], [2, 4, 0]), ([1], [1])]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens,slots", STEP_BATCHES)
+@pytest.mark.parametrize("N,C,cph,cpg,per_state,gated", [(4, 40, 1, 40, True, True), (16, 4608, 1, 4608, True, True), (8, 72, 8, 24, False, False),
+                                                        (32, 33, 1, 11, True, False), (64, 130, 65, 130, False, True), (128, 192, 64, 96, False, False)])
+def test_selective_scan_of_one_token_each(dtype, lens, slots, N, C, cph, cpg, per_state, gated):
+    g = torch.Generator().manual_seed(N + C)
+    T, groups, heads = sum(lens), C // cpg, C // cph
+    seq_slot, first, start, end = _step_tables(lens, slots)
+    mk = lambda *s: torch.randn(*s, generator=g)
+    u, dt, bc, z = (mk(T, w).to(dtype) for w in (C + 3, heads + 1, 2 * groups * N + 8, C + 1))
+    dt_bias, D, A = mk(heads) - 1.0, mk(heads), -torch.exp(mk(heads, N) if per_state else mk(heads))
+    state = mk(6, C, N)
+    out_dtype = dtype if gated else torch.float32
+    want, want_state = torch.zeros(T, C, dtype=out_dtype), state.clone()
+    args = lambda dev, st, out: (dev(u), 2, dev(dt), 1, dev(dt_bias), dev(A), per_state, dev(bc), 4, 4 + groups * N, dev(D), dev(z) if gated else None, 1,
+                                 dev(seq_slot), dev(first), dev(start), dev(end), len(lens), st, out, C, N, cph, cpg)
+    R.selective_scan(*args(lambda x: x, want_state, want))
+    got, got_state = torch.full((T, C), float("nan"), dtype=out_dtype, device=dev()), state.clone().to(dev())
+    ops().selective_scan(*args(lambda x: x.to(dev()), got_state, got))
+    close(got, want, tol_of(out_dtype) if out_dtype == torch.bfloat16 else 5e-5, "results")
+    close(got_state, want_state, 5e-5, "the states left behind")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("lens,slots", STEP_BATCHES)
+@pytest.mark.parametrize("H,d,dv", [(8, 128, 256), (2, 4, 7), (3, 132, 40), (1, 256, 33)])
+def test_gated_linear_attention_of_one_token_each(dtype, lens, slots, H, d, dv):
+    g = torch.Generator().manual_seed(d + dv)
+    T = sum(lens)
+    seq_slot, first, start, end = _step_tables(lens, slots)
+    width = (2 * H * d + H * dv + 7) // 4 * 4
+    rows, z, b = (torch.randn(*s, generator=g).to(dtype) for s in ((T, width), (T, H * d), (H * d,)))
+    state = torch.randn(6, H, dv, d, generator=g)
+    want, want_state = torch.zeros(T, H * dv), state.clone()
+    args = lambda dev, st, out: (dev(rows), 0, H * d, 2 * H * d, dev(z), dev(b), dev(seq_slot), dev(first), dev(start), dev(end), st, out, len(lens), H, d, dv,
+                                 d ** -0.5, 16.0)
+    R.gla_scan(*args(lambda x: x, want_state, want))
+    got, got_state, decay = torch.full((T, H * dv), float("nan"), device=dev()), state.clone().to(dev()), torch.zeros(T, H * d, device=dev())
+    ops().gla_scan(*args(lambda x: x.to(dev()), got_state, got), decay=decay)
+    close(got, want, 5e-5, "results")
+    close(got_state, want_state, 5e-5, "the states left behind")
+    close(decay, torch.sigmoid(z.double() + b.double()) ** (1 / 16.0), 1e-5, "the decays")
