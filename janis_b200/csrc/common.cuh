@@ -8,6 +8,7 @@
 #include <stdarg.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <string.h>
 
 #define JANIS_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -283,6 +284,33 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return t;
 }
 
+// exp(x) - 1 for x <= 0 without a branch, for kernels that form one per value and do little else.
+// x = j ln 2 + f with a whole j (Cody and Waite's reduction: ln 2 in two floats), e^f - 1 is its Taylor series up to f^8 (the
+// next term is 6e-10 of the sum at |f| = ln 2 / 2), and 2^j (e^f - 1) + (2^j - 1) has one rounding: within 0.881 units in the
+// last place of exp(x) - 1, as compared with 64 bits at every negative float.
+__host__ __device__ __forceinline__ float shrink_minus_one(float x) {
+    x = x < -30.f ? -30.f : x;                            // (-1 there already; a NaN stays one)
+    const float t = fmaf(x, 1.44269504f, 12582912.f), j = t - 12582912.f;      // x / ln 2 rounded, and in the low bits of t
+    const float f = fmaf(j, -1.42860682e-6f, fmaf(j, -0.693145751953125f, x));
+    float p = fmaf(1.f / 40320.f, f, 1.f / 5040.f);
+    p = fmaf(p, f, 1.f / 720.f);
+    p = fmaf(p, f, 1.f / 120.f);
+    p = fmaf(p, f, 1.f / 24.f);
+    p = fmaf(p, f, 1.f / 6.f);
+    p = fmaf(p, f, 0.5f);
+#ifdef __CUDA_ARCH__
+    const float s = __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
+#else
+    uint32_t bits;
+    float s;
+    memcpy(&bits, &t, 4);
+    bits = (bits << 23) + 0x3f800000u;
+    memcpy(&s, &bits, 4);
+#endif
+    const float q = fmaf(f * f, p, f);
+    return fmaf(s, q, s - 1.f);
+}
+
 __device__ __forceinline__ float gelu_tanh(float v) {
     const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
     return 0.5f * v * (1.0f + tanhf(inner));
@@ -298,7 +326,7 @@ __device__ __forceinline__ float clamped_gate(float gate, float up, float limit,
 // a_neg = 1/2 + softplus(q) formed on the host (z > 0: a_pos z^2 + z/2; z <= 0: a_neg (e^z - 1 - z) + z/2);
 // 2 the tanh form of gelu; 3 silu; 4 the square of relu.
 __device__ __forceinline__ float dense_act(float z, int act, float a_pos, float a_neg) {
-    if (act == 1) return z > 0.f ? fmaf(a_pos * z, z, 0.5f * z) : fmaf(a_neg, expm1f(z) - z, 0.5f * z);
+    if (act == 1) return z > 0.f ? fmaf(a_pos * z, z, 0.5f * z) : fmaf(a_neg, shrink_minus_one(z) - z, 0.5f * z);
     if (act == 2) return gelu_tanh(z);
     if (act == 3) return z / (1.0f + expf(-z));
     if (act == 4) return z > 0.f ? z * z : 0.f;

@@ -30,32 +30,6 @@ __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log
 // small against S and its rounding does not count; what remains is the one rounding of the sum.
 __device__ __forceinline__ float decay_minus_one(float x) { return expm1f(x); }
 
-// The same for x <= 0 without a branch, for the selective scan's prompts, which form one per state and token and do little else.
-// x = j ln 2 + f with a whole j (Cody and Waite's reduction: ln 2 in two floats), e^f - 1 is its Taylor series up to f^8 (the
-// next term is 6e-10 of the sum at |f| = ln 2 / 2), and 2^j (e^f - 1) + (2^j - 1) has one rounding: within 0.881 units in the
-// last place of exp(x) - 1, as compared with 64 bits at every negative float.
-__host__ __device__ __forceinline__ float shrink_minus_one(float x) {
-    x = x < -30.f ? -30.f : x;                            // (-1 there already; a NaN stays one)
-    const float t = fmaf(x, 1.44269504f, 12582912.f), j = t - 12582912.f;      // x / ln 2 rounded, and in the low bits of t
-    const float f = fmaf(j, -1.42860682e-6f, fmaf(j, -0.693145751953125f, x));
-    float p = fmaf(1.f / 40320.f, f, 1.f / 5040.f);
-    p = fmaf(p, f, 1.f / 720.f);
-    p = fmaf(p, f, 1.f / 120.f);
-    p = fmaf(p, f, 1.f / 24.f);
-    p = fmaf(p, f, 1.f / 6.f);
-    p = fmaf(p, f, 0.5f);
-#ifdef __CUDA_ARCH__
-    const float s = __int_as_float((__float_as_int(t) << 23) + 0x3f800000);
-#else
-    uint32_t bits;
-    float s;
-    memcpy(&bits, &t, 4);
-    bits = (bits << 23) + 0x3f800000u;
-    memcpy(&s, &bits, 4);
-#endif
-    const float q = fmaf(f * f, p, f);
-    return fmaf(s, q, s - 1.f);
-}
 __device__ __forceinline__ float decayed(float S, float grow, float input) { return S + fmaf(S, grow, input); }
 
 // ---------------------------------------------------------------------------
@@ -109,17 +83,31 @@ causal_conv_silu_kernel(const T* __restrict__ rows, int row_elems, int col_off, 
     }
 }
 
-// The same with 16 bytes of channels a thread, up to four taps: a thread takes its channels over a run of tokens in turn and
+__device__ __forceinline__ void load_channels(const float* p, float* o) { Vec16<float>::load(p, o); }
+__device__ __forceinline__ void load_channels(const bf16* p, float* o) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
+    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store_channels(float* p, const float* v) { Vec16<float>::store(p, v); }
+__device__ __forceinline__ void store_channels(bf16* p, const float* v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
+// The same with four channels a thread, up to four taps: a thread takes its channels over a run of tokens in turn and
 // keeps the last K - 1 inputs in registers while the tokens are one sequence's; four tokens' inputs are asked for together.
+// (Eight channels a thread took 136 registers, three CTAs an SM, and 0.31 instructions a scheduler's cycle: 2,048 tokens of 4,608
+// channels 42 us; four, 26.5.)
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 5)
 causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, int C, int K,
                        const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ state,
                        const int* __restrict__ tok_seq, const int* __restrict__ seq_slot,
                        const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
                        const int* __restrict__ seq_end, T* __restrict__ out, int n_tok, int run, int act,
                        const float* __restrict__ in_bias) {
-    constexpr int V = Vec16<T>::N, KM = 4, AHEAD = 4;
+    constexpr int V = 4, KM = 4, AHEAD = 4;
     const int per_row = C / V, idx = blockIdx.x * blockDim.x + threadIdx.x;
     const int piece = idx / per_row, c = (idx - piece * per_row) * V, t0 = piece * run, t1 = min(n_tok, t0 + run);
     grid_dependents_launch();
@@ -148,7 +136,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
         float x[AHEAD][V];
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
-            if (tb + a < t1) Vec16<T>::load(rows + (size_t)(tb + a) * row_elems + col_off + c, x[a]);
+            if (tb + a < t1) load_channels(rows + (size_t)(tb + a) * row_elems + col_off + c, x[a]);
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a) {
             const int t = tb + a;
@@ -163,7 +151,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
                 for (int j = 0; j < KM - 1; ++j) {
                     const int at = i - 1 - j;
                     if (j < K - 1 && at >= 0) {
-                        Vec16<T>::load(rows + (size_t)(t - 1 - j) * row_elems + col_off + c, past[j]);
+                        load_channels(rows + (size_t)(t - 1 - j) * row_elems + col_off + c, past[j]);
 #pragma unroll
                         for (int e = 0; e < V; ++e) past[j][e] += xb[e];
                     } else {
@@ -185,7 +173,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
                 for (int j = KM - 2; j > 0; --j) past[j][e] = past[j - 1][e];
                 past[0][e] = x[a][e];
             }
-            Vec16<T>::store(out + (size_t)t * C + c, y);
+            store_channels(out + (size_t)t * C + c, y);
             if (alone && st != nullptr) {                    // the sequence's only token of the step: the kept inputs move on
 #pragma unroll
                 for (int j = 0; j < KM - 1; ++j)
@@ -888,13 +876,13 @@ static int conv_launch(const void* rows, int row_elems, int col_off, int C, int 
                        int act, const float* in_bias, cudaStream_t stream) {
     const int by = (C + 255) / 256, tpc = n_tok >= 1024 ? 8 : 1;
     if (by > 65535) return fail("causal_conv_silu: too many channels (%d)", C);
-    constexpr int V = Vec16<T>::N;
+    constexpr int V = 4;
     if (K <= 4 && n_tok > 64 && C % V == 0 && col_off % V == 0 && row_elems % V == 0 &&
         (((uintptr_t)rows | (uintptr_t)out | (uintptr_t)state | (uintptr_t)w) & 15) == 0) {
-        // (few rows: a thread a channel and token has less to do.)  Runs of tokens as long as every SM still gets two CTAs
+        // (few rows: a thread a channel and token has less to do.)  Runs of tokens as long as every SM still gets six CTAs
         const int per_row = C / V;
         int run = 1;
-        while (run < 16 && (long long)((n_tok + 2 * run - 1) / (2 * run)) * per_row >= 148LL * 2 * 128) run *= 2;
+        while (run < 16 && (long long)((n_tok + 2 * run - 1) / (2 * run)) * per_row >= 148LL * 6 * 128) run *= 2;
         const long long threads = (long long)((n_tok + run - 1) / run) * per_row;
         if (launch_kernel("causal_conv_silu", causal_conv_vec_kernel<T>, dim3((unsigned)((threads + 127) / 128)), dim3(128), 0, stream, 1,
                           (const T*)rows, row_elems, col_off, C, K, w, bias, state, tok_seq, seq_slot, seq_first_row, seq_start,
