@@ -152,6 +152,8 @@ def mixers():
         lib.janis_talk_prompt_chunks.restype = I
         lib.janis_gla_chunks_floats.argtypes = [I, I, I, I, I]
         lib.janis_gla_chunks_floats.restype = c_longlong
+        lib.janis_gla_chunks_least.argtypes = [I, I, I, I, I]
+        lib.janis_gla_chunks_least.restype = c_longlong
         lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P, c_longlong, P]
         lib.janis_talk_attention_rows_mixed_floats.argtypes = [I, I, I, I, I, I, I]
         lib.janis_talk_attention_rows_mixed_floats.restype = c_longlong
@@ -1134,11 +1136,19 @@ def gla_chunks_floats(dtype, T: int, n_seq: int, H: int, d: int, dv: int) -> int
     if dtype != torch.bfloat16 or T < max(GLA_CHUNK_TOKENS * n_seq, GLA_CHUNK_STEP):
         return 0
     n = int(mixers().janis_gla_chunks_floats(int(T), int(n_seq), int(H), int(d), int(dv)))
+    return n if n <= GLA_CHUNK_FLOATS else _gla_chunks_least(dtype, T, n_seq, H, d, dv)
+
+
+def _gla_chunks_least(dtype, T: int, n_seq: int, H: int, d: int, dv: int) -> int:
+    """What the chunks alone take (`gla_chunks_floats` adds room in which few sequences' chains run in pieces)."""
+    if dtype != torch.bfloat16 or T < max(GLA_CHUNK_TOKENS * n_seq, GLA_CHUNK_STEP):
+        return 0
+    n = int(mixers().janis_gla_chunks_least(int(T), int(n_seq), int(H), int(d), int(dv)))
     return n if n <= GLA_CHUNK_FLOATS else 0
 
 
 def _gla_chunked(rows, v_off, state, o_out, T, n_seq, H, d, dv, chunks) -> bool:
-    need = gla_chunks_floats(rows.dtype, T, n_seq, H, d, dv)
+    need = _gla_chunks_least(rows.dtype, T, n_seq, H, d, dv)
     return (0 < need <= chunks.numel() and rows.shape[1] % 8 == 0 and v_off % 8 == 0 and (rows.data_ptr() | chunks.data_ptr()) % 16 == 0
             and (state.data_ptr() | o_out.data_ptr()) % 8 == 0)
 
@@ -1171,9 +1181,9 @@ def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_
         if _gla_chunked(rows, v_off, state, o_out, T, n_seq, H, d, dv, chunks):
             _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_start, seq_end, T, n_seq, H, d, dv)
             lib = mixers()
-            _check(lib, lib.janis_gla_chunks(rows.data_ptr(), width, q_off, k_off, v_off, z.data_ptr(), z_bias.data_ptr(), T, seq_slot.data_ptr(),
-                                             seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(),
-                                             n_seq, H, d, dv, float(q_scale), float(tau), chunks.data_ptr(), chunks.numel(), _stream()), kernels=2)
+            _check_counted(lib, lib.janis_gla_chunks, rows.data_ptr(), width, q_off, k_off, v_off, z.data_ptr(), z_bias.data_ptr(), T, seq_slot.data_ptr(),
+                           seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(),
+                           n_seq, H, d, dv, float(q_scale), float(tau), chunks.data_ptr(), chunks.numel(), _stream())
             return o_out
     if decay is None:
         decay = torch.empty((T, H * d), dtype=torch.float32, device=rows.device)

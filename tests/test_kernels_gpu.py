@@ -1214,3 +1214,27 @@ def test_gated_linear_attention_of_one_token_each(dtype, lens, slots, H, d, dv):
     close(got, want, 5e-5, "results")
     close(got_state, want_state, 5e-5, "the states left behind")
     close(decay, torch.sigmoid(z.double() + b.double()) ** (1 / 16.0), 1e-5, "the decays")
+
+
+@pytest.mark.parametrize("lens,slots", [([700], [1]), ([30, 600], [3, 0]), ([520, 0, 300], [-1, 2, 4])])
+@pytest.mark.parametrize("H,d,dv,strength", [(2, 128, 64, 1.0), (1, 64, 32, 0.02)])
+def test_gated_linear_attention_in_pieces(lens, slots, H, d, dv, strength):
+    """Chains cut into pieces of 16 chunks and more: against the recurrence in 64 bits, with states that forget and states that
+    remember hundreds of tokens, and beside whole chains (a scratch with no room for the pieces' states)."""
+    g = torch.Generator().manual_seed(d + len(lens))
+    T, n_seq = sum(lens), len(lens)
+    seq_slot, first, start, end = _step_tables(lens, slots)
+    rows, z = torch.randn(T, 2 * H * d + H * dv, generator=g).bfloat16(), (torch.randn(T, H * d, generator=g) * strength).bfloat16()
+    b = torch.full((H * d,), 0.0 if strength == 1.0 else 4.0).bfloat16()
+    state = torch.randn(6, H, dv, d, generator=g)
+    want, want_state = torch.zeros(T, H * dv), state.clone()
+    args = lambda dev, st, out: (dev(rows), 0, H * d, 2 * H * d, dev(z), dev(b), dev(seq_slot), dev(first), dev(start), dev(end), st, out, n_seq, H, d, dv,
+                                 d ** -0.5, 16.0)
+    R.gla_scan(*args(lambda x: x, want_state, want))
+    most, least = ops().gla_chunks_floats(torch.bfloat16, T, n_seq, H, d, dv), ops()._gla_chunks_least(torch.bfloat16, T, n_seq, H, d, dv)
+    assert most > least > 0
+    for room in (most, least):
+        got, got_state = torch.full((T, H * dv), float("nan"), device=dev()), state.clone().to(dev())
+        ops().gla_scan(*args(lambda x: x.to(dev()), got_state, got), chunks=torch.full((room,), float("nan"), device=dev()))
+        close(got, want, 2e-5, "results")
+        close(got_state, want_state, 2e-5, "the states left behind")
