@@ -24,7 +24,8 @@
 // states keeps whole chains).
 //
 // 8 heads of 128 x 256, against gla_scan_kernel (bound by shared memory: three 16-byte reads for 16 multiply-adds a lane) with its
-// kernel for the decays: one sequence of 2,048 tokens 374 -> 200 us, 300 tokens 60 -> 43, eight of 512 666 -> 210.  Errors
+// kernel for the decays: whole chains of one sequence of 2,048 tokens 374 -> 200 us (in pieces 140), 300 tokens 60 -> 43,
+// eight of 512 666 -> 210.  Errors
 // against 64 bits over 2,048 tokens: results 3.3e-7 -> 1.4e-7, states 3.2e-7 -> 0.7e-7; where the states remember a thousand tokens
 // 5.3e-6 -> 1.9e-7 and 7.3e-6 -> 2.1e-7.
 #include "mma_bf16.cuh"
