@@ -24,10 +24,10 @@
 // e^(c_t) S_0 C_t over its states, and gives its partner the sums of those 32 tokens of a chunk whose results the partner
 // finishes.  Tokens come by cp.async a chunk ahead, and one warp forms a chunk's decays while the chunk before is
 // computed.  What bounds it is the chain of a chunk: some 2,000 instructions a warp and three barriers.  Two warps a channel
-// tile instead of one hide each other's waits (328 us -> 218).
+// tile instead of one hide each other's waits (328 us -> 218); few sequences' chains are shared by two CTAs (220 -> 157).
 //
 // 72 heads of 64 channels, 128 states, with the scan of selective_scan_staged_kernel (an issue slot in two, 263 instructions
-// a token and warp) and its kernel for the step sizes: one sequence of 2,048 tokens 954 -> 209 us, 300 tokens 148 -> 39, eight
+// a token and warp) and its kernel for the step sizes: one sequence of 2,048 tokens 954 -> 209 us (157 shared), 300 tokens 148 -> 39, eight
 // of 512 1,400 -> 229, eight of 8 49 -> 29, one of 4 27 -> 23.  Errors against 64 bits over 2,048 tokens: results 1.1e-7 for
 // 1.0e-7, states 0.8e-7 for 0.7e-7; where the states remember a thousand tokens 1.5e-7 for 5.5e-7 and 1.2e-7 for 6.6e-7.
 #include "mma_bf16.cuh"
@@ -51,11 +51,21 @@ __host__ __device__ constexpr size_t duality_smem(int N) {
 
 __device__ __forceinline__ float duality_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
+// Where few sequences leave half of the SMs idle, two CTAs (a cluster) share a chain: the first runs its first part; the second takes
+// the state alone through that part, then runs the rest.  This is where the rest starts, in tokens: a chunk's state alone takes 0.58 of
+// a chunk's time (the decays, which one warp forms, stay), so that at seven tenths both take as long (x = 0.58 x + 1 - x; at three
+// fifths 166 us for 157).  n_tok for chains of less than four chunks, which one CTA runs.  The bits are those of one CTA: each chunk's
+// state is formed by the same instructions.
+__device__ __forceinline__ int duality_split(int n_tok) {
+    const int chunks = (n_tok + DQ - 1) / DQ;
+    return chunks < 4 ? n_tok : (7 * chunks + 5) / 10 * DQ;
+}
+
 template <int NK>                            // N = 16 NK states, NK even
 __global__ void __launch_bounds__(256)
 duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt_rows, const bf16* __restrict__ bc_rows,
                     const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
-                    DualityShape g, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
+                    DualityShape g, int parts, const int* __restrict__ seq_slot, const int* __restrict__ seq_first_row,
                     const int* __restrict__ seq_start, const int* __restrict__ seq_end, float* __restrict__ state,
                     float* __restrict__ out) {
     constexpr int N = 16 * NK, NH = NK / 2, LDN = N + 8, STAGE = duality_stage_elems(N), SCAL = 5 * DQ + 4;
@@ -64,14 +74,16 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
     bf16* m_s = stage_s + 2 * STAGE;                                       // [10 tiles on and below the diagonal][3][16][MTP]
     float* swap_s = reinterpret_cast<float*>(m_s + 10 * 3 * 16 * MTP);     // [64 tokens][DXP]: sums for the partner
     float* scal_s = swap_s + DQ * DXP;                                     // [2] of the decays below
-    const int seq = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5, npt = nwarp >> 1;
+    const int seq = blockIdx.x / parts, part = blockIdx.x % parts, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5, npt = nwarp >> 1;
     const int half = warp >= npt, pt = warp - half * npt;                  // half of the states, tile of 16 channels
     const int c0 = blockIdx.y * npt * 16, cw = c0 + pt * 16, head = c0 / g.cph, group = c0 / g.cpg;
     const int gr = lane >> 2, gc = (lane & 3) * 2;                         // a lane's row and first column of an 8 x 8 tile
     const int lr = lane & 7, lm = lane >> 3;                               // row and matrix that the lane addresses in ldmatrix
     grid_dependents_launch();
     const int slot = seq_slot[seq], row0 = seq_first_row[seq], n_tok = seq_end[seq] - seq_start[seq];
-    if (n_tok <= 0) return;
+    const int split = parts == 2 ? duality_split(n_tok) : n_tok;
+    if (n_tok <= 0 || (part == 1 && split == n_tok)) return;
+    const int stop = part == 0 ? split : n_tok;                            // (split < n_tok: whole chunks)
     const float Ah = A[head], Dh = D[head], bias = dt_bias[head];
     grid_dependency_wait();
 
@@ -89,7 +101,7 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         const int n = n_tok - t0;
         const bf16* b0 = bsrc + (size_t)t0 * g.bc_stride;
 #pragma unroll 4
-        for (int t = bt; t < DQ; t += b_step) {
+        for (int t = which && part == 1 && t0 < split ? DQ : bt; t < DQ; t += b_step) {              // (the state alone: no C)
             const bool ok = t < n;
             copy16_or_zero(b_to + t * LDN * 2, b0 + (ok ? (size_t)t * g.bc_stride : 0), ok);
         }
@@ -151,9 +163,11 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         }
         S[j][0] = a.x; S[j][1] = a.y; S[j][2] = b.x; S[j][3] = b.y;
     }
+    // (both CTAs have read the stored state before the second one writes it)
+    if (split < n_tok) asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
 
     // Tokens one after another: for the chunks that the products cannot take
-    auto plain = [&](int t0, int n_here, int buf) {
+    auto plain = [&](int t0, int n_here, int buf, bool results) {
         const bf16 *B_s = stage_s + (size_t)buf * STAGE + n0, *C_s = B_s + DQ * LDN, *u_s = stage_s + (size_t)buf * STAGE + 2 * DQ * LDN + pt * 16;
         const float* delta_s = scal_s + buf * SCAL + 2 * DQ;
         for (int t = 0; t < n_here; ++t) {
@@ -175,13 +189,13 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
                 yb += __shfl_xor_sync(0xffffffffu, yb, o);
             }
             if ((lane & 3) == 0 && half) swap_s[t * DXP + pt * 16 + gr] = ya, swap_s[t * DXP + pt * 16 + gr + 8] = yb;
-            if ((lane & 3) == 0 && !half) {
+            if ((lane & 3) == 0 && !half && results) {
                 float* y = out + (size_t)(row0 + t0 + t) * g.C + cw + gr;
                 y[0] = fmaf(Dh, ua, ya), y[8] = fmaf(Dh, ub, yb);
             }
         }
         __syncthreads();
-        for (int i = lane; i < 16 * n_here && !half; i += 32) {
+        for (int i = lane; i < 16 * n_here && !half && results; i += 32) {
             // (a lane's own warp wrote what it adds to, before the barrier)
             const int t = i >> 4, ch = i & 15;
             out[(size_t)(row0 + t0 + t) * g.C + cw + ch] += swap_s[t * DXP + pt * 16 + ch];
@@ -192,8 +206,8 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
     fetch(0, 0);
     if (warp == nwarp - 1) decays(0, scal_s);
     int buf = 0;
-    for (int t0 = 0; t0 < n_tok; t0 += DQ, buf ^= 1) {
-        const bool more = t0 + DQ < n_tok;
+    for (int t0 = 0; t0 < stop; t0 += DQ, buf ^= 1) {
+        const bool more = t0 + DQ < stop, results = part == 0 || t0 >= split;
         const int n_here = min(DQ, n_tok - t0), tiles = (n_here + 15) / 16;
         if (more) {
             fetch(t0 + DQ, buf ^ 1);
@@ -209,7 +223,7 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         }
         if (!__syncthreads_and(good)) {
             if (more && warp == nwarp - 1) decays(t0 + DQ, scal_s + (buf ^ 1) * SCAL);
-            plain(t0, n_here, buf);
+            plain(t0, n_here, buf, results);
             __syncthreads();                                               // the buffers have been read
             continue;
         }
@@ -219,7 +233,7 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
 
         // the chunk's start, over this warp's states; tiles of tokens 0 and 3 are the first warp's to finish, 1 and 2 the second's
         float mine[2][2][4];
-        {
+        if (results) {
             float hi[4][2][4], rest[4][2][4];
 #pragma unroll
             for (int i = 0; i < 4; ++i)
@@ -263,7 +277,7 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         }
 
         // M, a tile of 16 x 16 at a time
-        for (int m = warp; m < tiles * (tiles + 1) / 2; m += nwarp) {
+        for (int m = results ? warp : 10; m < tiles * (tiles + 1) / 2; m += nwarp) {
             const int i = m >= 6 ? 3 : m >= 3 ? 2 : m >= 1 ? 1 : 0, j = m - i * (i + 1) / 2;
             float acc[2][2][4];                                            // [even and odd k][8 columns each]
 #pragma unroll
@@ -306,18 +320,18 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
             }
         }
         if (more && warp == nwarp - 1) decays(t0 + DQ, scal_s + (buf ^ 1) * SCAL);
-        __syncthreads();
+        if (results) __syncthreads();
 
         // the chunk's own tokens, and the results of this warp's tiles of tokens
         const bf16* u_s = stage_s + (size_t)buf * STAGE + 2 * DQ * LDN;
         uint32_t ub[4][4];
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k < tiles) ldmatrix4_trans(ub[k], u_a + ((16 * k + lr + (lm & 1) * 8) * DUP + pt * 16 + (lm >> 1) * 8) * 2);
+            if (k < tiles && results) ldmatrix4_trans(ub[k], u_a + ((16 * k + lr + (lm & 1) * 8) * DUP + pt * 16 + (lm >> 1) * 8) * 2);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int i = half == 0 ? 3 * q : 1 + q;
-            if (i >= tiles) continue;
+            if (i >= tiles || !results) continue;
             float hi[2][2][4], rest[2][4];                                 // (hi: even and odd tiles)
 #pragma unroll
             for (int p = 0; p < 2; ++p)
@@ -400,7 +414,7 @@ duality_scan_kernel(const bf16* __restrict__ u_rows, const bf16* __restrict__ dt
         }
         __syncthreads();                                                   // the buffers have been read
     }
-    if (st != nullptr) {
+    if (st != nullptr && stop == n_tok) {
 #pragma unroll
         for (int j = 0; j < 2 * NH; ++j) {
             *reinterpret_cast<float2*>(st + (size_t)gr * N + 8 * j + gc) = make_float2(S[j][0], S[j][1]);
@@ -416,9 +430,10 @@ static int duality_launch(const bf16* u, const bf16* dt, const bf16* bc, const f
     constexpr size_t bytes = duality_smem(16 * NK);
     const cudaError_t e = cudaFuncSetAttribute(duality_scan_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail("duality_scan: shared memory of %zu bytes refused: %s", bytes, cudaGetErrorString(e));
-    // (launched once its predecessor is over: its few CTAs run long and have to lie on SMs of their own)
-    return launch_kernel_after("duality_scan", duality_scan_kernel<NK>, dim3(n_seq, g.C / (16 * tiles)), dim3(64 * tiles), bytes, stream, 1,
-                               u, dt, bc, dt_bias, A, D, g, seq_slot, seq_first_row, seq_start, seq_end, state, out);
+    // (launched once its predecessor is over: its few CTAs run long and have to lie on SMs of their own; 148 SMs)
+    const int parts = 2LL * n_seq * (g.C / (16 * tiles)) <= 148 ? 2 : 1;
+    return launch_kernel_after("duality_scan", duality_scan_kernel<NK>, dim3(n_seq * parts, g.C / (16 * tiles)), dim3(64 * tiles), bytes, stream, parts,
+                               u, dt, bc, dt_bias, A, D, g, parts, seq_slot, seq_first_row, seq_start, seq_end, state, out);
 }
 
 }  // namespace janis

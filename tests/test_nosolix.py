@@ -390,6 +390,38 @@ def test_chunked_duality_scan_against_its_statement(C, N, cph, cpg, lens):
 
 
 @GPU
+@pytest.mark.parametrize("C,N,cph,cpg", [(128, 128, 64, 64), (64, 32, 16, 64), (96, 64, 48, 96)])
+def test_chunked_duality_scan_shared_by_two(C, N, cph, cpg):
+    """A chain that two CTAs share (few sequences) gives the bits of the chain that one runs (many sequences): around the four chunks
+    from which on it is shared, long ones, with a stored state, a padding sequence and tokens that go one by one in either part."""
+    from janis_b200.kernels import ops
+    long = [192, 193, 256, 257, 320, 643, 1000, 300]
+    lens = long + [1 + i % 3 for i in range(72)]
+    slots = [7, 6, 5, 4, 3, 2, -1, 0] + list(range(8, 80))
+    _, seq_slot, first, seq_start, seq_end, T = _tables(lens, [30 * (i % 2) for i in range(80)], slots)
+    heads, groups = C // cph, C // cpg
+    g = torch.Generator().manual_seed(C + N)
+    u = torch.randn(T, C, generator=g).bfloat16()
+    u[sum(long[:3]) + 70, 3], u[sum(long[:5]) + 500, 17] = float("inf"), float("nan")
+    dt, bc = torch.randn(T, heads, generator=g).bfloat16(), torch.randn(T, 2 * groups * N, generator=g).bfloat16()
+    dt_bias, D, A = torch.randn(heads, generator=g) - 1.0, torch.randn(heads, generator=g), -torch.exp(torch.randn(heads, generator=g))
+    state = torch.randn(80, C, N, generator=g)
+    got = {}
+    ops.selective_scan_set_form(3)
+    try:
+        for n in (80, len(long)):
+            out, st = torch.zeros(T, C, device="cuda"), state.cuda()
+            ops.selective_scan(u.cuda(), 0, dt.cuda(), 0, dt_bias.cuda(), A.cuda(), False, bc.cuda(), 0, groups * N, D.cuda(), None, 0,
+                               *(x[:n].cuda() for x in (seq_slot, first, seq_start, seq_end)), n, st, out, C, N, cph, cpg)
+            got[n] = out[:sum(long)].cpu(), st[:8].cpu()
+    finally:
+        ops.selective_scan_set_form(0)
+    for whole, shared in zip(got[80], got[len(long)]):
+        assert torch.equal(whole.nan_to_num(7.0, 8.0, 9.0), shared.nan_to_num(7.0, 8.0, 9.0))
+    assert got[80][0].isnan().any() and torch.equal(got[80][1][1], state[1])
+
+
+@GPU
 @pytest.mark.parametrize("C,N,cph,cpg", [(128, 128, 64, 128), (64, 32, 16, 32)])
 @pytest.mark.parametrize("bad", ["input", "B", "C", "step", "growth"])
 def test_chunked_duality_scan_of_inputs_beyond_numbers(C, N, cph, cpg, bad):
