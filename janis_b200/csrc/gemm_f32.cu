@@ -38,10 +38,21 @@ namespace f32 {
 using namespace tc;
 
 constexpr int BK = 32, STAGES = 3;
-#ifndef JANIS_F32_CHUNK
-#define JANIS_F32_CHUNK 2             // blocks of 32 k between additions in registers (a tuning switch)
-#endif
-constexpr int CHUNK = JANIS_F32_CHUNK;
+constexpr int CHUNK = 2;              // blocks of 32 k between additions in registers
+// A wait by parity tells a barrier's phase only from the one beside it, so whoever waits for a phase has to have seen the one before.  A
+// stage's blocks go to both issuers and both groups of splitting warps in turn, and the copies of x of two stages may land in any order; so
+// a block's barriers are not its stage's but one of CYCLE pairs, which come back after whole rounds of stages, issuers and groups:
+//   full[b % CYCLE]   is waited for by the issuer of block b, who was the issuer of b - CYCLE and has seen that phase;
+//   empty[b % CYCLE]  by the group that splits block b + STAGES, which split b + STAGES - CYCLE, and by the thread that brings x (all blocks in turn).
+// None of them comes round again under a waiter: block b + CYCLE is brought to its stage after block b has been consumed, by that issuer, and
+// consumed after that group and that thread have passed their waits for block b's stage (tests run the waits in a model with random delays).
+constexpr int CYCLE = 12;
+__host__ __device__ constexpr int stage_of(int b) { return b % STAGES; }
+__host__ __device__ constexpr int pair_of(int b) { return b % CYCLE; }
+__host__ __device__ constexpr int parity_of(int b) { return (b / CYCLE) & 1; }
+__host__ __device__ constexpr int issuer_of(int b) { return (b / CHUNK) & 1; }
+__host__ __device__ constexpr int group_of(int b, int groups) { return b % groups; }
+static_assert(CYCLE % STAGES == 0 && CYCLE % (2 * CHUNK) == 0 && CYCLE % 2 == 0, "whole rounds of stages, issuers and groups of splitting warps");
 constexpr int W_ROWS = 128, W_PLANE = W_ROWS * 64;     // a plane: one of hi, mid, lo
 __host__ __device__ constexpr int stage_bytes(int cols) { return 3 * (W_PLANE + cols * 64); }
 __host__ __device__ constexpr int smem_bytes(int cols) { return STAGES * stage_bytes(cols) + 1024; }
@@ -113,14 +124,15 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
     constexpr int GROUPS = SUMS / 4, UNITS = MOST_COLS / 16 / GROUPS;       // units of 16 columns of sums in a thread
     constexpr int TURNS = SPLITS / 4, NW = W_ROWS / 16, AHEAD = 2;          // 16 rows of W a pass of four warps, 8 threads a row
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * STAGES + 5];
+    static_assert(CYCLE % TURNS == 0, "whole rounds of groups");
+    __shared__ __align__(8) unsigned long long bars[2 * CYCLE + 5];
     __shared__ uint32_t tmem_slot;
     __shared__ int low_bits[STAGES];                      // 1 + the last block whose W was not all bfloat16 numbers
     __shared__ int failed;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t stage0 = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023) & ~1023u;
-    const uint32_t full = (uint32_t)__cvta_generic_to_shared(bars), empty = full + 8 * STAGES;
-    const uint32_t sums_there = empty + 8 * STAGES, sums_taken = sums_there + 16, all_done = sums_taken + 16;
+    const uint32_t full = (uint32_t)__cvta_generic_to_shared(bars), empty = full + 8 * CYCLE;
+    const uint32_t sums_there = empty + 8 * CYCLE, sums_taken = sums_there + 16, all_done = sums_taken + 16;
     const int stage_size = stage_bytes(cols), x_plane = cols * 64;
     const int m_tiles = (M + cols - 1) / cols;            // neighbouring CTAs take the rows of x of one strip of W
     const int m0 = (int)(blockIdx.x % m_tiles) * cols, n0 = (int)(blockIdx.x / m_tiles) * W_ROWS;
@@ -128,11 +140,11 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
     const int tmem_cols = 2 * cols <= 32 ? 32 : (2 * cols <= 64 ? 64 : (2 * cols <= 128 ? 128 : (2 * cols <= 256 ? 256 : 512)));
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < STAGES; ++i) {
+        for (int i = 0; i < CYCLE; ++i) {
             mbar_init(full + 8 * i, 5);          // four warps of W, the copies of x
             mbar_init(empty + 8 * i, 1);
-            low_bits[i] = 0;
         }
+        for (int i = 0; i < STAGES; ++i) low_bits[i] = 0;
         for (int i = 0; i < 2; ++i) {
             mbar_init(sums_there + 8 * i, 1);
             mbar_init(sums_taken + 8 * i, SUMS);
@@ -163,12 +175,12 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
             const uint32_t plane16 = (uint32_t)x_plane >> 4;                    // (an address in a descriptor counts 16 bytes)
             const uint32_t d = tmem + issuer * cols;
             bool ok = true;
-            for (int c = issuer; c < n_chunks && ok; c += 2) {
+            for (int c = issuer; c < n_chunks && ok; c += 2) {              // (issuer_of)
                 if (c >= 2 && !__all_sync(0xffffffffu, mbar_wait(sums_taken + 8 * issuer, (c / 2 - 1) & 1))) { ok = false; break; }
                 const int first = c * CHUNK, last = min(first + CHUNK, n_blocks) - 1;
                 for (int b = first; b <= last; ++b) {
-                    const int s = b % STAGES;
-                    if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * s, (b / STAGES) & 1))) { ok = false; break; }
+                    const int s = stage_of(b);
+                    if (!__all_sync(0xffffffffu, mbar_wait(full + 8 * pair_of(b), parity_of(b)))) { ok = false; break; }
                     // The splitters' writes are fenced for the tensor cores here, behind the barrier that orders them.
                     fence_async_shared();
                     fence_after_sync();
@@ -191,7 +203,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
                         umma(d, w + 2, xs + plane16 + 2, idesc, 1);
                         umma(d, w, xs, idesc, 1);
                         umma(d, w + 2, xs + 2, idesc, 1);
-                        umma_commit(empty + 8 * s);
+                        umma_commit(empty + 8 * pair_of(b));
                         if (b == last) umma_commit(sums_there + 8 * issuer);
                     }
                     __syncwarp();
@@ -203,10 +215,10 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
             mbar_wait(all_done, 0);
         } else if (issuer == 2 && lane == 0) {            // brings the planes of x
             for (int b = 0; b < n_blocks; ++b) {
-                const int s = b % STAGES;
-                if (b >= STAGES && !mbar_wait_parked(empty + 8 * s, (b / STAGES - 1) & 1, &failed)) { atomicExch(&failed, 1); break; }
-                mbar_expect_tx(full + 8 * s, 3 * x_plane);
-                tma_load_3d(stage0 + s * stage_size + 3 * W_PLANE, &map_x, b * BK, m0, 0, full + 8 * s);
+                const int before = b - STAGES;            // what the stage held
+                if (before >= 0 && !mbar_wait_parked(empty + 8 * pair_of(before), parity_of(before), &failed)) { atomicExch(&failed, 1); break; }
+                mbar_expect_tx(full + 8 * pair_of(b), 3 * x_plane);
+                tma_load_3d(stage0 + stage_of(b) * stage_size + 3 * W_PLANE, &map_x, b * BK, m0, 0, full + 8 * pair_of(b));
             }
         }
         __syncwarp();
@@ -236,9 +248,9 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
             for (int a = 0; a < AHEAD; ++a) {
                 const int b = b0 + a * TURNS;
                 if (b >= n_blocks) break;
-                const int s = b % STAGES, round = b / STAGES;
+                const int s = stage_of(b), before = b - STAGES;
                 // (who gives up goes on without waiting: the other warps of the group count on its arrivals)
-                if (ok && round > 0) ok = mbar_wait_parked(empty + 8 * s, (round - 1) & 1, &failed);
+                if (ok && before >= 0) ok = mbar_wait_parked(empty + 8 * pair_of(before), parity_of(before), &failed);
                 const uint32_t to = stage0 + s * stage_size + place;
                 uint32_t low = 0;
 #pragma unroll
@@ -265,7 +277,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
                 }
                 if (b + AHEAD * TURNS < n_blocks) fetch(b + AHEAD * TURNS, a);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(full + 8 * s);
+                if (lane == 0) mbar_arrive(full + 8 * pair_of(b));
             }
         }
         if (!ok) atomicExch(&failed, 1);
@@ -352,6 +364,13 @@ static int launch(const CUtensorMap& map_x, const float* x, const float* W, floa
 using namespace janis;
 
 JANIS_EXPORT int janis_launches_made() { return launches_made(); }
+
+// How the kernel orders block b of 32 k, with `groups` groups of splitting warps (for tests): its stage, the pair of barriers and the
+// parity of their phase, its issuer, its group; then the numbers of stages and of pairs, blocks a chunk.
+JANIS_EXPORT void janis_gemm_f32_order(int b, int groups, int* out) {
+    const int v[8] = {f32::stage_of(b), f32::pair_of(b), f32::parity_of(b), f32::issuer_of(b), f32::group_of(b, groups), f32::STAGES, f32::CYCLE, f32::CHUNK};
+    for (int i = 0; i < 8; ++i) out[i] = v[i];
+}
 
 // rows of x whose planes take no more than 64 MB (256 at least): a product of more rows is made in parts
 static int f32_part_rows(int M, int K) {
