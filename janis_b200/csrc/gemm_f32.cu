@@ -214,12 +214,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
             __syncwarp();
             mbar_wait(all_done, 0);
         } else if (issuer == 2 && lane == 0) {            // brings the planes of x
-            for (int b = 0; b < n_blocks; ++b) {
+            int b = 0;
+            for (; b < n_blocks; ++b) {
                 const int before = b - STAGES;            // what the stage held
                 if (before >= 0 && !mbar_wait_parked(empty + 8 * pair_of(before), parity_of(before), &failed)) { atomicExch(&failed, 1); break; }
                 mbar_expect_tx(full + 8 * pair_of(b), 3 * x_plane);
                 tma_load_3d(stage0 + stage_of(b) * stage_size + 3 * W_PLANE, &map_x, b * BK, m0, 0, full + 8 * pair_of(b));
             }
+            // no copy is on its way when the CTA leaves, also where a wait was given up (then for some seconds at most)
+            for (int j = max(0, b - STAGES); j < b; ++j)
+                if (!mbar_wait_parked(full + 8 * pair_of(j), parity_of(j), &failed)) mbar_wait(full + 8 * pair_of(j), parity_of(j));
         }
         __syncwarp();
         asm volatile("bar.sync 0;" ::: "memory");         // the last sums have been read
@@ -249,7 +253,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
                 const int b = b0 + a * TURNS;
                 if (b >= n_blocks) break;
                 const int s = stage_of(b), before = b - STAGES;
-                // (who gives up goes on without waiting: the other warps of the group count on its arrivals)
+                // (who gives up goes on without waiting, as the other warps of the group count on it at their barrier, and arrives nowhere)
                 if (ok && before >= 0) ok = mbar_wait_parked(empty + 8 * pair_of(before), parity_of(before), &failed);
                 const uint32_t to = stage0 + s * stage_size + place;
                 uint32_t low = 0;
@@ -277,7 +281,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
                 }
                 if (b + AHEAD * TURNS < n_blocks) fetch(b + AHEAD * TURNS, a);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(full + 8 * pair_of(b));
+                if (lane == 0 && ok) mbar_arrive(full + 8 * pair_of(b));
             }
         }
         if (!ok) atomicExch(&failed, 1);
