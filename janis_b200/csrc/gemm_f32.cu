@@ -58,22 +58,32 @@ __host__ __device__ constexpr int stage_bytes(int cols) { return 3 * (W_PLANE + 
 __host__ __device__ constexpr int smem_bytes(int cols) { return STAGES * stage_bytes(cols) + 1024; }
 
 // Four floats from k on; zeros past the row's end and where !ok.  The loads are volatile so that they stay where they stand: the
-// compiler may move others down to the block that uses them.
-template <bool VEC>
+// compiler may move others down to the block that uses them.  CONSTANT: of a matrix that nobody writes while the kernel lives (W), through the
+// read-only path; x is the kernel before's result, which may still be at it when this one starts.
+template <bool VEC, bool CONSTANT>
 __device__ __forceinline__ float4 load4(const float* row, int k, int K, bool ok) {
     float4 v;
     if (VEC) {
-        asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n"
-                     "@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n}\n"
-                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                     : "l"(row + k), "r"((int)(ok && k < K)));
+#define JANIS_LOAD4(KIND)                                                                                                            \
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %5, 0;\nmov.b32 %0, 0;\nmov.b32 %1, 0;\nmov.b32 %2, 0;\nmov.b32 %3, 0;\n"         \
+                 "@p ld.global" KIND ".v4.f32 {%0, %1, %2, %3}, [%4];\n}\n"                                                          \
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)                                                                       \
+                 : "l"(row + k), "r"((int)(ok && k < K)))
+        if (CONSTANT) JANIS_LOAD4(".nc");
+        else JANIS_LOAD4("");
+#undef JANIS_LOAD4
     } else {
         float e[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.b32 %0, 0;\n@p ld.global.nc.f32 %0, [%1];\n}\n"
-                         : "=f"(e[j])
-                         : "l"(row + k + j), "r"((int)(ok && k + j < K)));
+        for (int j = 0; j < 4; ++j) {
+#define JANIS_LOAD1(KIND)                                                                                                            \
+    asm volatile("{\n.reg .pred p;\nsetp.ne.s32 p, %2, 0;\nmov.b32 %0, 0;\n@p ld.global" KIND ".f32 %0, [%1];\n}\n"                 \
+                 : "=f"(e[j])                                                                                                       \
+                 : "l"(row + k + j), "r"((int)(ok && k + j < K)))
+            if (CONSTANT) JANIS_LOAD1(".nc");
+            else JANIS_LOAD1("");
+#undef JANIS_LOAD1
+        }
         v = make_float4(e[0], e[1], e[2], e[3]);
     }
     return v;
@@ -102,7 +112,7 @@ split_rows_kernel(const float* x, bf16* __restrict__ planes, int M, int K, int K
     for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
         const size_t m = i / per_row;
         const int k = (int)(i - m * per_row) * 8;
-        const float4 a = load4<VEC>(x + m * K, k, K, true), b = load4<VEC>(x + m * K, k + 4, K, true);
+        const float4 a = load4<VEC, false>(x + m * K, k, K, true), b = load4<VEC, false>(x + m * K, k + 4, K, true);
         uint4 hi, mid, lo;
         split3(a.x, a.y, hi.x, mid.x, lo.x);
         split3(a.z, a.w, hi.y, mid.y, lo.y);
@@ -119,7 +129,7 @@ split_rows_kernel(const float* x, bf16* __restrict__ planes, int M, int K, int K
 // products and one brings x.  VEC: rows of W are 16-byte aligned, K a multiple of 4.
 template <int SUMS, int SPLITS, int MOST_COLS, bool VEC>
 __global__ void __launch_bounds__((SUMS + SPLITS + 4) * 32, SUMS == 8 ? 1 : 2)
-gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restrict__ x, const float* W, float* __restrict__ out,
+gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* x, const float* W, float* __restrict__ out,
                 int M, int N, int K, int cols, float cap, int* __restrict__ timeouts) {
     constexpr int GROUPS = SUMS / 4, UNITS = MOST_COLS / 16 / GROUPS;       // units of 16 columns of sums in a thread
     constexpr int TURNS = SPLITS / 4, NW = W_ROWS / 16, AHEAD = 2;          // 16 rows of W a pass of four warps, 8 threads a row
@@ -242,7 +252,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
         auto fetch = [&](int b, int a) {
             const int k = b * BK + quad * 4;
 #pragma unroll
-            for (int i = 0; i < NW; ++i) wv[a][i] = load4<VEC>(wr + (size_t)(i * 16) * K, k, K, i * 16 < rows);
+            for (int i = 0; i < NW; ++i) wv[a][i] = load4<VEC, true>(wr + (size_t)(i * 16) * K, k, K, i * 16 < rows);
         };
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a) fetch(turn + a * TURNS, a);
@@ -335,7 +345,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* __restri
                     odd &= odd - 1;
                     const float *xp = x + (size_t)m * K, *wp = W + (size_t)(n - lane + l) * K;
                     float plain = 0.f;
-                    for (int k = lane; k < K; k += 32) plain = fmaf(xp[k], wp[k], plain);
+                    for (int k = lane; k < K; k += 32) plain = fmaf(__ldcg(xp + k), wp[k], plain);
                     plain = warp_sum(plain);
                     if (lane == l) v = plain;
                 }
