@@ -115,8 +115,9 @@ class Stepper:
 
     def __init__(self, model: DecoderModel, cache: ModelCache, rt: Runtime, max_step_tokens: int = 16384,
                  use_graphs: bool = True):
-        self.model, self.cache, self.rt = model, cache, rt
+        self.model, self.cache = model, cache
         self.ws = Workspace(rt.device)
+        self.rt = rt.over(self.ws)
         self.max_step_tokens = max(1, int(max_step_tokens))
         self.use_graphs = bool(use_graphs) and torch.device(rt.device).type == "cuda" and model.graph_safe
         self._graphs: dict[tuple, tuple] = {}     # (padded batch, length bound, mean length in eighths of it, even) -> graph

@@ -422,15 +422,25 @@ def kv_store(qkv, tok_pos, tok_seq, seq_slot, seq_end, nq: int, nkv: int, hd: in
 # products
 # ---------------------------------------------------------------------------
 
-def gemm_f32(x, w, out, cap: float = 0.0):
+def gemm_f32_room(M: int, K: int) -> int:
+    """bfloat16 numbers of room in which `gemm_f32` keeps x's parts (at most 64 MB, or 256 rows of them: more rows go in turns)."""
+    return int(core().janis_gemm_f32_room(int(M), int(K)))
+
+
+def gemm_f32(x, w, out, cap: float = 0.0, planes=None):
     """out[M, N] = x[M, K] w[N, K]^T at float32's precision (floats as sums of bfloat16 numbers on the tensor cores);
-    optional cap * tanh(v / cap)."""
+    optional cap * tanh(v / cap).  planes: bfloat16 scratch of `gemm_f32_room(M, K)` numbers, 16-byte aligned (allocated where it is not given)."""
     M, K = x.shape
     N = w.shape[0]
     lib = core()
     xp, wp, op = _t(x, "x", torch.float32, (M, K)), _t(w, "w", torch.float32, (N, K)), _t(out, "out", torch.float32, (M, N))
-    planes = torch.empty(max(lib.janis_gemm_f32_room(M, K), 1), dtype=torch.bfloat16, device=x.device)
-    _check_counted(lib, lib.janis_gemm_f32, xp, wp, op, M, N, K, float(cap), planes.data_ptr(), _stream())
+    need = gemm_f32_room(M, K)
+    if planes is None:
+        planes = torch.empty(max(need, 1), dtype=torch.bfloat16, device=x.device)
+    pp = _t(planes, "planes", torch.bfloat16)
+    if planes.numel() < need:
+        raise KernelError(f"gemm_f32: planes of {planes.numel()} numbers, {need} wanted for {M} rows of {K}")
+    _check_counted(lib, lib.janis_gemm_f32, xp, wp, op, M, N, K, float(cap), pp, _stream())
     return out
 
 

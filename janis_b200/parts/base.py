@@ -43,6 +43,7 @@ parts chosen layer by layer is this library's.
 """
 from __future__ import annotations
 
+import copy
 from dataclasses import dataclass, field
 from typing import Any, Mapping
 
@@ -52,7 +53,8 @@ from ..weights.loader import TensorSpec
 
 
 class Runtime:
-    """The compute dtype, the device and the kernels a model runs with."""
+    """The compute dtype, the device and the kernels a model runs with.  `over(ws)`: the same with a workspace, in which
+    the products keep the room they need from step to step; without one they ask the allocator."""
 
     def __init__(self, dtype: torch.dtype, device, ops):
         if dtype not in (torch.float32, torch.bfloat16):
@@ -60,6 +62,7 @@ class Runtime:
         self.dtype = dtype
         self.device = device
         self.ops = ops
+        self.ws: Workspace | None = None
         dev = torch.device(device)
         self.sm_count = (torch.cuda.get_device_properties(dev).multi_processor_count
                          if dev.type == "cuda" else 1)
@@ -67,8 +70,20 @@ class Runtime:
     def linear(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """out = x w^T in the compute dtype, accumulated in float32."""
         if self.dtype == torch.float32:
-            return self.ops.gemm_f32(x, w, out)
+            return self.product_f32(x, w, out)
         return self.ops.linear_bf16(x, w, out)
+
+    def product_f32(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, cap: float = 0.0) -> torch.Tensor:
+        """out = x w^T of floats at their precision, then cap * tanh(v / cap)."""
+        room = getattr(self.ops, "gemm_f32_room", None)
+        if room is None or self.ws is None:
+            return self.ops.gemm_f32(x, w, out, cap)
+        return self.ops.gemm_f32(x, w, out, cap, self.ws.buf("f32.planes", (room(x.shape[0], x.shape[1]),), torch.bfloat16))
+
+    def over(self, ws: "Workspace") -> "Runtime":
+        rt = copy.copy(self)
+        rt.ws = ws
+        return rt
 
 
 class Workspace:

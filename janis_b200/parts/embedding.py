@@ -73,7 +73,7 @@ class LMHead(Part):
         ops = ctx.rt.ops
         R = y.shape[0]
         if ctx.rt.dtype == torch.float32:
-            return ops.gemm_f32(y, self.table, out, self.softcap)
+            return ctx.rt.product_f32(y, self.table, out, self.softcap)
         vec = self.hidden % 8 == 0        # the skinny products read 16 bytes at a time; other widths take the library's
         if R <= ops.GEMV_FAST_ROWS and vec:
             return ops.gemv_bf16(y, self.table, out, ops.EPI_SOFTCAP, self.softcap)

@@ -88,7 +88,7 @@ class MatrixMemory(Mixer):
         rt.linear(x, self.w_in, rows)
         z = ws.buf("mlstm.z", (T, 2 * H), torch.float32)
         if rt.dtype == torch.float32:
-            ops.gemm_f32(x, self.w_gates, z)
+            rt.product_f32(x, self.w_gates, z)
         elif T <= ops.GEMV_FAST_ROWS and self.hidden % 8 == 0:
             ops.gemv_bf16(x, self.w_gates, z)
         else:

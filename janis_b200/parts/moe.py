@@ -134,7 +134,7 @@ class RoutedExperts(FeedForward):
         n_weights = E + (1 if self.gated_shared else 0) + (1 if self.n_identity else 0)
         z = ws.buf("moe.logits", (T, n_route), torch.float32)
         if rt.dtype == torch.float32:
-            ops.gemm_f32(x, self.w_route, z)
+            rt.product_f32(x, self.w_route, z)
         elif T <= ops.GEMV_FAST_ROWS and self.hidden % 8 == 0:
             ops.gemv_bf16(x, self.w_route, z)
         else:

@@ -612,3 +612,69 @@ def test_schedules_are_checked():
     with pytest.raises(ValueError, match="never written"):
         mk([LayerCall(0, 1)])
     assert mk([LayerCall(0, 0), LayerCall(1, 1), LayerCall(0, 2)]).n_cache_lines == 3
+
+
+# ---------------------------------------------------------------------------
+# the float product's room
+# ---------------------------------------------------------------------------
+
+class _PlanesOps:
+    """The plain statements, with a float product that wants room for x's parts and notes which it is given."""
+
+    def __init__(self):
+        self.given = []
+
+    def __getattr__(self, name):
+        return getattr(kernel_refs, name)
+
+    def gemm_f32_room(self, M, K):
+        return 3 * M * ((K + 7) // 8 * 8)
+
+    def gemm_f32(self, x, w, out, cap=0.0, planes=None):
+        self.given.append(None if planes is None else planes.untyped_storage().data_ptr())
+        assert planes is None or (planes.dtype == torch.bfloat16 and planes.numel() == self.gemm_f32_room(*x.shape))
+        return kernel_refs.gemm_f32(x, w, out, cap)
+
+
+def test_float_products_keep_their_room_from_step_to_step(model_dirs):
+    """Every product of a step, the head's among them, works in one buffer of the stepper's workspace, which no later step of that size
+    or less makes larger: a step that runs once can be recorded."""
+    from janis_b200 import StepEntry
+    from janis_b200.config.base import read_config_json
+    from janis_b200.engine.engine import build_model
+    from janis_b200.weights.loader import load_tensors
+    ops = _PlanesOps()
+    _, _, model = build_model(read_config_json(model_dirs["A"]))
+    rt = Runtime(torch.float32, "cpu", ops)
+    model.load(WeightStore(load_tensors(model_dirs["A"], model.tensor_specs(), "cpu", model.ignorable_tensors)), rt)
+    eng = Engine(model, rt, 256, 4, 64, use_graphs=False)
+    tokens = random_tokens(model.vocab, 20, 5)
+    slots = [eng.alloc_slot(), eng.alloc_slot()]
+    eng.step([StepEntry(slots[0], tokens, (19,))])
+    eng.step([StepEntry(slots[0], tokens[:1], (0,))])
+    eng.step([StepEntry(slots[1], tokens[:7], (6,))])
+    ops.given.clear()
+    held = eng.stepper.ws.bytes()
+    eng.stepper.ws.begin_capture()                           # (whatever would have to grow raises)
+    eng.step([StepEntry(slots[0], tokens[1:2], (0,))])
+    eng.step([StepEntry(slots[1], tokens[7:14], (6,))])
+    eng.stepper.ws.end_capture()
+    assert len(ops.given) > 8 and set(ops.given) == {eng.stepper.ws.buf("f32.planes", (1,), torch.bfloat16).untyped_storage().data_ptr()}
+    assert eng.stepper.ws.bytes() == held
+
+
+@GPU
+def test_a_recorded_float_step_holds_no_memory_of_its_own(model_dirs):
+    from janis_b200 import StepEntry
+    eng = janis_b200.open(model_dirs["A"], dtype="float32", max_tokens=512, device="cuda:0")
+    tokens = random_tokens(eng.model.vocab, 20, 6)
+    for _ in range(3):                                       # (a prompt's shape is recorded when it comes again)
+        slot = eng.alloc_slot()
+        eng.step([StepEntry(slot, tokens, (19,))])
+        eng.step([StepEntry(slot, tokens[:1], (0,))])
+        eng.free_slot(slot)
+    graphs = [held[0] for of in (eng.stepper._prompt_graphs, eng.stepper._graphs) for held in of.values()]
+    assert len(graphs) == 2
+    pools = {tuple(g.pool()) for g in graphs}
+    assert not [s for s in torch.cuda.memory_snapshot() if tuple(s["segment_pool_id"]) in pools]
+    eng.close()
