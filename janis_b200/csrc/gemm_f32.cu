@@ -18,11 +18,11 @@
 // TMA; two warps issue the products into two accumulators in tensor memory, while others add the chunk before to their
 // registers.
 //
-// Against pairs of multiply-adds on the CUDA cores (the form before, 74 TFLOP/s at best), one B200, W of bfloat16 numbers (of any floats):
-// 683 x 18432 over 2304 1,309 -> 274 (356) us, 683 x 2304 over 9216 831 -> 156 (191), over 2048 187 -> 42 (52), 3 x 256000 over 2304
-// 1,650 -> 505 (568), 1 x 2304 over 9216 356 -> 175; errors against 64 bits over 2,304 k 6.1e-7 -> 2.1e-7 (3.4e-7) of the result, of
-// operands of one sign 3.3e-7 -> 2.5e-7.  What bounds it: an issuer's waits and commits, 1,100 cycles a block of which the products are
-// 300 to 550, two issuers beside each other; for few rows of x, W's way from memory.  Chunks of 32 x 2 k are as long as the cut-off
+// Against pairs of multiply-adds on the CUDA cores (the form before, 74 TFLOP/s at best), one B200, W of bfloat16 numbers (of any floats), L2 flushed:
+// 683 x 18432 over 2304 1,309 -> 180 (261) us, 683 x 2304 over 9216 831 -> 150 (189), over 2048 187 -> 42 (54), 3 x 256000 over 2304
+// 1,650 -> 502 (574), 1 x 2304 over 9216 356 -> 211 (249); errors against 64 bits over 2,304 k 6.1e-7 -> 2.1e-7 (3.4e-7) of the result, of
+// operands of one sign 3.3e-7 -> 2.5e-7.  What bounds it: many rows of x, the products and what a block costs besides (waits, commits, the
+// splitting of W where it is any floats); few rows, W's way from memory.  Chunks of 32 x 2 k are as long as the cut-off
 // bits allow: 32 x 4 has an error of 3.9e-7 (7.5e-7).
 #include "common.cuh"
 #include "mma_bf16.cuh"
@@ -330,6 +330,24 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* x, const
         if (failed) return;
 
         const int n = n0 + quarter * 32 + lane;           // neighbouring lanes hold neighbouring columns of out
+        bool finite = true;
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int col = (group + u * GROUPS) * 16;
+            if (col >= cols) break;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const int m = m0 + col + j;
+                if (m >= M || n >= N) break;
+                float v = acc[u][j];
+                finite &= fabsf(v) <= 3.402823466e38f;
+                if (cap > 0.f) v = cap * tanhf(v / cap);
+                out[(size_t)m * N + n] = v;
+            }
+        }
+        if (__all_sync(0xffffffffu, finite)) return;
+        // Hardly ever: a sum that is not finite is formed again by the warp, of plain products.  (A loop of its own: beside the stores
+        // above it cost every output, 683 x 18432 over 2304: 300 us with x read through the read-only path, 379 by plain loads, 180 apart.)
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
             const int col = (group + u * GROUPS) * 16;
@@ -338,20 +356,16 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* x, const
             for (int j = 0; j < 16; ++j) {
                 const int m = m0 + col + j;
                 if (m >= M) break;
-                float v = acc[u][j];
-                uint32_t odd = __ballot_sync(0xffffffffu, n < N && !(fabsf(v) <= 3.402823466e38f));
-                while (odd) {                             // (hardly ever) the warp forms such a sum of plain products
+                uint32_t odd = __ballot_sync(0xffffffffu, n < N && !(fabsf(acc[u][j]) <= 3.402823466e38f));
+                while (odd) {
                     const int l = __ffs(odd) - 1;
                     odd &= odd - 1;
                     const float *xp = x + (size_t)m * K, *wp = W + (size_t)(n - lane + l) * K;
                     float plain = 0.f;
                     for (int k = lane; k < K; k += 32) plain = fmaf(__ldcg(xp + k), wp[k], plain);
                     plain = warp_sum(plain);
-                    if (lane == l) v = plain;
-                }
-                if (n < N) {
-                    if (cap > 0.f) v = cap * tanhf(v / cap);
-                    out[(size_t)m * N + n] = v;
+                    if (cap > 0.f) plain = cap * tanhf(plain / cap);
+                    if (lane == l) out[(size_t)m * N + n] = plain;
                 }
             }
         }
