@@ -1,6 +1,6 @@
 // out[M, N] = x[M, K] * W[N, K]^T of float operands at float precision, on the tensor cores.
 //
-// A float is the sum of three bfloat16 numbers to its last bit (hi, mid, lo: 8 bits each of 24), products of bfloat16
+// A float of 2^-110 and more is the sum of three bfloat16 numbers to its last bit (hi, mid, lo: 8 bits each of 24), products of bfloat16
 // numbers are exact in float, and the tensor cores add them up in float: x w = (xh + xm + xl)(wh + wm + wl), of which
 // xm wl, xl wm and xl wl (2^-25 of the product and less) are left out.  Where a block of W holds nothing but bfloat16 numbers
 // (a bfloat16 checkpoint run in 32 bits) wm and wl are zero and three products are left; the kernel looks at every block it
@@ -10,7 +10,8 @@
 // of the same sign; so they only add up CHUNK blocks of 32 k at a time, and registers add the chunks, rounding to nearest.
 // Every output is formed from its own row of x and row of W in one order, whatever M, N and the tiling are.  An output
 // that does not come out finite (an infinity or NaN among the operands, or beyond the range) is formed again as a plain sum of
-// float products, so infinities and NaN go where they go in such a sum.  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
+// float products, so infinities and NaN go where they go in such a sum; and a smaller float whose last bits lo has no place for is split into NaN, so
+// that the outputs it counts in are such plain sums too (some 6 us a warp for each: such a row of x or W costs as much as the whole product).  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
 //
 // x is split once, by a kernel of its own, into three planes of bfloat16.  A CTA owns 128 rows of W (the lanes of tensor memory)
 // and up to 192 rows of x (its columns).  Some warps read a block of 32 k of W into registers, ahead, split it, and write it
@@ -89,6 +90,12 @@ __device__ __forceinline__ float4 load4(const float* row, int k, int K, bool ok)
     return v;
 }
 
+// Whether x is one of those that the three parts do not add up to: below 2^-110, the last of its 24 bits is below 2^-133, the smallest
+// bfloat16 number (one of bfloat16's own bits alone is hi itself).  A NaN takes its hi's place.
+constexpr float SPLIT_FROM = 0x1p-110f;
+__device__ __forceinline__ bool lost(float x) { return fabsf(x) < SPLIT_FROM && (__float_as_uint(x) & 0xffffu); }
+__device__ __forceinline__ uint32_t nan_where_lost(float x, float y, uint32_t hi) { return hi | (lost(x) ? 0x7fffu : 0u) | (lost(y) ? 0x7fff0000u : 0u); }
+
 __device__ __forceinline__ void store8(uint32_t shared, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(shared), "r"(a), "r"(b) : "memory");
 }
@@ -118,6 +125,10 @@ split_rows_kernel(const float* x, bf16* __restrict__ planes, int M, int K, int K
         split3(a.z, a.w, hi.y, mid.y, lo.y);
         split3(b.x, b.y, hi.z, mid.z, lo.z);
         split3(b.z, b.w, hi.w, mid.w, lo.w);
+        hi.x = nan_where_lost(a.x, a.y, hi.x);
+        hi.y = nan_where_lost(a.z, a.w, hi.y);
+        hi.z = nan_where_lost(b.x, b.y, hi.z);
+        hi.w = nan_where_lost(b.z, b.w, hi.w);
         bf16* to = planes + m * Kp + k;
         *reinterpret_cast<uint4*>(to) = hi;
         *reinterpret_cast<uint4*>(to + plane) = mid;
@@ -272,17 +283,29 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap map_x, const float* x, const
                     low |= __float_as_uint(wv[a][i].x) | __float_as_uint(wv[a][i].y) | __float_as_uint(wv[a][i].z) | __float_as_uint(wv[a][i].w);
                 // Whether mid and lo have to be written is asked of all four warps: the stage may hold what another group left there.
                 if (any_of_group(turn, (low & 0xffffu) != 0)) {
+                    float least[NW];
 #pragma unroll
                     for (int i = 0; i < NW; ++i) {
                         uint32_t h0, h1, m0_, m1, l0, l1;
                         split3(wv[a][i].x, wv[a][i].y, h0, m0_, l0);
                         split3(wv[a][i].z, wv[a][i].w, h1, m1, l1);
                         const uint32_t at = to + i * 16 * 64;
+                        least[i] = fminf(fminf(fabsf(wv[a][i].x), fabsf(wv[a][i].y)), fminf(fabsf(wv[a][i].z), fabsf(wv[a][i].w)));
                         store8(at, h0, h1);
                         store8(at + W_PLANE, m0_, m1);
                         store8(at + 2 * W_PLANE, l0, l1);
                     }
                     if ((thread & 127) == 0) *(volatile int*)&low_bits[s] = b + 1;
+#pragma unroll
+                    for (int i = NW / 2; i > 0; i >>= 1)
+#pragma unroll
+                        for (int j = 0; j < i; ++j) least[j] = fminf(least[j], least[j + i]);
+                    // (numbers as small are hardly ever there, and asking for each one in the loop above costs a quarter)
+                    if (least[0] < SPLIT_FROM) {
+#pragma unroll
+                        for (int i = 0; i < NW; ++i)
+                            if (lost(wv[a][i].x) || lost(wv[a][i].y) || lost(wv[a][i].z) || lost(wv[a][i].w)) store8(to + i * 16 * 64, 0x7fff7fffu, 0x7fff7fffu);
+                    }
                 } else {
 #pragma unroll
                     for (int i = 0; i < NW; ++i)

@@ -324,6 +324,27 @@ def test_gemm_f32_infinities_and_nan():
     assert got[50, 100].item() == 0.0                        # finite operands, a finite result
 
 
+@pytest.mark.parametrize("K", [40, 2304])
+@pytest.mark.parametrize("of_w", [False, True])
+def test_gemm_f32_smallest_numbers(of_w, K):
+    """Operands on both sides of 2^-110, where three bfloat16 numbers stop adding up to a float, and subnormal ones, against numbers large
+    enough that the result is an ordinary float; beside them rows that are zero, and rows of numbers of bfloat16's own bits.  A plain sum
+    rounds 77 times at most (72 products a lane, five times the lanes), partial sums that random signs keep below an eighth of the magnitudes'
+    sum: 77 / 8 2^-24 < 2^-20 of it."""
+    g = torch.Generator().manual_seed(64)
+    small = torch.randn(23, K, generator=g) * 2.0 ** torch.tensor([-100, -108, -109, -110, -111, -113, -118, -125, -130, -140, -112, -112] + [-120] * 11).view(-1, 1).float()
+    small[10, 1:] = 0.0                                      # one such number in a row
+    small[11] = torch.randn(K, generator=g)
+    small[11, K // 2] = 2.0 ** -115 * 1.2345678              # beside ordinary ones
+    small[12:14], small[14:18] = 0.0, small[14:18].bfloat16().float()
+    large = torch.randn(150, K, generator=g) * 2.0 ** 100
+    x, w = (large, small) if of_w else (small, large)
+    out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=dev())
+    ops().gemm_f32(x.to(dev()), w.to(dev()), out)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert ((out.cpu().double() - want).abs() <= 2.0 ** -20 * size).all()
+
+
 @pytest.mark.parametrize("dout", DTYPES)
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 33, 64])
 @pytest.mark.parametrize("N,K", [(16, 32), (40, 72), (384, 96), (2304, 2048), (1000, 328)])
