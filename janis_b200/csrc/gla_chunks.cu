@@ -125,10 +125,12 @@ __host__ __device__ constexpr int gla_chain_bytes(int d) { return GC_STAGES * gl
 
 // Where few sequences leave SMs idle a chain runs in pieces of `length` chunks at the same time, in two launches: STATES takes every piece
 // but a sequence's last from a state of zeros (its first from the stored state) to its end and leaves that, the piece's decay and a copy
-// of the stored state; then the pieces run as WHOLE chains do, each from the states before it folded together.
+// of the stored state; then the pieces run as WHOLE chains do, each from the states before it folded together.  The decay is kept as itself
+// and as decay - 1: what a piece of hundreds of tokens leaves of a state may be its ten-thousandth part, which S + S (decay - 1) has at
+// the precision of S, and of a state that hardly decays S decay rounds away what S + S (decay - 1) keeps.  The fold takes the one that does not cancel.
 struct GlaPieces {
     int length, most;                        // chunks a piece; pieces a sequence at most (0: whole chains)
-    float *ends, *grows;                     // [seq][most + 1][H][dv][d]: the stored state, then a piece's end; [seq][most][H][d]: decay - 1
+    float *ends, *grows;                     // [seq][most + 1][H][dv][d]: the stored state, then a piece's end; [seq][most][2][H][d]: decay - 1, decay
 };
 enum { GLA_WHOLE = 0, GLA_STATES = 1 };
 
@@ -214,20 +216,21 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
         // (the stored state's copy: the last piece may have written the state by now)
         load_state(end_of(piece == 0 ? 0 : 1), S);
         for (int q = 1; q < piece; ++q) {
-            const float* gq = pieces.grows + (((size_t)seq * pieces.most + q) * g.H + h) * D + n0;
+            const float* gq = pieces.grows + (((size_t)seq * pieces.most + q) * 2 * g.H + h) * D + n0;
             float e[2 * NK][4];
             load_state(end_of(q + 1), e);
 #pragma unroll
             for (int j = 0; j < 2 * NK; ++j) {
-                const float2 gw = *reinterpret_cast<const float2*>(gq + 8 * j + gc);
-                S[j][0] += fmaf(S[j][0], gw.x, e[j][0]);
-                S[j][1] += fmaf(S[j][1], gw.y, e[j][1]);
-                S[j][2] += fmaf(S[j][2], gw.x, e[j][2]);
-                S[j][3] += fmaf(S[j][3], gw.y, e[j][3]);
+                const float2 gw = *reinterpret_cast<const float2*>(gq + 8 * j + gc), keep = *reinterpret_cast<const float2*>(gq + hd + 8 * j + gc);
+                auto fold = [](float s, float grow, float decay, float end) { return decay < 0.5f ? fmaf(s, decay, end) : s + fmaf(s, grow, end); };
+                S[j][0] = fold(S[j][0], gw.x, keep.x, e[j][0]);
+                S[j][1] = fold(S[j][1], gw.y, keep.y, e[j][1]);
+                S[j][2] = fold(S[j][2], gw.x, keep.x, e[j][2]);
+                S[j][3] = fold(S[j][3], gw.y, keep.y, e[j][3]);
             }
         }
     }
-    float piece_grow = 0.f;                                                // of channel tid over the piece's chunks
+    float piece_grow = 0.f, piece_decay = 1.f;                             // of channel tid over the piece's chunks
     for (int c = 0; c < GC_STAGES - 1; ++c) fetch(c0 + c);
     for (int c = c0; c < c1; ++c) {
         asm volatile("cp.async.wait_group %0;" ::"n"(GC_STAGES - 2) : "memory");
@@ -235,7 +238,10 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
         fetch(c + GC_STAGES - 1);
         const uint32_t at = raw + (c % GC_STAGES) * STAGE;
         const float* grow = reinterpret_cast<const float*>(gla_raw + (c % GC_STAGES) * STAGE + G_AT);
-        if (PHASE == GLA_STATES && tid < D) piece_grow += fmaf(piece_grow, grow[tid], grow[tid]);
+        if (PHASE == GLA_STATES && tid < D) {
+            piece_grow += fmaf(piece_grow, grow[tid], grow[tid]);
+            piece_decay *= 1.f + grow[tid];
+        }
         // o: this quarter's channels of the state; the first quarter adds the chunk's own tokens
         if constexpr (PHASE != GLA_STATES) {
             float hi[2][4], rest[2][4];
@@ -352,7 +358,11 @@ gla_chain_kernel(const bf16* __restrict__ rows, GlaChunkShape g, GlaChunkScratch
     }
     if (PHASE == GLA_STATES) {
         store_state(end_of(piece + 1));
-        if (blockIdx.z == 0 && tid < D) pieces.grows[(((size_t)seq * pieces.most + piece) * g.H + h) * D + tid] = piece_grow;
+        if (blockIdx.z == 0 && tid < D) {
+            float* to = pieces.grows + (((size_t)seq * pieces.most + piece) * 2 * g.H + h) * D + tid;
+            to[0] = piece_grow;
+            to[hd] = piece_decay;
+        }
     } else if (st != nullptr && c1 == chunks) store_state(st);
 }
 
@@ -372,7 +382,7 @@ static GlaPieces gla_pieces(int n_tok, int n_seq, int H, int d, int dv) {
     return p;
 }
 static long long gla_piece_floats(const GlaPieces& p, int n_seq, int H, int d, int dv) {
-    return p.most ? (long long)n_seq * H * d * ((long long)(p.most + 1) * dv + p.most) : 0;
+    return p.most ? (long long)n_seq * H * d * ((long long)(p.most + 1) * dv + 2 * p.most) : 0;
 }
 
 template <int NK, int PHASE>

@@ -1259,3 +1259,33 @@ def test_gated_linear_attention_in_pieces(lens, slots, H, d, dv, strength):
         ops().gla_scan(*args(lambda x: x.to(dev()), got_state, got), chunks=torch.full((room,), float("nan"), device=dev()))
         close(got, want, 2e-5, "results")
         close(got_state, want_state, 2e-5, "the states left behind")
+
+
+@pytest.mark.parametrize("per_token", [0.05, 0.3, 8.0, 2.0 ** -12])
+def test_gated_linear_attention_in_pieces_of_what_is_left(per_token):
+    """A large stored state that decays by e^(-16 per_token) a chunk while next to nothing comes in, over pieces of 16 chunks and more: what is
+    left of it is as exact as in whole chains.  A chunk's decay is 1 + (e^b - 1) with one rounding of the second, 2^-25 of 1 at most beside
+    the state's own 2^-24, so after c chunks a state is within c (2^-24 + 2^-25 e^(16 per_token)) of itself.  A result has besides the error of
+    its own sum of 64 channels of one sign: five additions of the 16 channels of a quarter's products, each cut off within 2^-23 of what there
+    is by then, the quarters' three, and the query's and decay's roundings: 16 2^-24."""
+    H, d, dv, T = 2, 64, 64, 1024
+    g = torch.Generator().manual_seed(9)
+    rows = torch.cat([torch.rand(T, H * d, generator=g) + 0.5, torch.randn(T, H * d + H * dv, generator=g) * 1e-25], dim=1).bfloat16()
+    z = torch.full((T, H * d), -16.0 * per_token if per_token > 0.2 else math.log(1 / (math.exp(16.0 * per_token) - 1))).bfloat16()
+    b, state = torch.zeros(H * d).bfloat16(), torch.rand(1, H, dv, d, generator=g) * 1e4 + 1e3
+    step = torch.nn.functional.logsigmoid(z.double()) / 16.0                 # a token's logarithm of the decay
+    left = state.double()[0] * torch.exp(step.sum(0)).view(H, 1, d)
+    at = torch.exp(step.cumsum(0)).view(T, H, 1, d)
+    want = ((state.double() * at) @ (rows[:, :H * d].double() * d ** -0.5).view(T, H, d, 1)).reshape(T, H * dv)
+    i32 = lambda *v: torch.tensor(v, dtype=torch.int32, device=dev())
+    room = ops().gla_chunks_floats(torch.bfloat16, T, 1, H, d, dv)
+    assert room > ops()._gla_chunks_least(torch.bfloat16, T, 1, H, d, dv)
+    got, got_state = torch.empty(T, H * dv, device=dev()), state.to(dev())
+    ops().gla_scan(rows.to(dev()), 0, H * d, 2 * H * d, z.to(dev()), b.to(dev()), i32(0), i32(0), i32(0), i32(T), got_state, got, 1, H, d, dv, d ** -0.5, 16.0,
+                   chunks=torch.empty(room, device=dev()))
+    chunks = torch.arange(T, dtype=torch.float64).view(T, 1) // 16 + 2
+    bound = 2.0 ** -24 + 2.0 ** -25 * math.exp(-16 * step[0, 0].item())
+    alive = want > 1e-30                                     # (beyond, a float keeps no such numbers)
+    assert ((got.cpu().double() - want).abs()[alive] <= ((chunks * bound + 2.0 ** -20) * want)[alive]).all()
+    if left.min() > 1e-30:
+        assert ((got_state.cpu().double()[0] - left).abs() <= 66 * bound * left).all()
