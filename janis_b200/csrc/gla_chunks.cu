@@ -19,15 +19,17 @@
 // registers (as the accumulators of the last product, which are at the same time second operands of the first), and the
 // four sums of a result meet in shared memory.  The chain bounds it: some 250 instructions a warp and two barriers a chunk.
 //
-// Few sequences leave SMs idle: their chains run in up to four pieces at the same time, once for the pieces' end states alone and once
-// from the states that these give (one sequence of 2,048 tokens: 151 us for the chain -> 29 + 62; a scratch without room for the
-// states keeps whole chains).
+// Few sequences leave SMs idle: their chains run in pieces at the same time, as many as give two CTAs an SM, once for the pieces' end
+// states alone and once from the states that these give, where that takes less time (gla_pieces_pay; one sequence of 2,048 tokens: 151 us for
+// the chain -> 29 + 62; a scratch without room for the states keeps whole chains).
 //
 // 8 heads of 128 x 256, against gla_scan_kernel (bound by shared memory: three 16-byte reads for 16 multiply-adds a lane) with its
 // kernel for the decays: whole chains of one sequence of 2,048 tokens 374 -> 200 us (in pieces 140), 300 tokens 60 -> 43,
 // eight of 512 666 -> 210.  Errors
 // against 64 bits over 2,048 tokens: results 3.3e-7 -> 1.4e-7, states 3.2e-7 -> 0.7e-7; where the states remember a thousand tokens
 // 5.3e-6 -> 1.9e-7 and 7.3e-6 -> 2.1e-7.
+#include <math.h>
+
 #include "mma_bf16.cuh"
 
 namespace janis {
@@ -376,10 +378,20 @@ static GlaPieces gla_pieces(int n_tok, int n_seq, int H, int d, int dv) {
     long long length = (chunks + want - 1) / want;
     if (length < 16) length = 16;
     const long long most = (chunks + length - 1) / length;
-    if (most < 2) return p;
+    if (most < 2) return p;                               // (p.most is 0: no pieces)
     p.length = (int)length;
     p.most = (int)most;
     return p;
+}
+// Whether pieces take less time than whole chains, whose time is that of the longest sequence's.  In chunks of a CTA that has an SM to itself
+// (1.18 us at 128 key channels): of two CTAs on an SM each takes 1.64 a chunk; for the states alone 0.42 and 0.76; a launch and the fold
+// cost 8.5.  All of it, with the terms' kernel, 8 heads of 128 x 256, whole -> pieces: one sequence of 2,048 tokens 208 -> 153 us, of 1,024 112 -> 89,
+// of 600 79 -> 81 (whole), of 300 54 -> 62 (whole); two of 1,024 138 -> 153 (whole), of 2,000 and 50 204 -> 157; 4 heads, one of 600 75 -> 62.
+static bool gla_pieces_pay(const GlaPieces& p, int n_tok, int n_seq, int H, int dv, int longest) {
+    const int per = H * (dv / GC_COLS);                   // CTAs a piece
+    const int whole = (longest + GQ - 1) / GQ;
+    const double pieces = ceil(n_tok / GQ / (double)p.length + 0.5 * (n_seq - 1)), states = pieces - n_seq;
+    return p.length * ((pieces * per > 148 ? 1.64 : 1.0) + (states * per > 148 ? 0.76 : 0.42)) + 8.5 < whole;
 }
 static long long gla_piece_floats(const GlaPieces& p, int n_seq, int H, int d, int dv) {
     return p.most ? (long long)n_seq * H * d * ((long long)(p.most + 1) * dv + 2 * p.most) : 0;
@@ -416,9 +428,10 @@ JANIS_EXPORT long long janis_gla_chunks_least(int n_tok, int n_seq, int H, int d
     return janis_gla_chunks_floats(n_tok, n_seq, H, d, dv) ? gla_chunk_floats(n_tok, n_seq, H, d) : 0;
 }
 
+// longest: tokens of the longest sequence, for the choice between pieces and whole chains (0: taken to be the mean)
 JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, int k_off, int v_off, const void* z, const void* bias, int n_tok,
                                   const int* seq_slot, const int* seq_first_row, const int* seq_start, const int* seq_end, float* state,
-                                  float* o_out, int n_seq, int H, int d, int dv, float q_scale, float tau, void* scratch,
+                                  float* o_out, int n_seq, int H, int d, int dv, float q_scale, float tau, int longest, void* scratch,
                                   long long scratch_floats, cudaStream_t stream) {
     if (n_seq <= 0 || n_tok <= 0) return 0;
     const long long all = janis_gla_chunks_floats(n_tok, n_seq, H, d, dv), need = janis_gla_chunks_least(n_tok, n_seq, H, d, dv);
@@ -438,7 +451,8 @@ JANIS_EXPORT int janis_gla_chunks(const void* rows, int row_elems, int q_off, in
                       (const bf16*)z, (const bf16*)bias, g, n_seq, seq_first_row, seq_start, seq_end, s))
         return 1;
     GlaPieces pieces = gla_pieces(n_tok, n_seq, H, d, dv);
-    if (scratch_floats < all) pieces.most = 0;            // (a scratch for whole chains)
+    if (longest <= 0) longest = (n_tok + n_seq - 1) / n_seq;
+    if (scratch_floats < all || (pieces.most && !gla_pieces_pay(pieces, n_tok, n_seq, H, dv, longest))) pieces.most = 0;
     if (pieces.most) {
         pieces.ends = (float*)scratch + need;
         pieces.grows = pieces.ends + (long long)n_seq * (pieces.most + 1) * H * dv * d;

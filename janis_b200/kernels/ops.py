@@ -154,7 +154,7 @@ def mixers():
         lib.janis_gla_chunks_floats.restype = c_longlong
         lib.janis_gla_chunks_least.argtypes = [I, I, I, I, I]
         lib.janis_gla_chunks_least.restype = c_longlong
-        lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, P, c_longlong, P]
+        lib.janis_gla_chunks.argtypes = [P, I, I, I, I, P, P, I, P, P, P, P, P, P, I, I, I, I, F, F, I, P, c_longlong, P]
         lib.janis_talk_attention_rows_mixed_floats.argtypes = [I, I, I, I, I, I, I]
         lib.janis_talk_attention_rows_mixed_floats.restype = c_longlong
         lib.janis_talk_attention_rows_mixed.argtypes = [P, I, I, P, P, P, P, P, P, I, P, P, P, I, I, I, I, I, F, I, I, I, F, P, P, c_longlong, I, P]
@@ -1176,14 +1176,15 @@ def _gla_tables(rows, z, z_bias, state, o_out, seq_slot, seq_first_row, seq_star
 
 
 def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_first_row, seq_start, seq_end, state,
-             o_out, n_seq: int, H: int, d: int, dv: int, q_scale: float, tau: float, decay=None, chunks=None):
+             o_out, n_seq: int, H: int, d: int, dv: int, q_scale: float, tau: float, decay=None, chunks=None, longest: int = 0):
     """The recurrence of gated linear attention over the tokens each sequence brings to the step, in order:
     a = sigmoid(z + z_bias)^(1/tau) per key channel, S = diag(a) S + k v^T, o = S^T (q q_scale).
     rows [T, width] holds the projections (q [H, d] at q_off, k at k_off, v [H, dv] at v_off), z [T, H d] the
     projected decay logits; state float32 [slots, H, dv, d] (a column's key channels side by side) is read and written back for sequences whose slot is
     >= 0; o_out float32 [T, H dv]; decay float32 [T, H d] receives the decays (a kernel of its own forms them once
     for all the CTAs of a head; allocated here when not given).  `chunks` (float32 of at least `gla_chunks_floats`): scratch
-    with which a prompt runs 16 tokens at a time on the tensor cores; the decays are then not left in `decay`."""
+    with which a prompt runs 16 tokens at a time on the tensor cores; the decays are then not left in `decay`.  `longest`: tokens of the
+    step's longest sequence where the host knows it (0: taken to be the mean); with it few sequences' chains run whole or in pieces, whichever is sooner."""
     T, width = rows.shape
     if chunks is not None:
         _t(chunks, "chunks", torch.float32)
@@ -1193,7 +1194,7 @@ def gla_scan(rows, q_off: int, k_off: int, v_off: int, z, z_bias, seq_slot, seq_
             lib = mixers()
             _check_counted(lib, lib.janis_gla_chunks, rows.data_ptr(), width, q_off, k_off, v_off, z.data_ptr(), z_bias.data_ptr(), T, seq_slot.data_ptr(),
                            seq_first_row.data_ptr(), seq_start.data_ptr(), seq_end.data_ptr(), state.data_ptr(), o_out.data_ptr(),
-                           n_seq, H, d, dv, float(q_scale), float(tau), chunks.data_ptr(), chunks.numel(), _stream())
+                           n_seq, H, d, dv, float(q_scale), float(tau), int(longest), chunks.data_ptr(), chunks.numel(), _stream())
             return o_out
     if decay is None:
         decay = torch.empty((T, H * d), dtype=torch.float32, device=rows.device)

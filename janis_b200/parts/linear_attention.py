@@ -86,7 +86,7 @@ class GatedLinearAttention(Mixer):
                       ws.buf("gla.z", (T, H * d), rt.dtype))
         o = ws.buf("gla.o", (T, H * dv), torch.float32)
         room = getattr(ops, "gla_chunks_floats", lambda *a: 0)(rt.dtype, T, ctx.n_seq, H, d, dv) if ctx.mode == "prefill" else 0
-        how = dict(chunks=ws.buf("gla.chunks", (room,), torch.float32)) if room else dict(decay=ws.buf("gla.decay", (T, H * d), torch.float32))
+        how = dict(chunks=ws.buf("gla.chunks", (room,), torch.float32), longest=max(ctx.step_lens or (0,))) if room else dict(decay=ws.buf("gla.decay", (T, H * d), torch.float32))
         ops.gla_scan(rows, q_off, k_off, v_off, z, self.b_a2, ctx.seq_slot, ctx.seq_first_row, ctx.seq_start,
                      ctx.seq_end, st.data, o, ctx.n_seq, H, d, dv, self.q_scale, self.tau, **how)
         y = ws.buf("gla.y", (T, H * dv), rt.dtype)

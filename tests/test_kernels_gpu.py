@@ -1289,3 +1289,27 @@ def test_gated_linear_attention_in_pieces_of_what_is_left(per_token):
     assert ((got.cpu().double() - want).abs()[alive] <= ((chunks * bound + 2.0 ** -20) * want)[alive]).all()
     if left.min() > 1e-30:
         assert ((got_state.cpu().double()[0] - left).abs() <= 66 * bound * left).all()
+
+
+@pytest.mark.parametrize("lens,slots,launches", [([700], [1], 3), ([300], [1], 2), ([30, 600], [3, 0], 3), ([520, 0, 300], [-1, 2, 4], 3), ([340, 330], [0, 5], 2)])
+def test_gated_linear_attention_in_pieces_where_they_pay(lens, slots, launches):
+    """With the longest sequence's tokens known, unequal sequences run in pieces too (three kernels: the chunks' terms, the states, the pieces)
+    and sequences of few chunks whole; both are the recurrence, and without scratch for states the same call runs whole."""
+    H, d, dv = 2, 128, 64
+    g = torch.Generator().manual_seed(sum(lens))
+    T, n_seq = sum(lens), len(lens)
+    seq_slot, first, start, end = _step_tables(lens, slots)
+    rows, z, b = torch.randn(T, 2 * H * d + H * dv, generator=g).bfloat16(), torch.randn(T, H * d, generator=g).bfloat16(), torch.zeros(H * d).bfloat16()
+    state = torch.randn(6, H, dv, d, generator=g)
+    want, want_state = torch.zeros(T, H * dv), state.clone()
+    args = lambda dev, st, out: (dev(rows), 0, H * d, 2 * H * d, dev(z), dev(b), dev(seq_slot), dev(first), dev(start), dev(end), st, out, n_seq, H, d, dv,
+                                 d ** -0.5, 16.0)
+    R.gla_scan(*args(lambda x: x, want_state, want))
+    most, least = ops().gla_chunks_floats(torch.bfloat16, T, n_seq, H, d, dv), ops()._gla_chunks_least(torch.bfloat16, T, n_seq, H, d, dv)
+    for room, kernels in ((most, launches), (least, 2)):
+        got, got_state = torch.full((T, H * dv), float("nan"), device=dev()), state.clone().to(dev())
+        before = ops().launch_count()
+        ops().gla_scan(*args(lambda x: x.to(dev()), got_state, got), chunks=torch.full((room,), float("nan"), device=dev()), longest=max(lens))
+        assert ops().launch_count() - before == kernels
+        close(got, want, 2e-5, "results")
+        close(got_state, want_state, 2e-5, "the states left behind")
