@@ -246,6 +246,19 @@ template <> struct Vec16<bf16> {
     }
 };
 
+// four consecutive values, on the alignment of four
+__device__ __forceinline__ void load_four(const float* p, float* o) { Vec16<float>::load(p, o); }
+__device__ __forceinline__ void load_four(const bf16* p, float* o) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
+    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store_four(float* p, const float* v) { Vec16<float>::store(p, v); }
+__device__ __forceinline__ void store_four(bf16* p, const float* v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+
 // eight consecutive values, on 16 bytes
 template <typename T>
 __device__ __forceinline__ void load_eight(const T* p, float* out) {

@@ -214,13 +214,6 @@ gla_scan_kernel(const T* __restrict__ rows, GlaRows g, const float* __restrict__
     }
 }
 
-__device__ __forceinline__ void load_four(const float* p, float* o) { Vec16<float>::load(p, o); }
-__device__ __forceinline__ void load_four(const bf16* p, float* o) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p);
-    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
-    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
-}
-
 // One token a sequence (a decode step): the state comes and goes once.  A warp takes four columns of a head's state (two for more than
 // 128 key channels), a lane four channels of each, so that its accesses are whole lines; q, k and the decays, which are formed
 // here, lie in registers for all of them.  The state is asked for (into L2) before the kernel waits for the one that makes

@@ -83,18 +83,6 @@ causal_conv_silu_kernel(const T* __restrict__ rows, int row_elems, int col_off, 
     }
 }
 
-__device__ __forceinline__ void load_channels(const float* p, float* o) { Vec16<float>::load(p, o); }
-__device__ __forceinline__ void load_channels(const bf16* p, float* o) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p);
-    o[0] = __uint_as_float(v.x << 16); o[1] = __uint_as_float(v.x & 0xffff0000u);
-    o[2] = __uint_as_float(v.y << 16); o[3] = __uint_as_float(v.y & 0xffff0000u);
-}
-__device__ __forceinline__ void store_channels(float* p, const float* v) { Vec16<float>::store(p, v); }
-__device__ __forceinline__ void store_channels(bf16* p, const float* v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-}
-
 // The same with four channels a thread, up to four taps: a thread takes its channels over a run of tokens in turn and
 // keeps the last K - 1 inputs in registers while the tokens are one sequence's; four tokens' inputs are asked for together.
 // (Eight channels a thread took 136 registers, three CTAs an SM, and 0.31 instructions a scheduler's cycle: 2,048 tokens of 4,608
@@ -136,7 +124,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
         float x[AHEAD][V];
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a)
-            if (tb + a < t1) load_channels(rows + (size_t)(tb + a) * row_elems + col_off + c, x[a]);
+            if (tb + a < t1) load_four(rows + (size_t)(tb + a) * row_elems + col_off + c, x[a]);
 #pragma unroll
         for (int a = 0; a < AHEAD; ++a) {
             const int t = tb + a;
@@ -151,7 +139,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
                 for (int j = 0; j < KM - 1; ++j) {
                     const int at = i - 1 - j;
                     if (j < K - 1 && at >= 0) {
-                        load_channels(rows + (size_t)(t - 1 - j) * row_elems + col_off + c, past[j]);
+                        load_four(rows + (size_t)(t - 1 - j) * row_elems + col_off + c, past[j]);
 #pragma unroll
                         for (int e = 0; e < V; ++e) past[j][e] += xb[e];
                     } else {
@@ -173,7 +161,7 @@ causal_conv_vec_kernel(const T* __restrict__ rows, int row_elems, int col_off, i
                 for (int j = KM - 2; j > 0; --j) past[j][e] = past[j - 1][e];
                 past[0][e] = x[a][e];
             }
-            store_channels(out + (size_t)t * C + c, y);
+            store_four(out + (size_t)t * C + c, y);
             if (alone && st != nullptr) {                    // the sequence's only token of the step: the kept inputs move on
 #pragma unroll
                 for (int j = 0; j < KM - 1; ++j)
