@@ -7,11 +7,12 @@
 // splits, so nothing is remembered about a matrix.
 //
 // The tensor cores cut the sum's last bits off each time they add to it, which would show after thousands of additions
-// of the same sign; so they only add up CHUNK blocks of 32 k at a time, and registers add the chunks, rounding to nearest.
+// of the same sign; so they only add up CHUNK blocks of 32 k at a time, and registers add the chunks, rounding to nearest.  (An
+// output of one product is within 3.1 2^-24, where a float product has half a unit; large sums come out some 1.8e-7 of their size too small.)
 // Every output is formed from its own row of x and row of W in one order, whatever M, N and the tiling are.  An output
 // that does not come out finite (an infinity or NaN among the operands, or beyond the range) is formed again as a plain sum of
 // float products, so infinities and NaN go where they go in such a sum; and a smaller float whose last bits lo has no place for is split into NaN, so
-// that the outputs it counts in are such plain sums too (some 6 us a warp for each: such a row of x or W costs as much as the whole product).  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
+// that the outputs it counts in are such plain sums too (683 x 18432 over 2304: one such row of x or W 276 -> 530 us; one number in every row 23 ms).  Any M, N, K.  Optional epilogue: cap * tanh(v / cap).
 //
 // x is split once, by a kernel of its own, into three planes of bfloat16.  A CTA owns 128 rows of W (the lanes of tensor memory)
 // and up to 192 rows of x (its columns).  Some warps read a block of 32 k of W into registers, ahead, split it, and write it
@@ -21,7 +22,7 @@
 //
 // Against pairs of multiply-adds on the CUDA cores (the form before, 74 TFLOP/s at best), one B200, W of bfloat16 numbers (of any floats), L2 flushed:
 // 683 x 18432 over 2304 1,309 -> 180 (261) us, 683 x 2304 over 9216 831 -> 150 (189), over 2048 187 -> 42 (54), 3 x 256000 over 2304
-// 1,650 -> 502 (574), 1 x 2304 over 9216 356 -> 211 (249); errors against 64 bits over 2,304 k 6.1e-7 -> 2.1e-7 (3.4e-7) of the result, of
+// 1,650 -> 502 (587), 1 x 2304 over 9216 356 -> 212 (259); errors against 64 bits over 2,304 k 6.1e-7 -> 2.1e-7 (3.4e-7) of the result, of
 // operands of one sign 3.3e-7 -> 2.5e-7.  What bounds it: many rows of x, the products and what a block costs besides (waits, commits, the
 // splitting of W where it is any floats); few rows, W's way from memory.  Chunks of 32 x 2 k are as long as the cut-off
 // bits allow: 32 x 4 has an error of 3.9e-7 (7.5e-7).
